@@ -966,7 +966,16 @@ int32_t rfg_solve_device_noalloc(const RustyfemHandle* h, size_t nrhs_, double* 
         // scratch layout: X (n_sym · nr_max double), then the sweep workspace; the
         // caller-numbering maps live with the handle (uploaded when it was built)
         int64_t need = 0;
-        if (h->eng) need += r256(h->n_sym * nr_max * 8) + h->eng->sweep_workspace_bytes(nr_max);
+        bool chain = h->eng && h->eng->has_chain();
+        if (h->eng) {
+            const int64_t xb = r256(h->n_sym * nr_max * 8);
+            need = xb + h->eng->sweep_workspace_bytes(nr_max, chain);
+            if (need > NOALLOC_SCRATCH_BYTES && chain && h->eng->precision() == PREC_FP64) {
+                // an FP64 sweep whose solve chains do not fit runs every level stepped
+                chain = false;
+                need = xb + h->eng->sweep_workspace_bytes(nr_max, chain);
+            }
+        }
         if (need > NOALLOC_SCRATCH_BYTES) {
             set_error("rfg_solve_device_noalloc: this handle needs " + std::to_string(need) + " bytes of scratch for " +
                       std::to_string(nr_max) + " right-hand side(s) per sweep; the fixed scratch holds " +
@@ -987,7 +996,7 @@ int32_t rfg_solve_device_noalloc(const RustyfemHandle* h, size_t nrhs_, double* 
         order_after_caller(h, st);
         double* X = (double*)p;
         p += r256(h->n_sym * nr_max * 8);
-        const Engine::SweepWorkspace ws = E.carve_sweep_workspace(p, nr_max);
+        const Engine::SweepWorkspace ws = E.carve_sweep_workspace(p, nr_max, chain);
         for (int64_t j0 = 0; j0 < nrhs; j0 += CH) {
             int64_t nr = std::min(CH, nrhs - j0);
             double* bj = b + j0 * n;

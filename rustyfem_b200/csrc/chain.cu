@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "chain.h"
 #include "engine.h"
@@ -41,22 +42,34 @@ namespace {
 constexpr int CT = 256;             // threads per CTA
 constexpr int CQ = WS / 4;          // rows (forward) or columns (backward) of a block per CTA
 constexpr int CL = WS / CQ;         // CTAs per cluster: one block
-constexpr int FQP = CQ + 16;        // pitch (floats) of a forward tile quarter: float4 rows without conflicts
+// The tiles of a block stream in pieces of 256-byte rows, so that the ring is the same size for
+// an FP32 and an FP64 factor: forward 64 rows × FQC columns, backward BRC rows × 64 columns.
+template <typename T>
+constexpr int FQC = 256 / (int)sizeof(T);         // columns of a forward piece
+template <typename T>
+constexpr int FQP = FQC<T> + 64 / (int)sizeof(T); // its pitch: 16-byte row reads without conflicts
+template <typename T>
+constexpr int FPB = WS / FQC<T>;                  // forward pieces of a block
+template <typename T>
+constexpr int BRC = 256 / (int)sizeof(T);         // rows of a backward piece
+template <typename T>
+constexpr int BPB = WS / BRC<T>;                  // backward pieces of a block
 constexpr int FLP = WS + 4;         // pitch (doubles) of the forward inverse rows
-constexpr int BTP = CQ;             // pitch (floats) of a backward tile chunk
+constexpr int BTP = CQ;             // pitch of a backward piece
 constexpr long CHAIN_SPIN = 1L << 22;  // polls of a flag (about a second) before a wait gives up
 
 static_assert(CL == 4 && CT == 4 * CQ, "four CTAs of 256 threads per block");
 static_assert(CQ == CHAIN_PIECE, "the later-row pieces of the plan are one CTA's rows or columns");
 
 constexpr size_t fwd_smem(int R) {
-    return (size_t)CQ * FLP * 8 + (size_t)4 * CQ * FQP * 4 + (size_t)WS * R * 8 + (size_t)CQ * R * 8;
+    return (size_t)CQ * FLP * 8 + (size_t)4 * CQ * FQP<float> * sizeof(float) + (size_t)WS * R * 8 + (size_t)CQ * R * 8;
 }
 constexpr size_t bwd_smem(int R) {
-    return (size_t)WS * CQ * 8 + (size_t)4 * CQ * BTP * 4 + (size_t)4 * CQ * R * 8 + (size_t)WS * R * 8 +
+    return (size_t)WS * CQ * 8 + (size_t)4 * BRC<float> * BTP * sizeof(float) + (size_t)4 * CQ * R * 8 + (size_t)WS * R * 8 +
            (size_t)CQ * R * 8;
 }
-constexpr size_t INV_SMEM = (size_t)2 * NB * (NB + 1) * sizeof(double);
+static_assert(FQP<float> * sizeof(float) == FQP<double> * sizeof(double) && BRC<float> * sizeof(float) == BRC<double> * sizeof(double),
+              "the rings of both precisions have one size");
 static_assert(fwd_smem(4) <= 232448 && bwd_smem(4) <= 232448, "shared memory of a CTA");
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -127,50 +140,50 @@ __device__ __forceinline__ void quad_sum(double (&a)[R]) {
     }
 }
 
-// Forward tiles: acc (thread (i, q): row i, columns 4(q + 4v) .. of each 64-column quarter)
-// += Σ_{Q < nq} L[r0 + i, quarter Q]·y over the quarters of the blocks 0, 1, ...; quarter Q
-// in ring slot Q & 3, three quarters in flight. yload(j) fills yb with y_j (all threads,
+// Forward tiles: acc (thread (i, q): row i, 16-byte groups q, q + 4, ... of each piece's row)
+// += Σ_{Q < nq} L[r0 + i, piece Q]·y over the pieces of the blocks 0, 1, ...; piece Q in
+// ring slot Q & 3, three pieces in flight. yload(j) fills yb with y_j (all threads,
 // starting with a barrier that ends the previous block's use of yb).
-template <int R, typename YLoad>
-__device__ __forceinline__ void fwd_tiles(double (&acc)[R], float* ring, double* yb, const float* prow, int64_t ldp,
+template <typename T, int R, typename YLoad>
+__device__ __forceinline__ void fwd_tiles(double (&acc)[R], T* ring, double* yb, const T* prow, int64_t ldp,
                                           int64_t k, int nr, int nq, YLoad&& yload) {
+    constexpr int QC = FQC<T>, QP = FQP<T>, PB = FPB<T>, VEC = 16 / (int)sizeof(T);
+    using VT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
     const int tid = threadIdx.x, i = tid >> 2, q = tid & 3;
     auto issue = [&](int Q) {
-        const int64_t c0 = (int64_t)(Q >> 2) * WS + (Q & 3) * 64;
-        const int ncol = (int)max((int64_t)0, min((int64_t)64, k - c0));
-        if (ncol > 0 && nr > 0) cp_async_tile<float>(ring + (Q & 3) * CQ * FQP, FQP, prow + c0, ldp, nr, ncol, CQ, 64, CT);
+        const int64_t c0 = (int64_t)Q * QC;
+        const int ncol = (int)max((int64_t)0, min((int64_t)QC, k - c0));
+        if (ncol > 0 && nr > 0) cp_async_tile<T>(ring + (Q & 3) * CQ * QP, QP, prow + c0, ldp, nr, ncol, CQ, QC, CT);
         cp_async_commit();
     };
     for (int Q = 0; Q < min(3, nq); Q++) issue(Q);
     for (int Q = 0; Q < nq; Q++) {
-        const int64_t j = Q >> 2;
-        const int qq = Q & 3;
+        const int64_t j = Q / PB;
+        const int qq = Q % PB;
         if (qq == 0) yload(j);
         cp_wait_upto(min(2, nq - 1 - Q));
-        __syncthreads();  // quarter Q and y_j visible; every thread is done with quarter Q − 1
+        __syncthreads();  // piece Q and y_j visible; every thread is done with piece Q − 1
         if (Q + 3 < nq) issue(Q + 3);
-        if (j * WS + qq * 64 < k) {
-            const float* Lt = ring + qq * CQ * FQP + i * FQP;
-            const double* yq = yb + qq * 64 * R;
+        if ((int64_t)Q * QC < k) {
+            const T* Lt = ring + (Q & 3) * CQ * QP + i * QP;
+            const double* yq = yb + qq * QC * R;
 #pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const int c = 4 * (q + 4 * v);
-                const float4 l = *reinterpret_cast<const float4*>(Lt + c);
+            for (int v = 0; v < QC / (4 * VEC); v++) {
+                const int c = VEC * (q + 4 * v);
+                const VT l4 = *reinterpret_cast<const VT*>(Lt + c);
+                const T* l = reinterpret_cast<const T*>(&l4);
 #pragma unroll
-                for (int r = 0; r < R; r++) {
-                    acc[r] = fma((double)l.x, yq[c * R + r], acc[r]);
-                    acc[r] = fma((double)l.y, yq[(c + 1) * R + r], acc[r]);
-                    acc[r] = fma((double)l.z, yq[(c + 2) * R + r], acc[r]);
-                    acc[r] = fma((double)l.w, yq[(c + 3) * R + r], acc[r]);
-                }
+                for (int e = 0; e < VEC; e++)
+#pragma unroll
+                    for (int r = 0; r < R; r++) acc[r] = fma((double)l[e], yq[(c + e) * R + r], acc[r]);
             }
         }
     }
 }
 
-template <int R>
+template <typename T, int R>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
-    k_chain_fwd(const double* __restrict__ X, double* __restrict__ Y, const float* __restrict__ panel,
+    k_chain_fwd(const double* __restrict__ X, double* __restrict__ Y, const T* __restrict__ panel,
                 const double* __restrict__ cinv, const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
                 const int64_t* __restrict__ items, int64_t nitems, int* __restrict__ flags, int* __restrict__ counter,
                 int* __restrict__ err) {
@@ -178,8 +191,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     const int s = (int)cluster.block_rank();
     extern __shared__ __align__(16) double sm[];
     double* Lv = sm;                                                   // [CQ][FLP]: inverse rows 64s ..
-    float* ring = reinterpret_cast<float*>(sm + CQ * FLP);             // [4][CQ][FQP]: tile quarters
-    double* yb = reinterpret_cast<double*>(ring + 4 * CQ * FQP);       // [WS][R]: y_J, then x_B
+    T* ring = reinterpret_cast<T*>(sm + CQ * FLP);                     // [4][CQ][FQP]: tile pieces
+    double* yb = reinterpret_cast<double*>(ring + 4 * CQ * FQP<T>);    // [WS][R]: y_J, then x_B
     double* xo = yb + WS * R;                                          // [CQ][R]: this CTA's rows of x_B
     __shared__ int64_t s_item;
     const int tid = threadIdx.x, i = tid >> 2, q = tid & 3;
@@ -197,7 +210,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
         double acc[R];
 #pragma unroll
         for (int r = 0; r < R; r++) acc[r] = 0.0;
-        fwd_tiles<R>(acc, ring, yb, panel + f.poff + r0 * f.ldp, f.ldp, f.k, nr, 4 * (int)b, [&](int64_t j) {
+        fwd_tiles<T, R>(acc, ring, yb, panel + f.poff + r0 * f.ldp, f.ldp, f.k, nr, FPB<T> * (int)b, [&](int64_t j) {
             if (tid == 0) chain_wait(&flags[cb0 + j], CL, err);
             __syncthreads();
             const int wbj = (int)min((int64_t)WS, f.k - j * WS);
@@ -236,13 +249,13 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
 
 // The later rows of a chain level's fronts after the level's chain: V[rows] −= L21·y over
 // all the front's pivots, one CTA per CHAIN_PIECE rows.
-template <int R>
+template <typename T, int R>
 __global__ void __launch_bounds__(CT) k_chain_rows(const double* __restrict__ Y, double* __restrict__ V,
-                                                   const float* __restrict__ panel, const DFront* __restrict__ fr,
+                                                   const T* __restrict__ panel, const DFront* __restrict__ fr,
                                                    const int64_t* __restrict__ items) {
     extern __shared__ __align__(16) double sm[];
-    float* ring = reinterpret_cast<float*>(sm);                   // [4][CQ][FQP]
-    double* yb = reinterpret_cast<double*>(ring + 4 * CQ * FQP);  // [WS][R]
+    T* ring = reinterpret_cast<T*>(sm);                              // [4][CQ][FQP]
+    double* yb = reinterpret_cast<double*>(ring + 4 * CQ * FQP<T>);  // [WS][R]
     const int tid = threadIdx.x, i = tid >> 2, q = tid & 3;
     const int64_t t = items[2 * blockIdx.x], c = items[2 * blockIdx.x + 1];
     const DFront f = fr[t];
@@ -251,13 +264,13 @@ __global__ void __launch_bounds__(CT) k_chain_rows(const double* __restrict__ Y,
     double acc[R];
 #pragma unroll
     for (int r = 0; r < R; r++) acc[r] = 0.0;
-    fwd_tiles<R>(acc, ring, yb, panel + f.poff + r0 * f.ldp, f.ldp, f.k, nr, 4 * (int)((f.k + WS - 1) / WS),
-                 [&](int64_t j) {
-                     __syncthreads();
-                     const int wbj = (int)min((int64_t)WS, f.k - j * WS);
-                     const double* ys = Y + (f.start + j * WS) * R;
-                     for (int e = tid; e < WS * R; e += CT) yb[e] = e < wbj * R ? ys[e] : 0.0;
-                 });
+    fwd_tiles<T, R>(acc, ring, yb, panel + f.poff + r0 * f.ldp, f.ldp, f.k, nr, FPB<T> * (int)((f.k + WS - 1) / WS),
+                    [&](int64_t j) {
+                        __syncthreads();
+                        const int wbj = (int)min((int64_t)WS, f.k - j * WS);
+                        const double* ys = Y + (f.start + j * WS) * R;
+                        for (int e = tid; e < WS * R; e += CT) yb[e] = e < wbj * R ? ys[e] : 0.0;
+                    });
     quad_sum<R>(acc);
     if (q == 0 && i < nr) {
         double* vt = V + (f.vuoff + c * CQ + i) * R;
@@ -266,20 +279,20 @@ __global__ void __launch_bounds__(CT) k_chain_rows(const double* __restrict__ Y,
     }
 }
 
-// Backward chunks: acc (thread (c, g): column c, rows g, g + 4, ... of each 64-row chunk)
+// Backward chunks: acc (thread (c, g): column c, rows g, g + 4, ... of each BRC-row chunk)
 // += Σ_{h < nh} L[rows of chunk h, col0 + c]·y(rows); chunk h in ring slot h & 3, three in
 // flight. rows_of(h, ra) gives the chunk's first row and row count; yload(h) runs before
 // chunk h (all threads) and returns where the chunk's y values are in shared memory;
 // issue_y(h) queues the chunk's y values with its tile (cp.async) when it can.
-template <int R, typename Rows, typename YLoad, typename IssueY>
-__device__ __forceinline__ void bwd_tiles(double (&acc)[R], float* ring, const float* pcol, int64_t ldp, int nc, int nh,
+template <typename T, int R, typename Rows, typename YLoad, typename IssueY>
+__device__ __forceinline__ void bwd_tiles(double (&acc)[R], T* ring, const T* pcol, int64_t ldp, int nc, int nh,
                                           Rows&& rows_of, YLoad&& yload, IssueY&& issue_y) {
     const int tid = threadIdx.x, c = tid & (CQ - 1), g = tid >> 6;
     auto issue = [&](int h) {
         int64_t ra;
         const int nrr = rows_of(h, ra);
         if (nrr > 0 && nc > 0)
-            cp_async_tile<float>(ring + (h & 3) * CQ * BTP, BTP, pcol + ra * ldp, ldp, nrr, nc, CQ, CQ, CT);
+            cp_async_tile<T>(ring + (h & 3) * BRC<T> * BTP, BTP, pcol + ra * ldp, ldp, nrr, nc, BRC<T>, CQ, CT);
         issue_y(h, ra, nrr);
         cp_async_commit();
     };
@@ -292,9 +305,9 @@ __device__ __forceinline__ void bwd_tiles(double (&acc)[R], float* ring, const f
         __syncthreads();  // chunk h visible; every thread is done with chunk h − 1
         if (h + 3 < nh) issue(h + 3);
         if (nrr > 0) {
-            const float* Lt = ring + (h & 3) * CQ * BTP + c;
+            const T* Lt = ring + (h & 3) * BRC<T> * BTP + c;
 #pragma unroll 4
-            for (int u = 0; u < CQ / 4; u++) {
+            for (int u = 0; u < BRC<T> / 4; u++) {
                 const int rr = g + 4 * u;
                 const double l = Lt[rr * BTP];
 #pragma unroll
@@ -319,17 +332,17 @@ __device__ __forceinline__ void col_sum(double (&acc)[R], double* red) {
     }
 }
 
-template <int R>
+template <typename T, int R>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
-    k_chain_bwd(double* __restrict__ Y, const float* __restrict__ panel, const double* __restrict__ cinv,
+    k_chain_bwd(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ cinv,
                 const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk, const int64_t* __restrict__ items,
                 int64_t nitems, int* __restrict__ flags, int* __restrict__ counter, int* __restrict__ err) {
     cg::cluster_group cluster = cg::this_cluster();
     const int s = (int)cluster.block_rank();
     extern __shared__ __align__(16) double sm[];
     double* Lc = sm;                                               // [WS][CQ]: rows 64s .. of inverse columns 64s ..
-    float* ring = reinterpret_cast<float*>(sm + WS * CQ);          // [4][CQ][BTP]: tile chunks
-    double* yp = reinterpret_cast<double*>(ring + 4 * CQ * BTP);   // [WS][R]: y of a later block; then z_B
+    T* ring = reinterpret_cast<T*>(sm + WS * CQ);                  // [4][BRC][BTP]: tile chunks
+    double* yp = reinterpret_cast<double*>(ring + 4 * BRC<T> * BTP);  // [WS][R]: y of a later block; then z_B
     double* red = yp + WS * R;                                     // [4][CQ][R]
     double* zo = red + 4 * CQ * R;                                 // [CQ][R]: this CTA's columns of z_B
     __shared__ int64_t s_item;
@@ -350,23 +363,23 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
         double acc[R];
 #pragma unroll
         for (int r = 0; r < R; r++) acc[r] = 0.0;
-        // the chunks of blocks nb − 1, ..., b + 1, four per block
-        bwd_tiles<R>(
-            acc, ring, panel + f.poff + col0, f.ldp, nc, 4 * (int)(nb - 1 - b),
+        // the chunks of blocks nb − 1, ..., b + 1, BPB per block
+        bwd_tiles<T, R>(
+            acc, ring, panel + f.poff + col0, f.ldp, nc, BPB<T> * (int)(nb - 1 - b),
             [&](int h, int64_t& ra) -> int {
-                ra = (nb - 1 - h / 4) * WS + (h & 3) * CQ;
-                return (int)max((int64_t)0, min((int64_t)CQ, f.k - ra));
+                ra = (nb - 1 - h / BPB<T>) * WS + (h % BPB<T>) * BRC<T>;
+                return (int)max((int64_t)0, min((int64_t)BRC<T>, f.k - ra));
             },
             [&](int h) -> const double* {
-                if ((h & 3) == 0) {
-                    const int64_t bb = nb - 1 - h / 4;
+                if (h % BPB<T> == 0) {
+                    const int64_t bb = nb - 1 - h / BPB<T>;
                     if (tid == 0) chain_wait(&flags[cb0 + bb], CL, err);
                     __syncthreads();
                     const int wbb = (int)min((int64_t)WS, f.k - bb * WS);
                     const double* src = Y + (f.start + bb * WS) * R;
                     for (int e = tid; e < WS * R; e += CT) yp[e] = e < wbb * R ? __ldcg(src + e) : 0.0;
                 }
-                return yp + (h & 3) * CQ * R;
+                return yp + (h % BPB<T>) * BRC<T> * R;
             },
             [](int, int64_t, int) {});
         col_sum<R>(acc, red);
@@ -420,35 +433,36 @@ __global__ void __launch_bounds__(CT) k_chain_gather(const double* __restrict__ 
 // CHAIN_PIECE pivot columns and group of rows (blockIdx.y of CHAIN_GROUPS), into
 // part[(item · CHAIN_GROUPS + group) · CHAIN_PIECE + column]; k_chain_colsum subtracts them
 // from z in group order.
-template <int R>
+template <typename T, int R>
 __global__ void __launch_bounds__(CT) k_chain_cols(double* __restrict__ part, const double* __restrict__ V,
-                                                   const float* __restrict__ panel, const DFront* __restrict__ fr,
+                                                   const T* __restrict__ panel, const DFront* __restrict__ fr,
                                                    const int64_t* __restrict__ items) {
     extern __shared__ __align__(16) double sm[];
-    float* ring = reinterpret_cast<float*>(sm);                   // [4][CQ][BTP]
-    double* ys = reinterpret_cast<double*>(ring + 4 * CQ * BTP);  // [4][CQ][R]: y of a chunk, by slot
-    double* red = ys + 4 * CQ * R;                                // [4][CQ][R]
+    constexpr int RC = BRC<T>;
+    T* ring = reinterpret_cast<T*>(sm);                           // [4][RC][BTP]
+    double* ys = reinterpret_cast<double*>(ring + 4 * RC * BTP);  // [4][RC][R]: y of a chunk, by slot
+    double* red = ys + 4 * RC * R;                                // [4][CQ][R]
     const int tid = threadIdx.x, c = tid & (CQ - 1);
     const int64_t t = items[2 * blockIdx.x], cc = items[2 * blockIdx.x + 1];
     const DFront f = fr[t];
     const int64_t col0 = cc * CQ;
     const int nc = (int)min((int64_t)CQ, f.k - col0);
-    const int nchunk = (int)((f.u + CQ - 1) / CQ), g = blockIdx.y;
+    const int nchunk = (int)((f.u + RC - 1) / RC), g = blockIdx.y;
     const int h0 = nchunk * g / CHAIN_GROUPS, h1 = nchunk * (g + 1) / CHAIN_GROUPS;
     double acc[R];
 #pragma unroll
     for (int r = 0; r < R; r++) acc[r] = 0.0;
-    bwd_tiles<R>(
+    bwd_tiles<T, R>(
         acc, ring, panel + f.poff + col0, f.ldp, nc, h1 - h0,
         [&](int h, int64_t& ra) -> int {
-            ra = f.k + (int64_t)(h0 + h) * CQ;
-            return (int)min((int64_t)CQ, f.m - ra);
+            ra = f.k + (int64_t)(h0 + h) * RC;
+            return (int)min((int64_t)RC, f.m - ra);
         },
-        [&](int h) -> const double* { return ys + (h & 3) * CQ * R; },
+        [&](int h) -> const double* { return ys + (h & 3) * RC * R; },
         [&](int h, int64_t ra, int nrr) {
-            if (tid < CQ * R) {
+            if (tid < RC * R) {
                 const int rr = tid / R, r = tid - rr * R;
-                double* dst = ys + ((h & 3) * CQ + rr) * R + r;
+                double* dst = ys + ((h & 3) * RC + rr) * R + r;
                 if (rr < nrr)
                     cp_async8(dst, V + (f.vuoff + ra - f.k + rr) * R + r);
                 else
@@ -481,77 +495,104 @@ __global__ void __launch_bounds__(CT) k_chain_colsum(double* __restrict__ Y, con
 
 // The inverse of a chain block's unit-lower diagonal block, by block columns of NB:
 // M_jj = inv(L_jj) (from the factorization), M_ij = −inv(L_ii)·Σ_{j ≤ t < i} L_it·M_tj.
-__global__ void __launch_bounds__(256) k_chain_inverse(double* __restrict__ cinv, const float* __restrict__ panel,
+// The block columns are independent: one CTA (8 warps of 32×16 outputs) each, its M_tj kept
+// in shared memory, the products on the FP64 tensor-core path. It is bound by the chain of
+// 64³ products of block column 0 (nine for a full block) and by the loads of L between them.
+constexpr int IVP = NB + 4;  // pitch (doubles): fragment loads of both operands without conflicts
+constexpr size_t INV_SMEM = (size_t)5 * NB * IVP * sizeof(double);
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_chain_inverse(double* __restrict__ cinv, const T* __restrict__ panel,
                                                        const double* __restrict__ linv, const DFront* __restrict__ fr,
                                                        const int64_t* __restrict__ chain_blk,
                                                        const int64_t* __restrict__ chain_bfront) {
     extern __shared__ __align__(16) double sm[];
-    double(*A)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(sm);
-    double(*B)[NB + 1] = A + NB;
+    double* A = sm;                  // [NB][IVP]: L_it, then inv(L_ii)
+    double* B = sm + NB * IVP;       // [NB][IVP]: the sum
+    double* Mt = sm + 2 * NB * IVP;  // [3][NB][IVP]: M_jj, M_{j+1,j}, M_{j+2,j}
     const int64_t cb = blockIdx.x, ft = chain_bfront[cb];
+    const int j = blockIdx.y;
     const DFront f = fr[ft];
     const int64_t b = cb - chain_blk[ft], J0 = b * WS;
     const int wb = (int)min((int64_t)WS, f.k - J0), nbw = (wb + NB - 1) / NB;
-    double* M = cinv + cb * (int64_t)WS * WS;
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    for (int e = tid; e < WS * WS / 2; e += 256) reinterpret_cast<double2*>(M)[e] = make_double2(0.0, 0.0);
-    __syncthreads();
-    for (int j = 0; j < nbw; j++) {
-        const double* li = linv + (f.blk_off + 4 * b + j) * (int64_t)(NB * NB);
-        for (int e = tid; e < NB * NB; e += 256) M[(j * NB + e / NB) * WS + j * NB + e % NB] = li[e];
+    double* M = cinv + cb * (int64_t)WS * WS + j * NB;  // the block column
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    const int wm = warp & 1, wn = warp >> 1;
+    // zero above the diagonal block and beyond the block's width
+    for (int e = tid; e < WS * NB / 2; e += 256) {
+        const int r = e / (NB / 2), c = 2 * (e % (NB / 2));
+        if (j >= nbw || r < j * NB || r >= nbw * NB)
+            *reinterpret_cast<double2*>(M + (int64_t)r * WS + c) = make_double2(0.0, 0.0);
     }
-    __syncthreads();
-    auto gemm = [&](double (&acc)[4][4]) {
+    if (j >= nbw) return;
+    const double* li = linv + (f.blk_off + 4 * b) * (int64_t)(NB * NB);
+    for (int e = tid; e < NB * NB; e += 256) {
+        const double v = li[j * NB * NB + e];
+        Mt[(e / NB) * IVP + e % NB] = v;
+        M[(int64_t)(j * NB + e / NB) * WS + e % NB] = v;
+    }
+    // acc += A·B over NB: rows 32·wm + 8a + g, columns 16·wn + 8c + 2q + {0, 1}
+    auto gemm = [&](double (&acc)[4][2][2], const double* Bt) {
+        const double* a0 = A + (wm * 32 + g) * IVP + q;
+        const double* b0 = Bt + q * IVP + wn * 16 + g;
 #pragma unroll 4
-        for (int k = 0; k < NB; k++) {
-            double av[4], bv[4];
+        for (int k = 0; k < NB; k += 4) {
+            double fa[4], fb[2];
 #pragma unroll
-            for (int u = 0; u < 4; u++) av[u] = A[4 * ty + u][k];
+            for (int a = 0; a < 4; a++) fa[a] = a0[a * 8 * IVP + k];
 #pragma unroll
-            for (int v = 0; v < 4; v++) bv[v] = B[k][4 * tx + v];
+            for (int c = 0; c < 2; c++) fb[c] = b0[k * IVP + c * 8];
 #pragma unroll
-            for (int u = 0; u < 4; u++)
+            for (int a = 0; a < 4; a++)
 #pragma unroll
-                for (int v = 0; v < 4; v++) acc[u][v] = fma(av[u], bv[v], acc[u][v]);
+                for (int c = 0; c < 2; c++) dmma_884(acc[a][c][0], acc[a][c][1], fa[a], fb[c]);
         }
     };
-    for (int j = 0; j + 1 < nbw; j++)
-        for (int i = j + 1; i < nbw; i++) {
-            double acc[4][4] = {};
-            for (int tt = j; tt < i; tt++) {
-                for (int e = tid; e < NB * NB; e += 256) {
-                    const int r = e / NB, cc = e % NB, row = i * NB + r;
-                    A[r][cc] = row < wb ? (double)panel[f.poff + (J0 + row) * f.ldp + J0 + tt * NB + cc] : 0.0;
-                    B[r][cc] = __ldcg(&M[(tt * NB + r) * WS + j * NB + cc]);
-                }
-                __syncthreads();
-                gemm(acc);
-                __syncthreads();
+    for (int i = j + 1; i < nbw; i++) {
+        double acc[4][2][2] = {};
+        for (int t = j; t < i; t++) {
+            __syncthreads();  // A is read
+            for (int e = tid; e < NB * NB; e += 256) {
+                const int row = i * NB + e / NB;
+                A[(e / NB) * IVP + e % NB] =
+                    row < wb ? (double)panel[f.poff + (J0 + row) * f.ldp + J0 + t * NB + e % NB] : 0.0;
             }
-            // the sum becomes the right operand (B is free after the last product's barrier)
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int v = 0; v < 4; v++) B[4 * ty + u][4 * tx + v] = acc[u][v];
-            const double* li = linv + (f.blk_off + 4 * b + i) * (int64_t)(NB * NB);
-            for (int e = tid; e < NB * NB; e += 256) A[e / NB][e % NB] = li[e];
             __syncthreads();
-            double acc2[4][4] = {};
-            gemm(acc2);
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int v = 0; v < 4; v++) M[(i * NB + 4 * ty + u) * WS + j * NB + 4 * tx + v] = -acc2[u][v];
-            __syncthreads();
+            gemm(acc, Mt + (t - j) * NB * IVP);
         }
+        __syncthreads();
+        for (int e = tid; e < NB * NB; e += 256) A[(e / NB) * IVP + e % NB] = li[i * NB * NB + e];
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                    B[(wm * 32 + a * 8 + g) * IVP + wn * 16 + c * 8 + 2 * q + e] = acc[a][c][e];
+        __syncthreads();
+        double acc2[4][2][2] = {};
+        gemm(acc2, B);
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int r = wm * 32 + a * 8 + g, cc = wn * 16 + c * 8 + 2 * q + e;
+                    M[(int64_t)(i * NB + r) * WS + cc] = -acc2[a][c][e];
+                    if (i - j < 3) Mt[((i - j) * NB + r) * IVP + cc] = -acc2[a][c][e];
+                }
+    }
 }
 
 // per device: attributes set, the number of clusters that fit at once (forward, backward;
 // by right-hand sides 1 .. 4)
 struct ChainDev {
     bool done = false;
-    int fwd[5] = {0, 0, 0, 0, 0}, bwd[5] = {0, 0, 0, 0, 0};
+    int fwd[2][5] = {}, bwd[2][5] = {};  // [0] FP32, [1] FP64 factor
 };
+template <typename T>
+constexpr int chain_kind = sizeof(T) == 8 ? 1 : 0;
 
 template <typename K>
 int fit_clusters(K kern, size_t smem) {
@@ -572,13 +613,23 @@ int fit_clusters(K kern, size_t smem) {
     return n;
 }
 
-constexpr size_t rows_smem(int R) { return (size_t)4 * CQ * FQP * 4 + (size_t)WS * R * 8; }
-constexpr size_t cols_smem(int R) { return (size_t)4 * CQ * BTP * 4 + (size_t)8 * CQ * R * 8; }
+constexpr size_t rows_smem(int R) { return (size_t)4 * CQ * FQP<float> * sizeof(float) + (size_t)WS * R * 8; }
+constexpr size_t cols_smem(int R) { return (size_t)4 * BRC<float> * BTP * sizeof(float) + (size_t)8 * CQ * R * 8; }
 
-template <int R>
-void set_piece_attrs() {
-    RFG_CUDA(cudaFuncSetAttribute(k_chain_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(R)));
-    RFG_CUDA(cudaFuncSetAttribute(k_chain_cols<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_smem(R)));
+template <typename T, int R>
+void set_chain_attrs(ChainDev& d) {
+    d.fwd[chain_kind<T>][R] = fit_clusters(k_chain_fwd<T, R>, fwd_smem(R));
+    d.bwd[chain_kind<T>][R] = fit_clusters(k_chain_bwd<T, R>, bwd_smem(R));
+    RFG_CUDA(cudaFuncSetAttribute(k_chain_rows<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(R)));
+    RFG_CUDA(cudaFuncSetAttribute(k_chain_cols<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_smem(R)));
+}
+template <typename T>
+void set_chain_attrs_all(ChainDev& d) {
+    RFG_CUDA(cudaFuncSetAttribute(k_chain_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INV_SMEM));
+    set_chain_attrs<T, 1>(d);
+    set_chain_attrs<T, 2>(d);
+    set_chain_attrs<T, 3>(d);
+    set_chain_attrs<T, 4>(d);
 }
 
 const ChainDev& chain_dev() {
@@ -590,19 +641,8 @@ const ChainDev& chain_dev() {
     std::lock_guard<std::mutex> lock(mu);
     ChainDev& d = devs[dev];
     if (!d.done) {
-        RFG_CUDA(cudaFuncSetAttribute(k_chain_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INV_SMEM));
-        d.fwd[1] = fit_clusters(k_chain_fwd<1>, fwd_smem(1));
-        d.fwd[2] = fit_clusters(k_chain_fwd<2>, fwd_smem(2));
-        d.fwd[3] = fit_clusters(k_chain_fwd<3>, fwd_smem(3));
-        d.fwd[4] = fit_clusters(k_chain_fwd<4>, fwd_smem(4));
-        d.bwd[1] = fit_clusters(k_chain_bwd<1>, bwd_smem(1));
-        d.bwd[2] = fit_clusters(k_chain_bwd<2>, bwd_smem(2));
-        d.bwd[3] = fit_clusters(k_chain_bwd<3>, bwd_smem(3));
-        d.bwd[4] = fit_clusters(k_chain_bwd<4>, bwd_smem(4));
-        set_piece_attrs<1>();
-        set_piece_attrs<2>();
-        set_piece_attrs<3>();
-        set_piece_attrs<4>();
+        set_chain_attrs_all<float>(d);
+        set_chain_attrs_all<double>(d);
         d.done = true;
     }
     return d;
@@ -619,11 +659,13 @@ void check_nrhs(int nrhs) {
 
 }  // namespace
 
-void launch_chain_inverse(double* cinv, const float* panel, const double* linv, const DFront* fronts,
+template <typename T>
+void launch_chain_inverse(double* cinv, const T* panel, const double* linv, const DFront* fronts,
                           const int64_t* chain_blk, const int64_t* chain_bfront, int64_t nblocks, cudaStream_t st) {
     if (nblocks <= 0) return;
     chain_dev();
-    k_chain_inverse<<<(unsigned)nblocks, 256, INV_SMEM, st>>>(cinv, panel, linv, fronts, chain_blk, chain_bfront);
+    k_chain_inverse<T><<<dim3((unsigned)nblocks, CL), 256, INV_SMEM, st>>>(cinv, panel, linv, fronts, chain_blk,
+                                                                          chain_bfront);
     RFG_CUDA(cudaGetLastError());
 }
 
@@ -646,47 +688,66 @@ void launch_chain_inverse(double* cinv, const float* panel, const double* linv, 
         }                          \
     } while (0)
 
-void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, const float* panel, const double* cinv,
+template <typename T>
+void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, const T* panel, const double* cinv,
                       const DFront* fronts, const int64_t* chain_blk, const int64_t* items, int* flags, int* counter,
                       int* err, cudaStream_t st) {
     if (nitems <= 0) return;
     const ChainDev& d = chain_dev();
-    RFG_CHAIN_BY_R(nrhs, (k_chain_fwd<R><<<grid_for_items(d.fwd[R], nitems), CT, fwd_smem(R), st>>>(
+    RFG_CHAIN_BY_R(nrhs, (k_chain_fwd<T, R><<<grid_for_items(d.fwd[chain_kind<T>][R], nitems), CT, fwd_smem(R), st>>>(
                               X, Y, panel, cinv, fronts, chain_blk, items, nitems, flags, counter, err)));
     RFG_CUDA(cudaGetLastError());
 }
 
-void launch_chain_rows(int nrhs, int64_t nitems, const double* Y, double* V, const float* panel, const DFront* fronts,
+template <typename T>
+void launch_chain_rows(int nrhs, int64_t nitems, const double* Y, double* V, const T* panel, const DFront* fronts,
                        const int64_t* items, cudaStream_t st) {
     if (nitems <= 0) return;
     chain_dev();
-    RFG_CHAIN_BY_R(nrhs, (k_chain_rows<R><<<(unsigned)nitems, CT, rows_smem(R), st>>>(Y, V, panel, fronts, items)));
+    RFG_CHAIN_BY_R(nrhs, (k_chain_rows<T, R><<<(unsigned)nitems, CT, rows_smem(R), st>>>(Y, V, panel, fronts, items)));
     RFG_CUDA(cudaGetLastError());
 }
 
+template <typename T>
 void launch_chain_cols(int nrhs, int64_t ngather, const int64_t* gather_items, int64_t nitems, const int64_t* items,
-                       double* Y, double* V, double* part, const float* panel, const DFront* fronts,
+                       double* Y, double* V, double* part, const T* panel, const DFront* fronts,
                        const int64_t* rows, cudaStream_t st) {
     if (nitems <= 0) return;
     chain_dev();
     check_nrhs(nrhs);
     if (ngather > 0) k_chain_gather<<<(unsigned)ngather, CT, 0, st>>>(Y, V, fronts, rows, gather_items, nrhs);
-    RFG_CHAIN_BY_R(nrhs, (k_chain_cols<R><<<dim3((unsigned)nitems, CHAIN_GROUPS), CT, cols_smem(R), st>>>(
+    RFG_CHAIN_BY_R(nrhs, (k_chain_cols<T, R><<<dim3((unsigned)nitems, CHAIN_GROUPS), CT, cols_smem(R), st>>>(
                               part, V, panel, fronts, items)));
     k_chain_colsum<<<(unsigned)nitems, CT, 0, st>>>(Y, part, fronts, items, nrhs);
     RFG_CUDA(cudaGetLastError());
 }
 
-void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const float* panel, const double* cinv,
+template <typename T>
+void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const T* panel, const double* cinv,
                       const DFront* fronts, const int64_t* chain_blk, const int64_t* items, int* flags, int* counter,
                       int* err, cudaStream_t st) {
     if (nitems <= 0) return;
     const ChainDev& d = chain_dev();
-    RFG_CHAIN_BY_R(nrhs, (k_chain_bwd<R><<<grid_for_items(d.bwd[R], nitems), CT, bwd_smem(R), st>>>(
+    RFG_CHAIN_BY_R(nrhs, (k_chain_bwd<T, R><<<grid_for_items(d.bwd[chain_kind<T>][R], nitems), CT, bwd_smem(R), st>>>(
                               Y, panel, cinv, fronts, chain_blk, items, nitems, flags, counter, err)));
     RFG_CUDA(cudaGetLastError());
 }
 
 #undef RFG_CHAIN_BY_R
+
+#define RFG_CHAIN_INSTANCE(T)                                                                                       \
+    template void launch_chain_inverse<T>(double*, const T*, const double*, const DFront*, const int64_t*,          \
+                                          const int64_t*, int64_t, cudaStream_t);                                   \
+    template void launch_chain_fwd<T>(int, int64_t, const double*, double*, const T*, const double*, const DFront*, \
+                                      const int64_t*, const int64_t*, int*, int*, int*, cudaStream_t);              \
+    template void launch_chain_rows<T>(int, int64_t, const double*, double*, const T*, const DFront*,               \
+                                       const int64_t*, cudaStream_t);                                               \
+    template void launch_chain_cols<T>(int, int64_t, const int64_t*, int64_t, const int64_t*, double*, double*,     \
+                                       double*, const T*, const DFront*, const int64_t*, cudaStream_t);             \
+    template void launch_chain_bwd<T>(int, int64_t, double*, const T*, const double*, const DFront*,                \
+                                      const int64_t*, const int64_t*, int*, int*, int*, cudaStream_t);
+RFG_CHAIN_INSTANCE(float)
+RFG_CHAIN_INSTANCE(double)
+#undef RFG_CHAIN_INSTANCE
 
 }  // namespace rfg

@@ -23,33 +23,38 @@ inline int64_t chain_flag_words(const Plan& P) { return 2 * P.chain_blocks + 2 *
 
 // The inverse of every chain block's unit-lower diagonal block, WS × WS in FP64 (row-major,
 // zero above the diagonal and beyond the block's width), from the NB × NB inverses of the
-// factorization and the FP32 factor: cinv[(cb·WS + r)·WS + c].
-void launch_chain_inverse(double* cinv, const float* panel, const double* linv, const DFront* fronts,
+// factorization and the factor: cinv[(cb·WS + r)·WS + c].
+template <typename T>
+void launch_chain_inverse(double* cinv, const T* panel, const double* linv, const DFront* fronts,
                           const int64_t* chain_blk, const int64_t* chain_bfront, int64_t nblocks, cudaStream_t st);
 
 // Forward chain of one level: Y[pivot rows] = L⁻¹ x for the level's fronts, X (with the
 // children's update vectors added) as the right-hand side. items: the level's (front,
 // block) pairs; flags: the forward block flags; counter: the level's work counter; err: set
 // to 1 when a wait gave up (sticky).
-void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, const float* panel, const double* cinv,
+template <typename T>
+void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, const T* panel, const double* cinv,
                       const DFront* fronts, const int64_t* chain_blk, const int64_t* items, int* flags, int* counter,
                       int* err, cudaStream_t st);
 
 // After a level's forward chain: V[later rows] −= L21·y, items the (front, piece) pairs of
 // the level's later rows.
-void launch_chain_rows(int nrhs, int64_t nitems, const double* Y, double* V, const float* panel, const DFront* fronts,
+template <typename T>
+void launch_chain_rows(int nrhs, int64_t nitems, const double* Y, double* V, const T* panel, const DFront* fronts,
                        const int64_t* items, cudaStream_t st);
 
 // Before a level's backward chain: the solution of the fronts' later rows gathered into V
 // (gather_items: the level's later-row pieces), then z[pivot columns] −= L21ᵀ·y_later
 // (items: the level's pivot-column pieces), z the scaled forward result in Y; part holds
 // the row groups' partial sums (CHAIN_GROUPS · CHAIN_PIECE · nrhs values per item).
+template <typename T>
 void launch_chain_cols(int nrhs, int64_t ngather, const int64_t* gather_items, int64_t nitems, const int64_t* items,
-                       double* Y, double* V, double* part, const float* panel, const DFront* fronts,
+                       double* Y, double* V, double* part, const T* panel, const DFront* fronts,
                        const int64_t* rows, cudaStream_t st);
 
 // Backward chain of one level: Y[pivot rows] = L11⁻ᵀ z.
-void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const float* panel, const double* cinv,
+template <typename T>
+void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const T* panel, const double* cinv,
                       const DFront* fronts, const int64_t* chain_blk, const int64_t* items, int* flags, int* counter,
                       int* err, cudaStream_t st);
 

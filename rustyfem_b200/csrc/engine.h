@@ -158,11 +158,13 @@ class Engine {
     struct SweepWorkspace {
         double* y;        // n · nrhs
         double* v;        // vu_rows · nrhs
-        double* partial;  // partial_rows() · nrhs
+        double* partial;  // partial_rows · nrhs
         int* tickets;     // max_nact, then the flag words of the solve chains
+        bool chain;       // room for the solve chains; without it every level is stepped
     };
-    int64_t sweep_workspace_bytes(int64_t nrhs) const;
-    SweepWorkspace carve_sweep_workspace(void* base, int64_t nrhs) const;
+    bool has_chain() const { return chain_inv_ != nullptr; }
+    int64_t sweep_workspace_bytes(int64_t nrhs, bool chain) const;
+    SweepWorkspace carve_sweep_workspace(void* base, int64_t nrhs, bool chain) const;
     void solve_sweep_on(double* X, int64_t nrhs, const SweepWorkspace& ws);
 
     // Pivots D in the internal numbering (device array of n doubles).
@@ -218,8 +220,8 @@ class Engine {
     // the sweeps of nrhs right-hand sides run the solve chains of the plan's chain levels
     bool chain_on(int64_t nrhs) const;
     void ensure_chain_inverse();
-    int64_t ticket_words() const;
-    int64_t partial_rows() const;  // partial-sum values per right-hand side of a sweep
+    int64_t ticket_words(bool chain) const;
+    int64_t partial_rows(bool chain) const;  // partial-sum values per right-hand side of a sweep
     void init(bool use_tc);
     void upload_plan();
     void upload_scatter();
@@ -259,7 +261,7 @@ class Engine {
     bool tc_persistent_ = true;
     double* d_ = nullptr;
     double* linv_ = nullptr;      // inverse of each unit-lower NB×NB diagonal block (solves)
-    double* chain_inv_ = nullptr; // inverse of each solve-chain block (WS × WS), mixed precision
+    double* chain_inv_ = nullptr; // inverse of each solve-chain block (WS × WS)
     int* chain_err_ = nullptr;    // set by a solve-chain wait that gave up
     int64_t chain_inv_at_ = -1;   // the numeric phase (factor_calls_) chain_inv_ was formed for
     double* adiag_ = nullptr;

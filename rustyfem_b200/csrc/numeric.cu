@@ -44,14 +44,6 @@ namespace rfg {
 
 namespace {
 
-// D = A·B + D on the FP64 tensor-core path for one 8×8×4 block (mma.sync m8n8k4 f64):
-// lane l holds A[l / 4][l % 4], B[l % 4][l / 4] and D[l / 4][2·(l % 4) + {0, 1}].
-__device__ __forceinline__ void dmma_884(double& c0, double& c1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
-
 template <typename T>
 __global__ void k_scatter(T* __restrict__ panel, const double* __restrict__ src, const int64_t* __restrict__ dst,
                           const int64_t* __restrict__ seg_ptr, const int64_t* __restrict__ seg_src, int64_t lo,
@@ -1574,7 +1566,7 @@ void Engine::init(bool) {
     scr_l_ = dalloc(std::max<int64_t>(plan_.max_scr_rows, 1) * NBO * es);
     d_ = (double*)dalloc(std::max<int64_t>(plan_.n, 1) * sizeof(double));
     linv_ = (double*)dalloc(std::max<int64_t>(plan_.nblocks, 1) * NB * NB * sizeof(double));
-    if (prec_ == PREC_MIXED && plan_.chain_blocks > 0) {
+    if (plan_.chain_blocks > 0) {
         chain_inv_ = (double*)dalloc(plan_.chain_blocks * (int64_t)WS * WS * sizeof(double));
         chain_err_ = (int*)dalloc(sizeof(int));
         RFG_CUDA(cudaMemsetAsync(chain_err_, 0, sizeof(int), stream_));

@@ -397,10 +397,11 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
     // solve chains: forward items by block position (the fronts of the level interleaved),
     // backward items by distance from the front's last block; the later rows' pieces
     {
-        int64_t cf = tun.chain_fronts;
+        int64_t cf = tun.chain_fronts, min_k = 0;
         if (cf < 0) {
             const char* e = std::getenv("RFG_SOLVE_CHAIN");
             cf = e ? std::atoll(e) : CHAIN_FRONTS;
+            if (!e) min_k = CHAIN_MIN_K;
         }
         P.level_chain.assign(nlev, 0);
         P.chain_blk.assign(nt, -1);
@@ -410,7 +411,7 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
         P.chain_cols_off.assign(nlev + 1, 0);
         for (int64_t l = 0; l < nlev; l++) {
             const int64_t lo = P.level_off[l], hi = P.level_off[l + 1];
-            if (hi > lo && hi - lo <= cf) {
+            if (hi > lo && hi - lo <= cf && P.level_maxk[l] > min_k) {
                 P.level_chain[l] = 1;
                 int64_t maxnb = 0;
                 for (int64_t i = lo; i < hi; i++) {

@@ -144,8 +144,8 @@ struct Plan {
     std::vector<int64_t> pre_wrows, pre_wpart;
     int64_t max_wrows = 0, max_wpart = 0;
     // Solve chains. On the levels with at most chain_fronts fronts (the top of the tree,
-    // where a step's launches have a few CTAs of work) a sweep of the FP32 factor with at
-    // most four right-hand sides runs as one launch per level and direction instead of
+    // where a step's launches have a few CTAs of work) a sweep with at most
+    // four right-hand sides runs as one launch per level and direction instead of
     // two per WS-wide step: each WS-wide diagonal block of a front is one work item, done
     // by a cluster of four CTAs that waits for the blocks it depends on (chain.cu). The
     // block's solve multiplies by the inverse of its unit-lower diagonal block (WS × WS,
@@ -196,6 +196,10 @@ struct Tuning {
                                          // (-1: RFG_SOLVE_CHAIN, else CHAIN_FRONTS; 0: none)
 };
 constexpr int64_t CHAIN_FRONTS = 16;
+// Levels whose fronts are all one block wide have no chain to shorten: their two step launches
+// beat the chain's six (410-equation plate, FP64: 0.181 ms per solve call stepped, 0.271 ms on
+// chains; 22³ cube 0.831 against 0.851 ms).
+constexpr int64_t CHAIN_MIN_K = WS;
 constexpr int64_t CHAIN_PIECE = 64;  // rows or columns of a later-rows CTA of the solve chains
 constexpr int CHAIN_GROUPS = 4;      // row groups of a column piece (each its own CTA and partial sums)
 

@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(256) k_wbwd(double* __restrict__ Y, const T* _
 }
 
 // ---------------------------------------------------------------------------
-// Prefetching step kernels for an FP32 factor and at most PF_MAXR right-hand sides.
+// Prefetching step kernels for at most PF_MAXR right-hand sides.
 // Every kernel of a sweep is launched as a programmatic dependent of the one before it:
 // it starts while its predecessor runs, copies the factor data it needs (unchanged
 // during a solve) into shared memory with cp.async, and only then waits for the
@@ -393,18 +393,34 @@ constexpr int PF_MAXR = 4;
 // × cols floats (cols = the step's widest block rounded up to 32), row pitch cols + 4
 // (16-byte rows, conflict-free row reads); three such CTAs fit on an SM
 constexpr int PF_RPC = PR / 2;
+// The rows kernel takes 64 rows of an FP32 factor per CTA and 32 of an FP64 one (the same bytes);
+// the partial sums take 64 in both, so that the partial blocks of a chunk stay two.
+template <typename T>
+constexpr int PF_ROWS = PF_RPC * 4 / (int)sizeof(T);
+// row pitches: FP32 rows are read in two halves, FP64 rows by four lanes in 64-byte groups
+template <typename T>
+__host__ __device__ inline int pf_pitch(int cols) { return cols + (sizeof(T) == 4 ? 4 : 8); }
 inline int pf_cols(int64_t wb_max) { return (int)((wb_max + 31) / 32 * 32); }
-inline size_t pf_rows_smem(int cols, int nrhs) {
-    return (size_t)PF_RPC * (cols + 4) * sizeof(float) + (size_t)WS * nrhs * sizeof(double);
+template <typename T>
+size_t pf_rows_smem(int cols, int nrhs) {
+    return (size_t)PF_ROWS<T> * pf_pitch<T>(cols) * sizeof(T) + (size_t)WS * nrhs * sizeof(double);
 }
-inline size_t pf_part_smem(int cols, int nrhs) {
-    return (size_t)PF_RPC * (cols + 4) * sizeof(float) + (size_t)PF_RPC * nrhs * sizeof(double) +
+template <typename T>
+size_t pf_part_smem(int cols, int nrhs) {
+    return (size_t)PF_RPC * pf_pitch<T>(cols) * sizeof(T) + (size_t)PF_RPC * nrhs * sizeof(double) +
            (size_t)256 * nrhs * sizeof(double);
 }
 // diagonal kernels: min(nbw, 3) inverse blocks, nbw(nbw−1)/2 panel pieces (NB×NB), the
 // block's vectors; nbw = the step's largest number of NB sub-blocks
 __host__ __device__ inline int pf_nli(int nbw) { return nbw < 3 ? nbw : 3; }
 __host__ __device__ inline int pf_npc(int nbw) { return nbw * (nbw - 1) / 2; }
+// FP64 factor: the inverse blocks and pieces are tiles of one size, at most PD_SLOTS of them
+// resident (all ten of a full block are 320 KB)
+constexpr int PD_SLOTS = 6;
+__host__ __device__ inline int pd_slots(int nbw) { return nbw + pf_npc(nbw) < PD_SLOTS ? nbw + pf_npc(nbw) : PD_SLOTS; }
+inline size_t pd_diag_smem(int nbw, int nrhs) {
+    return (size_t)pd_slots(nbw) * NB * NB * sizeof(double) + (size_t)(WS + NB + 4 * NB) * nrhs * sizeof(double);
+}
 inline size_t pf_diag_smem(int nbw, int nrhs) {
     return (size_t)pf_nli(nbw) * NB * NB * sizeof(double) + (size_t)pf_npc(nbw) * NB * NB * sizeof(float) +
            (size_t)(WS + NB + 4 * NB) * nrhs * sizeof(double);
@@ -536,29 +552,31 @@ __global__ void __launch_bounds__(256) k_wfwd_diag_pf(const double* __restrict__
     }
 }
 
-// Rows below a wide block: X (pivot rows) or V (later rows) −= L[r, J0:J1]·y_B. Two CTAs
-// per PR-row chunk (PF_RPC rows each), two threads per row (half of the columns each),
-// the row tile prefetched before the wait for y_B.
-template <int R>
+// Rows below a wide block: X (pivot rows) or V (later rows) −= L[r, J0:J1]·y_B. PF_ROWS rows
+// per CTA (two or four CTAs per PR-row chunk), two (FP32) or four (FP64) threads per row, the
+// row tile prefetched before the wait for y_B.
+template <typename T, int R>
 __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, double* __restrict__ V,
-                                                     const double* __restrict__ Y, const float* __restrict__ panel,
+                                                     const double* __restrict__ Y, const T* __restrict__ panel,
                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ order,
                                                      int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
                                                      int64_t S, int cols) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
-    const int pitch = cols + 4;
-    float* Lt = reinterpret_cast<float*>(sm);  // [PF_RPC][pitch]
-    double* yB = sm + PF_RPC * pitch / 2;      // [WS][R]
-    const int64_t b = blockIdx.x >> 1;
+    constexpr int RPC = PF_ROWS<T>, SUB = PR / RPC, TPR = PR / RPC, VEC = 16 / (int)sizeof(T);
+    using VT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+    const int pitch = pf_pitch<T>(cols);
+    T* Lt = reinterpret_cast<T*>(sm);                              // [RPC][pitch]
+    double* yB = sm + RPC * pitch * sizeof(T) / sizeof(double);    // [WS][R]
+    const int64_t b = blockIdx.x / SUB;
     const int64_t i = find_slot_warp(pre, nact, b);
     const int64_t chunk = b - pre[i];
     const DFront f = fr[order[fr_off + i]];
     const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
     const int wb = (int)(J1 - J0);
-    const int64_t r0 = J1 + chunk * PR + (blockIdx.x & 1) * PF_RPC;
-    const int nr = (int)max((int64_t)0, min((int64_t)PF_RPC, f.m - r0));
-    if (nr > 0) cp_async_tile<float>(Lt, pitch, panel + f.poff + r0 * f.ldp + J0, f.ldp, nr, wb, nr, cols, PR);
+    const int64_t r0 = J1 + chunk * PR + (blockIdx.x % SUB) * RPC;
+    const int nr = (int)max((int64_t)0, min((int64_t)RPC, f.m - r0));
+    if (nr > 0) cp_async_tile<T>(Lt, pitch, panel + f.poff + r0 * f.ldp + J0, f.ldp, nr, wb, nr, cols, PR);
     cp_async_commit();
     pdl_wait();
     if (nr == 0) return;
@@ -566,28 +584,31 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
     for (int idx = threadIdx.x; idx < cols * R; idx += PR) yB[idx] = idx < wb * R ? ys[idx] : 0.0;
     cp_async_wait<0>();
     __syncthreads();
-    const int rr = threadIdx.x >> 1, h = threadIdx.x & 1;
+    const int rr = threadIdx.x / TPR, h = threadIdx.x % TPR;
     double acc[R][2];
 #pragma unroll
     for (int j = 0; j < R; j++) acc[j][0] = acc[j][1] = 0.0;
-    const int q0 = h * (cols / 8), q1 = q0 + cols / 8;
-    const float4* row = reinterpret_cast<const float4*>(Lt + rr * pitch);
+    // FP32: each thread a half of the row; FP64: every fourth 16-byte group
+    const int nq = cols / (VEC * TPR);
+    const int q0 = sizeof(T) == 4 ? h * nq : h, dq = sizeof(T) == 4 ? 1 : TPR;
+    const VT* row = reinterpret_cast<const VT*>(Lt + rr * pitch);
 #pragma unroll 4
-    for (int q = q0; q < q1; q++) {
-        const float4 l = row[q];
+    for (int u = 0; u < nq; u++) {
+        const int q = q0 + u * dq;
+        const VT lv = row[q];
+        const T* l = reinterpret_cast<const T*>(&lv);
 #pragma unroll
-        for (int j = 0; j < R; j++) {
-            acc[j][0] = fma((double)l.x, yB[(4 * q) * R + j], acc[j][0]);
-            acc[j][1] = fma((double)l.y, yB[(4 * q + 1) * R + j], acc[j][1]);
-            acc[j][0] = fma((double)l.z, yB[(4 * q + 2) * R + j], acc[j][0]);
-            acc[j][1] = fma((double)l.w, yB[(4 * q + 3) * R + j], acc[j][1]);
-        }
+        for (int j = 0; j < R; j++)
+#pragma unroll
+            for (int e = 0; e < VEC; e++)
+                acc[j][e & 1] = fma((double)l[e], yB[(VEC * q + e) * R + j], acc[j][e & 1]);
     }
     double v[R];
 #pragma unroll
     for (int j = 0; j < R; j++) {
         v[j] = acc[j][0] + acc[j][1];
         v[j] += __shfl_xor_sync(0xffffffffu, v[j], 1);
+        if (TPR == 4) v[j] += __shfl_xor_sync(0xffffffffu, v[j], 2);
     }
     if (h == 0 && rr < nr) {
         const int64_t r = r0 + rr;
@@ -600,8 +621,8 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
 // Backward partial sums: out[p][j] = Σ_rr L[r0+rr][J0+p]·y(r0+rr)[j] over the CTA's PF_RPC
 // rows (two CTAs per PR-row chunk, each with its own block of partials); G = 256/cols
 // thread groups take every G-th row, their sums added in group order.
-template <int R>
-__global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__ Y, const float* __restrict__ panel,
+template <typename T, int R>
+__global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__ Y, const T* __restrict__ panel,
                                                       const DFront* __restrict__ fr, const int64_t* __restrict__ order,
                                                       int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
                                                       const int64_t* __restrict__ pre_part,
@@ -609,10 +630,10 @@ __global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__
                                                       double* __restrict__ partial, int cols) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
-    const int pitch = cols + 4;
-    float* Lt = reinterpret_cast<float*>(sm);  // [PF_RPC][pitch]
-    double* yr = sm + PF_RPC * pitch / 2;      // [PF_RPC][R]
-    double* red = yr + PF_RPC * R;             // [256][R]
+    const int pitch = pf_pitch<T>(cols);
+    T* Lt = reinterpret_cast<T*>(sm);                               // [PF_RPC][pitch]
+    double* yr = sm + PF_RPC * pitch * sizeof(T) / sizeof(double);  // [PF_RPC][R]
+    double* red = yr + PF_RPC * R;                                  // [256][R]
     const int64_t b = blockIdx.x >> 1;
     const int64_t i = find_slot_warp(pre, nact, b);
     const int64_t chunk = b - pre[i];
@@ -621,7 +642,7 @@ __global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__
     const int wb = (int)(J1 - J0);
     const int64_t r0 = J1 + chunk * PR + (blockIdx.x & 1) * PF_RPC;
     const int nr = (int)max((int64_t)0, min((int64_t)PF_RPC, f.m - r0));
-    if (nr > 0) cp_async_tile<float>(Lt, pitch, panel + f.poff + r0 * f.ldp + J0, f.ldp, nr, wb, nr, cols, 256);
+    if (nr > 0) cp_async_tile<T>(Lt, pitch, panel + f.poff + r0 * f.ldp + J0, f.ldp, nr, wb, nr, cols, 256);
     cp_async_commit();
     pdl_wait();
     for (int idx = threadIdx.x; idx < PF_RPC * R; idx += 256) {
@@ -676,6 +697,39 @@ __global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__
     }
 }
 
+// z_B = y_B − Σ partial blocks (nc of them from block offset off), zero beyond the block.
+template <int R>
+__device__ __forceinline__ void wbwd_sum_partials(double* z, const double* Y, const double* partial, const DFront& f,
+                                                  int64_t J0, int wb, int nbw, int64_t nc, int64_t off) {
+    const int nout = wb * R;
+    const double* pbase = partial + off * R;
+    for (int o = threadIdx.x; o < nbw * NB * R; o += 256) {
+        double v = 0.0;
+        if (o < nout) {
+            // blocks added in order; loaded 32 at a time so the loads overlap (the
+            // top-of-tree steps have up to two hundred blocks)
+            int64_t c = 0;
+            for (; c + 32 <= nc; c += 32) {
+                double t[32];
+#pragma unroll
+                for (int u = 0; u < 32; u++) t[u] = __ldcg(&pbase[(c + u) * nout + o]);
+#pragma unroll
+                for (int u = 0; u < 32; u++) v += t[u];
+            }
+            for (; c + 8 <= nc; c += 8) {
+                double t[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) t[u] = __ldcg(&pbase[(c + u) * nout + o]);
+#pragma unroll
+                for (int u = 0; u < 8; u++) v += t[u];
+            }
+            for (; c < nc; c++) v += __ldcg(&pbase[c * nout + o]);
+            v = Y[(f.start + J0) * R + o] - v;
+        }
+        z[o] = v;
+    }
+}
+
 // Backward diagonal block: one CTA (256 threads) per active front. z_B = y_B − Σ partials
 // (chunks in order), then for sub-blocks bb from the last: y_bb = L_bb⁻ᵀ·z_bb and
 // z_b2 −= L[bb, b2]ᵀ·y_bb for b2 < bb. Pieces in row-block order (1,0) (2,0) (2,1) (3,0)
@@ -712,36 +766,7 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pf(double* __restrict__ Y, co
         }
     cp_async_commit();
     pdl_wait();
-    {
-        const int nout = wb * R;
-        const int64_t nc = 2 * (pre[i + 1] - pre[i]);  // two partial blocks per chunk
-        const double* pbase = partial + 2 * pre_part[i] * R;
-        for (int o = threadIdx.x; o < nbw * NB * R; o += 256) {
-            double v = 0.0;
-            if (o < nout) {
-                // blocks added in order; loaded 32 at a time so the loads overlap (the
-                // top-of-tree steps have up to two hundred blocks)
-                int64_t c = 0;
-                for (; c + 32 <= nc; c += 32) {
-                    double t[32];
-#pragma unroll
-                    for (int u = 0; u < 32; u++) t[u] = __ldcg(&pbase[(c + u) * nout + o]);
-#pragma unroll
-                    for (int u = 0; u < 32; u++) v += t[u];
-                }
-                for (; c + 8 <= nc; c += 8) {
-                    double t[8];
-#pragma unroll
-                    for (int u = 0; u < 8; u++) t[u] = __ldcg(&pbase[(c + u) * nout + o]);
-#pragma unroll
-                    for (int u = 0; u < 8; u++) v += t[u];
-                }
-                for (; c < nc; c++) v += __ldcg(&pbase[c * nout + o]);
-                v = Y[(f.start + J0) * R + o] - v;
-            }
-            z[o] = v;
-        }
-    }
+    wbwd_sum_partials<R>(z, Y, partial, f, J0, wb, nbw, 2 * (pre[i + 1] - pre[i]), 2 * pre_part[i]);
     cp_async_wait<0>();
     for (int bb = nbw - 1; bb >= 0; bb--) {
         const int jbb = min(NB, wb - bb * NB);
@@ -799,6 +824,203 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pf(double* __restrict__ Y, co
             cp_async_flat(Pr + 3 * NB * NB, lsrc, NB * NB / 2, 256);
             cp_async_commit();
         }
+    }
+}
+
+// The diagonal kernels of an FP64 factor: inverse blocks and pieces are 32 KB tiles, taken in
+// the order of use (forward: inverse b, then the pieces (b2, b) below it; backward: inverse
+// bb, then the pieces (bb, b2) left of it) through PD_SLOTS slots. A block of up to three
+// sub-blocks is prefetched whole before the wait for the vectors; of a full block the first
+// six tiles are, and the last four take the first slots when stage 0 is done with them.
+// A step is bound by the latency of its chain of launches and barriers, not by the factor's
+// bytes: with these kernels (launched as programmatic dependents) and the solve chains instead
+// of the plain step kernels, a refined-solve call with the FP64 factor of the 33³ cube went
+// from 3.72 to 1.79 ms, of the 45³ cube from 6.25 to 3.26 ms, of a 410-equation plate from
+// 0.224 to 0.181 ms.
+template <bool FWD>
+__device__ __forceinline__ void pd_issue(double* sm, int tile, const double* panel, const DFront& f,
+                                         const double* lsrc, int64_t J0, int wb, int nbw) {
+    double* dst = sm + (tile % PD_SLOTS) * NB * NB;
+    int st = 0, i = tile;  // stage st, the i-th tile of it
+    while (i > nbw - 1 - st) {
+        i -= nbw - st;
+        st++;
+    }
+    const int b = FWD ? st : nbw - 1 - st;
+    if (i == 0) {
+        cp_async_flat(dst, lsrc + b * NB * NB, NB * NB / 2, 256);
+    } else {
+        const int rb = FWD ? b + i : b, cb = FWD ? b : i - 1;
+        cp_async_tile<double>(dst, NB, panel + f.poff + (J0 + rb * NB) * f.ldp + J0 + cb * NB, f.ldp,
+                              min(NB, wb - rb * NB), NB, NB, NB, 256);
+    }
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) k_wfwd_diag_pd(const double* __restrict__ X, double* __restrict__ Y,
+                                                      const double* __restrict__ panel, const double* __restrict__ linv,
+                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ order,
+                                                      int64_t fr_off, int64_t S, int nbw_max) {
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) double sm[];
+    double* xB = sm + pd_slots(nbw_max) * NB * NB;  // [WS][R]
+    double* yb = xB + WS * R;                       // [NB][R]
+    const DFront f = fr[order[fr_off + blockIdx.x]];
+    const int64_t J0 = S * WS;
+    const int wb = (int)min((int64_t)WS, f.k - J0), nbw = (wb + NB - 1) / NB;
+    const double* lsrc = linv + (f.blk_off + S * 4) * (int64_t)(NB * NB);
+    const int ntile = nbw + pf_npc(nbw);
+    for (int i = 0; i < min(ntile, PD_SLOTS); i++) pd_issue<true>(sm, i, panel, f, lsrc, J0, wb, nbw);
+    cp_async_commit();
+    pdl_wait();
+    const double* xs = X + (f.start + J0) * R;
+    for (int idx = threadIdx.x; idx < nbw * NB * R; idx += 256) xB[idx] = idx < wb * R ? xs[idx] : 0.0;
+    cp_async_wait<0>();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sel = (lane >> 2) & 7;
+    int t0 = 0;  // the stage's first tile
+    for (int b = 0; b < nbw; b++) {
+        const int jbb = min(NB, wb - b * NB);
+        __syncthreads();
+        {
+            const double* L = sm + (t0 % PD_SLOTS) * NB * NB;
+            double x0[R], x1[R], v[8][R], out[R];
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                x0[j] = xB[(b * NB + lane) * R + j];
+                x1[j] = xB[(b * NB + lane + 32) * R + j];
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const double l0 = L[(8 * warp + i) * NB + lane], l1 = L[(8 * warp + i) * NB + lane + 32];
+#pragma unroll
+                for (int j = 0; j < R; j++) v[i][j] = fma(l0, x0[j], l1 * x1[j]);
+            }
+            warp_sum8<R>(v, out);
+            if ((lane & 3) == 0) {
+                const int p = 8 * warp + sel;
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    yb[p * R + j] = out[j];
+                    if (p < jbb) Y[(f.start + J0 + b * NB + p) * R + j] = out[j];
+                }
+            }
+        }
+        if (b == 1 && nbw == 4) cp_async_wait<0>();  // the last four tiles
+        __syncthreads();
+        if (b + 1 < nbw) {
+            double y0[R], y1[R];
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                y0[j] = yb[lane * R + j];
+                y1[j] = yb[(lane + 32) * R + j];
+            }
+            const int ngrp = (nbw - 1 - b) * NB / 8;
+            for (int g = warp; g < ngrp; g += 8) {
+                const double* Lp = sm + ((t0 + 1 + g / 8) % PD_SLOTS) * NB * NB;
+                double v[8][R], out[R];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const double* row = Lp + (8 * (g & 7) + i) * NB;
+                    const double l0 = row[lane], l1 = row[lane + 32];
+#pragma unroll
+                    for (int j = 0; j < R; j++) v[i][j] = fma(l0, y0[j], l1 * y1[j]);
+                }
+                warp_sum8<R>(v, out);
+                if ((lane & 3) == 0) {
+#pragma unroll
+                    for (int j = 0; j < R; j++) xB[((b + 1) * NB + 8 * g + sel) * R + j] -= out[j];
+                }
+            }
+            if (b == 0 && nbw == 4) {
+                __syncthreads();  // stage 0's four tiles are read
+                for (int i = PD_SLOTS; i < ntile; i++) pd_issue<true>(sm, i, panel, f, lsrc, J0, wb, nbw);
+                cp_async_commit();
+            }
+        }
+        t0 += nbw - b;
+    }
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) k_wbwd_diag_pd(double* __restrict__ Y, const double* __restrict__ panel,
+                                                      const double* __restrict__ linv, const DFront* __restrict__ fr,
+                                                      const int64_t* __restrict__ order, int64_t fr_off,
+                                                      const int64_t* __restrict__ pre,
+                                                      const int64_t* __restrict__ pre_part, int64_t S,
+                                                      const double* __restrict__ partial, int nbw_max) {
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) double sm[];
+    double* z = sm + pd_slots(nbw_max) * NB * NB;  // [WS][R]
+    double* yb = z + WS * R;                       // [NB][R]
+    double* red = yb + NB * R;                     // [4][NB][R]
+    const int64_t i = blockIdx.x;
+    const DFront f = fr[order[fr_off + i]];
+    const int64_t J0 = S * WS;
+    const int wb = (int)min((int64_t)WS, f.k - J0), nbw = (wb + NB - 1) / NB;
+    const double* lsrc = linv + (f.blk_off + S * 4) * (int64_t)(NB * NB);
+    const int ntile = nbw + pf_npc(nbw);
+    for (int t = 0; t < min(ntile, PD_SLOTS); t++) pd_issue<false>(sm, t, panel, f, lsrc, J0, wb, nbw);
+    cp_async_commit();
+    pdl_wait();
+    wbwd_sum_partials<R>(z, Y, partial, f, J0, wb, nbw, 2 * (pre[i + 1] - pre[i]), 2 * pre_part[i]);
+    cp_async_wait<0>();
+    int t0 = 0;  // the stage's first tile
+    for (int bb = nbw - 1; bb >= 0; bb--) {
+        const int jbb = min(NB, wb - bb * NB);
+        __syncthreads();
+        // y_bb = L_bb⁻ᵀ·z_bb: thread (p, g) sums rows q ∈ [16g, 16g+16) of column p
+        const double* L = sm + (t0 % PD_SLOTS) * NB * NB;
+        {
+            const int p = threadIdx.x & 63, g = threadIdx.x >> 6;
+            double acc[R][2];
+#pragma unroll
+            for (int j = 0; j < R; j++) acc[j][0] = acc[j][1] = 0.0;
+#pragma unroll
+            for (int q = 16 * g; q < 16 * g + 16; q += 2) {
+                const double l0 = L[q * NB + p], l1 = L[(q + 1) * NB + p];
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    acc[j][0] = fma(l0, z[(bb * NB + q) * R + j], acc[j][0]);
+                    acc[j][1] = fma(l1, z[(bb * NB + q + 1) * R + j], acc[j][1]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < R; j++) red[(g * NB + p) * R + j] = acc[j][0] + acc[j][1];
+        }
+        __syncthreads();
+        for (int o = threadIdx.x; o < NB * R; o += 256) {
+            const double v = red[o] + red[NB * R + o] + red[2 * NB * R + o] + red[3 * NB * R + o];
+            yb[o] = v;
+            if (o < jbb * R) Y[(f.start + J0 + bb * NB) * R + o] = v;
+        }
+        if (bb == 0) break;
+        if (bb == 2 && nbw == 4) cp_async_wait<0>();  // the last four tiles
+        __syncthreads();
+        // z_b2 −= L[bb, b2]ᵀ·y_bb, one thread per column of row block bb
+        if (threadIdx.x < bb * NB) {
+            const int b2 = threadIdx.x >> 6, c = threadIdx.x & 63;
+            const double* T = sm + ((t0 + 1 + b2) % PD_SLOTS) * NB * NB;
+            double acc[R][4];
+#pragma unroll
+            for (int j = 0; j < R; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0;
+#pragma unroll 4
+            for (int q = 0; q < NB; q += 4) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const double l = T[(q + u) * NB + c];
+#pragma unroll
+                    for (int j = 0; j < R; j++) acc[j][u] = fma(l, yb[(q + u) * R + j], acc[j][u]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < R; j++) z[(b2 * NB + c) * R + j] -= (acc[j][0] + acc[j][1]) + (acc[j][2] + acc[j][3]);
+        }
+        if (bb == 3) {
+            __syncthreads();  // stage 0's four tiles are read
+            for (int t = PD_SLOTS; t < ntile; t++) pd_issue<false>(sm, t, panel, f, lsrc, J0, wb, nbw);
+            cp_async_commit();
+        }
+        t0 += bb + 1;
     }
 }
 
@@ -1385,41 +1607,40 @@ void launch_chained(bool pdl, void (*kern)(KArgs...), unsigned grid, unsigned bl
     launch_pdl(pdl, kern, dim3(grid), dim3(block), smem, st, args...);
 }
 
-// the sweep of an FP32 factor with at most PF_MAXR right-hand sides runs the prefetching
-// kernels, all launched as programmatic dependents; other sweeps launch plainly
-template <typename T>
-bool pf_path(int64_t nrhs) {
-    return std::is_same<T, float>::value && nrhs <= PF_MAXR;
-}
+// a sweep with at most PF_MAXR right-hand sides runs the prefetching kernels
+inline bool pf_path(int64_t nrhs) { return nrhs <= PF_MAXR; }
 // steps with 5 to 32 right-hand sides whose blocks are at least NB wide run the register-
 // tiled kernels; narrower ones (the many small fronts of 2D models) the first kernels, whose
 // CTAs are sized to the rows they have
 inline bool mr_step(int64_t nrhs, int64_t level_maxk, int64_t S) {
     return nrhs > PF_MAXR && std::min<int64_t>(WS, level_maxk - S * WS) >= NB;
 }
-// sweeps whose step kernels prefetch (and so gain from programmatic dependent launches)
-template <typename T>
-bool chained_sweep(int64_t nrhs) {
-    return pf_path<T>(nrhs) || nrhs > PF_MAXR;
-}
-
-template <int R>
-void wfwd_pf(const WStep& w, int nbw_max, int cols, double* X, double* Y, double* V, const float* panel,
+template <typename T, int R>
+void wfwd_pf(const WStep& w, int nbw_max, int cols, double* X, double* Y, double* V, const T* panel,
              const double* linv, const DevPlan& dp, cudaStream_t st) {
-    launch_chained(true, k_wfwd_diag_pf<R>, (unsigned)w.nact, 256, pf_diag_smem(nbw_max, R), st, X, Y, panel, linv,
-                   dp.fronts, dp.level_order, w.fr_off, w.S, nbw_max);
-    launch_chained(true, k_wfwd_rows_pf<R>, (unsigned)(2 * w.n_rows), PR, pf_rows_smem(cols, R), st, X, V, Y, panel, dp.fronts,
-                   dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, w.S, cols);
+    if constexpr (sizeof(T) == 4)
+        launch_chained(true, k_wfwd_diag_pf<R>, (unsigned)w.nact, 256, pf_diag_smem(nbw_max, R), st, X, Y, panel, linv,
+                       dp.fronts, dp.level_order, w.fr_off, w.S, nbw_max);
+    else
+        launch_chained(true, k_wfwd_diag_pd<R>, (unsigned)w.nact, 256, pd_diag_smem(nbw_max, R), st, X, Y, panel, linv,
+                       dp.fronts, dp.level_order, w.fr_off, w.S, nbw_max);
+    launch_chained(true, k_wfwd_rows_pf<T, R>, (unsigned)(PR / PF_ROWS<T> * w.n_rows), PR, pf_rows_smem<T>(cols, R), st,
+                   X, V, Y, panel, dp.fronts, dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, w.S, cols);
 }
-template <int R>
-void wbwd_pf(const WStep& w, int nbw_max, int cols, double* Y, const float* panel, const double* linv,
+template <typename T, int R>
+void wbwd_pf(const WStep& w, int nbw_max, int cols, double* Y, const T* panel, const double* linv,
              const DevPlan& dp, double* partial, cudaStream_t st) {
-    launch_chained(true, k_wbwd_part_pf<R>, (unsigned)(2 * w.n_rows), 256, pf_part_smem(cols, R), st, Y, panel, dp.fronts,
-                   dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off, dp.rows, w.S,
-                   partial, cols);
-    launch_chained(true, k_wbwd_diag_pf<R>, (unsigned)w.nact, 256, pf_diag_smem(nbw_max, R), st, Y, panel, linv, dp.fronts,
-                   dp.level_order, w.fr_off, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off, w.S, partial,
-                   nbw_max);
+    launch_chained(true, k_wbwd_part_pf<T, R>, (unsigned)(2 * w.n_rows), 256, pf_part_smem<T>(cols, R), st, Y, panel,
+                   dp.fronts, dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off,
+                   dp.rows, w.S, partial, cols);
+    if constexpr (sizeof(T) == 4)
+        launch_chained(true, k_wbwd_diag_pf<R>, (unsigned)w.nact, 256, pf_diag_smem(nbw_max, R), st, Y, panel, linv,
+                       dp.fronts, dp.level_order, w.fr_off, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off, w.S,
+                       partial, nbw_max);
+    else
+        launch_chained(true, k_wbwd_diag_pd<R>, (unsigned)w.nact, 256, pd_diag_smem(nbw_max, R), st, Y, panel, linv,
+                       dp.fronts, dp.level_order, w.fr_off, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off, w.S,
+                       partial, nbw_max);
 }
 
 }  // namespace
@@ -1444,22 +1665,21 @@ int64_t Engine::forward_steps(int64_t l, double* X, double* Y, double* V, int nr
     int64_t launches = 0;
     if (chain && P.level_chain[l]) {
         const int64_t i0 = P.chain_fwd_off[l], r0 = P.chain_rows_off[l], nr = P.chain_rows_off[l + 1] - r0;
-        launch_chain_fwd(nrhs, P.chain_fwd_off[l + 1] - i0, X, Y, (const float*)panel_, chain_inv_, dp_.fronts,
+        launch_chain_fwd(nrhs, P.chain_fwd_off[l + 1] - i0, X, Y, panel, chain_inv_, dp_.fronts,
                          dp_.chain_blk, dp_.chain_fwd + 2 * i0, chain, chain + 2 * P.chain_blocks + 2 * l, chain_err_,
                          stream_);
-        launch_chain_rows(nrhs, nr, Y, V, (const float*)panel_, dp_.fronts, dp_.chain_rows + 2 * r0, stream_);
+        launch_chain_rows(nrhs, nr, Y, V, panel, dp_.fronts, dp_.chain_rows + 2 * r0, stream_);
         return nr > 0 ? 2 : 1;
     }
     for (int64_t wi = P.wstep_off[l]; wi < P.wstep_off[l + 1]; wi++) {
         const WStep& w = P.wsteps[wi];
-        if (pf_path<T>(nrhs)) {
-            const float* pf = (const float*)panel_;
+        if (pf_path(nrhs)) {
             const int64_t wb_max = std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS);
             const int nbw_max = (int)((wb_max + NB - 1) / NB), cols = pf_cols(wb_max);
-            if (nrhs == 1) wfwd_pf<1>(w, nbw_max, cols, X, Y, V, pf, linv_, dp_, stream_);
-            else if (nrhs == 2) wfwd_pf<2>(w, nbw_max, cols, X, Y, V, pf, linv_, dp_, stream_);
-            else if (nrhs == 3) wfwd_pf<3>(w, nbw_max, cols, X, Y, V, pf, linv_, dp_, stream_);
-            else wfwd_pf<4>(w, nbw_max, cols, X, Y, V, pf, linv_, dp_, stream_);
+            if (nrhs == 1) wfwd_pf<T, 1>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
+            else if (nrhs == 2) wfwd_pf<T, 2>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
+            else if (nrhs == 3) wfwd_pf<T, 3>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
+            else wfwd_pf<T, 4>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
         } else if (mr_step(nrhs, P.level_maxk[l], w.S)) {
             const int pr = wfwd_piece_rows(P.level_maxk[l], w.S);
             const int cols = pf_cols(std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS));
@@ -1498,22 +1718,21 @@ int64_t Engine::backward_steps(int64_t l, double* Y, double* V, int nrhs, double
         const int64_t i0 = P.chain_bwd_off[l], r0 = P.chain_rows_off[l], c0 = P.chain_cols_off[l];
         const int64_t nr = P.chain_rows_off[l + 1] - r0, nc = P.chain_cols_off[l + 1] - c0;
         launch_chain_cols(nrhs, nr, dp_.chain_rows + 2 * r0, nc, dp_.chain_cols + 2 * c0, Y, V, partial,
-                          (const float*)panel_, dp_.fronts, dp_.rows, stream_);
-        launch_chain_bwd(nrhs, P.chain_bwd_off[l + 1] - i0, Y, (const float*)panel_, chain_inv_, dp_.fronts,
+                          panel, dp_.fronts, dp_.rows, stream_);
+        launch_chain_bwd(nrhs, P.chain_bwd_off[l + 1] - i0, Y, panel, chain_inv_, dp_.fronts,
                          dp_.chain_blk, dp_.chain_bwd + 2 * i0, chain + P.chain_blocks,
                          chain + 2 * P.chain_blocks + 2 * l + 1, chain_err_, stream_);
         return nc > 0 ? 4 : 1;
     }
     for (int64_t wi = P.wstep_off[l + 1] - 1; wi >= P.wstep_off[l]; wi--) {
         const WStep& w = P.wsteps[wi];
-        if (pf_path<T>(nrhs)) {
-            const float* pf = (const float*)panel_;
+        if (pf_path(nrhs)) {
             const int64_t wb_max = std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS);
             const int nbw_max = (int)((wb_max + NB - 1) / NB), cols = pf_cols(wb_max);
-            if (nrhs == 1) wbwd_pf<1>(w, nbw_max, cols, Y, pf, linv_, dp_, partial, stream_);
-            else if (nrhs == 2) wbwd_pf<2>(w, nbw_max, cols, Y, pf, linv_, dp_, partial, stream_);
-            else if (nrhs == 3) wbwd_pf<3>(w, nbw_max, cols, Y, pf, linv_, dp_, partial, stream_);
-            else wbwd_pf<4>(w, nbw_max, cols, Y, pf, linv_, dp_, partial, stream_);
+            if (nrhs == 1) wbwd_pf<T, 1>(w, nbw_max, cols, Y, panel, linv_, dp_, partial, stream_);
+            else if (nrhs == 2) wbwd_pf<T, 2>(w, nbw_max, cols, Y, panel, linv_, dp_, partial, stream_);
+            else if (nrhs == 3) wbwd_pf<T, 3>(w, nbw_max, cols, Y, panel, linv_, dp_, partial, stream_);
+            else wbwd_pf<T, 4>(w, nbw_max, cols, Y, panel, linv_, dp_, partial, stream_);
             launches += 2;
         } else if (mr_step(nrhs, P.level_maxk[l], w.S)) {
             const int64_t wb_max = std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS);
@@ -1585,19 +1804,19 @@ void Engine::solve_impl(double* X, int64_t nrhs_total) {
     }
     int nrhs = (int)nrhs_total;
     RFG_CUDA(cudaMemsetAsync(vupd_, 0, std::max<int64_t>(P.vu_rows * nrhs, 1) * sizeof(double), stream_));
-    int* chain = std::is_same<T, float>::value && chain_on(nrhs) ? counters_ + std::max<int64_t>(P.max_nact, 1) : nullptr;
+    int* chain = chain_on(nrhs) ? counters_ + std::max<int64_t>(P.max_nact, 1) : nullptr;
     if (chain) RFG_CUDA(cudaMemsetAsync(chain, 0, chain_flag_words(P) * sizeof(int), stream_));
     for (int64_t l = 0; l < P.nlevels; l++) {
         for (int r = 0; r < 2; r++) {
             const DXadd& x = P.xadd[2 * l + r];
             if (x.nblk == 0) continue;
-            launch_chained(chained_sweep<T>(nrhs), k_vec_extend_add, (unsigned)x.nblk, 256, 0, stream_, X, vupd_, dp_.fronts,
+            launch_chained(true, k_vec_extend_add, (unsigned)x.nblk, 256, 0, stream_, X, vupd_, dp_.fronts,
                            (const int64_t*)(dp_.xadd_task + 4 * x.task_off), x.ntask, (const int32_t*)dp_.emap, nrhs);
             launches++;
         }
         launches += forward_steps<T>(l, X, ybuf_, vupd_, nrhs, chain);
     }
-    launch_chained(chained_sweep<T>(nrhs), k_divide_d, (unsigned)grid_for(P.n * nrhs), 256, 0, stream_, ybuf_, (const double*)d_, P.n, nrhs);
+    launch_chained(true, k_divide_d, (unsigned)grid_for(P.n * nrhs), 256, 0, stream_, ybuf_, (const double*)d_, P.n, nrhs);
     launches++;
     for (int64_t l = P.nlevels - 1; l >= 0; l--)
         launches += backward_steps<T>(l, ybuf_, vupd_, nrhs, partial_, counters_, chain);
@@ -1634,16 +1853,24 @@ static void solve_set_attributes_current_device() {
     RFG_CUDA(cudaFuncSetAttribute(k_wfwd_rows<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(WS * MAXR * sizeof(double))));
     RFG_CUDA(cudaFuncSetAttribute(k_wbwd<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wbwd_smem<double>(MAXR)));
-    auto pf_attrs = [](auto diag_f, auto rows_f, auto part_f, auto diag_b, int r) {
-        RFG_CUDA(cudaFuncSetAttribute(diag_f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf_diag_smem(4, r)));
-        RFG_CUDA(cudaFuncSetAttribute(rows_f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf_rows_smem(WS, r)));
-        RFG_CUDA(cudaFuncSetAttribute(part_f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf_part_smem(WS, r)));
-        RFG_CUDA(cudaFuncSetAttribute(diag_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pf_diag_smem(4, r)));
+    auto attr = [](auto kern, size_t bytes) {
+        RFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     };
-    pf_attrs(k_wfwd_diag_pf<1>, k_wfwd_rows_pf<1>, k_wbwd_part_pf<1>, k_wbwd_diag_pf<1>, 1);
-    pf_attrs(k_wfwd_diag_pf<2>, k_wfwd_rows_pf<2>, k_wbwd_part_pf<2>, k_wbwd_diag_pf<2>, 2);
-    pf_attrs(k_wfwd_diag_pf<3>, k_wfwd_rows_pf<3>, k_wbwd_part_pf<3>, k_wbwd_diag_pf<3>, 3);
-    pf_attrs(k_wfwd_diag_pf<4>, k_wfwd_rows_pf<4>, k_wbwd_part_pf<4>, k_wbwd_diag_pf<4>, 4);
+    auto pf_attrs = [&](auto r) {
+        constexpr int R = decltype(r)::value;
+        attr(k_wfwd_diag_pf<R>, pf_diag_smem(4, R));
+        attr(k_wbwd_diag_pf<R>, pf_diag_smem(4, R));
+        attr(k_wfwd_diag_pd<R>, pd_diag_smem(4, R));
+        attr(k_wbwd_diag_pd<R>, pd_diag_smem(4, R));
+        attr(k_wfwd_rows_pf<float, R>, pf_rows_smem<float>(WS, R));
+        attr(k_wfwd_rows_pf<double, R>, pf_rows_smem<double>(WS, R));
+        attr(k_wbwd_part_pf<float, R>, pf_part_smem<float>(WS, R));
+        attr(k_wbwd_part_pf<double, R>, pf_part_smem<double>(WS, R));
+    };
+    pf_attrs(std::integral_constant<int, 1>());
+    pf_attrs(std::integral_constant<int, 2>());
+    pf_attrs(std::integral_constant<int, 3>());
+    pf_attrs(std::integral_constant<int, 4>());
     RFG_CUDA(cudaFuncSetAttribute(k_wfwd_rows_mr<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)mr_rows_smem(WS, sizeof(float))));
     RFG_CUDA(cudaFuncSetAttribute(k_wfwd_rows_mr<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1679,10 +1906,10 @@ void Engine::solve_device(double* X, int64_t nrhs, bool allow_graph) {
             }
         }
         vupd_ = (double*)dalloc(std::max<int64_t>(plan_.vu_rows * w, 1) * sizeof(double));
-        partial_ = (double*)dalloc(std::max<int64_t>(partial_rows() * w, 1) * sizeof(double));
+        partial_ = (double*)dalloc(std::max<int64_t>(partial_rows(has_chain()) * w, 1) * sizeof(double));
         ybuf_ = (double*)dalloc(std::max<int64_t>(plan_.n * w, 1) * sizeof(double));
-        counters_ = (int*)dalloc(ticket_words() * sizeof(int));
-        RFG_CUDA(cudaMemsetAsync(counters_, 0, ticket_words() * sizeof(int), stream_));
+        counters_ = (int*)dalloc(ticket_words(has_chain()) * sizeof(int));
+        RFG_CUDA(cudaMemsetAsync(counters_, 0, ticket_words(has_chain()) * sizeof(int), stream_));
         ws_nrhs_ = w;
     }
     if (chain_on(nrhs)) ensure_chain_inverse();
@@ -1738,23 +1965,27 @@ int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }
 }  // namespace
 
 bool Engine::chain_on(int64_t nrhs) const {
-    return prec_ == PREC_MIXED && chain_inv_ != nullptr && nrhs >= 1 && nrhs <= PF_MAXR;
+    return chain_inv_ != nullptr && nrhs >= 1 && nrhs <= PF_MAXR;
 }
 
-int64_t Engine::partial_rows() const {
-    return std::max<int64_t>(2 * plan_.max_wpart, chain_inv_ ? plan_.chain_colpart : 0);
+int64_t Engine::partial_rows(bool chain) const {
+    return std::max<int64_t>(2 * plan_.max_wpart, chain ? plan_.chain_colpart : 0);
 }
 
-int64_t Engine::ticket_words() const {
-    return std::max<int64_t>(plan_.max_nact, 1) + (chain_inv_ ? chain_flag_words(plan_) : 0);
+int64_t Engine::ticket_words(bool chain) const {
+    return std::max<int64_t>(plan_.max_nact, 1) + (chain ? chain_flag_words(plan_) : 0);
 }
 
 // The chain blocks' inverses for the current factor: formed by the first sweep after each
 // numeric phase (on the engine's stream, before that sweep's launches or graph).
 void Engine::ensure_chain_inverse() {
     if (chain_inv_at_ == factor_calls_) return;
-    launch_chain_inverse(chain_inv_, (const float*)panel_, linv_, dp_.fronts, dp_.chain_blk, dp_.chain_bfront,
-                         plan_.chain_blocks, stream_);
+    if (prec_ == PREC_FP64)
+        launch_chain_inverse(chain_inv_, (const double*)panel_, linv_, dp_.fronts, dp_.chain_blk, dp_.chain_bfront,
+                             plan_.chain_blocks, stream_);
+    else
+        launch_chain_inverse(chain_inv_, (const float*)panel_, linv_, dp_.fronts, dp_.chain_blk, dp_.chain_bfront,
+                             plan_.chain_blocks, stream_);
     solve_launches++;
     chain_inv_at_ = factor_calls_;
 }
@@ -1770,13 +2001,13 @@ void Engine::chain_check() {
     }
 }
 
-int64_t Engine::sweep_workspace_bytes(int64_t nrhs) const {
+int64_t Engine::sweep_workspace_bytes(int64_t nrhs, bool chain) const {
     const Plan& P = plan_;
     return round256(std::max<int64_t>(P.n * nrhs, 1) * 8) + round256(std::max<int64_t>(P.vu_rows * nrhs, 1) * 8) +
-           round256(std::max<int64_t>(partial_rows() * nrhs, 1) * 8) + round256(ticket_words() * 4);
+           round256(std::max<int64_t>(partial_rows(chain) * nrhs, 1) * 8) + round256(ticket_words(chain) * 4);
 }
 
-Engine::SweepWorkspace Engine::carve_sweep_workspace(void* base, int64_t nrhs) const {
+Engine::SweepWorkspace Engine::carve_sweep_workspace(void* base, int64_t nrhs, bool chain) const {
     const Plan& P = plan_;
     char* p = (char*)base;
     SweepWorkspace ws;
@@ -1785,8 +2016,9 @@ Engine::SweepWorkspace Engine::carve_sweep_workspace(void* base, int64_t nrhs) c
     ws.v = (double*)p;
     p += round256(std::max<int64_t>(P.vu_rows * nrhs, 1) * 8);
     ws.partial = (double*)p;  // two blocks of partials per chunk on the prefetching path
-    p += round256(std::max<int64_t>(partial_rows() * nrhs, 1) * 8);
+    p += round256(std::max<int64_t>(partial_rows(chain) * nrhs, 1) * 8);
     ws.tickets = (int*)p;
+    ws.chain = chain;
     return ws;
 }
 
@@ -1796,18 +2028,18 @@ void Engine::solve_sweep_impl(double* X, int64_t nrhs_total, const SweepWorkspac
     const Plan& P = plan_;
     int nrhs = (int)nrhs_total;
     RFG_CUDA(cudaMemsetAsync(ws.v, 0, std::max<int64_t>(P.vu_rows * nrhs, 1) * sizeof(double), stream_));
-    RFG_CUDA(cudaMemsetAsync(ws.tickets, 0, ticket_words() * sizeof(int), stream_));
-    int* chain = std::is_same<T, float>::value && chain_on(nrhs) ? ws.tickets + std::max<int64_t>(P.max_nact, 1) : nullptr;
+    RFG_CUDA(cudaMemsetAsync(ws.tickets, 0, ticket_words(ws.chain) * sizeof(int), stream_));
+    int* chain = ws.chain && chain_on(nrhs) ? ws.tickets + std::max<int64_t>(P.max_nact, 1) : nullptr;
     for (int64_t l = 0; l < P.nlevels; l++) {
         for (int r = 0; r < 2; r++) {
             const DXadd& x = P.xadd[2 * l + r];
             if (x.nblk == 0) continue;
-            launch_chained(chained_sweep<T>(nrhs), k_vec_extend_add, (unsigned)x.nblk, 256, 0, stream_, X, ws.v, dp_.fronts,
+            launch_chained(true, k_vec_extend_add, (unsigned)x.nblk, 256, 0, stream_, X, ws.v, dp_.fronts,
                            (const int64_t*)(dp_.xadd_task + 4 * x.task_off), x.ntask, (const int32_t*)dp_.emap, nrhs);
         }
         forward_steps<T>(l, X, ws.y, ws.v, nrhs, chain);
     }
-    launch_chained(chained_sweep<T>(nrhs), k_divide_d, (unsigned)grid_for(P.n * nrhs), 256, 0, stream_, ws.y, (const double*)d_, P.n, nrhs);
+    launch_chained(true, k_divide_d, (unsigned)grid_for(P.n * nrhs), 256, 0, stream_, ws.y, (const double*)d_, P.n, nrhs);
     for (int64_t l = P.nlevels - 1; l >= 0; l--) backward_steps<T>(l, ws.y, ws.v, nrhs, ws.partial, ws.tickets, chain);
     RFG_CUDA(cudaMemcpyAsync(X, ws.y, P.n * nrhs * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
     RFG_CUDA(cudaGetLastError());
@@ -1817,7 +2049,7 @@ void Engine::solve_sweep_on(double* X, int64_t nrhs, const SweepWorkspace& ws) {
     if (nrhs <= 0 || plan_.n == 0) return;
     if (nrhs > MAXR) throw CudaError("solve_sweep_on: at most 32 right-hand sides per sweep");
     solve_set_attributes();
-    if (chain_on(nrhs)) ensure_chain_inverse();
+    if (ws.chain && chain_on(nrhs)) ensure_chain_inverse();
     if (prec_ == PREC_FP64)
         solve_sweep_impl<double>(X, nrhs, ws);
     else

@@ -93,6 +93,14 @@ __device__ __forceinline__ double recip_newton(double p) {
     return fma(r, e, r);
 }
 
+// D = A·B + D on the FP64 tensor-core path for one 8×8×4 block (mma.sync m8n8k4 f64):
+// lane l holds A[l / 4][l % 4], B[l % 4][l / 4] and D[l / 4][2·(l % 4) + {0, 1}].
+__device__ __forceinline__ void dmma_884(double& c0, double& c1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(a), "d"(b));
+}
+
 // Programmatic dependent launch (PDL): a kernel launched with the programmatic
 // stream-serialization attribute may start while its predecessor in the stream still
 // runs. pdl_wait() blocks until the predecessor grid has completed and its memory is
