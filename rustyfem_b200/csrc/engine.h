@@ -278,9 +278,11 @@ class Engine {
     std::vector<std::pair<std::pair<double*, int64_t>, int64_t>> solve_seen_;  // (X, nrhs) -> sweeps run
     // matrix for refinement (full CSR over the internal numbering)
     int64_t* a_rowptr_ = nullptr;
-    int64_t* a_col_ = nullptr;
-    int64_t* a_src_ = nullptr;
+    int32_t* a_col_ = nullptr;
+    uint32_t* a_src_ = nullptr;  // source value of each entry (a_direct_), or its segment
     double* a_val_ = nullptr;
+    bool a_direct_ = false;
+    int64_t a_val_at_ = -1;      // the numeric phase (factor_calls_) a_val_ and the norms belong to
     int64_t a_nnz_ = 0;
     bool matrix_built_ = false;  // a_* hold the FP64 matrix of the refinement
     double anorm_ = 0.0;

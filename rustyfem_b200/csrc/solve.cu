@@ -1422,52 +1422,59 @@ __global__ void k_place_rows(const int32_t* __restrict__ key, const uint64_t* __
     }
 }
 
-__global__ void k_split_entries(const uint64_t* __restrict__ val, int64_t cnt, int64_t* __restrict__ col,
-                                int64_t* __restrict__ seg) {
+// Columns and sources of the sorted entries in 32 bits. With direct_src the source is the index
+// of the entry's only source value, otherwise its segment.
+__global__ void k_split_entries(const uint64_t* __restrict__ val, int64_t cnt, int32_t* __restrict__ col,
+                                uint32_t* __restrict__ from, const int64_t* __restrict__ direct_src) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < cnt; e += (int64_t)gridDim.x * blockDim.x) {
-        col[e] = (int64_t)(val[e] >> 32);
-        seg[e] = (int64_t)(val[e] & 0xffffffffull);
+        const int64_t seg = (int64_t)(val[e] & 0xffffffffull);
+        col[e] = (int32_t)(val[e] >> 32);
+        from[e] = (uint32_t)(direct_src ? direct_src[seg] : seg);
     }
 }
 
-// value of each CSR entry: the sum of its segment's source values
-__global__ void k_gather_values(double* __restrict__ val, const double* __restrict__ src, const int64_t* __restrict__ seg,
-                                const int64_t* __restrict__ seg_ptr, const int64_t* __restrict__ seg_src, int64_t nnz) {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x) {
-        int64_t i = seg[e];
-        double s;
-        if (seg_ptr) {
-            s = 0.0;
-            for (int64_t j = seg_ptr[i]; j < seg_ptr[i + 1]; j++) s += src[seg_src[j]];
-        } else {
-            s = src[seg_src[i]];
-        }
-        val[e] = s;
-    }
-}
-
-// one warp per row; also accumulates |a| row sums when rowsum != null
-__global__ void k_spmv(const int64_t* __restrict__ rp, const int64_t* __restrict__ col, const double* __restrict__ val,
-                       const double* __restrict__ X, double* __restrict__ Y, int64_t n, int nrhs,
-                       double* __restrict__ rowsum) {
-    int lane = threadIdx.x & 31;
+// Values of the CSR entries of a factorization (the sum of each entry's source values) and the
+// rows' sums of |a|, one warp per row. Runs once per numeric phase.
+__global__ void k_gather_rows(const int64_t* __restrict__ rp, const uint32_t* __restrict__ from,
+                              const double* __restrict__ src, const int64_t* __restrict__ seg_ptr,
+                              const int64_t* __restrict__ seg_src, bool direct, int64_t n, double* __restrict__ val,
+                              double* __restrict__ rowsum) {
+    const int lane = threadIdx.x & 31;
     for (int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; row < n;
          row += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    int64_t e0 = rp[row], e1 = rp[row + 1];
-    for (int j = 0; j < nrhs; j++) {
-        double acc = 0.0;
-        for (int64_t e = e0 + lane; e < e1; e += 32) acc = fma(val[e], X[col[e] * nrhs + j], acc);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) Y[row * nrhs + j] = acc;
-    }
-    if (rowsum) {
+        const int64_t e1 = rp[row + 1];
         double a = 0.0;
-        for (int64_t e = e0 + lane; e < e1; e += 32) a += fabs(val[e]);
+        for (int64_t e = rp[row] + lane; e < e1; e += 32) {
+            double s = 0.0;
+            if (direct) {
+                s = src[from[e]];
+            } else if (seg_ptr) {
+                const int64_t i = from[e];
+                for (int64_t j = seg_ptr[i]; j < seg_ptr[i + 1]; j++) s += src[seg_src[j]];
+            } else {
+                s = src[seg_src[from[e]]];
+            }
+            val[e] = s;
+            a += fabs(s);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         if (lane == 0) rowsum[row] = a;
     }
+}
+
+// Y = A·X for one right-hand side, one warp per row: bound by the entries (12 bytes each)
+__global__ void k_spmv(const int64_t* __restrict__ rp, const int32_t* __restrict__ col, const double* __restrict__ val,
+                       const double* __restrict__ X, double* __restrict__ Y, int64_t n) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; row < n;
+         row += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+        const int64_t e1 = rp[row + 1];
+        double acc = 0.0;
+        for (int64_t e = rp[row] + lane; e < e1; e += 32) acc = fma(val[e], X[col[e]], acc);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) Y[row] = acc;
     }
 }
 
@@ -1475,7 +1482,7 @@ __global__ void k_spmv(const int64_t* __restrict__ rp, const int64_t* __restrict
 // (L a power of two, the smallest >= min(nrhs, 32)) take one row each and lane j of a
 // group right-hand side j (chunks of L for more), so an X row is read as L consecutive
 // doubles and the group's lanes read each matrix entry at the same address (one access).
-__global__ void k_spmm(const int64_t* __restrict__ rp, const int64_t* __restrict__ col,
+__global__ void k_spmm(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                        const double* __restrict__ val, const double* __restrict__ X, double* __restrict__ Y,
                        int64_t n, int nrhs, int L) {
     const int sub = (int)(threadIdx.x & (L - 1));
@@ -1487,17 +1494,19 @@ __global__ void k_spmm(const int64_t* __restrict__ rp, const int64_t* __restrict
             double a0 = 0.0, a1 = 0.0;
             int64_t e = e0;
             for (; e + 1 < e1; e += 2) {
-                a0 = fma(val[e], xj[col[e] * nrhs], a0);
-                a1 = fma(val[e + 1], xj[col[e + 1] * nrhs], a1);
+                a0 = fma(val[e], xj[(int64_t)col[e] * nrhs], a0);
+                a1 = fma(val[e + 1], xj[(int64_t)col[e + 1] * nrhs], a1);
             }
-            if (e < e1) a0 = fma(val[e], xj[col[e] * nrhs], a0);
+            if (e < e1) a0 = fma(val[e], xj[(int64_t)col[e] * nrhs], a0);
             Y[row * nrhs + j] = a0 + a1;
         }
     }
 }
 
-// R = B − AX (in R, AX given), per-RHS reductions: red[j·5 + {0..4}] =
-// {max|r|, max|x|, max|b|, Σr², Σb²} accumulated with atomics on nonnegative doubles
+// maxima of nonnegative doubles by their bits (a NaN stays the largest)
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+    return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
 __device__ __forceinline__ void atomic_max_nonneg(double* a, double v) {
     atomicMax((unsigned long long*)a, (unsigned long long)__double_as_longlong(v));
 }
@@ -1505,37 +1514,58 @@ __device__ __forceinline__ void atomic_max_nonneg(double* a, double v) {
 // Per-system reductions of the refinement residual. The internal rows are split into
 // segments (one per independent model of a batched factorization, else one), each
 // reduced by blocks of SEG_ROWS rows: R = B − AX, and red[(g·nrhs + j)·5 + {0..4}] =
-// {max|r|, max|x|, max|b|, Σr², Σb²} of segment g, right-hand side j.
-constexpr int64_t SEG_ROWS = 2048;
+// {max|r|, max|x|, max|b|, Σr², Σb²} of segment g, right-hand side j. The block takes whole
+// rows of right-hand sides at a time, so a thread keeps one right-hand side and its five
+// values in registers; the threads of a right-hand side are then combined in halves.
+// (Shared-memory atomics per entry, and 2048 rows per block, took 93 µs on the 33³ cube
+// with one right-hand side and 338 µs on the hex20 20³ cube with 32; now 6 and 40 µs.)
+constexpr int64_t SEG_ROWS = 512;
 
-__global__ void k_residual_seg(double* __restrict__ R, const double* __restrict__ AX, const double* __restrict__ B,
-                               const double* __restrict__ X, const int64_t* __restrict__ seg_off,
-                               const int64_t* __restrict__ blk_pre, int64_t nseg, int nrhs, double* __restrict__ red) {
-    __shared__ double s[5][MAXR];
-    for (int i = threadIdx.x; i < 5 * MAXR; i += blockDim.x) s[i / MAXR][i % MAXR] = 0.0;
-    __syncthreads();
-    int64_t g = find_slot2(blk_pre, nseg, blockIdx.x);
-    int64_t r0 = seg_off[g] + (blockIdx.x - blk_pre[g]) * SEG_ROWS;
-    int64_t r1 = min(seg_off[g + 1], r0 + SEG_ROWS);
-    for (int64_t e = r0 * nrhs + threadIdx.x; e < r1 * nrhs; e += blockDim.x) {
-        int j = (int)(e % nrhs);
-        double r = B[e] - AX[e];
-        R[e] = r;
-        atomic_max_nonneg(&s[0][j], fabs(r));
-        atomic_max_nonneg(&s[1][j], fabs(X[e]));
-        atomic_max_nonneg(&s[2][j], fabs(B[e]));
-        atomicAdd(&s[3][j], r * r);
-        atomicAdd(&s[4][j], B[e] * B[e]);
+__global__ void __launch_bounds__(256) k_residual_seg(double* __restrict__ R, const double* __restrict__ AX,
+                                                      const double* __restrict__ B, const double* __restrict__ X,
+                                                      const int64_t* __restrict__ seg_off,
+                                                      const int64_t* __restrict__ blk_pre, int64_t nseg, int nrhs,
+                                                      double* __restrict__ red) {
+    __shared__ double s[5][256];
+    const int64_t g = find_slot2(blk_pre, nseg, blockIdx.x);
+    const int64_t r0 = seg_off[g] + (blockIdx.x - blk_pre[g]) * SEG_ROWS;
+    const int64_t r1 = min(seg_off[g + 1], r0 + SEG_ROWS);
+    const int G = 256 / nrhs, T = G * nrhs, t = threadIdx.x;  // G rows at a time
+    double mr = 0.0, mx = 0.0, mb = 0.0, sr = 0.0, sb = 0.0;
+    if (t < T) {
+#pragma unroll 4
+        for (int64_t e = r0 * nrhs + t; e < r1 * nrhs; e += T) {
+            const double b = B[e], x = X[e], r = b - AX[e];
+            R[e] = r;
+            mr = max_nonneg(mr, fabs(r));
+            mx = max_nonneg(mx, fabs(x));
+            mb = max_nonneg(mb, fabs(b));
+            sr = fma(r, r, sr);
+            sb = fma(b, b, sb);
+        }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 5 * nrhs; i += blockDim.x) {
-        int w = i / nrhs, j = i % nrhs;
-        double v = s[w][j];
-        double* dst = &red[(g * nrhs + j) * 5 + w];
-        if (w < 3)
-            atomic_max_nonneg(dst, v);
-        else
-            atomicAdd(dst, v);
+    s[0][t] = mr;
+    s[1][t] = mx;
+    s[2][t] = mb;
+    s[3][t] = sr;
+    s[4][t] = sb;
+    const int row = t / nrhs;
+    for (int h = 128; h > 0; h >>= 1) {
+        __syncthreads();
+        if (row < h && row + h < G) {
+            const int o = t + h * nrhs;
+#pragma unroll
+            for (int w = 0; w < 3; w++) s[w][t] = max_nonneg(s[w][t], s[w][o]);
+            s[3][t] += s[3][o];
+            s[4][t] += s[4][o];
+        }
+    }
+    if (t < nrhs) {
+        double* dst = &red[(g * nrhs + t) * 5];
+#pragma unroll
+        for (int w = 0; w < 3; w++) atomic_max_nonneg(dst + w, s[w][t]);
+        atomicAdd(dst + 3, s[3][t]);
+        atomicAdd(dst + 4, s[4][t]);
     }
 }
 
@@ -2089,6 +2119,7 @@ void Engine::set_segments(const std::vector<int64_t>& off) {
         if (ref_r_) dev_free(ref_r_, stream_);
         if (ref_dx_) dev_free(ref_dx_, stream_);
         ref_r_ = ref_dx_ = nullptr;
+        a_val_at_ = -1;
     }
     seg_off_ = off;
     seg_blocks_ = pre[nseg];
@@ -2143,7 +2174,11 @@ void Engine::build_matrix() {
     RFG_CUDA(cudaMemcpyAsync(&nnz, rp + n, sizeof(int64_t), cudaMemcpyDeviceToHost, stream_));
     RFG_CUDA(cudaStreamSynchronize(stream_));
     a_nnz_ = nnz;
-    if (nnz > 0) k_split_entries<<<grid_for(nnz), 256, 0, stream_>>>(v1, nnz, a_col_, a_src_);
+    // one source per entry and 32-bit indices: the values are gathered without the segments
+    a_direct_ = !dp_.seg_ptr && nsrc_ <= ((int64_t)1 << 32);
+    if (nnz > 0)
+        k_split_entries<<<grid_for(nnz), 256, 0, stream_>>>(v1, nnz, a_col_, a_src_,
+                                                            a_direct_ ? (const int64_t*)dp_.seg_src : nullptr);
     if (!in_arena) dev_free(base, stream_);
     RFG_CUDA(cudaStreamSynchronize(stream_));
     matrix_built_ = true;
@@ -2152,7 +2187,7 @@ void Engine::build_matrix() {
 void Engine::matvec(const double* X, double* Y, int64_t nrhs) {
     const int64_t n = plan_.n;
     if (nrhs <= 1) {
-        k_spmv<<<grid_for(n * 32, 256), 256, 0, stream_>>>(a_rowptr_, a_col_, a_val_, X, Y, n, (int)nrhs, nullptr);
+        k_spmv<<<grid_for(n * 32, 256), 256, 0, stream_>>>(a_rowptr_, a_col_, a_val_, X, Y, n);
         return;
     }
     int L = 1;
@@ -2177,8 +2212,6 @@ SolveStats Engine::solve_refined(double* X, const double* B, int64_t nrhs, doubl
     // the first refined solve of an engine runs its sweeps without capturing graphs
     const bool graphs = refined_calls_++ > 0;
     int64_t l0 = solve_launches;
-    // the matrix values of the current factorization and ‖A‖∞
-    k_gather_values<<<grid_for(a_nnz_), 256, 0, stream_>>>(a_val_, src_, a_src_, dp_.seg_ptr, dp_.seg_src, a_nnz_);
     if (seg_off_.empty()) set_segments({0, n});
     const int64_t nseg = (int64_t)seg_off_.size() - 1;
     // red: 5 values per (segment, right-hand side), then anorm per segment, then ‖A‖∞
@@ -2192,15 +2225,22 @@ SolveStats Engine::solve_refined(double* X, const double* B, int64_t nrhs, doubl
         ref_dx_ = (double*)dev_alloc(n * MAXR * sizeof(double), stream_);
         ref_red_ = (double*)dev_alloc(nred * sizeof(double), stream_);
         ref_nrhs_ = MAXR;
+        a_val_at_ = -1;
     }
     double* seg_anorm = ref_red_ + 5 * nseg * MAXR;
     double* eta_out = seg_anorm + nseg + 1;
-    RFG_CUDA(cudaMemsetAsync(ref_red_, 0, nred * sizeof(double), stream_));
-    k_spmv<<<grid_for(n * 32, 256), 256, 0, stream_>>>(a_rowptr_, a_col_, a_val_, nullptr, nullptr, n, 0, ref_dx_);
-    k_max_reduce<<<grid_for(n), 256, 0, stream_>>>(ref_dx_, n, seg_anorm + nseg);
-    if (seg_blocks_ > 0)
-        k_seg_max<<<(unsigned)seg_blocks_, 256, 0, stream_>>>(ref_dx_, d_seg_off_, d_seg_blk_, nseg, seg_anorm);
-    RFG_CUDA(cudaMemcpyAsync(&anorm_, seg_anorm + nseg, sizeof(double), cudaMemcpyDeviceToHost, stream_));
+    if (a_val_at_ != factor_calls_) {
+        // the matrix values of the current factorization and its norms: formed by the first
+        // refined solve after each numeric phase
+        RFG_CUDA(cudaMemsetAsync(seg_anorm, 0, (nseg + 3) * sizeof(double), stream_));
+        k_gather_rows<<<grid_for(n * 32, 256), 256, 0, stream_>>>(a_rowptr_, a_src_, src_, dp_.seg_ptr, dp_.seg_src,
+                                                                 a_direct_, n, a_val_, ref_dx_);
+        k_max_reduce<<<grid_for(n), 256, 0, stream_>>>(ref_dx_, n, seg_anorm + nseg);
+        if (seg_blocks_ > 0)
+            k_seg_max<<<(unsigned)seg_blocks_, 256, 0, stream_>>>(ref_dx_, d_seg_off_, d_seg_blk_, nseg, seg_anorm);
+        RFG_CUDA(cudaMemcpyAsync(&anorm_, seg_anorm + nseg, sizeof(double), cudaMemcpyDeviceToHost, stream_));
+        a_val_at_ = factor_calls_;
+    }
     if (X != B) RFG_CUDA(cudaMemcpyAsync(X, B, n * nrhs * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
     lap("values, norms");
     solve_device(X, nrhs, graphs);
