@@ -7,12 +7,13 @@
 // work items are WS-wide diagonal blocks (and, forward, WS-row pieces of the later rows),
 // each done by a cluster of four CTAs:
 //   forward, block B of a front, CTA s owning the rows B·WS + 64s ... + 63:
-//       x_s = X[rows] − Σ_{J < B} L[rows, J]·y_J   (tile J as soon as block J's flag is up)
+//       x_s = X[rows] + (children's V) − Σ_{J < B} L[rows, J]·y_J   (tile J as soon as block
+//             J's flag is up)
 //       x_B gathered from the cluster's CTAs (distributed shared memory),
 //       y[rows] = inv(L_BB)[rows, :]·x_B, then the block's flag is raised;
-//   forward, later rows: V[rows] −= Σ_J L[rows, J]·y_J over all blocks J;
+//   forward, later rows: V[rows] = (children's V) − Σ_J L[rows, J]·y_J over all blocks J;
 //   backward, block B, CTA s owning the columns B·WS + 64s ... + 63:
-//       z_s = Y[cols] − Σ_{r later} L[r, cols]·y_r − Σ_{J > B} L[J, cols]ᵀ·y_J,
+//       z_s = Y[cols]/D − Σ_{r later} L[r, cols]·y_r − Σ_{J > B} L[J, cols]ᵀ·y_J,
 //       y[cols] = inv(L_BB)[:, cols]ᵀ·z_B.
 // The tiles of a block stream through a ring of four cp.async stages while the CTA waits
 // for the flags; the dependency chain from block to block is one flag wait, the last
@@ -24,6 +25,11 @@
 // resident clusters. Waits are bounded: a wait that gives up sets *err, the CTA goes on
 // with the values it finds, every later wait of the launch returns at once, and the host
 // reports the error (Engine::chain_check).
+//
+// One to four right-hand sides run on the CUDA cores. Five and more run the same chains in
+// groups of eight right-hand sides (the _mm kernels): the eight columns are the N of the FP64
+// tensor-core product, a group is a chain of its own with its own flags, and the later rows take
+// all groups in one CTA so that L21 is read once.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -184,9 +190,12 @@ __device__ __forceinline__ void fwd_tiles(double (&acc)[R], T* ring, double* yb,
 template <typename T, int R>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     k_chain_fwd(const double* __restrict__ X, double* __restrict__ Y, const T* __restrict__ panel,
+                const double* __restrict__ V, const int32_t* __restrict__ imap,
                 const double* __restrict__ cinv, const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
                 const int64_t* __restrict__ items, int64_t nitems, int* __restrict__ flags, int* __restrict__ counter,
                 int* __restrict__ err) {
+    pdl_launch_dependents();
+    pdl_wait();
     cg::cluster_group cluster = cg::this_cluster();
     const int s = (int)cluster.block_rank();
     extern __shared__ __align__(16) double sm[];
@@ -220,7 +229,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
         quad_sum<R>(acc);
         if (q == 0) {
 #pragma unroll
-            for (int r = 0; r < R; r++) xo[i * R + r] = i < nr ? X[(f.start + r0 + i) * R + r] - acc[r] : 0.0;
+            for (int r = 0; r < R; r++)
+                xo[i * R + r] =
+                    i < nr ? kids_add(X[(f.start + r0 + i) * R + r], V, imap, f, r0 + i, R, r) - acc[r] : 0.0;
         }
         cluster.sync();
         for (int e = tid; e < WS * R; e += CT) {
@@ -247,12 +258,14 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     }
 }
 
-// The later rows of a chain level's fronts after the level's chain: V[rows] −= L21·y over
-// all the front's pivots, one CTA per CHAIN_PIECE rows.
+// The later rows of a chain level's fronts after the level's chain: V[rows] = (children's V) −
+// L21·y over all the front's pivots, one CTA per CHAIN_PIECE rows.
 template <typename T, int R>
 __global__ void __launch_bounds__(CT) k_chain_rows(const double* __restrict__ Y, double* __restrict__ V,
-                                                   const T* __restrict__ panel, const DFront* __restrict__ fr,
-                                                   const int64_t* __restrict__ items) {
+                                                   const int32_t* __restrict__ imap, const T* __restrict__ panel,
+                                                   const DFront* __restrict__ fr, const int64_t* __restrict__ items) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) double sm[];
     T* ring = reinterpret_cast<T*>(sm);                              // [4][CQ][FQP]
     double* yb = reinterpret_cast<double*>(ring + 4 * CQ * FQP<T>);  // [WS][R]
@@ -275,7 +288,7 @@ __global__ void __launch_bounds__(CT) k_chain_rows(const double* __restrict__ Y,
     if (q == 0 && i < nr) {
         double* vt = V + (f.vuoff + c * CQ + i) * R;
 #pragma unroll
-        for (int r = 0; r < R; r++) vt[r] -= acc[r];
+        for (int r = 0; r < R; r++) vt[r] = kids_add(0.0, V, imap, f, r0 + i, R, r) - acc[r];
     }
 }
 
@@ -332,11 +345,29 @@ __device__ __forceinline__ void col_sum(double (&acc)[R], double* red) {
     }
 }
 
+// z of pivot column col of a front before the chain's own products: the forward result over D
+// minus the later rows' part (the row groups of k_chain_cols in order; cb < 0: no later rows).
+__device__ __forceinline__ double chain_z(const double* Y, const double* d, const double* part, int64_t cb,
+                                          const DFront& f, int64_t col, int nrhs, int r) {
+    double z = Y[(f.start + col) * nrhs + r] / d[f.start + col];
+    if (cb >= 0) {
+        const double* p = part + ((cb + col / CQ) * CHAIN_GROUPS * CQ + col % CQ) * (int64_t)nrhs + r;
+        double sum = 0.0;
+#pragma unroll
+        for (int g = 0; g < CHAIN_GROUPS; g++) sum += p[(int64_t)g * CQ * nrhs];
+        z -= sum;
+    }
+    return z;
+}
+
 template <typename T, int R>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     k_chain_bwd(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ cinv,
+                const double* __restrict__ d, const double* __restrict__ part, const int64_t* __restrict__ colbase,
                 const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk, const int64_t* __restrict__ items,
                 int64_t nitems, int* __restrict__ flags, int* __restrict__ counter, int* __restrict__ err) {
+    pdl_launch_dependents();
+    pdl_wait();
     cg::cluster_group cluster = cg::this_cluster();
     const int s = (int)cluster.block_rank();
     extern __shared__ __align__(16) double sm[];
@@ -385,7 +416,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
         col_sum<R>(acc, red);
         if (tid < CQ) {
 #pragma unroll
-            for (int r = 0; r < R; r++) zo[c * R + r] = c < nc ? Y[(f.start + col0 + c) * R + r] - acc[r] : 0.0;
+            for (int r = 0; r < R; r++)
+                zo[c * R + r] = c < nc ? chain_z(Y, d, part, colbase[t], f, col0 + c, R, r) - acc[r] : 0.0;
         }
         cluster.sync();
         double* zf = yp;
@@ -418,9 +450,11 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
 __global__ void __launch_bounds__(CT) k_chain_gather(const double* __restrict__ Y, double* __restrict__ V,
                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ rows,
                                                      const int64_t* __restrict__ items, int nrhs) {
+    pdl_launch_dependents();
     const int64_t t = items[2 * blockIdx.x], c = items[2 * blockIdx.x + 1];
     const DFront f = fr[t];
     const int64_t i0 = c * CQ;
+    pdl_wait();
     const int nr = (int)min((int64_t)CQ, f.u - i0);
     for (int e = threadIdx.x; e < nr * nrhs; e += CT) {
         const int ii = e / nrhs, r = e - ii * nrhs;
@@ -431,12 +465,14 @@ __global__ void __launch_bounds__(CT) k_chain_gather(const double* __restrict__ 
 // The later rows' part of a chain level's backward, before its chain: the partial sums
 // L21ᵀ·y of the front's later rows (their y in V, from k_chain_gather), one CTA per
 // CHAIN_PIECE pivot columns and group of rows (blockIdx.y of CHAIN_GROUPS), into
-// part[(item · CHAIN_GROUPS + group) · CHAIN_PIECE + column]; k_chain_colsum subtracts them
-// from z in group order.
+// part[(item · CHAIN_GROUPS + group) · CHAIN_PIECE + column]; the chain subtracts them in
+// group order (chain_z).
 template <typename T, int R>
 __global__ void __launch_bounds__(CT) k_chain_cols(double* __restrict__ part, const double* __restrict__ V,
                                                    const T* __restrict__ panel, const DFront* __restrict__ fr,
                                                    const int64_t* __restrict__ items) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) double sm[];
     constexpr int RC = BRC<T>;
     T* ring = reinterpret_cast<T*>(sm);                           // [4][RC][BTP]
@@ -477,20 +513,360 @@ __global__ void __launch_bounds__(CT) k_chain_cols(double* __restrict__ part, co
     }
 }
 
-// z[cols] −= the row groups' partial sums of k_chain_cols, added in group order.
-__global__ void __launch_bounds__(CT) k_chain_colsum(double* __restrict__ Y, const double* __restrict__ part,
-                                                     const DFront* __restrict__ fr, const int64_t* __restrict__ items,
-                                                     int nrhs) {
+// ---------------------------------------------------------------------------
+// Five to 32 right-hand sides: groups of eight (MG) on the FP64 tensor-core path (m8n8k4).
+// Warp w owns rows (forward) or columns (backward) 8w ... of the CTA's 64. The vectors of a
+// group are rows of eight doubles with the halves swapped on every second pair of rows (vsw),
+// so that a fragment load (four rows, eight columns) meets every bank once per half-warp.
+// Before, the wide steps ran one by one with the products on the CUDA cores and eight
+// right-hand sides per CTA of the diagonal kernels: 47.3 ms per refined solve of the hex20 20³
+// cube with 32 right-hand sides (four sweeps), now 11.7 ms.
+// ---------------------------------------------------------------------------
+constexpr int MG = 8;
+template <typename T>
+constexpr int MFP = FQC<T> + 4;                    // pitch of a forward piece: conflict-free row fragments
+template <typename T>
+constexpr int MBP = CQ + (sizeof(T) == 4 ? 8 : 4); // pitch of a backward piece: conflict-free column fragments
+constexpr int MLP = CQ + 4;                        // pitch of the backward inverse columns
+template <typename T>
+constexpr size_t mm_fwd_smem = (size_t)CQ * FLP * 8 + (size_t)4 * CQ * MFP<T> * sizeof(T) + (size_t)WS * MG * 8;
+template <typename T>
+constexpr size_t mm_bwd_smem = (size_t)WS * MLP * 8 + (size_t)4 * BRC<T> * MBP<T> * sizeof(T) + (size_t)WS * MG * 8;
+static_assert(mm_fwd_smem<float> <= 232000 && mm_fwd_smem<double> <= 232000 && mm_bwd_smem<float> <= 232000 &&
+                  mm_bwd_smem<double> <= 232000,
+              "shared memory of a CTA");
+
+__device__ __forceinline__ int vsw(int k, int n) { return k * MG + (n ^ ((k & 2) << 1)); }
+
+template <typename T>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
+    k_chain_fwd_mm(const double* __restrict__ X, double* __restrict__ Y, const T* __restrict__ panel,
+                   const double* __restrict__ V, const int32_t* __restrict__ imap, const double* __restrict__ cinv,
+                   const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
+                   const int64_t* __restrict__ items, int64_t nitems, int nrhs, int64_t nblocks,
+                   int* __restrict__ flags0, int* __restrict__ counter, int* __restrict__ err) {
+    pdl_launch_dependents();
+    pdl_wait();
+    cg::cluster_group cluster = cg::this_cluster();
+    const int s = (int)cluster.block_rank(), ngrp = (nrhs + MG - 1) / MG;
+    extern __shared__ __align__(16) double sm[];
+    constexpr int QC = FQC<T>, QP = MFP<T>, PB = FPB<T>;
+    double* Lv = sm;                                             // [CQ][FLP]: inverse rows 64s ..
+    T* ring = reinterpret_cast<T*>(sm + CQ * FLP);               // [4][CQ][QP]
+    double* yb = reinterpret_cast<double*>(ring + 4 * CQ * QP);  // [WS][MG]: y_J, then x_B
+    double* xo = reinterpret_cast<double*>(ring);                // [CQ][MG]: this CTA's rows of x_B (ring idle)
+    __shared__ int64_t s_item;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    for (;;) {
+        const int64_t it = grab(cluster, &s_item, counter);
+        if (it >= nitems * ngrp) break;
+        const int64_t item = it / ngrp;
+        const int jg = (int)(it - item * ngrp), j0 = jg * MG, rc = min(MG, nrhs - j0);
+        const int64_t t = items[2 * item], b = items[2 * item + 1];
+        const DFront f = fr[t];
+        int* flags = flags0 + jg * nblocks + chain_blk[t];
+        const int64_t r0 = b * WS + s * CQ;
+        const int nr = (int)max((int64_t)0, min((int64_t)CQ, f.k - r0));
+        const int cmax = CQ * (s + 1);  // inverse row 64s + i ends at the diagonal
+        cp_async_tile<double>(Lv, FLP, cinv + ((chain_blk[t] + b) * WS + s * CQ) * (int64_t)WS, WS, CQ, cmax, CQ, cmax,
+                              CT);
+        cp_async_commit();
+        const T* prow = panel + f.poff + r0 * f.ldp;
+        const int nq = PB * (int)b;
+        auto issue = [&](int Q) {
+            if (nr > 0) cp_async_tile<T>(ring + (Q & 3) * CQ * QP, QP, prow + (int64_t)Q * QC, f.ldp, nr, QC, CQ, QC, CT);
+            cp_async_commit();
+        };
+        double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+        for (int Q = 0; Q < min(3, nq); Q++) issue(Q);
+        for (int Q = 0; Q < nq; Q++) {
+            if (Q % PB == 0) {
+                const int64_t j = Q / PB;
+                if (tid == 0) chain_wait(&flags[j], CL, err);
+                __syncthreads();
+                const double* ys = Y + (f.start + j * WS) * nrhs + j0;
+                for (int e = tid; e < WS * MG; e += CT) {
+                    const int k = e / MG, n = e % MG;
+                    yb[vsw(k, n)] = n < rc ? __ldcg(ys + (int64_t)k * nrhs + n) : 0.0;
+                }
+            }
+            cp_wait_upto(min(2, nq - 1 - Q));
+            __syncthreads();  // piece Q and y_j visible; every thread is done with piece Q − 1
+            if (Q + 3 < nq) issue(Q + 3);
+            if (nr > 8 * w) {
+                const T* Lt = ring + (Q & 3) * CQ * QP + (8 * w + g) * QP + q;
+                const int kb = (Q % PB) * QC + q;
+#pragma unroll
+                for (int k = 0; k < QC; k += 8) {
+                    dmma_884(a0[0], a0[1], (double)Lt[k], yb[vsw(kb + k, g)]);
+                    dmma_884(a1[0], a1[1], (double)Lt[k + 4], yb[vsw(kb + k + 4, g)]);
+                }
+            }
+        }
+        __syncthreads();  // the ring is idle: it takes x_s
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int i = 8 * w + g, n = 2 * q + e;
+            double x = 0.0;
+            if (i < nr && n < rc)
+                x = kids_add(X[(f.start + r0 + i) * nrhs + j0 + n], V, imap, f, r0 + i, nrhs, j0 + n) - (a0[e] + a1[e]);
+            xo[i * MG + n] = x;
+        }
+        cluster.sync();
+        for (int e = tid; e < WS * MG; e += CT) {
+            const int k = e / MG;
+            yb[vsw(k, e % MG)] = cluster.map_shared_rank(xo, k / CQ)[e - (k / CQ) * CQ * MG];
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        {
+            double acc[2][2] = {};
+            const double* Lr = Lv + (8 * w + g) * FLP + q;
+            const int kmax = s * CQ + 8 * w + 8;  // the inverse rows 8w .. 8w+7 end at their diagonal
+            for (int k = 0; k < kmax; k += 8) {
+                dmma_884(acc[0][0], acc[0][1], Lr[k], yb[vsw(k + q, g)]);
+                dmma_884(acc[1][0], acc[1][1], Lr[k + 4], yb[vsw(k + 4 + q, g)]);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int i = 8 * w + g, n = 2 * q + e;
+                if (i < nr && n < rc) Y[(f.start + r0 + i) * nrhs + j0 + n] = acc[0][e] + acc[1][e];
+            }
+        }
+        chain_signal(&flags[b]);
+        cluster.sync();  // the cluster's x_B pieces may be overwritten after this
+    }
+}
+
+template <typename T>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
+    k_chain_bwd_mm(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ cinv,
+                   const double* __restrict__ d, const double* __restrict__ part, const int64_t* __restrict__ colbase,
+                   const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
+                   const int64_t* __restrict__ items, int64_t nitems, int nrhs, int64_t nblocks,
+                   int* __restrict__ flags0, int* __restrict__ counter, int* __restrict__ err) {
+    pdl_launch_dependents();
+    pdl_wait();
+    cg::cluster_group cluster = cg::this_cluster();
+    const int s = (int)cluster.block_rank(), ngrp = (nrhs + MG - 1) / MG;
+    extern __shared__ __align__(16) double sm[];
+    constexpr int RC = BRC<T>, BP = MBP<T>, PB = BPB<T>;
+    double* Lc = sm;                                             // [WS][MLP]: rows 64s .. of inverse columns 64s ..
+    T* ring = reinterpret_cast<T*>(sm + WS * MLP);               // [4][RC][BP]
+    double* yp = reinterpret_cast<double*>(ring + 4 * RC * BP);  // [WS][MG]: y of a later block; then z_B
+    double* zo = reinterpret_cast<double*>(ring);                // [CQ][MG]: this CTA's columns of z_B (ring idle)
+    __shared__ int64_t s_item;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    for (;;) {
+        const int64_t it = grab(cluster, &s_item, counter);
+        if (it >= nitems * ngrp) break;
+        const int64_t item = it / ngrp;
+        const int jg = (int)(it - item * ngrp), j0 = jg * MG, rc = min(MG, nrhs - j0);
+        const int64_t t = items[2 * item], b = items[2 * item + 1];
+        const DFront f = fr[t];
+        int* flags = flags0 + jg * nblocks + chain_blk[t];
+        const int64_t col0 = b * WS + s * CQ;
+        const int nc = (int)max((int64_t)0, min((int64_t)CQ, f.k - col0));
+        const int64_t nb = (f.k + WS - 1) / WS;
+        const int ninv = WS - s * CQ;  // inverse column 64s + c starts at its diagonal row
+        cp_async_tile<double>(Lc, MLP, cinv + ((chain_blk[t] + b) * WS + s * CQ) * (int64_t)WS + s * CQ, WS, ninv, CQ,
+                              ninv, CQ, CT);
+        cp_async_commit();
+        // the chunks of blocks nb − 1, ..., b + 1, PB per block
+        const T* pcol = panel + f.poff + col0;
+        const int nh = PB * (int)(nb - 1 - b);
+        auto issue = [&](int h) {
+            const int64_t ra = (nb - 1 - h / PB) * WS + (h % PB) * RC;
+            const int nrr = (int)max((int64_t)0, min((int64_t)RC, f.k - ra));
+            if (nc > 0)
+                cp_async_tile<T>(ring + (h & 3) * RC * BP, BP, nrr > 0 ? pcol + ra * f.ldp : pcol, f.ldp, nrr, nc, RC, CQ,
+                                 CT);
+            cp_async_commit();
+        };
+        double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+        for (int h = 0; h < min(3, nh); h++) issue(h);
+        for (int h = 0; h < nh; h++) {
+            if (h % PB == 0) {
+                const int64_t bb = nb - 1 - h / PB;
+                if (tid == 0) chain_wait(&flags[bb], CL, err);
+                __syncthreads();
+                const int wbb = (int)min((int64_t)WS, f.k - bb * WS);
+                const double* src = Y + (f.start + bb * WS) * nrhs + j0;
+                for (int e = tid; e < WS * MG; e += CT) {
+                    const int k = e / MG, n = e % MG;
+                    yp[vsw(k, n)] = (k < wbb && n < rc) ? __ldcg(src + (int64_t)k * nrhs + n) : 0.0;
+                }
+            }
+            cp_wait_upto(min(2, nh - 1 - h));
+            __syncthreads();  // chunk h visible; every thread is done with chunk h − 1
+            if (h + 3 < nh) issue(h + 3);
+            if (nc > 8 * w) {
+                const T* Lt = ring + (h & 3) * RC * BP + q * BP + 8 * w + g;
+                const int kb = (h % PB) * RC + q;
+#pragma unroll
+                for (int k = 0; k < RC; k += 8) {
+                    dmma_884(a0[0], a0[1], (double)Lt[k * BP], yp[vsw(kb + k, g)]);
+                    dmma_884(a1[0], a1[1], (double)Lt[(k + 4) * BP], yp[vsw(kb + k + 4, g)]);
+                }
+            }
+        }
+        __syncthreads();  // the ring is idle: it takes z_s
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int c = 8 * w + g, n = 2 * q + e;
+            zo[c * MG + n] =
+                c < nc && n < rc ? chain_z(Y, d, part, colbase[t], f, col0 + c, nrhs, j0 + n) - (a0[e] + a1[e]) : 0.0;
+        }
+        cluster.sync();
+        for (int e = tid; e < WS * MG; e += CT) {
+            const int k = e / MG;
+            yp[vsw(k, e % MG)] = cluster.map_shared_rank(zo, k / CQ)[e - (k / CQ) * CQ * MG];
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        {
+            double acc[2][2] = {};
+            const double* Lq = Lc + q * MLP + 8 * w + g;
+            // inverse columns 64s + 8w ...: rows from 8w (relative to 64s) to the block's end
+            for (int k = 8 * w; k < ninv; k += 8) {
+                dmma_884(acc[0][0], acc[0][1], Lq[k * MLP], yp[vsw(s * CQ + k + q, g)]);
+                dmma_884(acc[1][0], acc[1][1], Lq[(k + 4) * MLP], yp[vsw(s * CQ + k + 4 + q, g)]);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int c = 8 * w + g, n = 2 * q + e;
+                if (c < nc && n < rc) Y[(f.start + col0 + c) * nrhs + j0 + n] = acc[0][e] + acc[1][e];
+            }
+        }
+        chain_signal(&flags[b]);
+        cluster.sync();  // the cluster's z_B pieces may be overwritten after this
+    }
+}
+
+// Later rows, NT groups in one CTA: pieces of L and of the vectors (pitch 8·NT + 4 doubles)
+// stream together through a four-slot ring.
+template <int NT>
+constexpr int MVP = MG * NT + 4;
+template <typename T, int NT>
+constexpr size_t mm_rows_smem = (size_t)4 * CQ * MFP<T> * sizeof(T) + (size_t)4 * FQC<T> * MVP<NT> * 8;
+template <typename T, int NT>
+constexpr size_t mm_cols_smem = (size_t)4 * BRC<T> * MBP<T> * sizeof(T) + (size_t)4 * BRC<T> * MVP<NT> * 8;
+
+// cp.async of n rows of nrhs contiguous values into rows of pitch MVP, zero beyond the rows and
+// beyond nrhs; src rows are contiguous
+template <int NT>
+__device__ __forceinline__ void vec_piece(double* dst, const double* src, int n, int nrhs, int rows) {
+    for (int e = threadIdx.x; e < rows * MG * NT; e += CT) {
+        const int k = e / (MG * NT), c = e % (MG * NT);
+        double* o = dst + k * MVP<NT> + c;
+        if (k < n && c < nrhs)
+            cp_async8(o, src + (int64_t)k * nrhs + c);
+        else
+            *o = 0.0;
+    }
+}
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(CT) k_chain_rows_mm(const double* __restrict__ Y, double* __restrict__ V,
+                                                      const int32_t* __restrict__ imap, const T* __restrict__ panel,
+                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ items,
+                                                      int nrhs) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) double sm[];
+    constexpr int QC = FQC<T>, QP = MFP<T>, VP = MVP<NT>;
+    double* yr = sm;                                         // [4][QC][VP]
+    T* ring = reinterpret_cast<T*>(sm + 4 * QC * VP);        // [4][CQ][QP]
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    const int64_t t = items[2 * blockIdx.x], c = items[2 * blockIdx.x + 1];
+    const DFront f = fr[t];
+    const int64_t r0 = f.k + c * CQ;
+    const int nr = (int)min((int64_t)CQ, f.m - r0);
+    const int nq = (int)((f.k + QC - 1) / QC);
+    const T* prow = panel + f.poff + r0 * f.ldp;
+    auto issue = [&](int Q) {
+        const int64_t c0 = (int64_t)Q * QC;
+        const int ncol = (int)min((int64_t)QC, f.k - c0);
+        cp_async_tile<T>(ring + (Q & 3) * CQ * QP, QP, prow + c0, f.ldp, nr, ncol, CQ, QC, CT);
+        vec_piece<NT>(yr + (Q & 3) * QC * VP, Y + (f.start + c0) * nrhs, ncol, nrhs, QC);
+        cp_async_commit();
+    };
+    double acc[NT][2] = {};
+    for (int Q = 0; Q < min(3, nq); Q++) issue(Q);
+    for (int Q = 0; Q < nq; Q++) {
+        cp_wait_upto(min(2, nq - 1 - Q));
+        __syncthreads();
+        if (Q + 3 < nq) issue(Q + 3);
+        const T* Lt = ring + (Q & 3) * CQ * QP + (8 * w + g) * QP + q;
+        const double* yq = yr + (Q & 3) * QC * VP + q * VP + g;
+#pragma unroll 4
+        for (int k = 0; k < QC; k += 4) {
+            const double a = (double)Lt[k];
+#pragma unroll
+            for (int n = 0; n < NT; n++) dmma_884(acc[n][0], acc[n][1], a, yq[k * VP + n * MG]);
+        }
+    }
+    const int i = 8 * w + g;
+    if (i < nr) {
+        double* vt = V + (f.vuoff + c * CQ + i) * nrhs;
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int j = n * MG + 2 * q + e;
+                if (j < nrhs) vt[j] = kids_add(0.0, V, imap, f, r0 + i, nrhs, j) - acc[n][e];
+            }
+    }
+}
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(CT) k_chain_cols_mm(double* __restrict__ part, const double* __restrict__ V,
+                                                      const T* __restrict__ panel, const DFront* __restrict__ fr,
+                                                      const int64_t* __restrict__ items, int nrhs) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) double sm[];
+    constexpr int RC = BRC<T>, BP = MBP<T>, VP = MVP<NT>;
+    double* yr = sm;                                   // [4][RC][VP]
+    T* ring = reinterpret_cast<T*>(sm + 4 * RC * VP);  // [4][RC][BP]
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
     const int64_t t = items[2 * blockIdx.x], cc = items[2 * blockIdx.x + 1];
     const DFront f = fr[t];
     const int64_t col0 = cc * CQ;
     const int nc = (int)min((int64_t)CQ, f.k - col0);
-    for (int e = threadIdx.x; e < nc * nrhs; e += CT) {
-        const int c = e / nrhs, r = e - c * nrhs;
-        double sum = 0.0;
-        for (int g = 0; g < CHAIN_GROUPS; g++) sum += part[(((int64_t)blockIdx.x * CHAIN_GROUPS + g) * CQ + c) * nrhs + r];
-        Y[(f.start + col0 + c) * nrhs + r] -= sum;
+    const int nchunk = (int)((f.u + RC - 1) / RC), grp = blockIdx.y;
+    const int h0 = nchunk * grp / CHAIN_GROUPS, nh = nchunk * (grp + 1) / CHAIN_GROUPS - h0;
+    auto issue = [&](int h) {
+        const int64_t ra = (int64_t)(h0 + h) * RC;
+        const int nrr = (int)min((int64_t)RC, f.u - ra);
+        cp_async_tile<T>(ring + (h & 3) * RC * BP, BP, panel + f.poff + (f.k + ra) * f.ldp + col0, f.ldp, nrr, nc, RC, CQ,
+                         CT);
+        vec_piece<NT>(yr + (h & 3) * RC * VP, V + (f.vuoff + ra) * nrhs, nrr, nrhs, RC);
+        cp_async_commit();
+    };
+    double acc[NT][2] = {};
+    for (int h = 0; h < min(3, nh); h++) issue(h);
+    for (int h = 0; h < nh; h++) {
+        cp_wait_upto(min(2, nh - 1 - h));
+        __syncthreads();
+        if (h + 3 < nh) issue(h + 3);
+        const T* Lt = ring + (h & 3) * RC * BP + q * BP + 8 * w + g;
+        const double* yq = yr + (h & 3) * RC * VP + q * VP + g;
+#pragma unroll 4
+        for (int k = 0; k < RC; k += 4) {
+            const double a = (double)Lt[k * BP];
+#pragma unroll
+            for (int n = 0; n < NT; n++) dmma_884(acc[n][0], acc[n][1], a, yq[k * VP + n * MG]);
+        }
     }
+    double* out = part + (((int64_t)blockIdx.x * CHAIN_GROUPS + grp) * CQ + 8 * w + g) * nrhs;
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int j = n * MG + 2 * q + e;
+            if (j < nrhs) out[j] = acc[n][e];
+        }
 }
 
 // The inverse of a chain block's unit-lower diagonal block, by block columns of NB:
@@ -589,7 +965,7 @@ __global__ void __launch_bounds__(256) k_chain_inverse(double* __restrict__ cinv
 // by right-hand sides 1 .. 4)
 struct ChainDev {
     bool done = false;
-    int fwd[2][5] = {}, bwd[2][5] = {};  // [0] FP32, [1] FP64 factor
+    int fwd[2][5] = {}, bwd[2][5] = {};  // [0] FP32, [1] FP64 factor; by right-hand sides 1 .. 4, [0] the groups
 };
 template <typename T>
 constexpr int chain_kind = sizeof(T) == 8 ? 1 : 0;
@@ -616,20 +992,28 @@ int fit_clusters(K kern, size_t smem) {
 constexpr size_t rows_smem(int R) { return (size_t)4 * CQ * FQP<float> * sizeof(float) + (size_t)WS * R * 8; }
 constexpr size_t cols_smem(int R) { return (size_t)4 * BRC<float> * BTP * sizeof(float) + (size_t)8 * CQ * R * 8; }
 
+template <typename K>
+void set_smem(K kern, size_t bytes) {
+    RFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
 template <typename T, int R>
 void set_chain_attrs(ChainDev& d) {
     d.fwd[chain_kind<T>][R] = fit_clusters(k_chain_fwd<T, R>, fwd_smem(R));
     d.bwd[chain_kind<T>][R] = fit_clusters(k_chain_bwd<T, R>, bwd_smem(R));
-    RFG_CUDA(cudaFuncSetAttribute(k_chain_rows<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(R)));
-    RFG_CUDA(cudaFuncSetAttribute(k_chain_cols<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols_smem(R)));
+    set_smem(k_chain_rows<T, R>, rows_smem(R));
+    set_smem(k_chain_cols<T, R>, cols_smem(R));
+    set_smem(k_chain_rows_mm<T, R>, mm_rows_smem<T, R>);
+    set_smem(k_chain_cols_mm<T, R>, mm_cols_smem<T, R>);
 }
 template <typename T>
 void set_chain_attrs_all(ChainDev& d) {
-    RFG_CUDA(cudaFuncSetAttribute(k_chain_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INV_SMEM));
+    set_smem(k_chain_inverse<T>, INV_SMEM);
     set_chain_attrs<T, 1>(d);
     set_chain_attrs<T, 2>(d);
     set_chain_attrs<T, 3>(d);
     set_chain_attrs<T, 4>(d);
+    d.fwd[chain_kind<T>][0] = fit_clusters(k_chain_fwd_mm<T>, mm_fwd_smem<T>);
+    d.bwd[chain_kind<T>][0] = fit_clusters(k_chain_bwd_mm<T>, mm_bwd_smem<T>);
 }
 
 const ChainDev& chain_dev() {
@@ -654,7 +1038,7 @@ unsigned grid_for_items(int fit, int64_t nitems) {
 }
 
 void check_nrhs(int nrhs) {
-    if (nrhs < 1 || nrhs > 4) throw CudaError("solve chain: 1 to 4 right-hand sides");
+    if (nrhs < 1 || nrhs > 4 * MG) throw CudaError("solve chain: 1 to 32 right-hand sides");
 }
 
 }  // namespace
@@ -669,83 +1053,109 @@ void launch_chain_inverse(double* cinv, const T* panel, const double* linv, cons
     RFG_CUDA(cudaGetLastError());
 }
 
-// one of four instantiations by the number of right-hand sides
-#define RFG_CHAIN_BY_R(nrhs, CALL) \
-    do {                           \
-        check_nrhs(nrhs);          \
-        if ((nrhs) == 1) {         \
-            constexpr int R = 1;   \
-            CALL;                  \
-        } else if ((nrhs) == 2) {  \
-            constexpr int R = 2;   \
-            CALL;                  \
-        } else if ((nrhs) == 3) {  \
-            constexpr int R = 3;   \
-            CALL;                  \
-        } else {                   \
-            constexpr int R = 4;   \
-            CALL;                  \
-        }                          \
+// one of four instantiations (by the number of right-hand sides or of groups)
+#define RFG_CHAIN_BY_R(num, CALL) \
+    do {                          \
+        if ((num) == 1) {         \
+            constexpr int R = 1;  \
+            CALL;                 \
+        } else if ((num) == 2) {  \
+            constexpr int R = 2;  \
+            CALL;                 \
+        } else if ((num) == 3) {  \
+            constexpr int R = 3;  \
+            CALL;                 \
+        } else {                  \
+            constexpr int R = 4;  \
+            CALL;                 \
+        }                         \
     } while (0)
 
 template <typename T>
-void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, const T* panel, const double* cinv,
-                      const DFront* fronts, const int64_t* chain_blk, const int64_t* items, int* flags, int* counter,
-                      int* err, cudaStream_t st) {
+void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, const double* V, const T* panel,
+                      const ChainArgs& c, const int64_t* items, int* flags, int* counter, cudaStream_t st) {
     if (nitems <= 0) return;
+    check_nrhs(nrhs);
     const ChainDev& d = chain_dev();
-    RFG_CHAIN_BY_R(nrhs, (k_chain_fwd<T, R><<<grid_for_items(d.fwd[chain_kind<T>][R], nitems), CT, fwd_smem(R), st>>>(
-                              X, Y, panel, cinv, fronts, chain_blk, items, nitems, flags, counter, err)));
-    RFG_CUDA(cudaGetLastError());
+    if (nrhs > 4) {
+        const int64_t n = nitems * ((nrhs + MG - 1) / MG);
+        launch_pdl(true, k_chain_fwd_mm<T>, dim3(grid_for_items(d.fwd[chain_kind<T>][0], n)), dim3(CT), mm_fwd_smem<T>,
+                   st, X, Y, panel, V, c.imap, c.cinv, c.fronts, c.blk, items, nitems, nrhs, c.nblocks, flags, counter,
+                   c.err);
+        return;
+    }
+    RFG_CHAIN_BY_R(nrhs, launch_pdl(true, k_chain_fwd<T, R>, dim3(grid_for_items(d.fwd[chain_kind<T>][R], nitems)),
+                                    dim3(CT), fwd_smem(R), st, X, Y, panel, V, c.imap, c.cinv, c.fronts, c.blk, items,
+                                    nitems, flags, counter, c.err));
 }
 
 template <typename T>
-void launch_chain_rows(int nrhs, int64_t nitems, const double* Y, double* V, const T* panel, const DFront* fronts,
+void launch_chain_rows(int nrhs, int64_t nitems, const double* Y, double* V, const T* panel, const ChainArgs& c,
                        const int64_t* items, cudaStream_t st) {
     if (nitems <= 0) return;
+    check_nrhs(nrhs);
     chain_dev();
-    RFG_CHAIN_BY_R(nrhs, (k_chain_rows<T, R><<<(unsigned)nitems, CT, rows_smem(R), st>>>(Y, V, panel, fronts, items)));
-    RFG_CUDA(cudaGetLastError());
+    if (nrhs > 4) {
+        RFG_CHAIN_BY_R((nrhs + MG - 1) / MG,
+                       launch_pdl(true, k_chain_rows_mm<T, R>, dim3((unsigned)nitems), dim3(CT), mm_rows_smem<T, R>, st,
+                                  Y, V, c.imap, panel, c.fronts, items, nrhs));
+        return;
+    }
+    RFG_CHAIN_BY_R(nrhs, launch_pdl(true, k_chain_rows<T, R>, dim3((unsigned)nitems), dim3(CT), rows_smem(R), st, Y, V,
+                                    c.imap, panel, c.fronts, items));
 }
 
 template <typename T>
 void launch_chain_cols(int nrhs, int64_t ngather, const int64_t* gather_items, int64_t nitems, const int64_t* items,
-                       double* Y, double* V, double* part, const T* panel, const DFront* fronts,
-                       const int64_t* rows, cudaStream_t st) {
+                       const double* Y, double* V, double* part, const T* panel, const ChainArgs& c, cudaStream_t st) {
     if (nitems <= 0) return;
-    chain_dev();
     check_nrhs(nrhs);
-    if (ngather > 0) k_chain_gather<<<(unsigned)ngather, CT, 0, st>>>(Y, V, fronts, rows, gather_items, nrhs);
-    RFG_CHAIN_BY_R(nrhs, (k_chain_cols<T, R><<<dim3((unsigned)nitems, CHAIN_GROUPS), CT, cols_smem(R), st>>>(
-                              part, V, panel, fronts, items)));
-    k_chain_colsum<<<(unsigned)nitems, CT, 0, st>>>(Y, part, fronts, items, nrhs);
-    RFG_CUDA(cudaGetLastError());
+    chain_dev();
+    if (ngather > 0)
+        launch_pdl(true, k_chain_gather, dim3((unsigned)ngather), dim3(CT), 0, st, Y, V, c.fronts, c.rows, gather_items,
+                   nrhs);
+    const dim3 grid((unsigned)nitems, CHAIN_GROUPS);
+    if (nrhs > 4) {
+        RFG_CHAIN_BY_R((nrhs + MG - 1) / MG,
+                       launch_pdl(true, k_chain_cols_mm<T, R>, grid, dim3(CT), mm_cols_smem<T, R>, st, part,
+                                  (const double*)V, panel, c.fronts, items, nrhs));
+        return;
+    }
+    RFG_CHAIN_BY_R(nrhs, launch_pdl(true, k_chain_cols<T, R>, grid, dim3(CT), cols_smem(R), st, part, (const double*)V,
+                                    panel, c.fronts, items));
 }
 
 template <typename T>
-void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const T* panel, const double* cinv,
-                      const DFront* fronts, const int64_t* chain_blk, const int64_t* items, int* flags, int* counter,
-                      int* err, cudaStream_t st) {
+void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const double* part, const T* panel, const ChainArgs& c,
+                      const int64_t* items, int* flags, int* counter, cudaStream_t st) {
     if (nitems <= 0) return;
+    check_nrhs(nrhs);
     const ChainDev& d = chain_dev();
-    RFG_CHAIN_BY_R(nrhs, (k_chain_bwd<T, R><<<grid_for_items(d.bwd[chain_kind<T>][R], nitems), CT, bwd_smem(R), st>>>(
-                              Y, panel, cinv, fronts, chain_blk, items, nitems, flags, counter, err)));
-    RFG_CUDA(cudaGetLastError());
+    if (nrhs > 4) {
+        const int64_t n = nitems * ((nrhs + MG - 1) / MG);
+        launch_pdl(true, k_chain_bwd_mm<T>, dim3(grid_for_items(d.bwd[chain_kind<T>][0], n)), dim3(CT), mm_bwd_smem<T>,
+                   st, Y, panel, c.cinv, c.d, part, c.colbase, c.fronts, c.blk, items, nitems, nrhs, c.nblocks, flags,
+                   counter, c.err);
+        return;
+    }
+    RFG_CHAIN_BY_R(nrhs, launch_pdl(true, k_chain_bwd<T, R>, dim3(grid_for_items(d.bwd[chain_kind<T>][R], nitems)),
+                                    dim3(CT), bwd_smem(R), st, Y, panel, c.cinv, c.d, part, c.colbase, c.fronts, c.blk,
+                                    items, nitems, flags, counter, c.err));
 }
 
 #undef RFG_CHAIN_BY_R
 
-#define RFG_CHAIN_INSTANCE(T)                                                                                       \
-    template void launch_chain_inverse<T>(double*, const T*, const double*, const DFront*, const int64_t*,          \
-                                          const int64_t*, int64_t, cudaStream_t);                                   \
-    template void launch_chain_fwd<T>(int, int64_t, const double*, double*, const T*, const double*, const DFront*, \
-                                      const int64_t*, const int64_t*, int*, int*, int*, cudaStream_t);              \
-    template void launch_chain_rows<T>(int, int64_t, const double*, double*, const T*, const DFront*,               \
-                                       const int64_t*, cudaStream_t);                                               \
-    template void launch_chain_cols<T>(int, int64_t, const int64_t*, int64_t, const int64_t*, double*, double*,     \
-                                       double*, const T*, const DFront*, const int64_t*, cudaStream_t);             \
-    template void launch_chain_bwd<T>(int, int64_t, double*, const T*, const double*, const DFront*,                \
-                                      const int64_t*, const int64_t*, int*, int*, int*, cudaStream_t);
+#define RFG_CHAIN_INSTANCE(T)                                                                                        \
+    template void launch_chain_inverse<T>(double*, const T*, const double*, const DFront*, const int64_t*,           \
+                                          const int64_t*, int64_t, cudaStream_t);                                    \
+    template void launch_chain_fwd<T>(int, int64_t, const double*, double*, const double*, const T*,                 \
+                                      const ChainArgs&, const int64_t*, int*, int*, cudaStream_t);                   \
+    template void launch_chain_rows<T>(int, int64_t, const double*, double*, const T*, const ChainArgs&,             \
+                                       const int64_t*, cudaStream_t);                                                \
+    template void launch_chain_cols<T>(int, int64_t, const int64_t*, int64_t, const int64_t*, const double*,         \
+                                       double*, double*, const T*, const ChainArgs&, cudaStream_t);                  \
+    template void launch_chain_bwd<T>(int, int64_t, double*, const double*, const T*, const ChainArgs&,              \
+                                      const int64_t*, int*, int*, cudaStream_t);
 RFG_CHAIN_INSTANCE(float)
 RFG_CHAIN_INSTANCE(double)
 #undef RFG_CHAIN_INSTANCE

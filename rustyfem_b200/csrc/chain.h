@@ -6,9 +6,10 @@
 // flags of the blocks the item depends on.
 //
 // Flag region of a sweep (int words, zeroed before the sweep): forward block flags
-// [0, chain_blocks), backward block flags [chain_blocks, 2·chain_blocks), then the work
-// counter of each level and direction (2·nlevels). A block's flag counts the CTAs of its
-// cluster that have published their part of y (four when the block is done).
+// [0, 4·chain_blocks), one set per group of eight right-hand sides (sweeps of one to four use
+// the first), backward block flags [4·chain_blocks, 8·chain_blocks), then the work counter of
+// each level and direction (2·nlevels). A block's flag counts the CTAs of its cluster that have
+// published their part of y (four when the block is done).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -19,7 +20,20 @@
 
 namespace rfg {
 
-inline int64_t chain_flag_words(const Plan& P) { return 2 * P.chain_blocks + 2 * P.nlevels; }
+inline int64_t chain_flag_words(const Plan& P) { return 8 * P.chain_blocks + 2 * P.nlevels; }
+
+// What every launch of a handle's chains reads.
+struct ChainArgs {
+    const DFront* fronts;
+    const int64_t* rows;     // Plan::rows
+    const int32_t* imap;     // DevPlan::imap
+    const int64_t* blk;      // Plan::chain_blk
+    const int64_t* colbase;  // Plan::chain_colbase
+    const double* cinv;      // the blocks' inverses
+    const double* d;         // pivots
+    int64_t nblocks;         // Plan::chain_blocks
+    int* err;                // set to 1 when a wait gave up (sticky)
+};
 
 // The inverse of every chain block's unit-lower diagonal block, WS × WS in FP64 (row-major,
 // zero above the diagonal and beyond the block's width), from the NB × NB inverses of the
@@ -28,34 +42,32 @@ template <typename T>
 void launch_chain_inverse(double* cinv, const T* panel, const double* linv, const DFront* fronts,
                           const int64_t* chain_blk, const int64_t* chain_bfront, int64_t nblocks, cudaStream_t st);
 
-// Forward chain of one level: Y[pivot rows] = L⁻¹ x for the level's fronts, X (with the
-// children's update vectors added) as the right-hand side. items: the level's (front,
-// block) pairs; flags: the forward block flags; counter: the level's work counter; err: set
-// to 1 when a wait gave up (sticky).
+// Forward chain of one level: Y[pivot rows] = L⁻¹ x for the level's fronts, x = X plus the
+// children's update vectors in V. items: the level's (front, block) pairs; flags: the forward
+// block flags; counter: the level's work counter. 1 to 32 right-hand sides.
 template <typename T>
-void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, const T* panel, const double* cinv,
-                      const DFront* fronts, const int64_t* chain_blk, const int64_t* items, int* flags, int* counter,
-                      int* err, cudaStream_t st);
+void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, const double* V, const T* panel,
+                      const ChainArgs& c, const int64_t* items, int* flags, int* counter, cudaStream_t st);
 
-// After a level's forward chain: V[later rows] −= L21·y, items the (front, piece) pairs of
-// the level's later rows.
+// After a level's forward chain: V[later rows] = the children's V − L21·y, items the (front,
+// piece) pairs of the level's later rows.
 template <typename T>
-void launch_chain_rows(int nrhs, int64_t nitems, const double* Y, double* V, const T* panel, const DFront* fronts,
+void launch_chain_rows(int nrhs, int64_t nitems, const double* Y, double* V, const T* panel, const ChainArgs& c,
                        const int64_t* items, cudaStream_t st);
 
 // Before a level's backward chain: the solution of the fronts' later rows gathered into V
-// (gather_items: the level's later-row pieces), then z[pivot columns] −= L21ᵀ·y_later
-// (items: the level's pivot-column pieces), z the scaled forward result in Y; part holds
-// the row groups' partial sums (CHAIN_GROUPS · CHAIN_PIECE · nrhs values per item).
+// (gather_items: the level's later-row pieces), then L21ᵀ·y_later (items: the level's
+// pivot-column pieces) as partial sums of the row groups in part (CHAIN_GROUPS · CHAIN_PIECE ·
+// nrhs values per item).
 template <typename T>
 void launch_chain_cols(int nrhs, int64_t ngather, const int64_t* gather_items, int64_t nitems, const int64_t* items,
-                       double* Y, double* V, double* part, const T* panel, const DFront* fronts,
-                       const int64_t* rows, cudaStream_t st);
+                       const double* Y, double* V, double* part, const T* panel, const ChainArgs& c, cudaStream_t st);
 
-// Backward chain of one level: Y[pivot rows] = L11⁻ᵀ z.
+// Backward chain of one level: Y[pivot columns] = L⁻ᵀ z, z the forward result in Y over D minus
+// the partial sums in part. items: the level's (front, block) pairs from each front's last
+// block on; flags: the backward block flags; counter: the level's work counter.
 template <typename T>
-void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const T* panel, const double* cinv,
-                      const DFront* fronts, const int64_t* chain_blk, const int64_t* items, int* flags, int* counter,
-                      int* err, cudaStream_t st);
+void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const double* part, const T* panel, const ChainArgs& c,
+                      const int64_t* items, int* flags, int* counter, cudaStream_t st);
 
 }  // namespace rfg

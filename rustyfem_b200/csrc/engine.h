@@ -89,7 +89,6 @@ struct DevPlan {
     uint8_t* outer_mode = nullptr;    // Plan::outer_mode
     int64_t* pre_scr = nullptr;
     int64_t* xadd_child = nullptr;
-    int64_t* xadd_task = nullptr;
     int64_t* xadd_fpre = nullptr;
     int64_t* pre_wrows = nullptr;
     int64_t* pre_wpart = nullptr;
@@ -105,7 +104,11 @@ struct DevPlan {
     int64_t* chain_bwd = nullptr;     // Plan::chain_bwd
     int64_t* chain_rows = nullptr;    // Plan::chain_rows
     int64_t* chain_cols = nullptr;    // Plan::chain_cols
+    int64_t* chain_colbase = nullptr; // Plan::chain_colbase
+    int32_t* imap = nullptr;          // per front with children (DFront::imap_off) and child: the child row of each row
 };
+
+struct ChainArgs;
 
 struct FactorStats {
     double t_factor_ms = 0.0;     // device time of the numeric phase
@@ -153,13 +156,13 @@ class Engine {
     // The sweep of solve_device for nrhs ≤ 32 right-hand sides, launched directly (no
     // CUDA graph) on workspace the caller provides instead of the engine's own. The
     // workspace is sweep_workspace_bytes(nrhs) bytes at a 256-byte aligned address. It
-    // need hold nothing on entry: the sweep zeroes the ticket words and the update rows
-    // (v) itself, with memsets on the engine's stream. Allocates nothing.
+    // need hold nothing on entry: the sweep writes the update rows (v) before it reads them
+    // and zeroes the flag words itself, on the engine's stream. Allocates nothing.
     struct SweepWorkspace {
         double* y;        // n · nrhs
         double* v;        // vu_rows · nrhs
         double* partial;  // partial_rows · nrhs
-        int* tickets;     // max_nact, then the flag words of the solve chains
+        int* flags;       // the flag words of the solve chains
         bool chain;       // room for the solve chains; without it every level is stepped
     };
     bool has_chain() const { return chain_inv_ != nullptr; }
@@ -216,11 +219,12 @@ class Engine {
     template <typename T>
     int64_t forward_steps(int64_t level, double* X, double* Y, double* V, int nrhs, int* chain);
     template <typename T>
-    int64_t backward_steps(int64_t level, double* Y, double* V, int nrhs, double* partial, int* tickets, int* chain);
+    int64_t backward_steps(int64_t level, double* Y, double* V, int nrhs, double* partial, int* chain);
+    ChainArgs chain_args() const;
     // the sweeps of nrhs right-hand sides run the solve chains of the plan's chain levels
     bool chain_on(int64_t nrhs) const;
     void ensure_chain_inverse();
-    int64_t ticket_words(bool chain) const;
+    int64_t flag_words(bool chain) const;
     int64_t partial_rows(bool chain) const;  // partial-sum values per right-hand side of a sweep
     void init(bool use_tc);
     void upload_plan();

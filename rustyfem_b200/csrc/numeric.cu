@@ -1337,6 +1337,17 @@ __global__ void k_orig_diag(const double* __restrict__ src, const int64_t* __res
     }
 }
 
+// imap of a front's parent: the front's row x at the parent row emap[x]
+__global__ void k_imap_fill(const DFront* __restrict__ fr, const int32_t* __restrict__ emap,
+                            int32_t* __restrict__ imap) {
+    const int64_t c = blockIdx.x;
+    const DFront f = fr[c];
+    if (f.parent < 0 || f.u == 0) return;
+    const DFront p = fr[f.parent];
+    int32_t* m = imap + p.imap_off + (p.kid0 == c ? 0 : p.m);
+    for (int64_t x = threadIdx.x; x < f.u; x += blockDim.x) m[emap[f.emap_off + x]] = (int32_t)x;
+}
+
 __global__ void k_gather_i64(const int64_t* __restrict__ a, const int64_t* __restrict__ idx, int64_t n,
                              int64_t* __restrict__ out) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -1386,7 +1397,6 @@ void Engine::upload_plan() {
     dp_.panel_mode = up(plan_.panel_mode);
     dp_.outer_mode = up(plan_.outer_mode);
     dp_.xadd_child = up(plan_.xadd_child);
-    dp_.xadd_task = up(plan_.xadd_task);
     dp_.xadd_fpre = up(plan_.xadd_fpre);
     dp_.rows = up(plan_.rows);
     dp_.emap = up(plan_.emap);
@@ -1396,6 +1406,14 @@ void Engine::upload_plan() {
     dp_.chain_bwd = up(plan_.chain_bwd);
     dp_.chain_rows = up(plan_.chain_rows);
     dp_.chain_cols = up(plan_.chain_cols);
+    dp_.chain_colbase = up(plan_.chain_colbase);
+    // the child row of each front row, for either child: the inverse of emap, on the device
+    dp_.imap = (int32_t*)dalloc(std::max<int64_t>(plan_.imap_elems, 1) * sizeof(int32_t));
+    RFG_CUDA(cudaMemsetAsync(dp_.imap, 0xff, std::max<int64_t>(plan_.imap_elems, 1) * sizeof(int32_t), stream_));
+    if (plan_.nfronts > 0) {
+        k_imap_fill<<<(unsigned)plan_.nfronts, 128, 0, stream_>>>(dp_.fronts, dp_.emap, dp_.imap);
+        RFG_CUDA(cudaGetLastError());
+    }
     level_poff_.assign(plan_.nlevels + 1, plan_.panel_elems);
     for (int64_t l = 0; l < plan_.nlevels; l++)
         if (plan_.level_off[l + 1] > plan_.level_off[l]) level_poff_[l] = plan_.fronts[plan_.level_order[plan_.level_off[l]]].poff;

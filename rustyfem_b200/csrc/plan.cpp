@@ -129,6 +129,25 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
             d.blk_off = nblk;
             nblk += cdiv(f.k, NB);
         }
+    for (int64_t t = 0; t < nt; t++) {
+        // children come before their parent in level order: their vuoff is set
+        const SymFront& f = S.fronts[t];
+        DFront& d = P.fronts[t];
+        auto kid = [&](int64_t r) -> int64_t {
+            if (f.nchild <= r) return -1;
+            const int64_t c = S.children[f.child_off + r];
+            return S.fronts[c].u > 0 ? c : -1;
+        };
+        d.kid0 = kid(0);
+        d.kid1 = kid(1);
+        d.kv0 = d.kid0 >= 0 ? P.fronts[d.kid0].vuoff : 0;
+        d.kv1 = d.kid1 >= 0 ? P.fronts[d.kid1].vuoff : 0;
+        d.imap_off = -1;
+        if (d.kid0 >= 0 || d.kid1 >= 0) {
+            d.imap_off = P.imap_elems;
+            P.imap_elems += 2 * d.m;
+        }
+    }
     P.panel_elems = poff;
     P.vu_rows = vu;
     P.nblocks = nblk;
@@ -369,13 +388,15 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
     P.wstep_off.assign(nlev + 1, 0);
     for (int64_t l = 0; l < nlev; l++) {
         const int64_t lo = P.level_off[l], hi = P.level_off[l + 1];
-        const int64_t nws = cdiv(P.level_maxk[l], WS);
+        // the first step takes every front of the level: its rows kernel also passes the
+        // children's update vectors on, for a front without pivots too
+        const int64_t nws = hi > lo ? std::max<int64_t>(1, cdiv(P.level_maxk[l], WS)) : 0;
         for (int64_t S2 = 0; S2 < nws; S2++) {
             WStep w{};
             w.level = l;
             w.S = S2;
             w.fr_off = lo;
-            while (lo + w.nact < hi && S.fronts[P.level_order[lo + w.nact]].k > S2 * WS) w.nact++;
+            while (lo + w.nact < hi && (S2 == 0 || S.fronts[P.level_order[lo + w.nact]].k > S2 * WS)) w.nact++;
             w.pre_off = (int64_t)P.pre_wrows.size();
             P.pre_wrows.push_back(0);
             P.pre_wpart.push_back(0);
@@ -405,6 +426,7 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
         }
         P.level_chain.assign(nlev, 0);
         P.chain_blk.assign(nt, -1);
+        P.chain_colbase.assign(nt, -1);
         P.chain_fwd_off.assign(nlev + 1, 0);
         P.chain_bwd_off.assign(nlev + 1, 0);
         P.chain_rows_off.assign(nlev + 1, 0);
@@ -429,6 +451,7 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
                 for (int64_t i = lo; i < hi; i++) {
                     const int64_t t = P.level_order[i];
                     if (P.fronts[t].u == 0) continue;
+                    P.chain_colbase[t] = (int64_t)P.chain_cols.size() / 2 - P.chain_cols_off[l];
                     for (int64_t c = 0; c < cdiv(P.fronts[t].u, CHAIN_PIECE); c++) P.chain_rows.insert(P.chain_rows.end(), {t, c});
                     for (int64_t c = 0; c < cdiv(P.fronts[t].k, CHAIN_PIECE); c++) P.chain_cols.insert(P.chain_cols.end(), {t, c});
                 }
@@ -453,7 +476,6 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
         for (int r = 0; r < 2; r++) {
             DXadd& x = P.xadd[2 * l + r];
             x.off = (int64_t)P.xadd_child.size();
-            x.task_off = (int64_t)P.xadd_task.size() / 4;
             x.fpre_off = (int64_t)P.xadd_fpre.size();
             P.xadd_fpre.push_back(0);
             int64_t cnt = 0, fblk = 0;
@@ -464,16 +486,12 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
                 if (S.fronts[c].u == 0) continue;
                 P.xadd_child.push_back(c);
                 const int64_t uc = S.fronts[c].u;
-                for (int64_t x0 = 0; x0 < uc; x0 += XR)
-                    P.xadd_task.insert(P.xadd_task.end(), {c, P.level_order[i], x0, std::min<int64_t>(XR, uc - x0)});
                 const int64_t T = cdiv(uc, XT);
                 fblk += cdiv(T * (T + 1) / 2, 8);
                 P.xadd_fpre.push_back(fblk);
                 cnt++;
             }
             x.nchild = cnt;
-            x.ntask = (int64_t)P.xadd_task.size() / 4 - x.task_off;
-            x.nblk = cdiv(x.ntask, 8);
             x.fnblk = fblk;
         }
     if (std::any_of(S.fronts.begin(), S.fronts.end(), [](const SymFront& f) { return f.nchild > 2; }))

@@ -40,7 +40,6 @@ constexpr int NBO = 256;      // outer block: pivots applied together to the tra
 constexpr int KO = NBO / NB;
 constexpr int UT = 64;        // Schur-update tile (UT × UT of F)
 constexpr int PR = 128;       // panel rows per CTA
-constexpr int XR = 256;       // solve: update-vector rows of one warp's extend-add task
 constexpr int XT = 32;        // factor: tile (XT × XT of a child's update matrix) of one warp of the extend-add
 
 // per-front descriptor used by the kernels (int64 everywhere: offsets exceed 2^31)
@@ -53,6 +52,9 @@ struct DFront {
     int64_t emap_off;         // emap[] offset: local index in the parent of each later row
     int64_t vuoff;            // offset (in rows) of the front's solve update vector
     int64_t blk_off;          // first of the front's NB×NB diagonal blocks in the inverse store
+    int64_t kid0, kid1;       // children with later rows, by rank (-1: none)
+    int64_t kv0, kv1;         // their vuoff
+    int64_t imap_off;         // the front's child-row maps (two of m entries), -1 without children
 };
 
 // one step s of one level: the active fronts are the first nact of the level's
@@ -95,10 +97,7 @@ struct WStep {
 // extend-add work of one level and one child rank
 struct DXadd {
     int64_t off;              // offset into xadd_child
-    int64_t task_off;         // offset (in tasks) into xadd_task
-    int64_t ntask;            // solve: warp tasks (XR rows of one child each)
     int64_t nchild;
-    int64_t nblk;             // solve: CTAs (eight warp tasks each)
     int64_t fpre_off;         // offset into xadd_fpre (nchild + 1 entries)
     int64_t fnblk;            // total CTAs of the factor's extend-add (eight XT × XT tiles each)
 };
@@ -144,8 +143,8 @@ struct Plan {
     std::vector<int64_t> pre_wrows, pre_wpart;
     int64_t max_wrows = 0, max_wpart = 0;
     // Solve chains. On the levels with at most chain_fronts fronts (the top of the tree,
-    // where a step's launches have a few CTAs of work) a sweep with at most
-    // four right-hand sides runs as one launch per level and direction instead of
+    // where a step's launches have a few CTAs of work) a sweep
+    // runs as one launch per level and direction instead of
     // two per WS-wide step: each WS-wide diagonal block of a front is one work item, done
     // by a cluster of four CTAs that waits for the blocks it depends on (chain.cu). The
     // block's solve multiplies by the inverse of its unit-lower diagonal block (WS × WS,
@@ -162,16 +161,16 @@ struct Plan {
     // pivot columns CHAIN_PIECE·i ... (z −= L21ᵀ·y_later before it)
     std::vector<int64_t> chain_rows_off, chain_cols_off;  // nlevels + 1, in pairs
     std::vector<int64_t> chain_rows, chain_cols;
+    std::vector<int64_t> chain_colbase;  // per front: its first column piece of its level, or -1
     int64_t chain_colpart = 0;  // partial sums of a level's column pieces (CHAIN_GROUPS row groups), per rhs
     std::vector<uint8_t> front_tc;      // fronts whose large outer updates run on the tensor cores
     // extend-add lists, per level and rank (2 ranks)
     std::vector<DXadd> xadd;            // 2·nlevels
     std::vector<int64_t> xadd_child;    // child ids
-    std::vector<int64_t> xadd_task;     // solve: (child, parent, first row, rows) per warp task
-    std::vector<int64_t> xadd_fpre;     // the same for the factor's area-balanced chunks
+    std::vector<int64_t> xadd_fpre;     // prefix of the children's area-balanced chunks
     SegVec rows;                        // global equation of the later rows (Symbolic::rows)
     std::vector<int32_t> emap;          // local index in the parent of each later row
-    int64_t panel_elems = 0, upd_elems = 0, vu_rows = 0;
+    int64_t panel_elems = 0, upd_elems = 0, vu_rows = 0, imap_elems = 0;
     int64_t max_scr_rows = 0;           // largest scratch over all steps
     int64_t max_nact = 0;               // largest number of active fronts of a step
     int64_t nblocks = 0;                // NB×NB diagonal blocks of all fronts

@@ -3,20 +3,19 @@
 // The solve follows the level schedule of the factor (plan.h) in steps of WS = 4·NB
 // pivots (WStep), for nrhs right-hand sides stored as X[q·nrhs + j] (internal
 // numbering):
-//  forward  (leaves up)   per level, the children's update vectors are added into
-//                         their parents (k_vec_extend_add: pivot rows into X, later
-//                         rows into the parent's update vector V_t); then per step
-//                         k_wfwd_diag solves the step's diagonal block with its four
-//                         stored NB×NB inverse blocks (y_B → Y) and k_wfwd_rows
-//                         subtracts L[r, J0:J1]·y_B from the rows below (X or V_t);
-//  diagonal               Y /= D (k_divide_d);
+//  forward  (leaves up)   per level and step, a diagonal kernel solves the step's diagonal
+//                         block with its four stored NB×NB inverse blocks (y_B → Y) and a
+//                         rows kernel subtracts L[r, J0:J1]·y_B from the rows below (X or the
+//                         front's update vector V_t). The first step of a front adds the
+//                         children's update vectors on the way, through the map of each row
+//                         to the children's rows (kids_add: child 0 before child 1);
 //  backward (root down)   per step, last first: partial sums of Lᵀ·y over row chunks
-//                         below the block, then the diagonal block backwards
-//                         (k_wbwd_part_pf + k_wbwd_diag_pf for an FP32 factor and up
-//                         to four right-hand sides, else k_wbwd, whose last CTA per
-//                         front reduces the partials and solves the block).
+//                         below the block, then the diagonal block backwards from
+//                         z = Y/D − Σ partials.
+// One to four right-hand sides run the _pf (FP32 factor) and _pd (FP64) kernels, five to 32
+// the _mm kernels on the FP64 tensor-core path; the levels at the top run as chains (chain.h).
 // Every kernel of a sweep is launched as a programmatic dependent of the one before
-// (PDL): the _pf kernels copy their factor data into shared memory before they wait for
+// (PDL): the kernels copy their factor data into shared memory before they wait for
 // the vectors of the previous kernel.
 // This is the multifrontal form of Factor::solve (src/sparse.rs:615-652): the same
 // three sweeps, with the updates of each front gathered in its update vector instead
@@ -58,320 +57,6 @@ __device__ __forceinline__ int64_t find_slot2(const int64_t* pre, int64_t n, int
             hi = mid;
     }
     return lo;
-}
-
-// children's update vectors into the parent (one launch per child rank, so that no two
-// tasks of a launch add into the same entry): one warp per task of up to XR rows of one
-// child; the rows' targets in the parent are staged in shared memory before the wait for
-// the previous kernel, then the lanes run over (row, right-hand side) pairs
-__global__ void __launch_bounds__(256) k_vec_extend_add(double* __restrict__ X, double* __restrict__ V,
-                                                        const DFront* __restrict__ fr,
-                                                        const int64_t* __restrict__ tasks, int64_t ntask,
-                                                        const int32_t* __restrict__ emap, int nrhs) {
-    pdl_launch_dependents();
-    __shared__ int32_t spos[8][XR];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t tk = (int64_t)blockIdx.x * 8 + w;
-    if (tk >= ntask) return;
-    const int64_t c = tasks[4 * tk], p = tasks[4 * tk + 1], x0 = tasks[4 * tk + 2];
-    const int nx = (int)tasks[4 * tk + 3];
-    const DFront fc = fr[c], fp = fr[p];
-    for (int x = lane; x < nx; x += 32) spos[w][x] = emap[fc.emap_off + x0 + x];
-    __syncwarp();
-    pdl_wait();
-    for (int e = lane; e < nx * nrhs; e += 32) {
-        const int x = e / nrhs, j = e - x * nrhs;
-        const int pos = spos[w][x];
-        const double v = V[(fc.vuoff + x0 + x) * nrhs + j];
-        if (pos < fp.k)
-            X[(fp.start + pos) * nrhs + j] += v;
-        else
-            V[(fp.vuoff + pos - fp.k) * nrhs + j] += v;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Solve steps WS = 4·NB pivots wide (WStep). Forward: k_wfwd_diag (one CTA per active
-// front) solves the step's diagonal block with its four stored NB×NB inverses and the
-// panel pieces between them, writes y_B to Y, and k_wfwd_rows (PR rows per CTA)
-// subtracts L[r, J0:J1]·y_B from every row below the block. Backward: k_wbwd sums
-// L[r, J0:J1]ᵀ·y(r) over its rows into a per-CTA partial; the last CTA of the front
-// (atomic ticket) subtracts all partials from y_B and solves the diagonal block
-// backwards. One wide step replaces four NB steps, so the chain of dependent launches
-// at the top of the tree is four times shorter.
-// ---------------------------------------------------------------------------
-
-// rows of panel pieces the forward diagonal kernel stages for a level (multiple of NB)
-inline int wfwd_piece_rows(int64_t maxk_level, int64_t S) {
-    const int64_t wbmax = std::min<int64_t>(WS, std::max<int64_t>(0, maxk_level - S * WS));
-    const int64_t rows = std::min<int64_t>(3 * NB, std::max<int64_t>(0, wbmax - NB));
-    return (int)((rows + NB - 1) / NB * NB);
-}
-template <typename T>
-size_t wfwd_diag_smem(int piece_rows, int nrhs) {
-    return NB * (NB + 1) * sizeof(double) + ((size_t)piece_rows * (NB + 1) * sizeof(T) + 7) / 8 * 8 +
-           (size_t)(WS + NB) * nrhs * sizeof(double);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_wfwd_diag(const double* __restrict__ X, double* __restrict__ Y,
-                                                   const T* __restrict__ panel, const double* __restrict__ linv,
-                                                   const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                   int64_t fr_off, int64_t S, int nrhs, int piece_rows, int cgrp) {
-    pdl_launch_dependents();
-    pdl_wait();
-    // this CTA: right-hand sides [jc0, jc0 + rc) of front blockIdx.x
-    const int jc0 = blockIdx.y * cgrp, rc = min(cgrp, nrhs - jc0);
-    extern __shared__ double sm[];
-    double(*Li)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(sm);
-    T(*Lp)[NB + 1] = reinterpret_cast<T(*)[NB + 1]>(sm + NB * (NB + 1));
-    double* xB = sm + NB * (NB + 1) + ((size_t)piece_rows * (NB + 1) * sizeof(T) + 7) / 8;  // [WS][rc]
-    double* yb = xB + WS * rc;                                                                // [NB][rc]
-    const DFront f = fr[order[fr_off + blockIdx.x]];
-    const int64_t J0 = S * WS;
-    const int wb = (int)min((int64_t)WS, f.k - J0), nbw = (wb + NB - 1) / NB;
-    const double* xs = X + (f.start + J0) * nrhs + jc0;
-    for (int idx = threadIdx.x; idx < nbw * NB * rc; idx += blockDim.x) {
-        const int q = idx / rc, j = idx - q * rc;
-        xB[idx] = q < wb ? xs[(int64_t)q * nrhs + j] : 0.0;
-    }
-    for (int b = 0; b < nbw; b++) {
-        const int jbb = min(NB, wb - b * NB);
-        const int nbelow = wb - (b + 1) * NB;  // rows of the block below sub-block b
-        __syncthreads();
-        load_linv<256>(Li, linv + (f.blk_off + S * 4 + b) * (int64_t)(NB * NB));
-        for (int c = 0; c * NB < nbelow; c++)
-            load_tile<T, NB, 256>(Lp + c * NB, panel + f.poff + (J0 + (b + 1 + c) * NB) * f.ldp + J0 + b * NB, f.ldp,
-                                  min(NB, nbelow - c * NB), jbb);
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < NB * rc; idx += blockDim.x) {
-            const int p = idx / rc, j = idx - p * rc;
-            double a0 = 0.0, a1 = 0.0;
-            int q = 0;
-            for (; q + 1 <= p; q += 2) {
-                a0 = fma(Li[p][q], xB[(b * NB + q) * rc + j], a0);
-                a1 = fma(Li[p][q + 1], xB[(b * NB + q + 1) * rc + j], a1);
-            }
-            if (q <= p) a0 = fma(Li[p][q], xB[(b * NB + q) * rc + j], a0);
-            yb[idx] = a0 + a1;
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < jbb * rc; idx += blockDim.x) {
-            const int p = idx / rc, j = idx - p * rc;
-            Y[(f.start + J0 + b * NB + p) * nrhs + jc0 + j] = yb[idx];
-        }
-        for (int idx = threadIdx.x; idx < max(0, nbelow) * rc; idx += blockDim.x) {
-            const int i = idx / rc, j = idx - i * rc;
-            double a0 = 0.0, a1 = 0.0;
-            for (int p = 0; p < NB; p += 2) {
-                a0 = fma((double)Lp[i][p], yb[p * rc + j], a0);
-                a1 = fma((double)Lp[i][p + 1], yb[(p + 1) * rc + j], a1);
-            }
-            xB[((b + 1) * NB + i) * rc + j] -= a0 + a1;
-        }
-    }
-}
-
-// rows below the wide block: X (pivot rows) or V (later rows) −= L[r, J0:J1]·y_B
-template <typename T>
-__global__ void __launch_bounds__(PR) k_wfwd_rows(double* __restrict__ X, double* __restrict__ V,
-                                                  const double* __restrict__ Y, const T* __restrict__ panel,
-                                                  const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                  int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
-                                                  int64_t S, int nrhs) {
-    pdl_launch_dependents();
-    pdl_wait();
-    extern __shared__ double sm[];
-    double* yB = sm;  // [⌈wb/NB⌉·NB][nrhs]
-    const int64_t b = blockIdx.x;
-    const int64_t i = find_slot_warp(pre, nact, b);
-    const int64_t chunk = b - pre[i];
-    const DFront f = fr[order[fr_off + i]];
-    const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
-    const int wb = (int)(J1 - J0), nbw = (wb + NB - 1) / NB;
-    const int64_t r0 = J1 + chunk * PR;
-    const int nr = (int)max((int64_t)0, min((int64_t)PR, f.m - r0));
-    if (nr == 0) return;
-    const double* ys = Y + (f.start + J0) * nrhs;
-    for (int idx = threadIdx.x; idx < nbw * NB * nrhs; idx += blockDim.x) yB[idx] = idx < wb * nrhs ? ys[idx] : 0.0;
-    __syncthreads();
-    const int rr = threadIdx.x;
-    if (rr >= nr) return;
-    const int64_t r = r0 + rr;
-    double* tgt = r < f.k ? X + (f.start + r) * nrhs : V + (f.vuoff + r - f.k) * nrhs;
-    const T* rowp = panel + f.poff + r * f.ldp + J0;
-    constexpr int VEC = 16 / (int)sizeof(T);
-    using VT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-    for (int c = 0; c < nbw; c++) {
-        const int jc = min(NB, wb - c * NB);
-        T lv[NB];
-#pragma unroll
-        for (int q = 0; q < NB / VEC; q++) {
-            const int p = q * VEC;
-            if (p + VEC <= jc) {
-                *reinterpret_cast<VT*>(&lv[p]) = __ldg(reinterpret_cast<const VT*>(rowp + c * NB + p));
-            } else {
-#pragma unroll
-                for (int e = 0; e < VEC; e++) lv[p + e] = p + e < jc ? rowp[c * NB + p + e] : T(0);
-            }
-        }
-        for (int j = 0; j < nrhs; j++) {
-            double acc = 0.0;
-#pragma unroll
-            for (int p = 0; p < NB; p++) acc = fma((double)lv[p], yB[(c * NB + p) * nrhs + j], acc);
-            tgt[j] -= acc;
-        }
-    }
-}
-
-// shared memory of k_wbwd (layout in the kernel)
-template <typename T>
-constexpr size_t wbwd_smem(int nrhs) {
-    return ((std::max<size_t>(PR * (NB + 1) * sizeof(T), NB * (NB + 1) * 8) + 7) / 8 +
-            std::max<size_t>(PR * (nrhs + 1), WS * (nrhs + 1) + NB * nrhs + 256) + 256) *
-           sizeof(double);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_wbwd(double* __restrict__ Y, const T* __restrict__ panel,
-                                              const double* __restrict__ linv, const DFront* __restrict__ fr,
-                                              const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
-                                              const int64_t* __restrict__ pre, const int64_t* __restrict__ pre_part,
-                                              const int64_t* __restrict__ rows, int64_t S, int nrhs,
-                                              double* __restrict__ partial, int* __restrict__ tickets) {
-    pdl_launch_dependents();
-    pdl_wait();
-    // region 0: the panel tile (storage type T), later an inverse block or a panel piece;
-    // region 1: y of the CTA's rows (row stride nrhs+1), later z_B, y_b and group sums;
-    // then 256 doubles for the partial-sum reduction
-    extern __shared__ double sm[];
-    T(*Lt)[NB + 1] = reinterpret_cast<T(*)[NB + 1]>(sm);
-    const int region0 = (int)((max(PR * (NB + 1) * (int)sizeof(T), NB * (NB + 1) * 8) + 7) / 8);
-    const int xs = nrhs + 1;
-    double* xr = sm + region0;
-    const int region1 = max(PR * xs, WS * xs + NB * nrhs + 256);
-    double* red = xr + region1;
-    __shared__ int last;
-    const int64_t b = blockIdx.x;
-    const int64_t i = find_slot_warp(pre, nact, b);
-    const int64_t chunk = b - pre[i];
-    const DFront f = fr[order[fr_off + i]];
-    const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
-    const int wb = (int)(J1 - J0), nbw = (wb + NB - 1) / NB;
-    const int64_t r0 = J1 + chunk * PR;
-    const int nr = (int)max((int64_t)0, min((int64_t)PR, f.m - r0));
-#pragma unroll 4
-    for (int idx = threadIdx.x; idx < PR * nrhs; idx += 256) {
-        int rr = idx / nrhs, j = idx - rr * nrhs;
-        double v = 0.0;
-        if (rr < nr) {
-            int64_t r = r0 + rr;
-            int64_t q = r < f.k ? f.start + r : rows[f.rows_off + r - f.k];
-            v = Y[q * nrhs + j];
-        }
-        xr[rr * xs + j] = v;
-    }
-    // out[p·nrhs + j] = Σ_rr L[r][J0+p]·y(r)[j], column chunk by column chunk; with few
-    // outputs, G thread groups take every G-th row, their sums added in group order
-    double* out = partial + (pre_part[i] + chunk * wb) * nrhs;
-    for (int c = 0; c < nbw; c++) {
-        const int jc = min(NB, wb - c * NB);
-        __syncthreads();
-        load_tile<T, PR, 256>(Lt, panel + f.poff + r0 * f.ldp + J0 + c * NB, f.ldp, nr, jc);
-        __syncthreads();
-        const int nout = jc * nrhs;
-        const int G = nout >= 256 ? 1 : 256 / nout;
-        for (int idx = threadIdx.x; idx < nout * G; idx += 256) {
-            int g = idx / nout, o = idx - g * nout;
-            int p = o / nrhs, j = o - p * nrhs;
-            double acc = 0.0;
-            for (int rr = g; rr < nr; rr += G) acc = fma((double)Lt[rr][p], xr[rr * xs + j], acc);
-            if (G == 1)
-                out[c * NB * nrhs + o] = acc;
-            else
-                red[g * nout + o] = acc;
-        }
-        if (G > 1) {
-            __syncthreads();
-            for (int o = threadIdx.x; o < nout; o += 256) {
-                double v = 0.0;
-                for (int g = 0; g < G; g++) v += red[g * nout + o];
-                out[c * NB * nrhs + o] = v;
-            }
-        }
-    }
-    __threadfence();
-    __syncthreads();
-    const int64_t c0 = pre[i], c1 = pre[i + 1];
-    if (threadIdx.x == 0) last = (atomicAdd(&tickets[i], 1) == (int)(c1 - c0 - 1));
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // the last CTA: z_B = y_B − Σ partials (CTAs in order), then the block solved backwards
-    double(*Li)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(sm);
-    double* z = xr;                   // [nbw·NB][xs]
-    double* yb = xr + WS * xs;        // [NB][nrhs]
-    double* gsum = yb + NB * nrhs;    // [G][nout] when nout < 256
-    {
-        const int nout = wb * nrhs;
-        const int G = nout >= 256 ? 1 : 256 / nout;
-        const int64_t nc = c1 - c0, per = (nc + G - 1) / G;
-        const double* pbase = partial + pre_part[i] * nrhs;
-        for (int idx = threadIdx.x; idx < nout * G; idx += 256) {
-            int g = idx / nout, o = idx - g * nout;
-            int64_t ca = g * per, cb = min(nc, ca + per);
-            double v = 0.0;
-#pragma unroll 4
-            for (int64_t c = ca; c < cb; c++) v += __ldcg(&pbase[c * nout + o]);
-            if (G == 1) {
-                int p = o / nrhs, j = o - p * nrhs;
-                z[p * xs + j] = Y[(f.start + J0 + p) * nrhs + j] - v;
-            } else {
-                gsum[g * nout + o] = v;
-            }
-        }
-        if (G > 1) {
-            __syncthreads();
-            for (int o = threadIdx.x; o < nout; o += 256) {
-                double v = 0.0;
-                for (int g = 0; g < G; g++) v += gsum[g * nout + o];
-                int p = o / nrhs, j = o - p * nrhs;
-                z[p * xs + j] = Y[(f.start + J0 + p) * nrhs + j] - v;
-            }
-        }
-        for (int idx = threadIdx.x; idx < (nbw * NB - wb) * nrhs; idx += 256) {
-            int p = wb + idx / nrhs, j = idx % nrhs;
-            z[p * xs + j] = 0.0;
-        }
-    }
-    for (int bb = nbw - 1; bb >= 0; bb--) {
-        const int jbb = min(NB, wb - bb * NB);
-        __syncthreads();
-        load_linv<256>(Li, linv + (f.blk_off + S * 4 + bb) * (int64_t)(NB * NB));
-        __syncthreads();
-        // y_b = L_bb⁻ᵀ·z_b
-        for (int idx = threadIdx.x; idx < NB * nrhs; idx += 256) {
-            const int p = idx / nrhs, j = idx - p * nrhs;
-            double acc = 0.0;
-            for (int q = p; q < NB; q++) acc = fma(Li[q][p], z[(bb * NB + q) * xs + j], acc);
-            yb[idx] = acc;
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < jbb * nrhs; idx += 256) Y[(f.start + J0 + bb * NB) * nrhs + idx] = yb[idx];
-        // the earlier sub-blocks: z_b2 −= L[rows of bb, columns of b2]ᵀ·y_b
-        for (int b2 = 0; b2 < bb; b2++) {
-            __syncthreads();
-            load_tile<T, NB, 256>(Lt, panel + f.poff + (J0 + bb * NB) * f.ldp + J0 + b2 * NB, f.ldp, jbb, NB);
-            __syncthreads();
-            for (int idx = threadIdx.x; idx < NB * nrhs; idx += 256) {
-                const int c = idx / nrhs, j = idx - c * nrhs;
-                double acc = 0.0;
-                for (int q = 0; q < jbb; q++) acc = fma((double)Lt[q][c], yb[q * nrhs + j], acc);
-                z[(b2 * NB + c) * xs + j] -= acc;
-            }
-        }
-    }
-    if (threadIdx.x == 0) tickets[i] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -465,7 +150,8 @@ template <int R>
 __global__ void __launch_bounds__(256) k_wfwd_diag_pf(const double* __restrict__ X, double* __restrict__ Y,
                                                       const float* __restrict__ panel, const double* __restrict__ linv,
                                                       const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                      int64_t fr_off, int64_t S, int nbw_max) {
+                                                      int64_t fr_off, int64_t S, int nbw_max,
+                                                      const double* __restrict__ V, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
     double* Li = sm;                                                     // [nli][NB][NB]
@@ -486,7 +172,15 @@ __global__ void __launch_bounds__(256) k_wfwd_diag_pf(const double* __restrict__
     cp_async_commit();
     pdl_wait();
     const double* xs = X + (f.start + J0) * R;
-    for (int idx = threadIdx.x; idx < nbw * NB * R; idx += 256) xB[idx] = idx < wb * R ? xs[idx] : 0.0;
+    if (threadIdx.x < nbw * NB) {
+        const int p = threadIdx.x;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            double x = p < wb ? xs[p * R + r] : 0.0;
+            if (S == 0 && p < wb) x = kids_add(x, V, imap, f, p, R, r);
+            xB[p * R + r] = x;
+        }
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sel = (lane >> 2) & 7;
     for (int b = 0; b < nbw; b++) {
         const int jbb = min(NB, wb - b * NB);
@@ -560,7 +254,7 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
                                                      const double* __restrict__ Y, const T* __restrict__ panel,
                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ order,
                                                      int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
-                                                     int64_t S, int cols) {
+                                                     int64_t S, int cols, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
     constexpr int RPC = PF_ROWS<T>, SUB = PR / RPC, TPR = PR / RPC, VEC = 16 / (int)sizeof(T);
@@ -613,8 +307,14 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
     if (h == 0 && rr < nr) {
         const int64_t r = r0 + rr;
         double* tgt = r < f.k ? X + (f.start + r) * R : V + (f.vuoff + r - f.k) * R;
+        if (S == 0) {
+            // the first step of the front: the children's part on the way (V starts from it)
 #pragma unroll
-        for (int j = 0; j < R; j++) tgt[j] -= v[j];
+            for (int j = 0; j < R; j++) tgt[j] = kids_add(r < f.k ? tgt[j] : 0.0, V, imap, f, r, R, j) - v[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < R; j++) tgt[j] -= v[j];
+        }
     }
 }
 
@@ -697,9 +397,10 @@ __global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__
     }
 }
 
-// z_B = y_B − Σ partial blocks (nc of them from block offset off), zero beyond the block.
+// z_B = y_B/D − Σ partial blocks (nc of them from block offset off), zero beyond the block.
 template <int R>
-__device__ __forceinline__ void wbwd_sum_partials(double* z, const double* Y, const double* partial, const DFront& f,
+__device__ __forceinline__ void wbwd_sum_partials(double* z, const double* Y, const double* __restrict__ d,
+                                                  const double* partial, const DFront& f,
                                                   int64_t J0, int wb, int nbw, int64_t nc, int64_t off) {
     const int nout = wb * R;
     const double* pbase = partial + off * R;
@@ -724,7 +425,7 @@ __device__ __forceinline__ void wbwd_sum_partials(double* z, const double* Y, co
                 for (int u = 0; u < 8; u++) v += t[u];
             }
             for (; c < nc; c++) v += __ldcg(&pbase[c * nout + o]);
-            v = Y[(f.start + J0) * R + o] - v;
+            v = Y[(f.start + J0) * R + o] / d[f.start + J0 + o / R] - v;
         }
         z[o] = v;
     }
@@ -741,7 +442,8 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pf(double* __restrict__ Y, co
                                                       const int64_t* __restrict__ order, int64_t fr_off,
                                                       const int64_t* __restrict__ pre,
                                                       const int64_t* __restrict__ pre_part, int64_t S,
-                                                      const double* __restrict__ partial, int nbw_max) {
+                                                      const double* __restrict__ partial, int nbw_max,
+                                                      const double* __restrict__ d) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
     double* Li = sm;                                                       // [nli][NB][NB]
@@ -766,7 +468,7 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pf(double* __restrict__ Y, co
         }
     cp_async_commit();
     pdl_wait();
-    wbwd_sum_partials<R>(z, Y, partial, f, J0, wb, nbw, 2 * (pre[i + 1] - pre[i]), 2 * pre_part[i]);
+    wbwd_sum_partials<R>(z, Y, d, partial, f, J0, wb, nbw, 2 * (pre[i + 1] - pre[i]), 2 * pre_part[i]);
     cp_async_wait<0>();
     for (int bb = nbw - 1; bb >= 0; bb--) {
         const int jbb = min(NB, wb - bb * NB);
@@ -860,7 +562,8 @@ template <int R>
 __global__ void __launch_bounds__(256) k_wfwd_diag_pd(const double* __restrict__ X, double* __restrict__ Y,
                                                       const double* __restrict__ panel, const double* __restrict__ linv,
                                                       const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                      int64_t fr_off, int64_t S, int nbw_max) {
+                                                      int64_t fr_off, int64_t S, int nbw_max,
+                                                      const double* __restrict__ V, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
     double* xB = sm + pd_slots(nbw_max) * NB * NB;  // [WS][R]
@@ -874,7 +577,15 @@ __global__ void __launch_bounds__(256) k_wfwd_diag_pd(const double* __restrict__
     cp_async_commit();
     pdl_wait();
     const double* xs = X + (f.start + J0) * R;
-    for (int idx = threadIdx.x; idx < nbw * NB * R; idx += 256) xB[idx] = idx < wb * R ? xs[idx] : 0.0;
+    if (threadIdx.x < nbw * NB) {
+        const int p = threadIdx.x;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            double x = p < wb ? xs[p * R + r] : 0.0;
+            if (S == 0 && p < wb) x = kids_add(x, V, imap, f, p, R, r);
+            xB[p * R + r] = x;
+        }
+    }
     cp_async_wait<0>();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sel = (lane >> 2) & 7;
     int t0 = 0;  // the stage's first tile
@@ -947,7 +658,8 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pd(double* __restrict__ Y, co
                                                       const int64_t* __restrict__ order, int64_t fr_off,
                                                       const int64_t* __restrict__ pre,
                                                       const int64_t* __restrict__ pre_part, int64_t S,
-                                                      const double* __restrict__ partial, int nbw_max) {
+                                                      const double* __restrict__ partial, int nbw_max,
+                                                      const double* __restrict__ d) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
     double* z = sm + pd_slots(nbw_max) * NB * NB;  // [WS][R]
@@ -962,7 +674,7 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pd(double* __restrict__ Y, co
     for (int t = 0; t < min(ntile, PD_SLOTS); t++) pd_issue<false>(sm, t, panel, f, lsrc, J0, wb, nbw);
     cp_async_commit();
     pdl_wait();
-    wbwd_sum_partials<R>(z, Y, partial, f, J0, wb, nbw, 2 * (pre[i + 1] - pre[i]), 2 * pre_part[i]);
+    wbwd_sum_partials<R>(z, Y, d, partial, f, J0, wb, nbw, 2 * (pre[i + 1] - pre[i]), 2 * pre_part[i]);
     cp_async_wait<0>();
     int t0 = 0;  // the stage's first tile
     for (int bb = nbw - 1; bb >= 0; bb--) {
@@ -1025,332 +737,365 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pd(double* __restrict__ Y, co
 }
 
 // ---------------------------------------------------------------------------
-// Step kernels for 5 to 32 right-hand sides (a block of load cases, the subspace
-// iteration of an eigen solver): the rows below a wide block and the partial sums of the
-// backward step are small GEMMs (PF_RPC rows × up to WS columns × nrhs), register-tiled
-// with eight right-hand sides per thread so that every factor entry is converted to FP64
-// and read from shared memory once per eight products; the row tile is prefetched
-// before the wait for the vectors (PDL). The partial sums of a backward step are added
-// (chunks in order) into y_B by k_wred, then k_wbwd_diag_mr solves the diagonal block.
+// Step kernels for 5 to 32 right-hand sides (a block of load cases, the subspace iteration of
+// an eigen solver) on the FP64 tensor-core path (m8n8k4). The diagonal kernels take one front
+// and eight right-hand sides per CTA: warp w owns rows (columns backward) 8w ... of each
+// sub-block, the inverse blocks and panel pieces stream through MM_SLOTS slots in the order of
+// use with one barrier per tile. The rows and partial kernels take all right-hand sides of a
+// block (NT groups of eight), so that the factor is read once. Vectors stand in rows of
+// 8·NT + 4 doubles: a fragment load (four rows, eight columns) meets every bank once per
+// half-warp. They are bound by the latency of a step's launches and tiles (the hex20 20³ cube
+// with 32 right-hand sides: 0.5 GB of factor and 16 GFLOP per sweep); with CUDA-core products,
+// a warp per 256 rows for the children's vectors and one CTA per 256 pivots a refined solve of
+// it (four sweeps) took 47.3 ms, now 11.7 ms; the FP64 solve of 160 batched plates with 8
+// right-hand sides went from 3.25 to 1.16 ms.
 // ---------------------------------------------------------------------------
-// rows kernel: the row tile transposed (k-major, PF_RPC + 4 elements per k) in region 0,
-// which later holds the four k-groups' partial sums; then Y_B ([cols][MAXR] doubles)
-__host__ __device__ inline size_t mr_rows_region0(int cols, size_t elt) {
-    const size_t tile = (size_t)cols * (PF_RPC + 4) * elt, sums = (size_t)4 * PF_RPC * MAXR * sizeof(double);
-    return tile > sums ? tile : sums;
+constexpr int MM_SLOTS = 5;
+constexpr int MM_P = NB + 4;       // tile pitch (elements): conflict-free row fragments
+constexpr int MM_TILE = NB * MM_P; // doubles per slot
+constexpr int MM_V = 12;           // pitch of a group's vector rows
+constexpr int MM_ROWS = 64;        // rows of a rows CTA
+// rows of a stage of the partial-sum kernel (two stages, PR rows per CTA), and its tile pitch
+template <typename T>
+constexpr int MM_PST = 256 / (int)sizeof(T);
+template <typename T>
+__host__ __device__ inline int mm_part_pitch(int cols) { return cols + (sizeof(T) == 4 ? 8 : 4); }
+__host__ __device__ inline int mm_slots(int nbw) { return nbw + pf_npc(nbw) < MM_SLOTS ? nbw + pf_npc(nbw) : MM_SLOTS; }
+inline size_t mm_diag_smem(int nbw) {
+    return ((size_t)mm_slots(nbw) * MM_TILE + (size_t)(nbw * NB + NB) * MM_V) * sizeof(double);
 }
-inline size_t mr_rows_smem(int cols, size_t elt) {
-    return mr_rows_region0(cols, elt) + (size_t)cols * MAXR * sizeof(double);
+template <typename T>
+size_t mm_rows_smem(int cols, int nt) {
+    return (size_t)MM_ROWS * (cols + 4) * sizeof(T) + (size_t)cols * (8 * nt + 4) * sizeof(double);
+}
+template <typename T>
+size_t mm_part_smem(int cols, int nt) {
+    return (size_t)2 * MM_PST<T> * mm_part_pitch<T>(cols) * sizeof(T) + (size_t)PR * (8 * nt + 4) * sizeof(double);
 }
 
-// Rows below a wide block: X (pivot rows) or V (later rows) −= L[r, J0:J1]·Y_B for PF_RPC
-// rows per CTA. The row tile is read into registers before the wait for Y_B and stored
-// k-major; thread (k-group of cols/4 columns, 4 rows, 8 right-hand sides) accumulates 32
-// products per k from one 4-row load and one 8-vector load; the four k-groups' sums are
-// added in order through shared memory.
+// The tile-th tile of a diagonal block into its slot (nothing past the last): the used part of
+// inverse block b (its first jb rows and columns, rounded up to eight) or of panel piece
+// (rb, cb), rows padded with zeros to eight. A tile counts as one commit group either way.
+template <typename T, bool FWD>
+__device__ __forceinline__ void mm_issue(double* sm, int tile, int ntile, const T* panel, const DFront& f,
+                                         const double* lsrc, int64_t J0, int wb, int nbw) {
+    if (tile < ntile) {
+        double* dst = sm + (tile % MM_SLOTS) * MM_TILE;
+        int st = 0, i = tile;  // stage st, the i-th tile of it
+        while (i > nbw - 1 - st) {
+            i -= nbw - st;
+            st++;
+        }
+        const int b = FWD ? st : nbw - 1 - st;
+        if (i == 0) {
+            const int jr = (min(NB, wb - b * NB) + 7) & ~7;
+            cp_async_tile<double>(dst, MM_P, lsrc + b * NB * NB, NB, jr, jr, jr, jr, 256);
+        } else {
+            const int rb = FWD ? b + i : b, cb = FWD ? b : i - 1, nr = min(NB, wb - rb * NB);
+            cp_async_tile<T>(reinterpret_cast<T*>(dst), MM_P, panel + f.poff + (J0 + rb * NB) * f.ldp + J0 + cb * NB,
+                             f.ldp, nr, NB, (nr + 7) & ~7, NB, 256);
+        }
+    }
+    cp_async_commit();
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_wfwd_rows_mr(double* __restrict__ X, double* __restrict__ V,
-                                                      const double* __restrict__ Y, const T* __restrict__ panel,
-                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                      int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
-                                                      int64_t S, int nrhs, int cols) {
+__global__ void __launch_bounds__(256) k_mm_fwd_diag(const double* __restrict__ X, double* __restrict__ Y,
+                                                     const double* __restrict__ V, const T* __restrict__ panel,
+                                                     const double* __restrict__ linv, const DFront* __restrict__ fr,
+                                                     const int64_t* __restrict__ order, int64_t fr_off, int64_t S,
+                                                     int nrhs, int nbw_max, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
-    constexpr int VEC = 16 / (int)sizeof(T);                 // elements per 16-byte load
-    constexpr int LP = PF_RPC + 4;                           // k-major pitch
-    constexpr int NPRE = PF_RPC * WS * 4 / 16 / 256;  // 16-byte loads held per thread (an FP32 tile; half an FP64 one)
-    using VT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-    T* LT = reinterpret_cast<T*>(sm);                                           // [cols][LP]
-    double* red = sm;                                                           // [4][PF_RPC][MAXR] (after use)
-    double* yB = sm + mr_rows_region0(cols, sizeof(T)) / sizeof(double);        // [cols][MAXR]
-    const int64_t b = blockIdx.x >> 1;
-    const int64_t i = find_slot_warp(pre, nact, b);
-    const int64_t chunk = b - pre[i];
-    const DFront f = fr[order[fr_off + i]];
-    const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
-    const int wb = (int)(J1 - J0);
-    const int64_t r0 = J1 + chunk * PR + (blockIdx.x & 1) * PF_RPC;
-    const int nr = (int)max((int64_t)0, min((int64_t)PF_RPC, f.m - r0));
-    // 16-byte pieces (row rr = idx % PF_RPC, columns VEC·(idx / PF_RPC) ..): a warp reads
-    // one column piece of 32 rows and stores it k-major without bank conflicts
-    const int npiece = PF_RPC * (cols / VEC);
-    const T* src = panel + f.poff + r0 * f.ldp + J0;
-    VT pre_v[NPRE];
-#pragma unroll
-    for (int u = 0; u < NPRE; u++) {
-        const int idx = threadIdx.x + 256 * u;
-        const int rr = idx % PF_RPC, c = (idx / PF_RPC) * VEC;
-        VT v;
-        T* ve = reinterpret_cast<T*>(&v);
-#pragma unroll
-        for (int e = 0; e < VEC; e++) ve[e] = T(0);
-        if (idx < npiece && rr < nr) {
-            if (c + VEC <= wb)
-                v = __ldg(reinterpret_cast<const VT*>(src + (int64_t)rr * f.ldp + c));
-            else
-#pragma unroll
-                for (int e = 0; e < VEC; e++) ve[e] = c + e < wb ? src[(int64_t)rr * f.ldp + c + e] : T(0);
-        }
-        pre_v[u] = v;
-    }
+    double* xB = sm + mm_slots(nbw_max) * MM_TILE;  // [nbw·NB][MM_V]
+    double* yb = xB + nbw_max * NB * MM_V;          // [NB][MM_V]
+    const DFront f = fr[order[fr_off + blockIdx.x]];
+    const int j0 = blockIdx.y * 8, rc = min(8, nrhs - j0);
+    const int64_t J0 = S * WS;
+    const int wb = (int)min((int64_t)WS, f.k - J0), nbw = (wb + NB - 1) / NB;
+    const double* lsrc = linv + (f.blk_off + S * 4) * (int64_t)(NB * NB);
+    const int ntile = nbw + pf_npc(nbw);
+    for (int i = 0; i < MM_SLOTS - 1; i++) mm_issue<T, true>(sm, i, ntile, panel, f, lsrc, J0, wb, nbw);
     pdl_wait();
-    if (nr == 0) return;
-#pragma unroll
-    for (int u = 0; u < NPRE; u++) {
-        const int idx = threadIdx.x + 256 * u;
-        if (idx < npiece) {
-            const int rr = idx % PF_RPC, c = (idx / PF_RPC) * VEC;
-            const T* ve = reinterpret_cast<const T*>(&pre_v[u]);
-#pragma unroll
-            for (int e = 0; e < VEC; e++) LT[(c + e) * LP + rr] = ve[e];
+    for (int e = threadIdx.x; e < nbw * NB * 8; e += 256) {
+        const int p = e >> 3, n = e & 7;
+        double x = 0.0;
+        if (p < wb && n < rc) {
+            x = X[(f.start + J0 + p) * nrhs + j0 + n];
+            if (S == 0) x = kids_add(x, V, imap, f, p, nrhs, j0 + n);
         }
+        xB[p * MM_V + n] = x;
     }
-    // pieces beyond the registers (FP64 tiles wider than 128 columns)
-    for (int idx = threadIdx.x + 256 * NPRE; idx < npiece; idx += 256) {
-        const int rr = idx % PF_RPC, c = (idx / PF_RPC) * VEC;
-#pragma unroll
-        for (int e = 0; e < VEC; e++)
-            LT[(c + e) * LP + rr] = (rr < nr && c + e < wb) ? src[(int64_t)rr * f.ldp + c + e] : T(0);
-    }
-    const double* ys = Y + (f.start + J0) * nrhs;
-    for (int idx = threadIdx.x; idx < cols * MAXR; idx += 256) {
-        const int p = idx / MAXR, j = idx - p * MAXR;
-        yB[idx] = (p < wb && j < nrhs) ? ys[p * nrhs + j] : 0.0;
-    }
-    __syncthreads();
-    const int kg = threadIdx.x >> 6, q = threadIdx.x & 63, rg = q >> 2, g = q & 3;
-    const int kq = cols / 4, k0 = kg * kq;
-    double acc[4][8];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int u = 0; u < 8; u++) acc[a][u] = 0.0;
-    if (8 * g < nrhs) {
-#pragma unroll 2
-        for (int k = k0; k < k0 + kq; k++) {
-            double l[4];
-            if constexpr (sizeof(T) == 4) {
-                const float4 lv = *reinterpret_cast<const float4*>(LT + k * LP + 4 * rg);
-                l[0] = lv.x; l[1] = lv.y; l[2] = lv.z; l[3] = lv.w;
-            } else {
-                const double2 l01 = *reinterpret_cast<const double2*>(LT + k * LP + 4 * rg);
-                const double2 l23 = *reinterpret_cast<const double2*>(LT + k * LP + 4 * rg + 2);
-                l[0] = l01.x; l[1] = l01.y; l[2] = l23.x; l[3] = l23.y;
-            }
-            const double2* y2 = reinterpret_cast<const double2*>(yB + k * MAXR + 8 * g);
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const double2 y = y2[u];
-#pragma unroll
-                for (int a = 0; a < 4; a++) {
-                    acc[a][2 * u] = fma(l[a], y.x, acc[a][2 * u]);
-                    acc[a][2 * u + 1] = fma(l[a], y.y, acc[a][2 * u + 1]);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    int i = 0;
+    for (int b = 0; b < nbw; b++) {
+        const int jb = min(NB, wb - b * NB), jr = (jb + 7) & ~7;
+        for (int b2 = b; b2 < nbw; b2++, i++) {
+            cp_async_wait<MM_SLOTS - 2>();
+            __syncthreads();  // tile i and the last stage's vectors visible; tile i − 1 is read
+            mm_issue<T, true>(sm, i + MM_SLOTS - 1, ntile, panel, f, lsrc, J0, wb, nbw);
+            const double* tile = sm + (i % MM_SLOTS) * MM_TILE;
+            double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+            if (b2 == b) {
+                // y_b = L_bb⁻¹·x_b: rows 8w ... of the lower triangle
+                if (8 * w >= jr) continue;
+                const double* A = tile + (8 * w + g) * MM_P + q;
+                const double* B = xB + (b * NB + q) * MM_V + g;
+                for (int k = 0; k < 8 * w + 8; k += 8) {
+                    dmma_884(a0[0], a0[1], A[k], B[k * MM_V]);
+                    dmma_884(a1[0], a1[1], A[k + 4], B[(k + 4) * MM_V]);
                 }
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int p = 8 * w + g, n = 2 * q + e;
+                    const double y = p < jb ? a0[e] + a1[e] : 0.0;
+                    yb[p * MM_V + n] = y;
+                    if (p < jb && n < rc) Y[(f.start + J0 + b * NB + p) * nrhs + j0 + n] = y;
+                }
+            } else {
+                // x_b2 −= L[b2, b]·y_b (b is a full sub-block)
+                if (8 * w >= min(NB, wb - b2 * NB)) continue;
+                const T* A = reinterpret_cast<const T*>(tile) + (8 * w + g) * MM_P + q;
+                const double* B = yb + q * MM_V + g;
+#pragma unroll
+                for (int k = 0; k < NB; k += 8) {
+                    dmma_884(a0[0], a0[1], (double)A[k], B[k * MM_V]);
+                    dmma_884(a1[0], a1[1], (double)A[k + 4], B[(k + 4) * MM_V]);
+                }
+                double* x = xB + (b2 * NB + 8 * w + g) * MM_V + 2 * q;
+                x[0] -= a0[0] + a1[0];
+                x[1] -= a0[1] + a1[1];
             }
         }
-    }
-    __syncthreads();  // the tile is read: region 0 takes the k-groups' sums
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int u = 0; u < 8; u++) red[(kg * PF_RPC + 4 * rg + a) * MAXR + 8 * g + u] = acc[a][u];
-    __syncthreads();
-    for (int o = threadIdx.x; o < PF_RPC * MAXR; o += 256) {
-        const int rr = o / MAXR, j = o - rr * MAXR;
-        if (rr >= nr || j >= nrhs) continue;
-        const double v = ((red[o] + red[PF_RPC * MAXR + o]) + red[2 * PF_RPC * MAXR + o]) + red[3 * PF_RPC * MAXR + o];
-        const int64_t r = r0 + rr;
-        double* tgt = r < f.k ? X + (f.start + r) * nrhs : V + (f.vuoff + r - f.k) * nrhs;
-        tgt[j] -= v;
     }
 }
 
-// Backward partial sums for 5 to 32 right-hand sides: out[p][j] = Σ_rr L[r0+rr][J0+p]·
-// y(r0+rr)[j] over the CTA's PF_RPC rows; thread (four columns, eight right-hand sides).
-template <typename T>
-__global__ void __launch_bounds__(256) k_wbwd_part_mr(const double* __restrict__ Y, const T* __restrict__ panel,
-                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                      int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
-                                                      const int64_t* __restrict__ pre_part,
-                                                      const int64_t* __restrict__ rows, int64_t S, int nrhs,
-                                                      double* __restrict__ partial, int cols) {
+// Rows below a wide block: X (pivot rows) or V (later rows) −= L[r, J0:J1]·Y_B, MM_ROWS rows per
+// CTA (two CTAs per PR-row chunk), warp w rows 8w ....
+template <typename T, int NT>
+__global__ void __launch_bounds__(256) k_mm_fwd_rows(double* __restrict__ X, double* __restrict__ V,
+                                                     const double* __restrict__ Y, const T* __restrict__ panel,
+                                                     const DFront* __restrict__ fr, const int64_t* __restrict__ order,
+                                                     int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
+                                                     int64_t S, int nrhs, int cols, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
-    constexpr int VEC = 16 / (int)sizeof(T);
-    const int pitch = cols + VEC;
-    T* Lt = reinterpret_cast<T*>(sm);                                      // [PF_RPC][pitch]
-    double* yr = sm + ((size_t)PF_RPC * pitch * sizeof(T) + 15) / 16 * 2;  // [PF_RPC][MAXR]
+    constexpr int VP = 8 * NT + 4;
+    const int pitch = cols + 4;
+    double* yB = sm;                                 // [cols][VP]
+    T* Lt = reinterpret_cast<T*>(sm + cols * VP);    // [MM_ROWS][pitch]
     const int64_t b = blockIdx.x >> 1;
     const int64_t i = find_slot_warp(pre, nact, b);
     const int64_t chunk = b - pre[i];
     const DFront f = fr[order[fr_off + i]];
     const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
     const int wb = (int)(J1 - J0);
-    const int64_t r0 = J1 + chunk * PR + (blockIdx.x & 1) * PF_RPC;
-    const int nr = (int)max((int64_t)0, min((int64_t)PF_RPC, f.m - r0));
-    // rows beyond nr are zero-filled (they are summed below); with no rows the source is
-    // the front's first row, from which nothing is read
-    cp_async_tile<T>(Lt, pitch, panel + f.poff + (nr > 0 ? r0 * f.ldp + J0 : 0), f.ldp, nr, wb, PF_RPC, cols, 256);
+    const int64_t r0 = J1 + chunk * PR + (blockIdx.x & 1) * MM_ROWS;
+    const int nr = (int)max((int64_t)0, min((int64_t)MM_ROWS, f.m - r0));
+    if (nr > 0) cp_async_tile<T>(Lt, pitch, panel + f.poff + r0 * f.ldp + J0, f.ldp, nr, wb, (nr + 7) & ~7, cols, 256);
     cp_async_commit();
     pdl_wait();
-    for (int idx = threadIdx.x; idx < PF_RPC * MAXR; idx += 256) {
-        const int q = idx / MAXR, j = idx - q * MAXR;
-        double v = 0.0;
-        if (q < nr && j < nrhs) {
-            const int64_t r = r0 + q;
-            const int64_t e = r < f.k ? f.start + r : rows[f.rows_off + r - f.k];
-            v = Y[e * nrhs + j];
-        }
-        yr[idx] = v;
+    if (nr == 0) return;
+    const double* ys = Y + (f.start + J0) * nrhs;
+    for (int e = threadIdx.x; e < cols * 8 * NT; e += 256) {
+        const int p = e / (8 * NT), n = e % (8 * NT);
+        yB[p * VP + n] = (p < wb && n < nrhs) ? ys[p * nrhs + n] : 0.0;
     }
     cp_async_wait<0>();
     __syncthreads();
-    const int pg = threadIdx.x >> 2, g = threadIdx.x & 3;  // columns 4pg .. 4pg+3, right-hand sides 8g ..
-    if (4 * pg >= cols || 8 * g >= nrhs) return;
-    double acc[4][8];
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-#pragma unroll
-        for (int u = 0; u < 8; u++) acc[c][u] = 0.0;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    if (8 * w >= nr) return;
+    double acc[2][NT][2] = {};
+    const T* A = Lt + (8 * w + g) * pitch + q;
+    const double* B = yB + q * VP + g;
+    const int kend = (wb + 7) & ~7;
 #pragma unroll 2
-    for (int q = 0; q < PF_RPC; q++) {
-        double l[4];
+    for (int k = 0; k < kend; k += 8) {
 #pragma unroll
-        for (int c = 0; c < 4; c++) l[c] = (double)Lt[q * pitch + 4 * pg + c];
-        const double2* y2 = reinterpret_cast<const double2*>(yr + q * MAXR + 8 * g);
+        for (int h = 0; h < 2; h++) {
+            const double a = (double)A[k + 4 * h];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const double2 y = y2[u];
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                acc[c][2 * u] = fma(l[c], y.x, acc[c][2 * u]);
-                acc[c][2 * u + 1] = fma(l[c], y.y, acc[c][2 * u + 1]);
-            }
+            for (int n = 0; n < NT; n++) dmma_884(acc[h][n][0], acc[h][n][1], a, B[(k + 4 * h) * VP + 8 * n]);
         }
     }
-    double* out = partial + (2 * (pre_part[i] + chunk * wb) + (blockIdx.x & 1) * wb) * nrhs;
+    const int rr = 8 * w + g;
+    if (rr >= nr) return;
+    const int64_t r = r0 + rr;
+    double* tgt = r < f.k ? X + (f.start + r) * nrhs : V + (f.vuoff + r - f.k) * nrhs;
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const int p = 4 * pg + c;
-        if (p >= wb) break;
+    for (int n = 0; n < NT; n++)
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (8 * g + u < nrhs) out[p * nrhs + 8 * g + u] = acc[c][u];
-    }
+        for (int e = 0; e < 2; e++) {
+            const int j = 8 * n + 2 * q + e;
+            if (j >= nrhs) continue;
+            double x = (S > 0 || r < f.k) ? tgt[j] : 0.0;
+            if (S == 0) x = kids_add(x, V, imap, f, r, nrhs, j);
+            tgt[j] = x - (acc[0][n][e] + acc[1][n][e]);
+        }
 }
 
-// y_B −= Σ partial blocks (two per row chunk, in order): grid (front, slice of 256 outputs).
-__global__ void __launch_bounds__(256) k_wred(double* __restrict__ Y, const DFront* __restrict__ fr,
-                                              const int64_t* __restrict__ order, int64_t fr_off,
-                                              const int64_t* __restrict__ pre, const int64_t* __restrict__ pre_part,
-                                              int64_t S, int nrhs, const double* __restrict__ partial) {
-    pdl_launch_dependents();
-    const int64_t i = blockIdx.x;
-    const DFront f = fr[order[fr_off + i]];
-    const int64_t J0 = S * WS;
-    const int wb = (int)min((int64_t)WS, f.k - J0);
-    const int nout = wb * nrhs;
-    const int o = blockIdx.y * 256 + threadIdx.x;
-    pdl_wait();
-    if (o >= nout) return;
-    const int64_t nc = 2 * (pre[i + 1] - pre[i]);
-    const double* pbase = partial + 2 * pre_part[i] * nrhs;
-    double v = 0.0;
-    int64_t c = 0;
-    for (; c + 32 <= nc; c += 32) {
-        double t[32];
-#pragma unroll
-        for (int u = 0; u < 32; u++) t[u] = __ldcg(&pbase[(c + u) * nout + o]);
-#pragma unroll
-        for (int u = 0; u < 32; u++) v += t[u];
-    }
-    for (; c + 8 <= nc; c += 8) {
-        double t[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) t[u] = __ldcg(&pbase[(c + u) * nout + o]);
-#pragma unroll
-        for (int u = 0; u < 8; u++) v += t[u];
-    }
-    for (; c < nc; c++) v += __ldcg(&pbase[c * nout + o]);
-    Y[(f.start + J0) * nrhs + o] -= v;
-}
-
-// Diagonal block of a backward step, y_B already reduced: for sub-blocks bb from the last,
-// y_bb = L_bb⁻ᵀ·z_bb and z_b2 −= L[bb, b2]ᵀ·y_bb for b2 < bb. One CTA per front.
-template <typename T>
-__global__ void __launch_bounds__(256) k_wbwd_diag_mr(double* __restrict__ Y, const T* __restrict__ panel,
-                                                      const double* __restrict__ linv, const DFront* __restrict__ fr,
-                                                      const int64_t* __restrict__ order, int64_t fr_off, int64_t S,
-                                                      int nrhs, int cgrp) {
+// Backward partial sums: out[p][j] = Σ_rr L[r0+rr][J0+p]·y(r0+rr)[j] over a chunk's PR rows, one
+// block of partials per chunk; warp w takes the columns 8w + 64i ....
+template <typename T, int NT>
+__global__ void __launch_bounds__(256) k_mm_bwd_part(const double* __restrict__ Y, const T* __restrict__ panel,
+                                                     const DFront* __restrict__ fr, const int64_t* __restrict__ order,
+                                                     int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
+                                                     const int64_t* __restrict__ pre_part,
+                                                     const int64_t* __restrict__ rows, int64_t S, int nrhs,
+                                                     double* __restrict__ partial, int cols) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
-    // this CTA: right-hand sides [jc0, jc0 + rc) of front blockIdx.x
-    const int jc0 = blockIdx.y * cgrp, rc = min(cgrp, nrhs - jc0);
-    double(*Li)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(sm);
-    T(*Lt)[NB + 1] = reinterpret_cast<T(*)[NB + 1]>(sm + NB * (NB + 1));
-    double* z = sm + 2 * NB * (NB + 1);  // [WS][rc]
-    double* yb = z + WS * rc;            // [NB][rc]
-    const DFront f = fr[order[fr_off + blockIdx.x]];
-    const int64_t J0 = S * WS;
-    const int wb = (int)min((int64_t)WS, f.k - J0), nbw = (wb + NB - 1) / NB;
-    double* yB = Y + (f.start + J0) * nrhs + jc0;
+    constexpr int VP = 8 * NT + 4, ST = MM_PST<T>;
+    const int pitch = mm_part_pitch<T>(cols);
+    double* yr = sm;                            // [PR][VP]
+    T* ring = reinterpret_cast<T*>(sm + PR * VP);  // [2][ST][pitch]
+    const int64_t i = find_slot_warp(pre, nact, blockIdx.x);
+    const int64_t chunk = blockIdx.x - pre[i];
+    const DFront f = fr[order[fr_off + i]];
+    const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
+    const int wb = (int)(J1 - J0);
+    const int64_t r0 = J1 + chunk * PR;
+    const int nr = (int)max((int64_t)0, min((int64_t)PR, f.m - r0)), nst = (nr + ST - 1) / ST;
+    auto issue = [&](int h) {
+        if (h < nst)
+            cp_async_tile<T>(ring + (h & 1) * ST * pitch, pitch, panel + f.poff + (r0 + h * ST) * f.ldp + J0, f.ldp,
+                             nr - h * ST, wb, min(ST, (nr - h * ST + 7) & ~7), cols, 256);
+        cp_async_commit();
+    };
+    issue(0);
+    issue(1);
     pdl_wait();
-    for (int idx = threadIdx.x; idx < nbw * NB * rc; idx += 256) {
-        const int q = idx / rc, j = idx - q * rc;
-        z[idx] = q < wb ? yB[(int64_t)q * nrhs + j] : 0.0;
+    for (int e = threadIdx.x; e < ((nr + 7) & ~7) * 8 * NT; e += 256) {
+        const int rr = e / (8 * NT), n = e % (8 * NT);
+        double v = 0.0;
+        if (rr < nr && n < nrhs) {
+            const int64_t r = r0 + rr;
+            v = Y[(r < f.k ? f.start + r : rows[f.rows_off + r - f.k]) * nrhs + n];
+        }
+        yr[rr * VP + n] = v;
     }
-    for (int bb = nbw - 1; bb >= 0; bb--) {
-        const int jbb = min(NB, wb - bb * NB);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    double acc[4][NT][2] = {};
+    for (int h = 0; h < nst; h++) {
+        cp_async_wait<1>();
         __syncthreads();
-        load_linv<256>(Li, linv + (f.blk_off + S * 4 + bb) * (int64_t)(NB * NB));
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < NB * rc; idx += 256) {
-            const int p = idx / rc, j = idx - p * rc;
-            double a0 = 0.0, a1 = 0.0;
-            int q = p;
-            for (; q + 1 < NB; q += 2) {
-                a0 = fma(Li[q][p], z[(bb * NB + q) * rc + j], a0);
-                a1 = fma(Li[q + 1][p], z[(bb * NB + q + 1) * rc + j], a1);
-            }
-            if (q < NB) a0 = fma(Li[q][p], z[(bb * NB + q) * rc + j], a0);
-            yb[idx] = a0 + a1;
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < jbb * rc; idx += 256) {
-            const int p = idx / rc, j = idx - p * rc;
-            yB[(int64_t)(bb * NB + p) * nrhs + j] = yb[idx];
-        }
-        for (int b2 = 0; b2 < bb; b2++) {
-            __syncthreads();
-            load_tile<T, NB, 256>(Lt, panel + f.poff + (J0 + bb * NB) * f.ldp + J0 + b2 * NB, f.ldp, jbb, NB);
-            __syncthreads();
-            for (int idx = threadIdx.x; idx < NB * rc; idx += 256) {
-                const int c = idx / rc, j = idx - c * rc;
-                double a0 = 0.0, a1 = 0.0;
-                int q = 0;
-                for (; q + 1 < jbb; q += 2) {
-                    a0 = fma((double)Lt[q][c], yb[q * rc + j], a0);
-                    a1 = fma((double)Lt[q + 1][c], yb[(q + 1) * rc + j], a1);
+        const T* A = ring + (h & 1) * ST * pitch + q * pitch + 8 * w + g;
+        const double* B = yr + (h * ST + q) * VP + g;
+        const int kend = min(ST, (nr - h * ST + 7) & ~7);
+#pragma unroll 2
+        for (int k = 0; k < kend; k += 4) {
+            double fb[NT];
+#pragma unroll
+            for (int n = 0; n < NT; n++) fb[n] = B[k * VP + 8 * n];
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+                if (64 * m + 8 * w < wb) {
+                    const double a = (double)A[k * pitch + 64 * m];
+#pragma unroll
+                    for (int n = 0; n < NT; n++) dmma_884(acc[m][n][0], acc[m][n][1], a, fb[n]);
                 }
-                if (q < jbb) a0 = fma((double)Lt[q][c], yb[q * rc + j], a0);
-                z[(b2 * NB + c) * rc + j] -= a0 + a1;
-            }
         }
+        if (h + 2 < nst) __syncthreads();  // stage h is read
+        issue(h + 2);
     }
-}
-inline size_t mr_diag_smem(int cgrp) {
-    return 2 * NB * (NB + 1) * sizeof(double) + (size_t)(WS + NB) * cgrp * sizeof(double);
-}
-inline size_t mr_part_smem(int cols, size_t elt) {
-    const int vec = (int)(16 / elt);
-    return ((size_t)PF_RPC * (cols + vec) * elt + 15) / 16 * 16 + (size_t)PF_RPC * MAXR * sizeof(double);
+    double* out = partial + (pre_part[i] + chunk * wb) * nrhs;
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        const int p = 64 * m + 8 * w + g;
+        if (p >= wb) continue;
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int j = 8 * n + 2 * q + e;
+                if (j < nrhs) out[p * nrhs + j] = acc[m][n][e];
+            }
+    }
 }
 
-__global__ void k_divide_d(double* __restrict__ X, const double* __restrict__ d, int64_t n, int nrhs) {
+// Backward diagonal block: z_B = y_B/D − Σ partial blocks (chunks in order), then for sub-blocks
+// bb from the last: y_bb = L_bb⁻ᵀ·z_bb and z_b2 −= L[bb, b2]ᵀ·y_bb for b2 < bb.
+template <typename T>
+__global__ void __launch_bounds__(256) k_mm_bwd_diag(double* __restrict__ Y, const T* __restrict__ panel,
+                                                     const double* __restrict__ linv, const double* __restrict__ d,
+                                                     const DFront* __restrict__ fr, const int64_t* __restrict__ order,
+                                                     int64_t fr_off, const int64_t* __restrict__ pre,
+                                                     const int64_t* __restrict__ pre_part, int64_t S, int nrhs,
+                                                     int nbw_max, const double* __restrict__ partial) {
     pdl_launch_dependents();
+    extern __shared__ __align__(16) double sm[];
+    double* z = sm + mm_slots(nbw_max) * MM_TILE;  // [nbw·NB][MM_V]
+    double* yb = z + nbw_max * NB * MM_V;          // [NB][MM_V]
+    const int64_t fi = blockIdx.x;
+    const DFront f = fr[order[fr_off + fi]];
+    const int j0 = blockIdx.y * 8, rc = min(8, nrhs - j0);
+    const int64_t J0 = S * WS;
+    const int wb = (int)min((int64_t)WS, f.k - J0), nbw = (wb + NB - 1) / NB;
+    const double* lsrc = linv + (f.blk_off + S * 4) * (int64_t)(NB * NB);
+    const int ntile = nbw + pf_npc(nbw);
+    for (int i = 0; i < MM_SLOTS - 1; i++) mm_issue<T, false>(sm, i, ntile, panel, f, lsrc, J0, wb, nbw);
     pdl_wait();
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n * nrhs; e += (int64_t)gridDim.x * blockDim.x)
-        X[e] /= d[e / nrhs];
+    {
+        const int64_t nc = pre[fi + 1] - pre[fi], bs = (int64_t)wb * nrhs;
+        const double* pb = partial + pre_part[fi] * nrhs + j0;
+        for (int e = threadIdx.x; e < nbw * NB * 8; e += 256) {
+            const int p = e >> 3, n = e & 7;
+            double v = 0.0;
+            if (p < wb && n < rc) {
+                const double* pe = pb + (int64_t)p * nrhs + n;
+                int64_t c = 0;
+                for (; c + 8 <= nc; c += 8) {
+                    double t[8];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) t[u] = __ldcg(pe + (c + u) * bs);
+#pragma unroll
+                    for (int u = 0; u < 8; u++) v += t[u];
+                }
+                for (; c < nc; c++) v += __ldcg(pe + c * bs);
+                v = Y[(f.start + J0 + p) * nrhs + j0 + n] / d[f.start + J0 + p] - v;
+            }
+            z[p * MM_V + n] = v;
+        }
+    }
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    int i = 0;
+    for (int bb = nbw - 1; bb >= 0; bb--) {
+        const int jb = min(NB, wb - bb * NB), jr = (jb + 7) & ~7;
+        for (int b2 = -1; b2 < bb; b2++, i++) {
+            cp_async_wait<MM_SLOTS - 2>();
+            __syncthreads();  // tile i and the last stage's vectors visible; tile i − 1 is read
+            mm_issue<T, false>(sm, i + MM_SLOTS - 1, ntile, panel, f, lsrc, J0, wb, nbw);
+            const double* tile = sm + (i % MM_SLOTS) * MM_TILE;
+            double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+            if (b2 < 0) {
+                // y_bb = L_bb⁻ᵀ·z_bb: columns 8w ..., rows from 8w on
+                if (8 * w >= jr) continue;
+                const double* A = tile + q * MM_P + 8 * w + g;
+                const double* B = z + (bb * NB + q) * MM_V + g;
+                for (int k = 8 * w; k < jr; k += 8) {
+                    dmma_884(a0[0], a0[1], A[k * MM_P], B[k * MM_V]);
+                    dmma_884(a1[0], a1[1], A[(k + 4) * MM_P], B[(k + 4) * MM_V]);
+                }
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int p = 8 * w + g, n = 2 * q + e;
+                    const double y = p < jb ? a0[e] + a1[e] : 0.0;
+                    yb[p * MM_V + n] = y;
+                    if (p < jb && n < rc) Y[(f.start + J0 + bb * NB + p) * nrhs + j0 + n] = y;
+                }
+            } else {
+                const T* A = reinterpret_cast<const T*>(tile) + q * MM_P + 8 * w + g;
+                const double* B = yb + q * MM_V + g;
+                for (int k = 0; k < jr; k += 8) {
+                    dmma_884(a0[0], a0[1], (double)A[k * MM_P], B[k * MM_V]);
+                    dmma_884(a1[0], a1[1], (double)A[(k + 4) * MM_P], B[(k + 4) * MM_V]);
+                }
+                double* zz = z + (b2 * NB + 8 * w + g) * MM_V + 2 * q;
+                zz[0] -= a0[0] + a1[0];
+                zz[1] -= a0[1] + a1[1];
+            }
+        }
+    }
 }
 
 // caller column-major b (ncaller × nrhs) -> internal X (nsym × nrhs, row-major)
@@ -1637,40 +1382,71 @@ void launch_chained(bool pdl, void (*kern)(KArgs...), unsigned grid, unsigned bl
     launch_pdl(pdl, kern, dim3(grid), dim3(block), smem, st, args...);
 }
 
-// a sweep with at most PF_MAXR right-hand sides runs the prefetching kernels
-inline bool pf_path(int64_t nrhs) { return nrhs <= PF_MAXR; }
-// steps with 5 to 32 right-hand sides whose blocks are at least NB wide run the register-
-// tiled kernels; narrower ones (the many small fronts of 2D models) the first kernels, whose
-// CTAs are sized to the rows they have
-inline bool mr_step(int64_t nrhs, int64_t level_maxk, int64_t S) {
-    return nrhs > PF_MAXR && std::min<int64_t>(WS, level_maxk - S * WS) >= NB;
-}
 template <typename T, int R>
 void wfwd_pf(const WStep& w, int nbw_max, int cols, double* X, double* Y, double* V, const T* panel,
              const double* linv, const DevPlan& dp, cudaStream_t st) {
+    const int32_t* imap = dp.imap;
     if constexpr (sizeof(T) == 4)
         launch_chained(true, k_wfwd_diag_pf<R>, (unsigned)w.nact, 256, pf_diag_smem(nbw_max, R), st, X, Y, panel, linv,
-                       dp.fronts, dp.level_order, w.fr_off, w.S, nbw_max);
+                       dp.fronts, dp.level_order, w.fr_off, w.S, nbw_max, V, imap);
     else
         launch_chained(true, k_wfwd_diag_pd<R>, (unsigned)w.nact, 256, pd_diag_smem(nbw_max, R), st, X, Y, panel, linv,
-                       dp.fronts, dp.level_order, w.fr_off, w.S, nbw_max);
+                       dp.fronts, dp.level_order, w.fr_off, w.S, nbw_max, V, imap);
     launch_chained(true, k_wfwd_rows_pf<T, R>, (unsigned)(PR / PF_ROWS<T> * w.n_rows), PR, pf_rows_smem<T>(cols, R), st,
-                   X, V, Y, panel, dp.fronts, dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, w.S, cols);
+                   X, V, Y, panel, dp.fronts, dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, w.S, cols, imap);
 }
 template <typename T, int R>
 void wbwd_pf(const WStep& w, int nbw_max, int cols, double* Y, const T* panel, const double* linv,
-             const DevPlan& dp, double* partial, cudaStream_t st) {
+             const double* d, const DevPlan& dp, double* partial, cudaStream_t st) {
     launch_chained(true, k_wbwd_part_pf<T, R>, (unsigned)(2 * w.n_rows), 256, pf_part_smem<T>(cols, R), st, Y, panel,
                    dp.fronts, dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off,
                    dp.rows, w.S, partial, cols);
     if constexpr (sizeof(T) == 4)
         launch_chained(true, k_wbwd_diag_pf<R>, (unsigned)w.nact, 256, pf_diag_smem(nbw_max, R), st, Y, panel, linv,
                        dp.fronts, dp.level_order, w.fr_off, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off, w.S,
-                       partial, nbw_max);
+                       partial, nbw_max, d);
     else
         launch_chained(true, k_wbwd_diag_pd<R>, (unsigned)w.nact, 256, pd_diag_smem(nbw_max, R), st, Y, panel, linv,
                        dp.fronts, dp.level_order, w.fr_off, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off, w.S,
-                       partial, nbw_max);
+                       partial, nbw_max, d);
+}
+
+
+// five to 32 right-hand sides, NT groups of eight
+template <typename T, int NT>
+void wfwd_mm(const WStep& w, int nbw_max, int cols, double* X, double* Y, double* V, const T* panel,
+             const double* linv, const DevPlan& dp, int nrhs, cudaStream_t st) {
+    launch_pdl(true, k_mm_fwd_diag<T>, dim3((unsigned)w.nact, NT), dim3(256), mm_diag_smem(nbw_max), st,
+               (const double*)X, Y, (const double*)V, panel, linv, (const DFront*)dp.fronts,
+               (const int64_t*)dp.level_order, w.fr_off, w.S, nrhs, nbw_max, (const int32_t*)dp.imap);
+    launch_pdl(true, k_mm_fwd_rows<T, NT>, dim3((unsigned)(2 * w.n_rows)), dim3(256), mm_rows_smem<T>(cols, NT), st, X,
+               V, (const double*)Y, panel, (const DFront*)dp.fronts, (const int64_t*)dp.level_order, w.fr_off, w.nact,
+               (const int64_t*)(dp.pre_wrows + w.pre_off), w.S, nrhs, cols, (const int32_t*)dp.imap);
+}
+template <typename T, int NT>
+void wbwd_mm(const WStep& w, int nbw_max, int cols, double* Y, const T* panel, const double* linv, const double* d,
+             const DevPlan& dp, double* partial, int nrhs, cudaStream_t st) {
+    launch_pdl(true, k_mm_bwd_part<T, NT>, dim3((unsigned)w.n_rows), dim3(256), mm_part_smem<T>(cols, NT), st,
+               (const double*)Y, panel, (const DFront*)dp.fronts, (const int64_t*)dp.level_order, w.fr_off, w.nact,
+               (const int64_t*)(dp.pre_wrows + w.pre_off), (const int64_t*)(dp.pre_wpart + w.pre_off),
+               (const int64_t*)dp.rows, w.S, nrhs, partial, cols);
+    launch_pdl(true, k_mm_bwd_diag<T>, dim3((unsigned)w.nact, NT), dim3(256), mm_diag_smem(nbw_max), st, Y, panel, linv,
+               d, (const DFront*)dp.fronts, (const int64_t*)dp.level_order, w.fr_off,
+               (const int64_t*)(dp.pre_wrows + w.pre_off), (const int64_t*)(dp.pre_wpart + w.pre_off), w.S, nrhs,
+               nbw_max, (const double*)partial);
+}
+
+// fn(std::integral_constant<int, n>) for n = 1 .. 4
+template <typename F>
+void by_count(int n, F&& fn) {
+    if (n <= 1)
+        fn(std::integral_constant<int, 1>());
+    else if (n == 2)
+        fn(std::integral_constant<int, 2>());
+    else if (n == 3)
+        fn(std::integral_constant<int, 3>());
+    else
+        fn(std::integral_constant<int, 4>());
 }
 
 }  // namespace
@@ -1688,126 +1464,68 @@ void launch_scatter_rhs(double* b, const double* X, const int64_t* eq, const int
     if (niso * nrhs > 0) k_iso_divide<<<grid_for(niso * nrhs), 256, 0, st>>>(b, iso_idx, iso_d, niso, ncaller, (int)nrhs);
 }
 
+ChainArgs Engine::chain_args() const {
+    return ChainArgs{dp_.fronts, dp_.rows, dp_.imap, dp_.chain_blk, dp_.chain_colbase, chain_inv_, d_,
+                     plan_.chain_blocks, chain_err_};
+}
+
 template <typename T>
 int64_t Engine::forward_steps(int64_t l, double* X, double* Y, double* V, int nrhs, int* chain) {
     const Plan& P = plan_;
     const T* panel = (const T*)panel_;
-    int64_t launches = 0;
     if (chain && P.level_chain[l]) {
         const int64_t i0 = P.chain_fwd_off[l], r0 = P.chain_rows_off[l], nr = P.chain_rows_off[l + 1] - r0;
-        launch_chain_fwd(nrhs, P.chain_fwd_off[l + 1] - i0, X, Y, panel, chain_inv_, dp_.fronts,
-                         dp_.chain_blk, dp_.chain_fwd + 2 * i0, chain, chain + 2 * P.chain_blocks + 2 * l, chain_err_,
-                         stream_);
-        launch_chain_rows(nrhs, nr, Y, V, panel, dp_.fronts, dp_.chain_rows + 2 * r0, stream_);
+        launch_chain_fwd(nrhs, P.chain_fwd_off[l + 1] - i0, (const double*)X, Y, (const double*)V, panel, chain_args(),
+                         dp_.chain_fwd + 2 * i0, chain, chain + 8 * P.chain_blocks + 2 * l, stream_);
+        launch_chain_rows(nrhs, nr, (const double*)Y, V, panel, chain_args(), dp_.chain_rows + 2 * r0, stream_);
         return nr > 0 ? 2 : 1;
     }
+    int64_t launches = 0;
     for (int64_t wi = P.wstep_off[l]; wi < P.wstep_off[l + 1]; wi++) {
         const WStep& w = P.wsteps[wi];
-        if (pf_path(nrhs)) {
-            const int64_t wb_max = std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS);
-            const int nbw_max = (int)((wb_max + NB - 1) / NB), cols = pf_cols(wb_max);
-            if (nrhs == 1) wfwd_pf<T, 1>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
-            else if (nrhs == 2) wfwd_pf<T, 2>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
-            else if (nrhs == 3) wfwd_pf<T, 3>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
-            else wfwd_pf<T, 4>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
-        } else if (mr_step(nrhs, P.level_maxk[l], w.S)) {
-            const int pr = wfwd_piece_rows(P.level_maxk[l], w.S);
-            const int cols = pf_cols(std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS));
-            {
-                // eight right-hand sides per CTA: the stages of a wide block run in parallel over the columns
-                cudaLaunchConfig_t cfg{};
-                cfg.gridDim = dim3((unsigned)w.nact, (unsigned)((nrhs + 7) / 8));
-                cfg.blockDim = dim3(256);
-                cfg.dynamicSmemBytes = wfwd_diag_smem<T>(pr, 8);
-                cfg.stream = stream_;
-                RFG_CUDA(cudaLaunchKernelEx(&cfg, k_wfwd_diag<T>, (const double*)X, Y, panel, (const double*)linv_,
-                                            (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, w.fr_off, w.S,
-                                            nrhs, pr, 8));
-            }
-            launch_chained(true, k_wfwd_rows_mr<T>, (unsigned)(2 * w.n_rows), 256, mr_rows_smem(cols, sizeof(T)), stream_,
-                           X, V, Y, panel, dp_.fronts, dp_.level_order, w.fr_off, w.nact, dp_.pre_wrows + w.pre_off, w.S,
-                           nrhs, cols);
-        } else {
-            const int pr = wfwd_piece_rows(P.level_maxk[l], w.S);
-            launch_chained(false, k_wfwd_diag<T>, (unsigned)w.nact, 256, wfwd_diag_smem<T>(pr, nrhs), stream_, X, Y, panel,
-                           linv_, dp_.fronts, dp_.level_order, w.fr_off, w.S, nrhs, pr, nrhs);
-            launch_chained(false, k_wfwd_rows<T>, (unsigned)w.n_rows, PR, (size_t)WS * nrhs * sizeof(double), stream_, X, V, Y,
-                           panel, dp_.fronts, dp_.level_order, w.fr_off, w.nact, dp_.pre_wrows + w.pre_off, w.S, nrhs);
-        }
+        const int64_t wb_max = std::max<int64_t>(1, std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS));
+        const int nbw_max = (int)((wb_max + NB - 1) / NB), cols = pf_cols(wb_max);
+        if (nrhs <= PF_MAXR)
+            by_count(nrhs, [&](auto r) {
+                wfwd_pf<T, decltype(r)::value>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, stream_);
+            });
+        else
+            by_count((nrhs + 7) / 8, [&](auto nt) {
+                wfwd_mm<T, decltype(nt)::value>(w, nbw_max, cols, X, Y, V, panel, linv_, dp_, nrhs, stream_);
+            });
         launches += 2;
     }
     return launches;
 }
 
 template <typename T>
-int64_t Engine::backward_steps(int64_t l, double* Y, double* V, int nrhs, double* partial, int* tickets, int* chain) {
+int64_t Engine::backward_steps(int64_t l, double* Y, double* V, int nrhs, double* partial, int* chain) {
     const Plan& P = plan_;
     const T* panel = (const T*)panel_;
-    int64_t launches = 0;
     if (chain && P.level_chain[l]) {
         const int64_t i0 = P.chain_bwd_off[l], r0 = P.chain_rows_off[l], c0 = P.chain_cols_off[l];
         const int64_t nr = P.chain_rows_off[l + 1] - r0, nc = P.chain_cols_off[l + 1] - c0;
-        launch_chain_cols(nrhs, nr, dp_.chain_rows + 2 * r0, nc, dp_.chain_cols + 2 * c0, Y, V, partial,
-                          panel, dp_.fronts, dp_.rows, stream_);
-        launch_chain_bwd(nrhs, P.chain_bwd_off[l + 1] - i0, Y, panel, chain_inv_, dp_.fronts,
-                         dp_.chain_blk, dp_.chain_bwd + 2 * i0, chain + P.chain_blocks,
-                         chain + 2 * P.chain_blocks + 2 * l + 1, chain_err_, stream_);
-        return nc > 0 ? 4 : 1;
+        launch_chain_cols(nrhs, nr, dp_.chain_rows + 2 * r0, nc, dp_.chain_cols + 2 * c0, (const double*)Y, V, partial,
+                          panel, chain_args(), stream_);
+        launch_chain_bwd(nrhs, P.chain_bwd_off[l + 1] - i0, Y, (const double*)partial, panel, chain_args(),
+                         dp_.chain_bwd + 2 * i0, chain + 4 * P.chain_blocks, chain + 8 * P.chain_blocks + 2 * l + 1,
+                         stream_);
+        return nc > 0 ? 3 : 1;
     }
+    int64_t launches = 0;
     for (int64_t wi = P.wstep_off[l + 1] - 1; wi >= P.wstep_off[l]; wi--) {
         const WStep& w = P.wsteps[wi];
-        if (pf_path(nrhs)) {
-            const int64_t wb_max = std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS);
-            const int nbw_max = (int)((wb_max + NB - 1) / NB), cols = pf_cols(wb_max);
-            if (nrhs == 1) wbwd_pf<T, 1>(w, nbw_max, cols, Y, panel, linv_, dp_, partial, stream_);
-            else if (nrhs == 2) wbwd_pf<T, 2>(w, nbw_max, cols, Y, panel, linv_, dp_, partial, stream_);
-            else if (nrhs == 3) wbwd_pf<T, 3>(w, nbw_max, cols, Y, panel, linv_, dp_, partial, stream_);
-            else wbwd_pf<T, 4>(w, nbw_max, cols, Y, panel, linv_, dp_, partial, stream_);
-            launches += 2;
-        } else if (mr_step(nrhs, P.level_maxk[l], w.S)) {
-            const int64_t wb_max = std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS);
-            const int cols = pf_cols(wb_max);
-            launch_chained(true, k_wbwd_part_mr<T>, (unsigned)(2 * w.n_rows), 256, mr_part_smem(cols, sizeof(T)), stream_, Y,
-                           panel, dp_.fronts, dp_.level_order, w.fr_off, w.nact, dp_.pre_wrows + w.pre_off,
-                           dp_.pre_wpart + w.pre_off, dp_.rows, w.S, nrhs, partial, cols);
-            {
-                cudaLaunchConfig_t cfg{};
-                cfg.gridDim = dim3((unsigned)w.nact, (unsigned)((wb_max * nrhs + 255) / 256));
-                cfg.blockDim = dim3(256);
-                cfg.stream = stream_;
-                cudaLaunchAttribute at[1];
-                at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                at[0].val.programmaticStreamSerializationAllowed = 1;
-                cfg.attrs = at;
-                cfg.numAttrs = pdl_enabled() ? 1 : 0;
-                RFG_CUDA(cudaLaunchKernelEx(&cfg, k_wred, Y, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order,
-                                            w.fr_off, (const int64_t*)(dp_.pre_wrows + w.pre_off),
-                                            (const int64_t*)(dp_.pre_wpart + w.pre_off), w.S, nrhs,
-                                            (const double*)partial));
-            }
-            {
-                // eight right-hand sides per CTA
-                cudaLaunchConfig_t cfg{};
-                cfg.gridDim = dim3((unsigned)w.nact, (unsigned)((nrhs + 7) / 8));
-                cfg.blockDim = dim3(256);
-                cfg.dynamicSmemBytes = mr_diag_smem(8);
-                cfg.stream = stream_;
-                cudaLaunchAttribute at[1];
-                at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                at[0].val.programmaticStreamSerializationAllowed = 1;
-                cfg.attrs = at;
-                cfg.numAttrs = pdl_enabled() ? 1 : 0;
-                RFG_CUDA(cudaLaunchKernelEx(&cfg, k_wbwd_diag_mr<T>, Y, panel, (const double*)linv_,
-                                            (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, w.fr_off, w.S,
-                                            nrhs, 8));
-            }
-            launches += 3;
-        } else {
-            launch_chained(false, k_wbwd<T>, (unsigned)w.n_rows, 256, wbwd_smem<T>(nrhs), stream_, Y, panel, linv_, dp_.fronts,
-                           dp_.level_order, w.fr_off, w.nact, dp_.pre_wrows + w.pre_off, dp_.pre_wpart + w.pre_off,
-                           dp_.rows, w.S, nrhs, partial, tickets);
-            launches++;
-        }
+        const int64_t wb_max = std::max<int64_t>(1, std::min<int64_t>(WS, P.level_maxk[l] - w.S * WS));
+        const int nbw_max = (int)((wb_max + NB - 1) / NB), cols = pf_cols(wb_max);
+        if (nrhs <= PF_MAXR)
+            by_count(nrhs, [&](auto r) {
+                wbwd_pf<T, decltype(r)::value>(w, nbw_max, cols, Y, panel, linv_, d_, dp_, partial, stream_);
+            });
+        else
+            by_count((nrhs + 7) / 8, [&](auto nt) {
+                wbwd_mm<T, decltype(nt)::value>(w, nbw_max, cols, Y, panel, linv_, d_, dp_, partial, nrhs, stream_);
+            });
+        launches += 2;
     }
     return launches;
 }
@@ -1833,23 +1551,11 @@ void Engine::solve_impl(double* X, int64_t nrhs_total) {
         return;
     }
     int nrhs = (int)nrhs_total;
-    RFG_CUDA(cudaMemsetAsync(vupd_, 0, std::max<int64_t>(P.vu_rows * nrhs, 1) * sizeof(double), stream_));
-    int* chain = chain_on(nrhs) ? counters_ + std::max<int64_t>(P.max_nact, 1) : nullptr;
+    int* chain = chain_on(nrhs) ? counters_ : nullptr;
     if (chain) RFG_CUDA(cudaMemsetAsync(chain, 0, chain_flag_words(P) * sizeof(int), stream_));
-    for (int64_t l = 0; l < P.nlevels; l++) {
-        for (int r = 0; r < 2; r++) {
-            const DXadd& x = P.xadd[2 * l + r];
-            if (x.nblk == 0) continue;
-            launch_chained(true, k_vec_extend_add, (unsigned)x.nblk, 256, 0, stream_, X, vupd_, dp_.fronts,
-                           (const int64_t*)(dp_.xadd_task + 4 * x.task_off), x.ntask, (const int32_t*)dp_.emap, nrhs);
-            launches++;
-        }
-        launches += forward_steps<T>(l, X, ybuf_, vupd_, nrhs, chain);
-    }
-    launch_chained(true, k_divide_d, (unsigned)grid_for(P.n * nrhs), 256, 0, stream_, ybuf_, (const double*)d_, P.n, nrhs);
-    launches++;
+    for (int64_t l = 0; l < P.nlevels; l++) launches += forward_steps<T>(l, X, ybuf_, vupd_, nrhs, chain);
     for (int64_t l = P.nlevels - 1; l >= 0; l--)
-        launches += backward_steps<T>(l, ybuf_, vupd_, nrhs, partial_, counters_, chain);
+        launches += backward_steps<T>(l, ybuf_, vupd_, nrhs, partial_, chain);
     RFG_CUDA(cudaMemcpyAsync(X, ybuf_, P.n * nrhs * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
     RFG_CUDA(cudaGetLastError());
     solve_launches += launches;
@@ -1874,15 +1580,6 @@ void solve_set_attributes() {
 }
 
 static void solve_set_attributes_current_device() {
-    RFG_CUDA(cudaFuncSetAttribute(k_wfwd_diag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wfwd_diag_smem<double>(3 * NB, MAXR)));
-    RFG_CUDA(cudaFuncSetAttribute(k_wfwd_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)wfwd_diag_smem<float>(3 * NB, MAXR)));
-    RFG_CUDA(cudaFuncSetAttribute(k_wfwd_rows<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(WS * MAXR * sizeof(double))));
-    RFG_CUDA(cudaFuncSetAttribute(k_wfwd_rows<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(WS * MAXR * sizeof(double))));
-    RFG_CUDA(cudaFuncSetAttribute(k_wbwd<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wbwd_smem<double>(MAXR)));
     auto attr = [](auto kern, size_t bytes) {
         RFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     };
@@ -1896,24 +1593,16 @@ static void solve_set_attributes_current_device() {
         attr(k_wfwd_rows_pf<double, R>, pf_rows_smem<double>(WS, R));
         attr(k_wbwd_part_pf<float, R>, pf_part_smem<float>(WS, R));
         attr(k_wbwd_part_pf<double, R>, pf_part_smem<double>(WS, R));
+        attr(k_mm_fwd_rows<float, R>, mm_rows_smem<float>(WS, R));
+        attr(k_mm_fwd_rows<double, R>, mm_rows_smem<double>(WS, R));
+        attr(k_mm_bwd_part<float, R>, mm_part_smem<float>(WS, R));
+        attr(k_mm_bwd_part<double, R>, mm_part_smem<double>(WS, R));
     };
-    pf_attrs(std::integral_constant<int, 1>());
-    pf_attrs(std::integral_constant<int, 2>());
-    pf_attrs(std::integral_constant<int, 3>());
-    pf_attrs(std::integral_constant<int, 4>());
-    RFG_CUDA(cudaFuncSetAttribute(k_wfwd_rows_mr<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mr_rows_smem(WS, sizeof(float))));
-    RFG_CUDA(cudaFuncSetAttribute(k_wfwd_rows_mr<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mr_rows_smem(WS, sizeof(double))));
-    RFG_CUDA(cudaFuncSetAttribute(k_wbwd_part_mr<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mr_part_smem(WS, sizeof(float))));
-    RFG_CUDA(cudaFuncSetAttribute(k_wbwd_part_mr<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mr_part_smem(WS, sizeof(double))));
-    RFG_CUDA(cudaFuncSetAttribute(k_wbwd_diag_mr<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mr_diag_smem(8)));
-    RFG_CUDA(cudaFuncSetAttribute(k_wbwd_diag_mr<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)mr_diag_smem(8)));
-    RFG_CUDA(cudaFuncSetAttribute(k_wbwd<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wbwd_smem<float>(MAXR)));
+    attr(k_mm_fwd_diag<float>, mm_diag_smem(4));
+    attr(k_mm_fwd_diag<double>, mm_diag_smem(4));
+    attr(k_mm_bwd_diag<float>, mm_diag_smem(4));
+    attr(k_mm_bwd_diag<double>, mm_diag_smem(4));
+    for (int n = 1; n <= 4; n++) by_count(n, pf_attrs);
 }
 
 void Engine::solve_device(double* X, int64_t nrhs, bool allow_graph) {
@@ -1938,8 +1627,7 @@ void Engine::solve_device(double* X, int64_t nrhs, bool allow_graph) {
         vupd_ = (double*)dalloc(std::max<int64_t>(plan_.vu_rows * w, 1) * sizeof(double));
         partial_ = (double*)dalloc(std::max<int64_t>(partial_rows(has_chain()) * w, 1) * sizeof(double));
         ybuf_ = (double*)dalloc(std::max<int64_t>(plan_.n * w, 1) * sizeof(double));
-        counters_ = (int*)dalloc(ticket_words(has_chain()) * sizeof(int));
-        RFG_CUDA(cudaMemsetAsync(counters_, 0, ticket_words(has_chain()) * sizeof(int), stream_));
+        counters_ = (int*)dalloc(flag_words(has_chain()) * sizeof(int));
         ws_nrhs_ = w;
     }
     if (chain_on(nrhs)) ensure_chain_inverse();
@@ -1995,15 +1683,15 @@ int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }
 }  // namespace
 
 bool Engine::chain_on(int64_t nrhs) const {
-    return chain_inv_ != nullptr && nrhs >= 1 && nrhs <= PF_MAXR;
+    return chain_inv_ != nullptr && nrhs >= 1 && nrhs <= MAXR;
 }
 
 int64_t Engine::partial_rows(bool chain) const {
     return std::max<int64_t>(2 * plan_.max_wpart, chain ? plan_.chain_colpart : 0);
 }
 
-int64_t Engine::ticket_words(bool chain) const {
-    return std::max<int64_t>(plan_.max_nact, 1) + (chain ? chain_flag_words(plan_) : 0);
+int64_t Engine::flag_words(bool chain) const {
+    return std::max<int64_t>(1, chain ? chain_flag_words(plan_) : 0);
 }
 
 // The chain blocks' inverses for the current factor: formed by the first sweep after each
@@ -2034,7 +1722,7 @@ void Engine::chain_check() {
 int64_t Engine::sweep_workspace_bytes(int64_t nrhs, bool chain) const {
     const Plan& P = plan_;
     return round256(std::max<int64_t>(P.n * nrhs, 1) * 8) + round256(std::max<int64_t>(P.vu_rows * nrhs, 1) * 8) +
-           round256(std::max<int64_t>(partial_rows(chain) * nrhs, 1) * 8) + round256(ticket_words(chain) * 4);
+           round256(std::max<int64_t>(partial_rows(chain) * nrhs, 1) * 8) + round256(flag_words(chain) * 4);
 }
 
 Engine::SweepWorkspace Engine::carve_sweep_workspace(void* base, int64_t nrhs, bool chain) const {
@@ -2047,7 +1735,7 @@ Engine::SweepWorkspace Engine::carve_sweep_workspace(void* base, int64_t nrhs, b
     p += round256(std::max<int64_t>(P.vu_rows * nrhs, 1) * 8);
     ws.partial = (double*)p;  // two blocks of partials per chunk on the prefetching path
     p += round256(std::max<int64_t>(partial_rows(chain) * nrhs, 1) * 8);
-    ws.tickets = (int*)p;
+    ws.flags = (int*)p;
     ws.chain = chain;
     return ws;
 }
@@ -2057,20 +1745,10 @@ template <typename T>
 void Engine::solve_sweep_impl(double* X, int64_t nrhs_total, const SweepWorkspace& ws) {
     const Plan& P = plan_;
     int nrhs = (int)nrhs_total;
-    RFG_CUDA(cudaMemsetAsync(ws.v, 0, std::max<int64_t>(P.vu_rows * nrhs, 1) * sizeof(double), stream_));
-    RFG_CUDA(cudaMemsetAsync(ws.tickets, 0, ticket_words(ws.chain) * sizeof(int), stream_));
-    int* chain = ws.chain && chain_on(nrhs) ? ws.tickets + std::max<int64_t>(P.max_nact, 1) : nullptr;
-    for (int64_t l = 0; l < P.nlevels; l++) {
-        for (int r = 0; r < 2; r++) {
-            const DXadd& x = P.xadd[2 * l + r];
-            if (x.nblk == 0) continue;
-            launch_chained(true, k_vec_extend_add, (unsigned)x.nblk, 256, 0, stream_, X, ws.v, dp_.fronts,
-                           (const int64_t*)(dp_.xadd_task + 4 * x.task_off), x.ntask, (const int32_t*)dp_.emap, nrhs);
-        }
-        forward_steps<T>(l, X, ws.y, ws.v, nrhs, chain);
-    }
-    launch_chained(true, k_divide_d, (unsigned)grid_for(P.n * nrhs), 256, 0, stream_, ws.y, (const double*)d_, P.n, nrhs);
-    for (int64_t l = P.nlevels - 1; l >= 0; l--) backward_steps<T>(l, ws.y, ws.v, nrhs, ws.partial, ws.tickets, chain);
+    int* chain = ws.chain && chain_on(nrhs) ? ws.flags : nullptr;
+    if (chain) RFG_CUDA(cudaMemsetAsync(chain, 0, chain_flag_words(P) * sizeof(int), stream_));
+    for (int64_t l = 0; l < P.nlevels; l++) forward_steps<T>(l, X, ws.y, ws.v, nrhs, chain);
+    for (int64_t l = P.nlevels - 1; l >= 0; l--) backward_steps<T>(l, ws.y, ws.v, nrhs, ws.partial, chain);
     RFG_CUDA(cudaMemcpyAsync(X, ws.y, P.n * nrhs * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
     RFG_CUDA(cudaGetLastError());
 }

@@ -101,6 +101,18 @@ __device__ __forceinline__ void dmma_884(double& c0, double& c1, double a, doubl
                  : "d"(a), "d"(b));
 }
 
+// x plus the children's update-vector entries of local row p of front f, right-hand side j,
+// child 0 before child 1. imap holds, per front with children, the child row (or −1) of each of
+// its rows for either child.
+__device__ __forceinline__ double kids_add(double x, const double* V, const int32_t* __restrict__ imap,
+                                           const DFront& f, int64_t p, int nrhs, int j) {
+    if (f.imap_off < 0) return x;
+    const int32_t i0 = imap[f.imap_off + p], i1 = imap[f.imap_off + f.m + p];
+    if (i0 >= 0) x += V[(f.kv0 + i0) * nrhs + j];
+    if (i1 >= 0) x += V[(f.kv1 + i1) * nrhs + j];
+    return x;
+}
+
 // Programmatic dependent launch (PDL): a kernel launched with the programmatic
 // stream-serialization attribute may start while its predecessor in the stream still
 // runs. pdl_wait() blocks until the predecessor grid has completed and its memory is
