@@ -11,10 +11,9 @@
 //                       block in shared memory (FP64), with the reference's
 //                       positive definite rule (src/sparse.rs:528-531), and the
 //                       inverse of its unit-lower factor (for panels and solves);
-//        k_panel        PR rows below the block per CTA, as a small GEMM with
-//                       that inverse (FP64 tensor-core path): W = F·L⁻ᵀ,
-//                       L = W·D⁻¹, plus the W and L operands of the Schur update
-//                       in a scratch of NB-wide rows;
+//        k_panel        PNR rows below the block per CTA (FP64 tensor-core path):
+//                       W = F·L⁻ᵀ, L = W·D⁻¹, plus the W and L operands of the Schur
+//                       update in a scratch of NB-wide rows;
 //        k_schur*       lower-triangular tiles of the trailing matrix,
 //                       F −= W·Lᵀ (src/sparse.rs:559-573), written to the panel
 //                       (pivot columns) or the update block (F22): in FP64 on the
@@ -472,57 +471,6 @@ __global__ void __launch_bounds__(PBT, 2) k_pivot_block(T* __restrict__ panel, d
     for (int idx = threadIdx.x; idx < NB * NB; idx += blockDim.x) out[idx] = X[idx / NB][idx % NB];
 }
 
-// Panel of one step as a small GEMM against the inverse of the diagonal block stored by
-// k_pivot_block: for the PR rows r in [j1, m) of a CTA,
-//     W[r, :] = F[r, j0:j1]·L_bb⁻ᵀ,   L[r, :] = W[r, :]·D⁻¹
-// (the forward substitution w ← w·L⁻ᵀ of src/sparse.rs:547-558, applied as a product).
-// L goes to the panel; W and L to the outer block's scratch (front row r is scratch
-// row pre_scr[i] + r − J0, columns j0 − J0 ..); in the tensor-core path also their TF32
-// head and tail. 256 threads; the products run on the FP64 tensor-core path (8 warps of
-// 32 rows × 32 columns, mma.sync m8n8k4 f64) from shared tiles with a row pitch of
-// PNP = NB + 4 doubles (the fragment loads, 8 rows × 4 columns per warp, hit distinct
-// banks in each half-warp); FP64 arithmetic in both precisions.
-constexpr int PNP = NB + 4;
-constexpr size_t PANEL_SMEM = (PR + NB) * PNP * sizeof(double) + NB * sizeof(double) +
-                              NB * sizeof(double) + PR * sizeof(float);  // + FP16 split: D^(1/2) (FP32), row scales
-constexpr size_t PANEL_SMEM_D = PANEL_SMEM + NB * PNP * sizeof(double);  // FP64: + L_bb
-
-// acc[a][c] (+)= ±A·Bᵀ for the warp's 32×32 outputs (rows 32·wm + 8a + g, columns
-// 32·wn + 8c + 2q + {0, 1}), A = [PR][PNP] and B = [NB][PNP] in shared memory, over the
-// columns [0, 4·ksteps) of both.
-template <bool NEG>
-__device__ __forceinline__ void panel_mma(double (&acc)[4][4][2], const double* A, const double* B, int ksteps,
-                                          int wm, int wn, int g, int q) {
-    const double* a0 = A + (wm * 32 + g) * PNP + q;
-    const double* b0 = B + (wn * 32 + g) * PNP + q;
-#pragma unroll 4
-    for (int k = 0; k < 4 * ksteps; k += 4) {
-        double fa[4], fb[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) fa[a] = NEG ? -a0[a * 8 * PNP + k] : a0[a * 8 * PNP + k];
-#pragma unroll
-        for (int c = 0; c < 4; c++) fb[c] = b0[c * 8 * PNP + k];
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) dmma_884(acc[a][c][0], acc[a][c][1], fa[a], fb[c]);
-    }
-}
-
-// The warp's accumulators into the shared tile (columns >= jb as zero).
-__device__ __forceinline__ void panel_store(double* Fs, const double (&acc)[4][4][2], int jb, int wm, int wn, int g,
-                                            int q) {
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int col = wn * 32 + c * 8 + 2 * q + e;
-                Fs[(wm * 32 + a * 8 + g) * PNP + col] = col < jb ? acc[a][c][e] : 0.0;
-            }
-}
-
 // FP16 split of the tensor-core update: the power-of-two scale of a row of U = L·D^(1/2)
 // from the row's diagonal a_rr in the original matrix. Every Schur complement of a
 // positive definite matrix has its diagonal below the original one and U[r, p]² is at
@@ -536,163 +484,264 @@ __device__ __forceinline__ float u16_row_scale(double arr) {
     return (float)ldexp(1.0, 12 - e);
 }
 
-// Rows of a panel CTA after its loads: W = F·L_bb⁻ᵀ over the jb pivots (FP64 panels add
-// one refinement step against L_bb), L = W·D⁻¹, stores: L into the panel, and as the
-// plan's mode says, W and L rows in the storage precision (PANEL_SCR) and the split
-// operands of the tensor cores (PANEL_SPLIT): the TF32 heads and tails of W and L (whi
-// non-null) or the FP16 head and tail of U·s_r = L·D^(1/2)·s_r (uhi non-null; usq the
-// step's D^(1/2) in FP32, rsc the rows' scales s_r, powers of two). U is formed in FP32 from L
-// as stored (one FP64 → FP32 conversion per entry for L and U together: the conversions, not
-// the products, bound these stores). A scaled U entry outside the FP16 range sets *err = 21.
-template <typename T, typename S>
-__device__ __forceinline__ void panel_rows(T* __restrict__ panel, const DFront& f, double* Fs, const double* Li,
-                                           const double* dinv, double* pnl_smem, int64_t r0, int nr, int jb,
-                                           int64_t j0, int64_t J0, int64_t scr0, S* __restrict__ scr_w,
-                                           S* __restrict__ scr_l, float* __restrict__ whi, float* __restrict__ wlo,
-                                           float* __restrict__ lhi, float* __restrict__ llo, bool scr,
-                                           __half* __restrict__ uhi, __half* __restrict__ ulo, const float* usq,
-                                           const float* rsc, int* __restrict__ err) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, q = lane & 3;
-    const int wm = warp & 3, wn = warp >> 2;
-    const bool busy = wm * 32 < nr;  // warps whose rows are all past the chunk's end idle
-    const int ksteps = (jb + 3) / 4;
-    double acc[4][4][2];
+// Panel of one step: for the PNR rows r in [j1, m) of a CTA, W[r, :] = F[r, j0:j1]·L_bb⁻ᵀ and
+// L[r, :] = W[r, :]·D⁻¹ (the forward substitution w ← w·L⁻ᵀ of src/sparse.rs:547-558), on the
+// FP64 tensor-core path (m8n8k4) in both precisions. A warp keeps 16 rows in registers from
+// the load to the store: lane (g, q) holds the columns 16G + 4q ... + 3 of the rows g and 8 + g.
+// The two n-tiles of a 16-column group take the columns 4q + {0, 1} and 4q + {2, 3}, so that
+// a result fragment is an operand fragment of the next product as it stands (the k index runs
+// over q), and loads and stores are four consecutive columns a lane. The other operand
+// (L_bb or its inverse) stands in shared memory in rows of PNP doubles: the 16-byte fragment
+// loads (two rows, four lanes each 32 bytes apart) meet every bank once.
+//   FP32 factor: one product with the FP64 inverse of the block stored by k_pivot_block, groups
+//   on or below the diagonal only;
+//   FP64 factor: substitution by 16-column groups, T = F_b − Σ_{a<b} W_a·L_baᵀ,
+//   W_b = T·L_bb⁻ᵀ with the inverse of the 16 × 16 diagonal block and one refinement step against
+//   that block (R = T − W_b·L_bbᵀ, W_b += R·L_bb⁻ᵀ).
+// L goes to the panel, and as the plan's mode says, W and L rows to the outer block's scratch in
+// the storage precision (PANEL_SCR; front row r is scratch row pre_scr[i] + r − J0, columns
+// j0 − J0 ...) and the split operands of the tensor cores (PANEL_SPLIT): the TF32 heads and
+// tails of W and L (whi non-null) or the FP16 head and tail of U·s_r = L·D^(1/2)·s_r (uhi
+// non-null). U is formed in FP32 from L as stored (one FP64 → FP32 conversion per entry for L
+// and U together). A scaled U entry outside the FP16 range sets *err = 21.
+// Near the top of the tree a launch has a few rows per SM and its time is one CTA's: with 128
+// rows per CTA through shared memory and (FP64) three full 64-column products the panel launches
+// of a factorization took 6.2 ms on the 33³ cube (FP64, 173 launches; now 3.5 ms), 2.8 ms for 160
+// batched plates (0.8 ms) and 17.4 ms on the 60³ cube (mixed, 415 launches; 11.8 ms). At the
+// leaves it is bound by the stores.
+constexpr int PNP = NB + 2;   // pitch of L_bb or its inverse (doubles)
+constexpr int PNI = 18;       // pitch of the 16-column diagonal inverses
+constexpr int PNT = 128;      // threads
+constexpr size_t PANEL_SMEM = NB * PNP * sizeof(double);
+constexpr size_t PANEL_SMEM_D = PANEL_SMEM + NB * PNI * sizeof(double);
+
+// acc (two n-tiles of two row tiles) += ±A·Bᵀ over one 16-column group: A the lane's four values
+// per row tile, B rows at b0 (n-tile 0) and b0 + 2 rows (n-tile 1).
+template <bool NEG, int P>
+__device__ __forceinline__ void panel_group(double (&acc)[2][4], const double (&a)[2][4], const double* b0) {
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int h = 0; h < 2; h++) {
+        const double2 u = *reinterpret_cast<const double2*>(b0 + 2 * h * P);
+        const double2 v = *reinterpret_cast<const double2*>(b0 + 2 * h * P + 2);
+        const double b[4] = {u.x, u.y, v.x, v.y};
 #pragma unroll
-        for (int c = 0; c < 4; c++) acc[a][c][0] = acc[a][c][1] = 0.0;
-    if constexpr (sizeof(T) == sizeof(double)) {
-        // FP64 panels: one refinement step against the triangular system itself,
-        // R = F − W·L_bbᵀ, W += R·L⁻ᵀ, so that W matches forward substitution to
-        // rounding even when the product with the explicit inverse loses digits
-        double* Lb = pnl_smem + (PR + NB) * PNP + NB;
-        const T* blk = panel + f.poff + j0 * f.ldp + j0;
-        for (int idx = threadIdx.x; idx < NB * NB; idx += blockDim.x) {
-            const int p = idx / NB, c = idx - p * NB;
-            Lb[p * PNP + c] = (p < jb && c < p) ? (double)blk[(int64_t)p * f.ldp + c] : (p == c ? 1.0 : 0.0);
-        }
-        double rv[4][4][2];
+        for (int k = 0; k < 4; k++)
 #pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) rv[a][c][e] = Fs[(wm * 32 + a * 8 + g) * PNP + wn * 32 + c * 8 + 2 * q + e];
-        if (busy) panel_mma<false>(acc, Fs, Li, ksteps, wm, wn, g, q);
-        __syncthreads();  // every warp has read F (and Lb is in)
-        panel_store(Fs, acc, jb, wm, wn, g, q);
-        __syncthreads();
-        if (busy) panel_mma<true>(rv, Fs, Lb, ksteps, wm, wn, g, q);
-        __syncthreads();
-        panel_store(Fs, rv, jb, wm, wn, g, q);
-        __syncthreads();
-        if (busy) panel_mma<false>(acc, Fs, Li, ksteps, wm, wn, g, q);
-    } else {
-        if (busy) panel_mma<false>(acc, Fs, Li, ksteps, wm, wn, g, q);
-    }
-    __syncthreads();
-    panel_store(Fs, acc, jb, wm, wn, g, q);
-    __syncthreads();
-    // stores: 16 consecutive columns per half-warp row
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-#pragma unroll
-    for (int a = 0; a < PR / 16; a++) {
-        const int rr = ty + 16 * a;
-        if (rr >= nr) continue;
-        const int64_t r = r0 + rr;
-        const int64_t so = (scr0 + (r - J0)) * NBO + (j0 - J0);
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int p = tx + 16 * c;
-            const double w = Fs[rr * PNP + p], l = w * dinv[p];
-            const T lt = (T)l;
-            if (p < jb) panel[f.poff + r * f.ldp + j0 + p] = lt;
-            if (scr) {
-                scr_w[so + p] = (S)w;
-                scr_l[so + p] = (S)l;
-            }
-            if (whi) {
-                float wf = (float)w, lf = (float)l;
-                float wh = tc::to_tf32(wf), lh = tc::to_tf32(lf);
-                whi[so + p] = wh;
-                wlo[so + p] = tc::to_tf32(wf - wh);
-                lhi[so + p] = lh;
-                llo[so + p] = tc::to_tf32(lf - lh);
-            }
-            if (uhi) {
-                const float u = (float)lt * usq[p] * rsc[rr];
-                const __half h = __float2half_rn(u);
-                uhi[so + p] = h;
-                ulo[so + p] = __float2half_rn(u - __half2float(h));
-                if (!(fabsf(u) < 65504.f)) atomicExch(err, 21);
-            }
-        }
+            for (int m = 0; m < 2; m++)
+                dmma_884(acc[m][2 * h], acc[m][2 * h + 1], NEG ? -a[m][k] : a[m][k], b[k]);
     }
 }
 
-template <typename T, typename S>
-__global__ void __launch_bounds__(256) k_panel(T* __restrict__ panel, const double* __restrict__ d,
+template <typename T>
+__global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const double* __restrict__ d,
                                                const double* __restrict__ linv, const DFront* __restrict__ fr,
                                                const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
                                                const int64_t* __restrict__ pre_panel, const int64_t* __restrict__ pre_scr,
-                                               int64_t s, S* __restrict__ scr_w, S* __restrict__ scr_l,
+                                               int64_t s, T* __restrict__ scr_w, T* __restrict__ scr_l,
                                                const int64_t* __restrict__ status, float* __restrict__ whi,
                                                float* __restrict__ wlo, float* __restrict__ lhi, float* __restrict__ llo,
                                                const uint8_t* __restrict__ mode, const int64_t* __restrict__ rows,
                                                const double* __restrict__ adiag0, __half* __restrict__ uhi,
                                                __half* __restrict__ ulo, float* __restrict__ uscale,
                                                int* __restrict__ err) {
-    extern __shared__ double pnl_smem[];
-    double* Fs = pnl_smem;                // [PR][PNP]
-    double* Li = pnl_smem + PR * PNP;     // [NB][PNP]
-    double* dinv = pnl_smem + (PR + NB) * PNP;
-    int64_t b = blockIdx.x;
-    int64_t i = find_slot_warp(pre_panel, nact, b);
-    int64_t chunk = b - pre_panel[i];
-    int64_t t = order[fr_off + i];
+    extern __shared__ __align__(16) double pnl_smem[];
+    double* Lb = pnl_smem;             // [NB][PNP]: L_bb (FP64) or its inverse
+    double* Iv = pnl_smem + NB * PNP;  // [NB][PNI]: the diagonal 16 × 16 inverses (FP64)
+    __shared__ double dinv[NB];
+    __shared__ float usq[NB];
+    const int64_t i = find_slot_warp(pre_panel, nact, blockIdx.x);
+    const int64_t chunk = blockIdx.x - pre_panel[i];
+    const int64_t t = order[fr_off + i];
     const DFront f = fr[t];
-    int64_t j0 = s * NB;
-    int jb = (int)min((int64_t)NB, f.k - j0);
-    int64_t j1 = j0 + jb;
-    int64_t J0 = (s / KO) * NBO;
-    int64_t r0 = j1 + chunk * PR;
-    int nr = (int)min((int64_t)PR, f.m - r0);
+    const int64_t j0 = s * NB;
+    const int jb = (int)min((int64_t)NB, f.k - j0);
+    const int64_t j1 = j0 + jb;
+    const int64_t J0 = (s / KO) * NBO;
+    const int64_t r0 = j1 + chunk * PNR;
+    const int nr = (int)min((int64_t)PNR, f.m - r0);
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
     // the chunk's rows of the step's columns are final once the update kernel before the
     // pivot kernel has completed, which the pivot kernel waited for before it let this
-    // kernel start (programmatic launch): they are loaded while the pivot block is factored
-    load_tile_p<T, PR, 256, PNP>(Fs, panel + f.poff + r0 * f.ldp + j0, f.ldp, nr, jb);
+    // kernel start (programmatic launch): they are loaded while the pivot block is factored.
+    // A group of four columns that starts below jb ends inside the row's padding (zeros).
+    double F[4][2][4];
+#pragma unroll
+    for (int G = 0; G < 4; G++)
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const int rr = 16 * w + 8 * m + g, c = 16 * G + 4 * q;
+            const bool ok = rr < nr && c < jb;
+            const T* p = panel + f.poff + (r0 + rr) * f.ldp + j0 + c;
+            if constexpr (sizeof(T) == 4) {
+                const float4 v = ok ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+                F[G][m][0] = v.x;
+                F[G][m][1] = v.y;
+                F[G][m][2] = v.z;
+                F[G][m][3] = v.w;
+            } else {
+                const double2 z = make_double2(0.0, 0.0);
+                const double2 u = ok ? *reinterpret_cast<const double2*>(p) : z;
+                const double2 v = ok ? *reinterpret_cast<const double2*>(p + 2) : z;
+                F[G][m][0] = u.x;
+                F[G][m][1] = u.y;
+                F[G][m][2] = v.x;
+                F[G][m][3] = v.y;
+            }
+        }
     // the scratch rows and the split operands only where an update reads them
     const uint8_t md = mode[i];
     if (!(md & PANEL_SPLIT)) {
         whi = nullptr;
         uhi = nullptr;
     }
-    float* usq = reinterpret_cast<float*>(pnl_smem + (PR + NB) * PNP + NB);
-    float* rsc = reinterpret_cast<float*>(pnl_smem + (PR + NB) * PNP + 2 * NB);
-    if (sizeof(T) == sizeof(float) && uhi) {
+    const bool scr = (md & PANEL_SCR) != 0;
+    const int64_t sr0 = pre_scr[i] + (r0 - J0);  // scratch row of the chunk's first row
+    float rsc = 0.f;  // the scale of the warp's row `lane` (lanes 0 .. 15)
+    if (sizeof(T) == sizeof(float) && uhi && lane < 16 && 16 * w + lane < nr) {
         // the rows' scales from their original diagonal (known since the assembly), also
         // kept per scratch row for the tensor-core epilogue: while the pivot block runs
-        const int64_t sr0 = pre_scr[i] + (r0 - J0);
-        for (int rr = threadIdx.x; rr < nr; rr += blockDim.x) {
-            const int64_t r = r0 + rr;
-            const int64_t q = r < f.k ? f.start + r : rows[f.rows_off + r - f.k];
-            const float sc = u16_row_scale(adiag0[q]);
-            if (sc == 0.f) atomicExch(err, 21);
-            uscale[sr0 + rr] = sc;
-            rsc[rr] = sc;
-        }
+        const int64_t r = r0 + 16 * w + lane;
+        rsc = u16_row_scale(adiag0[r < f.k ? f.start + r : rows[f.rows_off + r - f.k]]);
+        if (rsc == 0.f) atomicExch(err, 21);
+        uscale[sr0 + 16 * w + lane] = rsc;
     }
     pdl_wait();
     pdl_launch_dependents();
     if (status[t] != -1) return;
-    load_linv_p<256, PNP>(Li, linv + (f.blk_off + s) * (int64_t)(NB * NB));
-    for (int p = threadIdx.x; p < NB; p += blockDim.x) dinv[p] = p < jb ? 1.0 / d[f.start + j0 + p] : 0.0;
-    if (sizeof(T) == sizeof(float) && uhi)
-        for (int p = threadIdx.x; p < NB; p += blockDim.x) usq[p] = p < jb ? (float)sqrt(d[f.start + j0 + p]) : 0.f;
+    {
+        const double* li = linv + (f.blk_off + s) * (int64_t)(NB * NB);
+        constexpr int PER = NB * NB / 2 / PNT;  // 16-byte loads per thread, all issued before any store
+        double2 v[PER];
+        if constexpr (sizeof(T) == 4) {
+#pragma unroll
+            for (int u = 0; u < PER; u++) v[u] = __ldg(reinterpret_cast<const double2*>(li) + u * PNT + tid);
+        } else {
+            // L_bb: strictly lower from the panel, unit diagonal; rows beyond jb are unit rows
+            const T* blk = panel + f.poff + j0 * f.ldp + j0;
+#pragma unroll
+            for (int u = 0; u < PER; u++) {
+                const int e = 2 * (u * PNT + tid), r = e / NB, c = e % NB;
+                v[u] = r < jb && c < r ? *reinterpret_cast<const double2*>(blk + (int64_t)r * f.ldp + c)
+                                       : make_double2(0.0, 0.0);
+                if (c >= r) v[u].x = c == r ? 1.0 : 0.0;
+                if (c + 1 >= r) v[u].y = c + 1 == r ? 1.0 : 0.0;
+            }
+            for (int e = tid; e < NB * 8; e += PNT) {
+                const int r = e / 8, c = 2 * (e % 8);
+                *reinterpret_cast<double2*>(Iv + r * PNI + c) =
+                    __ldg(reinterpret_cast<const double2*>(li + r * NB + (r & ~15) + c));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int e = 2 * (u * PNT + tid);
+            *reinterpret_cast<double2*>(Lb + (e / NB) * PNP + e % NB) = v[u];
+        }
+    }
+    if (tid < NB) {
+        const double dv = tid < jb ? d[f.start + j0 + tid] : 0.0;
+        dinv[tid] = tid < jb ? 1.0 / dv : 0.0;
+        if (sizeof(T) == sizeof(float)) usq[tid] = tid < jb ? (float)sqrt(dv) : 0.f;
+    }
     __syncthreads();
-    panel_rows<T, S>(panel, f, Fs, Li, dinv, pnl_smem, r0, nr, jb, j0, J0, pre_scr[i], scr_w, scr_l, whi, wlo, lhi,
-                     llo, (md & PANEL_SCR) != 0, uhi, ulo, usq, rsc, err);
+    if (16 * w >= nr) return;
+    const int orow = 4 * (g >> 1) + (g & 1);  // n-tile 0: output column 16G + orow, n-tile 1: + 2
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+        for (int G = 3; G >= 0; G--) {
+            double acc[2][4] = {};
+#pragma unroll
+            for (int a = 0; a <= G; a++) panel_group<false, PNP>(acc, F[a], Lb + (16 * G + orow) * PNP + 16 * a + 4 * q);
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) F[G][m][e] = acc[m][e];
+        }
+    } else {
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            if (16 * b >= jb) break;
+            const double* Lr = Lb + (16 * b + orow) * PNP + 4 * q;
+            const double* Ir = Iv + (16 * b + orow) * PNI + 4 * q;
+#pragma unroll
+            for (int a = 0; a < b; a++) panel_group<true, PNP>(F[b], F[a], Lr + 16 * a);
+            double x[2][4] = {};
+            panel_group<false, PNI>(x, F[b], Ir);
+            panel_group<true, PNP>(F[b], x, Lr + 16 * b);
+            panel_group<false, PNI>(x, F[b], Ir);
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) F[b][m][e] = x[m][e];
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+        const int rr = 16 * w + 8 * m + g;
+        const float rs = __shfl_sync(0xffffffffu, rsc, 8 * m + g);
+        if (rr >= nr) continue;
+        T* prow = panel + f.poff + (r0 + rr) * f.ldp + j0;
+        const int64_t so = (sr0 + rr) * NBO + (j0 - J0);
+#pragma unroll
+        for (int G = 0; G < 4; G++) {
+            const int c = 16 * G + 4 * q;
+            const double(&wv)[4] = F[G][m];
+            double l[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) l[e] = wv[e] * dinv[c + e];
+            if constexpr (sizeof(T) == 4) {
+                const float4 lf = make_float4((float)l[0], (float)l[1], (float)l[2], (float)l[3]);
+                if (c < jb) *reinterpret_cast<float4*>(prow + c) = lf;
+                if (scr) {
+                    *reinterpret_cast<float4*>(scr_l + so + c) = lf;
+                    *reinterpret_cast<float4*>(scr_w + so + c) =
+                        make_float4((float)wv[0], (float)wv[1], (float)wv[2], (float)wv[3]);
+                }
+                const float la[4] = {lf.x, lf.y, lf.z, lf.w};
+                if (whi) {
+                    float wh[4], wl[4], lh[4], ll[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const float wf = (float)wv[e];
+                        wh[e] = tc::to_tf32(wf);
+                        wl[e] = tc::to_tf32(wf - wh[e]);
+                        lh[e] = tc::to_tf32(la[e]);
+                        ll[e] = tc::to_tf32(la[e] - lh[e]);
+                    }
+                    *reinterpret_cast<float4*>(whi + so + c) = make_float4(wh[0], wh[1], wh[2], wh[3]);
+                    *reinterpret_cast<float4*>(wlo + so + c) = make_float4(wl[0], wl[1], wl[2], wl[3]);
+                    *reinterpret_cast<float4*>(lhi + so + c) = make_float4(lh[0], lh[1], lh[2], lh[3]);
+                    *reinterpret_cast<float4*>(llo + so + c) = make_float4(ll[0], ll[1], ll[2], ll[3]);
+                }
+                if (uhi) {
+                    __half2 hi[2], lo[2];
+#pragma unroll
+                    for (int e = 0; e < 4; e += 2) {
+                        const float u0 = la[e] * usq[c + e] * rs, u1 = la[e + 1] * usq[c + e + 1] * rs;
+                        const __half h0 = __float2half_rn(u0), h1 = __float2half_rn(u1);
+                        hi[e / 2] = __halves2half2(h0, h1);
+                        lo[e / 2] = __halves2half2(__float2half_rn(u0 - __half2float(h0)),
+                                                   __float2half_rn(u1 - __half2float(h1)));
+                        if (!(fabsf(u0) < 65504.f) || !(fabsf(u1) < 65504.f)) atomicExch(err, 21);
+                    }
+                    *reinterpret_cast<uint2*>(uhi + so + c) = *reinterpret_cast<const uint2*>(hi);
+                    *reinterpret_cast<uint2*>(ulo + so + c) = *reinterpret_cast<const uint2*>(lo);
+                }
+            } else {
+                const double2 l0 = make_double2(l[0], l[1]), l1 = make_double2(l[2], l[3]);
+                if (c < jb) {
+                    *reinterpret_cast<double2*>(prow + c) = l0;
+                    *reinterpret_cast<double2*>(prow + c + 2) = l1;
+                }
+                if (scr) {
+                    *reinterpret_cast<double2*>(scr_l + so + c) = l0;
+                    *reinterpret_cast<double2*>(scr_l + so + c + 2) = l1;
+                    *reinterpret_cast<double2*>(scr_w + so + c) = make_double2(wv[0], wv[1]);
+                    *reinterpret_cast<double2*>(scr_w + so + c + 2) = make_double2(wv[2], wv[3]);
+                }
+            }
+        }
+    }
 }
 
 // Tile lt of a step's update on the UT×UT grid, with the pivots it applies (kofs, klen:
@@ -1632,8 +1681,8 @@ void Engine::set_attributes() {
     RFG_CUDA(cudaFuncSetAttribute(k_schur_dmma64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D64_SMEM));
     RFG_CUDA(cudaFuncSetAttribute(k_schur_big<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)big_smem<float>()));
-    RFG_CUDA(cudaFuncSetAttribute(k_panel<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM_D));
-    RFG_CUDA(cudaFuncSetAttribute(k_panel<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
+    RFG_CUDA(cudaFuncSetAttribute(k_panel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM_D));
+    RFG_CUDA(cudaFuncSetAttribute(k_panel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
     RFG_CUDA(cudaFuncSetAttribute(k_pivot_block<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
     RFG_CUDA(cudaFuncSetAttribute(k_pivot_block<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
     const size_t s32 = 2 * NB * (UT + 1) * sizeof(float);
@@ -1760,7 +1809,7 @@ void Engine::factor_impl() {
             if (st.n_panel > 0) {
                 // this outer block's buffer of the split operands
                 const int64_t so = use_tc_ ? ((st.s / KO) & 1) * std::max<int64_t>(plan_.max_scr_rows, 1) * NBO : 0;
-                launch_pdl(true, k_panel<T, S>, dim3((unsigned)st.n_panel), dim3(256),
+                launch_pdl(true, k_panel<T>, dim3((unsigned)st.n_panel), dim3(PNT),
                            sizeof(T) == 8 ? PANEL_SMEM_D : PANEL_SMEM, stream_, panel, (const double*)d_,
                            (const double*)linv_, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, st.fr_off,
                            st.nact, (const int64_t*)(dp_.pre_panel + st.pre_off),

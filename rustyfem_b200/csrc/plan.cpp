@@ -282,7 +282,7 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
                 int64_t jb = j1 - j0;
                 int64_t J1e = std::min<int64_t>(J1, d.k);
                 int64_t R = d.m - j1;
-                cp += cdiv(R, PR);
+                cp += cdiv(R, PNR);
                 {
                     // what the panel writes for the inner update of this step and the outer
                     // update of this outer block (rows [J1e, m), decided as below)

@@ -39,7 +39,8 @@ constexpr int NB = 64;        // pivot block width (factor and solve steps)
 constexpr int NBO = 256;      // outer block: pivots applied together to the trailing matrix
 constexpr int KO = NBO / NB;
 constexpr int UT = 64;        // Schur-update tile (UT × UT of F)
-constexpr int PR = 128;       // panel rows per CTA
+constexpr int PR = 128;       // rows of a row chunk of the solve steps
+constexpr int PNR = 64;       // panel rows per CTA
 constexpr int XT = 32;        // factor: tile (XT × XT of a child's update matrix) of one warp of the extend-add
 
 // per-front descriptor used by the kernels (int64 everywhere: offsets exceed 2^31)
