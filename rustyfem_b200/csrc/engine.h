@@ -105,6 +105,7 @@ struct DevPlan {
     int64_t* chain_rows = nullptr;    // Plan::chain_rows
     int64_t* chain_cols = nullptr;    // Plan::chain_cols
     int64_t* chain_colbase = nullptr; // Plan::chain_colbase
+    uint8_t* blk_width = nullptr;     // Plan::blk_width
     int32_t* imap = nullptr;          // per front with children (DFront::imap_off) and child: the child row of each row
 };
 

@@ -9,8 +9,9 @@
 //   3. factored in steps of NB pivots over all fronts of the level at once:
 //        k_pivot_block  one CTA per front: blocked LDLᵀ of the NB×NB diagonal
 //                       block in shared memory (FP64), with the reference's
-//                       positive definite rule (src/sparse.rs:528-531), and the
-//                       inverse of its unit-lower factor (for panels and solves);
+//                       positive definite rule (src/sparse.rs:528-531); the
+//                       blocks' inverses, for the solves, all at the end
+//                       (k_block_inverse);
 //        k_panel        PNR rows below the block per CTA (FP64 tensor-core path):
 //                       W = F·L⁻ᵀ, L = W·D⁻¹, plus the W and L operands of the Schur
 //                       update in a scratch of NB-wide rows;
@@ -162,173 +163,122 @@ __global__ void __launch_bounds__(256, 4) k_extend_add(T* __restrict__ panel, T*
     }
 }
 
-// LDLᵀ of the NB×NB diagonal block [j0, j1) of each active front in FP64 shared memory,
-// with the inverse of its unit lower factor (stored as a full NB×NB block, identity
-// beyond jb) for the panels and the solves. One CTA of PBT threads per front.
-//
-// The block is factored in four sub-panels of SB = 16 pivots. A sub-panel is factored
-// by at most three warps with one row per lane (lanes 0..15 the diagonal sub-block, which
-// every such warp computes, lanes 16..31 sixteen rows below it); within a warp the pivot
-// column is passed through shared memory, so the 16 pivots take no CTA barrier. The
-// sub-panel's rank-16 update of the trailing block is split: its update of the next
-// sub-panel's columns (look-ahead) is applied by all threads right away, the rest by
-// warps 3..7 while the next sub-panel is factored, together with the inverse of the
-// finished diagonal sub-block and the block row of the inverse below it:
-//     X_pp = L_pp⁻¹,   X[p, :p] = −X_pp·(L[p, :p]·X[:p, :p]).
-// This is the factorization of the reference's diagonal block (row by row there,
-// src/sparse.rs:516-537) with the same sums taken in another order; the pivot test
+// LDLᵀ of the NB×NB diagonal block [j0, j1) of each active front in FP64, one CTA of PBT
+// threads per front. A launch is a chain of 64 dependent pivots, so the kernel is built around
+// the length of that chain. The block is factored in sub-panels of PB = 8 pivots. Warps 0 and 1
+// hold one row below the sub-panel's diagonal 8×8 block per lane, and every lane also holds the
+// whole diagonal block and eliminates it for itself: from pivot to pivot there is no exchange,
+// only the reciprocal and one multiply-add on registers. The sub-panel's rank-8 update of the
+// trailing block runs on the FP64 tensor-core path (two m8n8k4 products per 8×8 tile), first for
+// the next sub-panel's columns, then, while the next sub-panel is eliminated, for the rest
+// (warps 2 to 6); warp 7 tests the pivots and inverts the finished 16×16 diagonal blocks. The block's slot of `linv`
+// receives L in FP64 strictly below the diagonal (unit rows beyond jb) and the inverse of each
+// 16×16 diagonal block, transposed, above it: what the panels need. The inverse of the whole
+// block, which only the solves read, is formed for all blocks at once at the end of the numeric
+// phase (k_block_inverse). This is the factorization of the reference's diagonal block (row by
+// row there, src/sparse.rs:516-537) with the same sums taken in another order; the pivot test
 // (src/sparse.rs:528-531) runs on every pivot in order and stops the front at the first
-// failure, recording that equation.
-constexpr int PBT = 256;  // threads of the pivot-block kernel
-constexpr int SB = 16;    // pivots per sub-panel
+// failure, recording that equation. (With 16-pivot sub-panels whose pivot columns went through
+// shared memory, the block's inverse inside and uncoalesced block loads and stores, the pivot
+// launches of a factorization took 4.1 ms on the 33³ cube, 174 of them, 1.47 ms on the 22³ cube
+// and 10.2 ms on the 60³ cube; now 3.0, 1.07 and 8.2 ms with k_block_inverse. A single launch is
+// about 21,000 cycles: 2,800 to load, 1,750 per sub-panel, of which the elimination takes 1,100
+// and the two barriers with the look-ahead between them the rest, 2,800 for the last inverse and
+// the stores.)
+constexpr int PBT = 256;       // threads
+constexpr int PB = 8;          // pivots per sub-panel
+constexpr int SB = 16;         // diagonal blocks inverted for the panels
+constexpr int PBP = NB + 2;    // pitch of the block (doubles)
+constexpr int PBW = 12;        // pitch of the sub-panel operands: conflict-free fragments
+constexpr size_t PB_SMEM = (size_t)(NB * (PBP + 4 * PBW) + SB * PBW) * sizeof(double);
 
-// X_pp = L_pp⁻¹ of the SB×SB diagonal sub-block at cp, one column c per lane:
-// x_r = −Σ_{q<r} L[r][q]·x_q; lanes c ≥ SB store nothing.
-__device__ __forceinline__ void pb_diag_inverse(const double (*A)[NB + 1], double (*X)[NB + 1], int cp, int c) {
-    double xv[SB];
-#pragma unroll
-    for (int r = 0; r < SB; r++) xv[r] = (r == c) ? 1.0 : 0.0;
-#pragma unroll
-    for (int r = 1; r < SB; r++) {
-        double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-        for (int q = 0; q < r; q++) {
-            const double lq = A[cp + r][cp + q];
-            if (q & 1)
-                s1 -= lq * xv[q];
-            else
-                s0 -= lq * xv[q];
-        }
-        if (r > c) xv[r] = s0 + s1;
-    }
-    if (c < SB) {
-#pragma unroll
-        for (int r = 0; r < SB; r++)
-            if (r >= c) X[cp + r][cp + c] = xv[r];
-    }
+// Rank-8 update of the 8×8 tile (ti, tj) of the block: A −= W[ti]·L[tj]ᵀ. All lanes of a warp.
+__device__ __forceinline__ void pb_tile(double* A, const double* W, const double* L, int ti, int tj) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    double2* c = reinterpret_cast<double2*>(A + (8 * ti + g) * PBP + 8 * tj + 2 * q);
+    double2 v = *c;
+    const double* w = W + (8 * ti + g) * PBW + q;
+    const double* l = L + (8 * tj + g) * PBW + q;
+    dmma_884(v.x, v.y, -w[0], l[0]);
+    dmma_884(v.x, v.y, -w[4], l[4]);
+    *c = v;
 }
 
-// Work of warps 3..7 (160 threads) for the finished sub-panel p while sub-panel p+1 is
-// factored: warp 3 inverts the diagonal sub-block; warps 4..7 apply the rest of the
-// sub-panel's trailing update (rows/cols from cp + 2·SB, when a later sub-panel needs it)
-// and Y = −L[p, :p]·X[:p, :p] (X is lower triangular, zero above the diagonal); then all
-// five form X[p, :p] = X_pp·Y.
-__device__ __forceinline__ void pb_group(double (*A)[NB + 1], double (*X)[NB + 1], const double (*Wq)[SB + 1],
-                                         double (*Y)[NB - SB + 1], int p, bool rest) {
-    const int gt = threadIdx.x - 96;
-    const int cp = p * SB;
-    if (gt < 32) {
-        pb_diag_inverse(A, X, cp, gt);
-    } else {
-        const int g4 = gt - 32;  // 0..127
-        if (rest) {
-            const int base = cp + 2 * SB, T = NB - base;
-            const int ty = g4 >> 3, tx = g4 & 7;
-            if (T == 32) {
-                double acc[2][4];
+// The same for the tiles (t0 + i, t0 + j), j <= i < n, numbered along the rows: warp x of PBR
+// takes the tiles x, x + PBR, ..., all operands loaded before any store.
+constexpr int PBR = 5;
+__device__ __noinline__ void pb_rest(double* A, const double* W, const double* L, int t0, int n, int x) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, cnt = n * (n + 1) / 2;
+    constexpr int M = 5;  // 21 tiles at most: n <= 6
+    double2 v[M];
+    double w0[M], w1[M], l0[M], l1[M];
+    int off[M];
 #pragma unroll
-                for (int i = 0; i < 2; i++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++) acc[i][k] = A[base + ty + 16 * i][base + tx + 8 * k];
-#pragma unroll 4
-                for (int q = 0; q < SB; q++) {
-                    double w[2], lv[4];
-#pragma unroll
-                    for (int i = 0; i < 2; i++) w[i] = Wq[base + ty + 16 * i][q];
-#pragma unroll
-                    for (int k = 0; k < 4; k++) lv[k] = A[base + tx + 8 * k][cp + q];
-#pragma unroll
-                    for (int i = 0; i < 2; i++)
-#pragma unroll
-                        for (int k = 0; k < 4; k++) acc[i][k] -= w[i] * lv[k];
-                }
-#pragma unroll
-                for (int i = 0; i < 2; i++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        if (ty + 16 * i >= tx + 8 * k) A[base + ty + 16 * i][base + tx + 8 * k] = acc[i][k];
-            } else if (T == 16) {
-                double acc[2];
-#pragma unroll
-                for (int k = 0; k < 2; k++) acc[k] = A[base + ty][base + tx + 8 * k];
-#pragma unroll 4
-                for (int q = 0; q < SB; q++) {
-                    const double w = Wq[base + ty][q];
-#pragma unroll
-                    for (int k = 0; k < 2; k++) acc[k] -= w * A[base + tx + 8 * k][cp + q];
-                }
-#pragma unroll
-                for (int k = 0; k < 2; k++)
-                    if (ty >= tx + 8 * k) A[base + ty][base + tx + 8 * k] = acc[k];
-            }
-        }
-        if (p > 0) {
-            const int rr = g4 & 15, cg = g4 >> 4;  // columns cg + 8m
-            double acc[6][2];
-#pragma unroll
-            for (int m = 0; m < 6; m++) acc[m][0] = acc[m][1] = 0.0;
-            for (int q = 0; q < cp; q += 2) {
-                const double l0 = A[cp + rr][q], l1 = A[cp + rr][q + 1];
-#pragma unroll
-                for (int m = 0; m < 6; m++)
-                    if (8 * m < cp) {
-                        acc[m][0] -= l0 * X[q][cg + 8 * m];
-                        acc[m][1] -= l1 * X[q + 1][cg + 8 * m];
-                    }
-            }
-#pragma unroll
-            for (int m = 0; m < 6; m++)
-                if (8 * m < cp) Y[rr][cg + 8 * m] = acc[m][0] + acc[m][1];
-        }
+    for (int u = 0; u < M; u++) {
+        const int e = x + PBR * u;
+        if (e >= cnt) continue;
+        const int i = (e >= 1) + (e >= 3) + (e >= 6) + (e >= 10) + (e >= 15), j = e - i * (i + 1) / 2;
+        off[u] = (8 * (t0 + i) + g) * PBP + 8 * (t0 + j) + 2 * q;
+        v[u] = *reinterpret_cast<const double2*>(A + off[u]);
+        const double* w = W + (8 * (t0 + i) + g) * PBW + q;
+        const double* l = L + (8 * (t0 + j) + g) * PBW + q;
+        w0[u] = -w[0];
+        w1[u] = -w[4];
+        l0[u] = l[0];
+        l1[u] = l[4];
     }
-    asm volatile("bar.sync 1, 160;" ::: "memory");  // warps 3..7 only
-    if (p > 0) {
-        for (int idx = gt; idx < SB * cp; idx += 160) {
-            const int rr = idx & 15, c = idx >> 4;
-            double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-            for (int q = 0; q < SB; q += 2) {
-                s0 += X[cp + rr][cp + q] * Y[q][c];
-                s1 += X[cp + rr][cp + q + 1] * Y[q + 1][c];
-            }
-            X[cp + rr][c] = s0 + s1;
+    for (int u = 0; u < M; u++)
+        if (x + PBR * u < cnt) dmma_884(v[u].x, v[u].y, w0[u], l0[u]);
+#pragma unroll
+    for (int u = 0; u < M; u++)
+        if (x + PBR * u < cnt) {
+            dmma_884(v[u].x, v[u].y, w1[u], l1[u]);
+            *reinterpret_cast<double2*>(A + off[u]) = v[u];
         }
-    }
 }
 
-// The last sub-panel's block row of the inverse, with the whole CTA: warp 0 the diagonal
-// sub-block, warps 2..7 Y (four columns cg + 12m each), then X[p, :p] = X_pp·Y.
-__device__ __forceinline__ void pb_final(const double (*A)[NB + 1], double (*X)[NB + 1], double (*Y)[NB - SB + 1],
-                                         int p) {
-    const int cp = p * SB;
-    if (threadIdx.x < 32) {
-        pb_diag_inverse(A, X, cp, threadIdx.x);
-    } else if (threadIdx.x >= 64 && p > 0) {
-        const int g = threadIdx.x - 64, rr = g & 15, cg = g >> 4;
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int q = 0; q < cp; q++) {
-            const double l = A[cp + rr][q];
+// Inverse of the unit lower SB×SB diagonal block at cp into the upper half of the slot,
+// transposed (out[cp + c][cp + r] = X[r][c]), by one warp: the two 8×8 diagonal inverses a column
+// per lane (lanes 0 .. 15), then X21 = −X22·(L21·X11) as two tensor-core products. S: a work tile
+// of SB rows of PBW doubles.
+__device__ __noinline__ void pb_diag_inverse(const double* A, double* S, double* out, int cp) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    if (lane < SB) {
+        const int c = lane & 7, b8 = cp + (lane & 8);
+        double x[PB];
 #pragma unroll
-            for (int m = 0; m < 4; m++)
-                if (12 * m < cp) acc[m] -= l * X[q][cg + 12 * m];
+        for (int r = 0; r < PB; r++) {
+            double v = r == c ? 1.0 : 0.0;
+#pragma unroll
+            for (int k = 0; k < r; k++) v -= A[(b8 + r) * PBP + b8 + k] * x[k];
+            x[r] = v;  // zero above the diagonal: x[k] = 0 for k < c
         }
 #pragma unroll
-        for (int m = 0; m < 4; m++)
-            if (cg + 12 * m < cp) Y[rr][cg + 12 * m] = acc[m];
-    }
-    __syncthreads();
-    if (p > 0) {
-        for (int idx = threadIdx.x; idx < SB * cp; idx += PBT) {
-            const int rr = idx & 15, c = idx >> 4;
-            double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int q = 0; q < SB; q += 2) {
-                s0 += X[cp + rr][cp + q] * Y[q][c];
-                s1 += X[cp + rr][cp + q + 1] * Y[q + 1][c];
-            }
-            X[cp + rr][c] = s0 + s1;
+        for (int r = 0; r < PB; r++) {
+            S[((lane & 8) + r) * PBW + c] = x[r];
+            if (r > c) out[(b8 + c) * NB + b8 + r] = x[r];
         }
     }
+    __syncwarp();
+    const double* l = A + (cp + PB + g) * PBP + cp + q;
+    double y0 = 0.0, y1 = 0.0;
+    dmma_884(y0, y1, l[0], S[q * PBW + g]);
+    dmma_884(y0, y1, l[4], S[(q + 4) * PBW + g]);
+    // Y as the right operand: Y[k][n] is in lane 4k + n/2, element n & 1
+    double b[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int src = 4 * (q + 4 * h) + (g >> 1);
+        const double v0 = __shfl_sync(0xffffffffu, y0, src), v1 = __shfl_sync(0xffffffffu, y1, src);
+        b[h] = g & 1 ? v1 : v0;
+    }
+    double x0 = 0.0, x1 = 0.0;
+    dmma_884(x0, x1, -S[(PB + g) * PBW + q], b[0]);
+    dmma_884(x0, x1, -S[(PB + g) * PBW + q + 4], b[1]);
+    out[(cp + 2 * q) * NB + cp + PB + g] = x0;
+    out[(cp + 2 * q + 1) * NB + cp + PB + g] = x1;
+    __syncwarp();  // S is read
 }
 
 template <typename T>
@@ -337,138 +287,250 @@ __global__ void __launch_bounds__(PBT, 2) k_pivot_block(T* __restrict__ panel, d
                                                         const DFront* __restrict__ fr, const int64_t* __restrict__ order,
                                                         int64_t fr_off, int64_t s, int64_t* __restrict__ status,
                                                         double* __restrict__ linv) {
-    pdl_wait();  // wait first: a dependent launched early may then read our inputs
-    pdl_launch_dependents();
-    extern __shared__ double pb_smem[];
-    double(*A)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(pb_smem);
-    double(*X)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(pb_smem + NB * (NB + 1));
-    __shared__ double Wp[2][NB][SB + 1];        // unscaled W = L·D of the last two sub-panels
-    __shared__ double Y[SB][NB - SB + 1];       // a block row of the inverse before X_pp
-    __shared__ __align__(16) double colbuf[3][2][SB];  // pivot column of the sub-panel warps
+    extern __shared__ __align__(16) double pb_smem[];
+    double* A = pb_smem;                // [NB][PBP]
+    double* Wq = pb_smem + NB * PBP;    // [2][NB][PBW]: the sub-panel's W = L·D and L rows, by parity
+    double* Lq = Wq + 2 * NB * PBW;     // [2][NB][PBW]
+    double* Sv = Lq + 2 * NB * PBW;     // [SB][PBW]: work tile of the inverses
     __shared__ double orig[NB];
-    __shared__ int failed;
+    __shared__ int bad;                 // first pivot of the block that breaks the rule, or NB
     const int64_t t = order[fr_off + blockIdx.x];
-    if (status[t] != -1) return;
     const DFront f = fr[t];
+    pdl_wait();
+    pdl_launch_dependents();
+    if (status[t] != -1) return;
     const int64_t j0 = s * NB;
-    const int jb = (int)min((int64_t)NB, f.k - j0);
+    const int jb = (int)min((int64_t)NB, f.k - j0), nsp = (jb + PB - 1) / PB;
     T* blk = panel + f.poff + j0 * f.ldp + j0;
-    {
-        // each thread loads EPT consecutive entries of one row (all issued before any
-        // store); rows beyond jb get a unit diagonal so the sub-panels need no bounds
-        constexpr int EPT = NB * NB / PBT, TPR = NB / EPT;
-        const int r = threadIdx.x / TPR, c0 = (threadIdx.x % TPR) * EPT;
-        T v[EPT];
-#pragma unroll
-        for (int e = 0; e < EPT; e++) {
-            const int c = c0 + e;
-            v[e] = (r < jb && c <= r) ? blk[(int64_t)r * f.ldp + c] : T(0);
-        }
-#pragma unroll
-        for (int e = 0; e < EPT; e++) {
-            const int c = c0 + e;
-            A[r][c] = (r >= jb && c == r) ? 1.0 : (double)v[e];
-            X[r][c] = (r == c) ? 1.0 : 0.0;
-        }
-    }
-    for (int p = threadIdx.x; p < jb; p += blockDim.x) orig[p] = adiag[f.start + j0 + p];
-    if (threadIdx.x == 0) failed = 0;
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nsub = (jb + SB - 1) / SB;
-    for (int b = 0; b < nsub; b++) {
-        const int c0 = b * SB;
-        const int nbelow = NB - c0 - SB;
-        const int nw = nbelow > 0 ? (nbelow + 15) / 16 : 1;
-        if (warp < nw) {
-            const bool dlane = lane < SB;
-            const int r = dlane ? c0 + lane : c0 + SB + warp * 16 + (lane - 16);
-            const bool live = r < NB;
-            double(*Wb)[SB + 1] = Wp[b & 1];
-            double a[SB];  // row r, columns c0 .. c0+SB−1
-#pragma unroll
-            for (int c = 0; c < SB; c++) a[c] = live ? A[r][c0 + c] : 0.0;
-#pragma unroll
-            for (int jj = 0; jj < SB; jj++) {
-                // column jj of the diagonal sub-block (final after pivot jj−1) to every
-                // lane; two buffers by parity, so one __syncwarp per pivot suffices
-                double* cb = colbuf[warp][jj & 1];
-                if (dlane && lane >= jj) cb[lane] = a[jj];
-                __syncwarp();
-                double acj[SB];
-#pragma unroll
-                for (int c = jj & ~1; c < SB; c += 2) {
-                    const double2 v = *reinterpret_cast<const double2*>(cb + c);
-                    acj[c] = v.x;
-                    acj[c + 1] = v.y;
-                }
-                const double piv = acj[jj];
-                const int j = c0 + jj;
-                if (j < jb && (!(orig[j] > 0.0) || !(piv > 1e-12 * orig[j]))) {
-                    if (warp == 0 && lane == 0) {
-                        failed = 1;
-                        status[t] = f.start + j0 + j;
-                    }
-                    break;
-                }
-                if (warp == 0 && lane == jj && j < jb) d[f.start + j0 + j] = piv;
-                const double l = a[jj] * recip_newton(piv);  // piv > 0, tested above
-                if (!dlane || lane > jj) {
-#pragma unroll
-                    for (int c = jj + 1; c < SB; c++) a[c] -= l * acj[c];
-                    if (live) Wb[r][jj] = a[jj];
-                    a[jj] = l;
-                }
-            }
-            if (live && (!dlane || warp == 0)) {
-#pragma unroll
-                for (int c = 0; c < SB; c++)
-                    if (!dlane || c <= lane) A[r][c0 + c] = a[c];
-            }
-        } else if (warp >= 3 && b > 0) {
-            pb_group(A, X, Wp[(b - 1) & 1], Y, b - 1, b + 1 < nsub);
-        }
-        __syncthreads();
-        if (failed) return;
-        if (b + 1 < nsub) {
-            // look-ahead: this sub-panel's update of the next sub-panel's columns
-            const int cn = c0 + SB, R = NB - cn;
-            const int cc = threadIdx.x & 15, rg = threadIdx.x >> 4;
-            const int c = cn + cc;
-            const double(*Wb)[SB + 1] = Wp[b & 1];
-            double lv[SB];
-#pragma unroll
-            for (int q = 0; q < SB; q++) lv[q] = A[c][c0 + q];
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                const int r = cn + rg + 16 * i;
-                if (16 * i < R && r >= c) {
-                    double s0 = A[r][c], s1 = 0.0;
-#pragma unroll
-                    for (int q = 0; q < SB; q += 2) {
-                        s0 -= Wb[r][q] * lv[q];
-                        s1 -= Wb[r][q + 1] * lv[q + 1];
-                    }
-                    A[r][c] = s0 + s1;
-                }
-            }
-        }
-        __syncthreads();
-    }
-    pb_final(A, X, Y, nsub - 1);
-    __syncthreads();
-    {
-        constexpr int EPT = NB * NB / PBT, TPR = NB / EPT;
-        const int r = threadIdx.x / TPR, c0 = (threadIdx.x % TPR) * EPT;
-        if (r < jb)
-#pragma unroll
-            for (int e = 0; e < EPT; e++) {
-                const int c = c0 + e;
-                if (c <= r) blk[(int64_t)r * f.ldp + c] = (T)A[r][c];
-            }
-    }
     double* out = linv + (f.blk_off + s) * (int64_t)(NB * NB);
-    for (int idx = threadIdx.x; idx < NB * NB; idx += blockDim.x) out[idx] = X[idx / NB][idx % NB];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    using VT = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+    {
+        // warp w: rows w, w + 8, ... (two columns per lane, all loads issued before any store).
+        // Rows and columns beyond jb get a unit diagonal so the sub-panels need no bounds
+        VT v[NB / 8];
+#pragma unroll
+        for (int i = 0; i < NB / 8; i++) {
+            const int r = warp + 8 * i;
+            v[i] = VT{};
+            if (r < jb && 2 * lane <= r) v[i] = *reinterpret_cast<const VT*>(blk + (int64_t)r * f.ldp + 2 * lane);
+        }
+        for (int p = tid; p < NB; p += PBT) orig[p] = p < jb ? adiag[f.start + j0 + p] : 1.0;
+        if (tid == 0) bad = NB;
+#pragma unroll
+        for (int i = 0; i < NB / 8; i++) {
+            const int r = warp + 8 * i, c = 2 * lane;
+            double2 w = make_double2((double)v[i].x, (double)v[i].y);
+            if (r >= jb && c == r) w.x = 1.0;
+            if (r >= jb && c + 1 == r) w.y = 1.0;
+            *reinterpret_cast<double2*>(A + r * PBP + c) = w;
+        }
+    }
+    __syncthreads();
+    for (int b = 0; b < nsp; b++) {
+        const int c0 = b * PB;
+        double* const W = Wq + (b & 1) * NB * PBW;
+        double* const L = Lq + (b & 1) * NB * PBW;
+        if (warp < 2) {
+            // lane: row c0 + 8 + tid below the diagonal block (rows past the block idle along)
+            const int r = c0 + PB + tid;
+            const bool live = r < NB;
+            double D[PB][PB], a[PB];
+            double* const wr = W + (live ? r : c0) * PBW;  // an idle lane's entries are read by nobody
+#pragma unroll
+            for (int i = 0; i < PB; i++)
+#pragma unroll
+                for (int k = 0; k <= i; k += 2) {
+                    const double2 v = *reinterpret_cast<const double2*>(A + (c0 + i) * PBP + c0 + k);
+                    D[i][k] = v.x;
+                    if (k + 1 <= i) D[i][k + 1] = v.y;
+                }
+            const double* row = A + (live ? r : c0) * PBP + c0;
+#pragma unroll
+            for (int k = 0; k < PB; k += 2) {
+                const double2 v = *reinterpret_cast<const double2*>(row + k);
+                a[k] = v.x;
+                a[k + 1] = v.y;
+            }
+            // the eight pivots without a branch: the rule is checked on all of them afterwards (a
+            // bad pivot spoils only values that nobody reads, the front stops here)
+#pragma unroll
+            for (int j = 0; j < PB; j++) {
+                const double rinv = recip_newton(D[j][j]);
+                double l[PB];
+#pragma unroll
+                for (int i = j + 1; i < PB; i++) {
+                    l[i] = D[i][j] * rinv;
+#pragma unroll
+                    for (int k = j + 1; k <= i; k++) D[i][k] -= l[i] * D[k][j];
+                }
+                wr[j] = a[j];
+                a[j] *= rinv;
+#pragma unroll
+                for (int k = j + 1; k < PB; k++) a[k] -= a[j] * D[k][j];
+#pragma unroll
+                for (int i = j + 1; i < PB; i++) D[i][j] = l[i];
+            }
+            if (live) {
+                double* const ar = A + r * PBP + c0;
+                double* const lr = L + r * PBW;
+#pragma unroll
+                for (int k = 0; k < PB; k += 2) {
+                    const double2 v = make_double2(a[k], a[k + 1]);
+                    *reinterpret_cast<double2*>(ar + k) = v;
+                    *reinterpret_cast<double2*>(lr + k) = v;
+                }
+            }
+            if (tid == 32) {
+#pragma unroll
+                for (int i = 0; i < PB; i++)
+#pragma unroll
+                    for (int k = 0; k <= i; k += 2) {
+                        if (k + 1 <= i)
+                            *reinterpret_cast<double2*>(A + (c0 + i) * PBP + c0 + k) = make_double2(D[i][k], D[i][k + 1]);
+                        else
+                            A[(c0 + i) * PBP + c0 + k] = D[i][k];
+                    }
+            }
+        } else if (b > 0) {
+            // the previous sub-panel's update right of this one, and the finished inverses
+            const double* Wp = Wq + ((b - 1) & 1) * NB * PBW;
+            const double* Lp = Lq + ((b - 1) & 1) * NB * PBW;
+            if (warp == 7) {
+                if ((b & 1) == 0) pb_diag_inverse(A, Sv, out, (b - 2) * PB);
+            } else {
+                pb_rest(A, Wp, Lp, b + 1, nsp - b - 1, warp - 2);
+            }
+        }
+        __syncthreads();
+        // look-ahead: this sub-panel's update of the next one's columns; warp 7, which has none of it,
+        // tests the sub-panel's pivots
+        if (warp < 7) {
+            if (b + 1 + warp < nsp) pb_tile(A, W, L, b + 1 + warp, b + 1);
+        } else {
+            const int p = c0 + lane;
+            const bool mine = lane < PB && p < jb;
+            const double pv = mine ? A[p * PBP + p] : 1.0, o = mine ? orig[p] : 1.0;
+            const unsigned fail = __ballot_sync(0xffffffffu, !(o > 0.0) || !(pv > 1e-12 * o));
+            const int first = fail ? c0 + __ffs(fail) - 1 : NB;
+            if (mine && p < first) d[f.start + j0 + p] = pv;
+            if (fail && lane == 0) {
+                bad = first;
+                status[t] = f.start + j0 + first;
+            }
+        }
+        __syncthreads();
+        if (bad < NB) return;
+    }
+    // the last 16×16 block's inverse beside the stores of L: the slot's rows and columns of whole
+    // 16×16 blocks (beyond them the slot is the identity since the engine was set up)
+    const int nd = (jb + SB - 1) / SB * SB;
+    if (warp == 0) {
+        pb_diag_inverse(A, Sv, out, nd - SB);
+    } else {
+        const int c = 2 * lane;
+#pragma unroll
+        for (int i = 0; i < (NB + 6) / 7; i++) {
+            const int r = warp - 1 + 7 * i;
+            if (r >= nd || c > r) continue;
+            const double2 w = *reinterpret_cast<const double2*>(A + r * PBP + c);
+            if (r < jb) {
+                T* const o = blk + (int64_t)r * f.ldp + c;
+                if (c + 1 <= r) {
+                    VT v;
+                    v.x = (T)w.x;
+                    v.y = (T)w.y;
+                    *reinterpret_cast<VT*>(o) = v;
+                } else {
+                    o[0] = (T)w.x;
+                }
+            }
+            if (c + 1 < r) {
+                *reinterpret_cast<double2*>(out + r * NB + c) = w;
+            } else if (c < r) {
+                out[r * NB + c] = w.x;
+            }
+        }
+    }
+}
+
+// Unit lower slots (the identity): rows and columns that no block fills stay so.
+__global__ void k_slot_identity(double* __restrict__ linv) {
+    double* slot = linv + blockIdx.x * (int64_t)(NB * NB);
+    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) slot[e] = e / NB == e % NB ? 1.0 : 0.0;
+}
+
+// The slots of linv from L and the transposed 16×16 inverses (k_pivot_block) to the inverses of
+// the whole blocks (lower triangular, zeros above), which the solves read: by block rows,
+// X_pp given, X[p, :p] = −X_pp·(L[p, :p]·X[:p, :p]). One CTA of four warps per slot, products on the
+// FP64 tensor-core path, only the 16×16 blocks that hold pivots (width[slot] pivots); bound by the
+// bytes a slot reads and writes.
+constexpr int BIP = NB + 4;
+constexpr size_t BI_SMEM = (size_t)(2 * NB + SB) * BIP * sizeof(double);
+__global__ void __launch_bounds__(128) k_block_inverse(double* __restrict__ linv, const uint8_t* __restrict__ width) {
+    extern __shared__ __align__(16) double bi_smem[];
+    double* L = bi_smem;             // [NB][BIP]
+    double* X = bi_smem + NB * BIP;  // [NB][BIP]
+    double* Y = X + NB * BIP;        // [SB][BIP]
+    double* slot = linv + blockIdx.x * (int64_t)(NB * NB);
+    const int nb = (width[blockIdx.x] + SB - 1) / SB, nd = nb * SB;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    pdl_wait();
+    pdl_launch_dependents();
+    for (int r = w; r < nd; r += 4) {
+        const int c = 2 * lane;
+        if (c >= nd) continue;
+        const double2 v = *reinterpret_cast<const double2*>(slot + r * NB + c);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const double x = u ? v.y : v.x;
+            const int cc = c + u;
+            L[r * BIP + cc] = cc < r ? x : 0.0;
+            // a diagonal 16×16 block holds its inverse transposed above the diagonal
+            if ((cc ^ r) < SB)
+                X[cc * BIP + r] = cc > r ? x : (cc == r ? 1.0 : 0.0);
+            else if (cc > r)
+                X[r * BIP + cc] = 0.0;
+        }
+    }
+    __syncthreads();
+    for (int p = 1; p < nb; p++) {
+        const int cp = p * SB;
+        // 8×8 tiles: two tile rows, 2p tile columns, of which warp w takes w and w + 4
+        for (int ct = w; ct < 2 * p; ct += 4) {
+            double acc[2][2] = {};
+            for (int k = (ct & ~1) * 8; k < cp; k += 4) {  // X is zero above its diagonal blocks
+                const double b = X[(k + q) * BIP + 8 * ct + g];
+#pragma unroll
+                for (int m = 0; m < 2; m++) dmma_884(acc[m][0], acc[m][1], L[(cp + 8 * m + g) * BIP + k + q], b);
+            }
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                Y[(8 * m + g) * BIP + 8 * ct + 2 * q] = acc[m][0];
+                Y[(8 * m + g) * BIP + 8 * ct + 2 * q + 1] = acc[m][1];
+            }
+        }
+        __syncwarp();  // a warp's columns of Y are its own
+        for (int ct = w; ct < 2 * p; ct += 4) {
+            double acc[2][2] = {};
+#pragma unroll
+            for (int k = 0; k < SB; k += 4) {
+                const double b = Y[(k + q) * BIP + 8 * ct + g];
+#pragma unroll
+                for (int m = 0; m < 2; m++) dmma_884(acc[m][0], acc[m][1], X[(cp + 8 * m + g) * BIP + cp + k + q], b);
+            }
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                X[(cp + 8 * m + g) * BIP + 8 * ct + 2 * q] = -acc[m][0];
+                X[(cp + 8 * m + g) * BIP + 8 * ct + 2 * q + 1] = -acc[m][1];
+            }
+        }
+        __syncthreads();
+    }
+    for (int r = w; r < nd; r += 4) {
+        const int c = 2 * lane;
+        if (c < nd) *reinterpret_cast<double2*>(slot + r * NB + c) = *reinterpret_cast<const double2*>(X + r * BIP + c);
+    }
 }
 
 // FP16 split of the tensor-core update: the power-of-two scale of a row of U = L·D^(1/2)
@@ -491,13 +553,11 @@ __device__ __forceinline__ float u16_row_scale(double arr) {
 // The two n-tiles of a 16-column group take the columns 4q + {0, 1} and 4q + {2, 3}, so that
 // a result fragment is an operand fragment of the next product as it stands (the k index runs
 // over q), and loads and stores are four consecutive columns a lane. The other operand
-// (L_bb or its inverse) stands in shared memory in rows of PNP doubles: the 16-byte fragment
+// stands in shared memory in rows of PNP doubles: the 16-byte fragment
 // loads (two rows, four lanes each 32 bytes apart) meet every bank once.
-//   FP32 factor: one product with the FP64 inverse of the block stored by k_pivot_block, groups
-//   on or below the diagonal only;
-//   FP64 factor: substitution by 16-column groups, T = F_b − Σ_{a<b} W_a·L_baᵀ,
-//   W_b = T·L_bb⁻ᵀ with the inverse of the 16 × 16 diagonal block and one refinement step against
-//   that block (R = T − W_b·L_bbᵀ, W_b += R·L_bb⁻ᵀ).
+// The substitution goes by 16-column groups, T = F_b − Σ_{a<b} W_a·L_baᵀ, W_b = T·L_bb⁻ᵀ with the
+// inverse of the 16 × 16 diagonal block, and for an FP64 factor one refinement step against that
+// block (R = T − W_b·L_bbᵀ, W_b += R·L_bb⁻ᵀ).
 // L goes to the panel, and as the plan's mode says, W and L rows to the outer block's scratch in
 // the storage precision (PANEL_SCR; front row r is scratch row pre_scr[i] + r − J0, columns
 // j0 − J0 ...) and the split operands of the tensor cores (PANEL_SPLIT): the TF32 heads and
@@ -509,11 +569,10 @@ __device__ __forceinline__ float u16_row_scale(double arr) {
 // of a factorization took 6.2 ms on the 33³ cube (FP64, 173 launches; now 3.5 ms), 2.8 ms for 160
 // batched plates (0.8 ms) and 17.4 ms on the 60³ cube (mixed, 415 launches; 11.8 ms). At the
 // leaves it is bound by the stores.
-constexpr int PNP = NB + 2;   // pitch of L_bb or its inverse (doubles)
+constexpr int PNP = NB + 2;   // pitch of L_bb (doubles)
 constexpr int PNI = 18;       // pitch of the 16-column diagonal inverses
 constexpr int PNT = 128;      // threads
-constexpr size_t PANEL_SMEM = NB * PNP * sizeof(double);
-constexpr size_t PANEL_SMEM_D = PANEL_SMEM + NB * PNI * sizeof(double);
+constexpr size_t PANEL_SMEM = NB * (PNP + PNI) * sizeof(double);
 
 // acc (two n-tiles of two row tiles) += ±A·Bᵀ over one 16-column group: A the lane's four values
 // per row tile, B rows at b0 (n-tile 0) and b0 + 2 rows (n-tile 1).
@@ -545,8 +604,8 @@ __global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const doub
                                                __half* __restrict__ ulo, float* __restrict__ uscale,
                                                int* __restrict__ err) {
     extern __shared__ __align__(16) double pnl_smem[];
-    double* Lb = pnl_smem;             // [NB][PNP]: L_bb (FP64) or its inverse
-    double* Iv = pnl_smem + NB * PNP;  // [NB][PNI]: the diagonal 16 × 16 inverses (FP64)
+    double* Lb = pnl_smem;             // [NB][PNP]: L_bb
+    double* Iv = pnl_smem + NB * PNP;  // [NB][PNI]: the inverses of its 16 × 16 diagonal blocks
     __shared__ double dinv[NB];
     __shared__ float usq[NB];
     const int64_t i = find_slot_warp(pre_panel, nact, blockIdx.x);
@@ -609,33 +668,23 @@ __global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const doub
     pdl_launch_dependents();
     if (status[t] != -1) return;
     {
+        // the block's slot: L strictly below the diagonal, the 16 × 16 inverses transposed above
         const double* li = linv + (f.blk_off + s) * (int64_t)(NB * NB);
         constexpr int PER = NB * NB / 2 / PNT;  // 16-byte loads per thread, all issued before any store
         double2 v[PER];
-        if constexpr (sizeof(T) == 4) {
 #pragma unroll
-            for (int u = 0; u < PER; u++) v[u] = __ldg(reinterpret_cast<const double2*>(li) + u * PNT + tid);
-        } else {
-            // L_bb: strictly lower from the panel, unit diagonal; rows beyond jb are unit rows
-            const T* blk = panel + f.poff + j0 * f.ldp + j0;
-#pragma unroll
-            for (int u = 0; u < PER; u++) {
-                const int e = 2 * (u * PNT + tid), r = e / NB, c = e % NB;
-                v[u] = r < jb && c < r ? *reinterpret_cast<const double2*>(blk + (int64_t)r * f.ldp + c)
-                                       : make_double2(0.0, 0.0);
-                if (c >= r) v[u].x = c == r ? 1.0 : 0.0;
-                if (c + 1 >= r) v[u].y = c + 1 == r ? 1.0 : 0.0;
-            }
-            for (int e = tid; e < NB * 8; e += PNT) {
-                const int r = e / 8, c = 2 * (e % 8);
-                *reinterpret_cast<double2*>(Iv + r * PNI + c) =
-                    __ldg(reinterpret_cast<const double2*>(li + r * NB + (r & ~15) + c));
-            }
-        }
+        for (int u = 0; u < PER; u++) v[u] = __ldg(reinterpret_cast<const double2*>(li) + u * PNT + tid);
 #pragma unroll
         for (int u = 0; u < PER; u++) {
-            const int e = 2 * (u * PNT + tid);
-            *reinterpret_cast<double2*>(Lb + (e / NB) * PNP + e % NB) = v[u];
+            const int e = 2 * (u * PNT + tid), r = e / NB, c = e % NB;
+            double2 l = v[u];
+            if (c >= r) l.x = c == r ? 1.0 : 0.0;
+            if (c + 1 >= r) l.y = c + 1 == r ? 1.0 : 0.0;
+            *reinterpret_cast<double2*>(Lb + r * PNP + c) = l;
+            if ((c ^ r) < 16) {
+                Iv[c * PNI + (r & 15)] = c > r ? v[u].x : (c == r ? 1.0 : 0.0);
+                Iv[(c + 1) * PNI + (r & 15)] = c + 1 > r ? v[u].y : (c + 1 == r ? 1.0 : 0.0);
+            }
         }
     }
     if (tid < NB) {
@@ -646,34 +695,23 @@ __global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const doub
     __syncthreads();
     if (16 * w >= nr) return;
     const int orow = 4 * (g >> 1) + (g & 1);  // n-tile 0: output column 16G + orow, n-tile 1: + 2
-    if constexpr (sizeof(T) == 4) {
 #pragma unroll
-        for (int G = 3; G >= 0; G--) {
-            double acc[2][4] = {};
+    for (int b = 0; b < 4; b++) {
+        if (16 * b >= jb) break;
+        const double* Lr = Lb + (16 * b + orow) * PNP + 4 * q;
+        const double* Ir = Iv + (16 * b + orow) * PNI + 4 * q;
 #pragma unroll
-            for (int a = 0; a <= G; a++) panel_group<false, PNP>(acc, F[a], Lb + (16 * G + orow) * PNP + 16 * a + 4 * q);
-#pragma unroll
-            for (int m = 0; m < 2; m++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) F[G][m][e] = acc[m][e];
-        }
-    } else {
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-            if (16 * b >= jb) break;
-            const double* Lr = Lb + (16 * b + orow) * PNP + 4 * q;
-            const double* Ir = Iv + (16 * b + orow) * PNI + 4 * q;
-#pragma unroll
-            for (int a = 0; a < b; a++) panel_group<true, PNP>(F[b], F[a], Lr + 16 * a);
-            double x[2][4] = {};
-            panel_group<false, PNI>(x, F[b], Ir);
+        for (int a = 0; a < b; a++) panel_group<true, PNP>(F[b], F[a], Lr + 16 * a);
+        double x[2][4] = {};
+        panel_group<false, PNI>(x, F[b], Ir);
+        if constexpr (sizeof(T) == 8) {
             panel_group<true, PNP>(F[b], x, Lr + 16 * b);
             panel_group<false, PNI>(x, F[b], Ir);
-#pragma unroll
-            for (int m = 0; m < 2; m++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) F[b][m][e] = x[m][e];
         }
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) F[b][m][e] = x[m][e];
     }
 #pragma unroll
     for (int m = 0; m < 2; m++) {
@@ -865,8 +903,6 @@ __global__ void __launch_bounds__(256) k_schur(T* __restrict__ panel, T* __restr
         }
     }
 }
-
-constexpr size_t PB_SMEM = 2 * NB * (NB + 1) * sizeof(double);
 
 // Outer update of large fronts on the CUDA cores: 128×128 tiles (the tile grid of the
 // tensor-core kernel), 256 threads with 8×8 outputs each, K in chunks of 16 through
@@ -1456,6 +1492,7 @@ void Engine::upload_plan() {
     dp_.chain_rows = up(plan_.chain_rows);
     dp_.chain_cols = up(plan_.chain_cols);
     dp_.chain_colbase = up(plan_.chain_colbase);
+    dp_.blk_width = up(plan_.blk_width);
     // the child row of each front row, for either child: the inverse of emap, on the device
     dp_.imap = (int32_t*)dalloc(std::max<int64_t>(plan_.imap_elems, 1) * sizeof(int32_t));
     RFG_CUDA(cudaMemsetAsync(dp_.imap, 0xff, std::max<int64_t>(plan_.imap_elems, 1) * sizeof(int32_t), stream_));
@@ -1633,6 +1670,10 @@ void Engine::init(bool) {
     scr_l_ = dalloc(std::max<int64_t>(plan_.max_scr_rows, 1) * NBO * es);
     d_ = (double*)dalloc(std::max<int64_t>(plan_.n, 1) * sizeof(double));
     linv_ = (double*)dalloc(std::max<int64_t>(plan_.nblocks, 1) * NB * NB * sizeof(double));
+    if (plan_.nblocks > 0) {
+        k_slot_identity<<<(unsigned)plan_.nblocks, 256, 0, stream_>>>(linv_);
+        RFG_CUDA(cudaGetLastError());
+    }
     if (plan_.chain_blocks > 0) {
         chain_inv_ = (double*)dalloc(plan_.chain_blocks * (int64_t)WS * WS * sizeof(double));
         chain_err_ = (int*)dalloc(sizeof(int));
@@ -1681,10 +1722,11 @@ void Engine::set_attributes() {
     RFG_CUDA(cudaFuncSetAttribute(k_schur_dmma64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D64_SMEM));
     RFG_CUDA(cudaFuncSetAttribute(k_schur_big<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)big_smem<float>()));
-    RFG_CUDA(cudaFuncSetAttribute(k_panel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM_D));
+    RFG_CUDA(cudaFuncSetAttribute(k_panel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
     RFG_CUDA(cudaFuncSetAttribute(k_panel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
     RFG_CUDA(cudaFuncSetAttribute(k_pivot_block<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
     RFG_CUDA(cudaFuncSetAttribute(k_pivot_block<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PB_SMEM));
+    RFG_CUDA(cudaFuncSetAttribute(k_block_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BI_SMEM));
     const size_t s32 = 2 * NB * (UT + 1) * sizeof(float);
     RFG_CUDA(cudaFuncSetAttribute(k_schur<float, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s32));
     RFG_CUDA(cudaFuncSetAttribute(k_schur<float, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s32));
@@ -1810,7 +1852,7 @@ void Engine::factor_impl() {
                 // this outer block's buffer of the split operands
                 const int64_t so = use_tc_ ? ((st.s / KO) & 1) * std::max<int64_t>(plan_.max_scr_rows, 1) * NBO : 0;
                 launch_pdl(true, k_panel<T>, dim3((unsigned)st.n_panel), dim3(PNT),
-                           sizeof(T) == 8 ? PANEL_SMEM_D : PANEL_SMEM, stream_, panel, (const double*)d_,
+                           PANEL_SMEM, stream_, panel, (const double*)d_,
                            (const double*)linv_, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, st.fr_off,
                            st.nact, (const int64_t*)(dp_.pre_panel + st.pre_off),
                            (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, sw, sl, (const int64_t*)status_,
@@ -1884,6 +1926,12 @@ void Engine::factor_impl() {
                 }
             }
         }
+    }
+    if (P.nblocks > 0) {
+        launch_pdl(true, k_block_inverse, dim3((unsigned)P.nblocks), dim3(128), BI_SMEM, stream_, linv_,
+                   (const uint8_t*)dp_.blk_width);
+        launches++;
+        mark(2);
     }
     RFG_CUDA(cudaGetLastError());
     last_factor.launches = launches;

@@ -151,6 +151,9 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
     P.panel_elems = poff;
     P.vu_rows = vu;
     P.nblocks = nblk;
+    P.blk_width.assign(nblk, (uint8_t)NB);
+    for (const DFront& d : P.fronts)
+        if (d.k % NB) P.blk_width[d.blk_off + d.k / NB] = (uint8_t)(d.k % NB);
     timer.lap("descriptors");
     // update arena with reuse: U_t lives from level(t) to level(parent(t))
     {

@@ -175,6 +175,7 @@ struct Plan {
     int64_t max_scr_rows = 0;           // largest scratch over all steps
     int64_t max_nact = 0;               // largest number of active fronts of a step
     int64_t nblocks = 0;                // NB×NB diagonal blocks of all fronts
+    std::vector<uint8_t> blk_width;     // their pivots (NB but for a front's last block)
     std::vector<int64_t> front_of_dof;  // front owning each equation
     double work = 0.0;
     double inner_flops = 0.0, outer_flops = 0.0;  // Σ over all steps

@@ -79,18 +79,16 @@ __device__ __forceinline__ void load_linv(double (*dst)[NB + 1], const double* _
     load_linv_p<NT, NB + 1>(&dst[0][0], src);
 }
 
-// 1/p for a positive normal p: Newton–Raphson iteration on f(r) = 1/r − p,
-// r ← r + r·(1 − p·r), from the hardware's approximate reciprocal (rcp.approx.ftz.f64, a
-// relative error near 2^-23); each step squares the relative error, so two steps leave the
-// rounding of the last fused multiply-add: within one unit in the last place of 1/p. Several
-// times shorter as a dependency chain than the IEEE division 1.0 / p.
+// 1/p for a positive normal p, from the hardware's approximate reciprocal r0
+// (rcp.approx.ftz.f64): with e = 1 − p·r0, 1/p = r0/(1 − e) = r0·(1 + e + e² + ...); r0 has a relative error
+// near 2^-23, so the terms past e² are below 2^-68 and the rounding of the last fused
+// multiply-add is left: within one unit in the last place of 1/p. Three dependent operations
+// after r0, a fraction of the IEEE division's chain.
 __device__ __forceinline__ double recip_newton(double p) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(p));
-    double e = fma(-p, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-p, r, 1.0);
-    return fma(r, e, r);
+    const double e = fma(-p, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 }
 
 // D = A·B + D on the FP64 tensor-core path for one 8×8×4 block (mma.sync m8n8k4 f64):
