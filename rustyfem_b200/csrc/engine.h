@@ -88,8 +88,7 @@ struct DevPlan {
     uint8_t* panel_mode = nullptr;    // Plan::panel_mode
     uint8_t* outer_mode = nullptr;    // Plan::outer_mode
     int64_t* pre_scr = nullptr;
-    int64_t* xadd_child = nullptr;
-    int64_t* xadd_fpre = nullptr;
+    int64_t* asm_pre = nullptr;       // Plan::asm_pre
     int64_t* pre_wrows = nullptr;
     int64_t* pre_wpart = nullptr;
     int64_t* rows = nullptr;
@@ -237,13 +236,12 @@ class Engine {
     void launch_schur_tc_inner(const DStep& st);
 
     Plan plan_;
-    Scatter scatter_;  // host lists (level_seg, front_seg kept; dst/src released after upload)
+    Scatter scatter_;  // host lists (front_seg kept; dst/src released after upload)
     int64_t nseg_ = 0;  // scatter segments (entries read from the caller's values)
     int64_t nsrc_;
     Precision prec_;
     cudaStream_t stream_ = nullptr;
     DevPlan dp_;
-    std::vector<int64_t> level_poff_;  // panel-arena range of each level
     void* panel_ = nullptr;
     void* upd_ = nullptr;
     void* scr_w_ = nullptr;

@@ -1,12 +1,11 @@
 // Numeric phase of the multifrontal LDLᵀ on the GPU (sm_100a).
 //
 // Level by level (see plan.h), each level of the elimination tree is
-//   1. zero-filled (its panel range with one memset, its update blocks by kernel),
-//   2. assembled: original entries stored into the panels (k_scatter), the
-//      original diagonal captured for the pivot test (k_capture_diag), then the
-//      children's update matrices added in child order (k_extend_add, one launch
-//      per child rank, so no two CTAs add into the same entry),
-//   3. factored in steps of NB pivots over all fronts of the level at once:
+//   1. assembled: the children's update matrices gathered into its fronts in child
+//      order (k_assemble); before the first level the panels of all levels are
+//      zeroed, the original entries stored (k_scatter) and the original diagonal
+//      captured for the pivot test (k_capture_diag),
+//   2. factored in steps of NB pivots over all fronts of the level at once:
 //        k_pivot_block  one CTA per front: blocked LDLᵀ of the NB×NB diagonal
 //                       block in shared memory (FP64), with the reference's
 //                       positive definite rule (src/sparse.rs:528-531); the
@@ -71,95 +70,121 @@ __global__ void k_capture_diag(const T* __restrict__ panel, double* __restrict__
     for (int64_t i = threadIdx.x; i < f.k; i += blockDim.x) adiag[f.start + i] = (double)panel[f.poff + i * f.ldp + i];
 }
 
-// zero the lower triangle of the update blocks of a level: warp w of block (i, y) clears
-// rows 8y + w, 8y + w + 8·gridDim.y, ... of front order[lo + i], its lanes in 16-byte stores
-// along the row (rows are 16-byte aligned and ldu ≥ ⌈u⌉₈, so rounding a row's length up
-// stays inside the row); gridDim.y follows the level's largest update block
-template <typename T>
-__global__ void k_zero_update(T* __restrict__ upd, const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                              int64_t lo) {
-    pdl_wait();  // wait first: a dependent launched early may then read our inputs
-    pdl_launch_dependents();
-    using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-    constexpr int VEC = 16 / (int)sizeof(T);
-    const DFront f = fr[order[lo + blockIdx.x]];
-    const V z{};
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int64_t x = (int64_t)blockIdx.y * 8 + warp; x < f.u; x += (int64_t)gridDim.y * 8) {
-        V* row = reinterpret_cast<V*>(upd + f.uoff + x * f.ldu);
-        for (int64_t y = lane; y * VEC <= x; y += 32) row[y] = z;
+// Children's update matrices into the fronts of a level, by gathering: the lower triangle of a
+// front is cut into XT × XT tiles (the update block's triangle alone for a front without
+// children), one warp per tile and eight tiles per CTA, lane l takes column C0 + l of the
+// tile's rows. imap gives the child row (or none) of each front row; the maps grow with the
+// row, so a child's entry (x, y), y <= x, lies in the front's lower triangle too. An update-block
+// entry is written once (child 0 + child 1, zeros where there is neither), a panel entry gets
+// both children on top of the original entry, and only where one of them has something. The
+// least traffic is each child entry read once and each update entry written once; what bounds
+// the kernel is the latency of the rows' loads, so every lane first asks for one row's part of
+// the children (the whole tile on its way into L2), six CTAs fit on an SM, a lane without a
+// child column reads a zero at stride 0 instead of a predicate, and a tile that only one child
+// reaches leaves the other out. (Zeroing, then one read-modify-write pass per child, took, with
+// the original entries stored level by level, 14.5 ms of a 60³ mixed factorization, 8.7 ms of a
+// 45³ FP64 one, 1.17 ms of 160 batched plates and 0.44 ms of a 9³ one; now 11.4, 5.8, 0.66 and
+// 0.19 ms. Two columns per lane with four CTAs per SM were as fast at 60³ and slower below.)
+static __device__ double g_zero = 0.0;
+
+template <typename T, bool PANEL, bool K0, bool K1>
+__device__ __forceinline__ void asm_rows(T* col, const T* p0, const T* p1, int s0, int s1, bool put, int cr, int ld,
+                                         int nr, int32_t r0, int32_t r1) {
+    constexpr int U = 4;
+    for (int x0 = 0; x0 < nr; x0 += U) {
+        T v0[U], v1[U], old[U];
+        bool some[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            // rows past the tile have no child row (r0 = r1 = -1)
+            const int32_t a0 = K0 ? __shfl_sync(0xffffffffu, r0, (x0 + u) & (XT - 1)) : -1;
+            const int32_t a1 = K1 ? __shfl_sync(0xffffffffu, r1, (x0 + u) & (XT - 1)) : -1;
+            some[u] = a0 >= 0 || a1 >= 0;
+            v0[u] = K0 && a0 >= 0 ? p0[(int64_t)a0 * s0] : T(0);
+            v1[u] = K1 && a1 >= 0 ? p1[(int64_t)a1 * s1] : T(0);
+            if (PANEL) old[u] = put && some[u] ? col[(int64_t)(x0 + u) * ld] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (put && (!PANEL || some[u]) && x0 + u >= cr && x0 + u < nr)
+                col[(int64_t)(x0 + u) * ld] = PANEL ? (old[u] + v0[u]) + v1[u] : v0[u] + v1[u];
     }
 }
 
-// F_parent[emap[x], emap[y]] += U_child[x, y] for y <= x, one launch per child rank. The
-// child's lower triangle is cut into XT × XT tiles (tile rows by tile columns, row-major
-// over the lower triangle), one warp per tile and eight tiles per CTA: lane l takes column
-// Y0 + l of the tile's rows (the child row read as one 128-byte segment, the parent's
-// column index once per tile, the parent rows of the tile's rows shuffled from one load),
-// eight rows in flight before any store; no per-row pointers are held, so four CTAs fit
-// on an SM. Child and parent
-// never overlap, and no two lanes of a launch touch one entry.
+// The part [lo, hi] of a child's row of this lane into L2, lo and hi over the warp's columns.
 template <typename T>
-__global__ void __launch_bounds__(256, 4) k_extend_add(T* __restrict__ panel, T* __restrict__ upd,
-                                                    const DFront* __restrict__ fr, const int64_t* __restrict__ child,
-                                                    const int64_t* __restrict__ pre, int64_t nchild,
-                                                    const int32_t* __restrict__ emap, int64_t* __restrict__ status) {
-    pdl_wait();  // wait first: a dependent launched early may then read our inputs
-    pdl_launch_dependents();
-    int64_t b = blockIdx.x;
-    int64_t i = find_slot_warp(pre, nchild, b);
-    int64_t c = child[i];
-    int64_t chunk = b - pre[i];
-    const DFront fc = fr[c];
-    const DFront fp = fr[fc.parent];
-    if (status[c] != -1) {
-        if (chunk == 0 && threadIdx.x == 0) status[fc.parent] = -2;  // an ancestor of a failed front
-        return;
-    }
+__device__ __forceinline__ void asm_prefetch(const T* base, int64_t ldu, int32_t row, int32_t c) {
+    const int lo = (int)__reduce_min_sync(0xffffffffu, (uint32_t)c), hi = __reduce_max_sync(0xffffffffu, c);
+    if (row < 0) return;
+    const char* p = reinterpret_cast<const char*>(base + row * ldu + lo);
+    const char* e = reinterpret_cast<const char*>(base + row * ldu + hi);
+    for (; p <= e; p += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 6) k_assemble(T* __restrict__ panel, T* __restrict__ upd,
+                                                     const DFront* __restrict__ fr, const int64_t* __restrict__ order,
+                                                     const int64_t* __restrict__ pre, int64_t nfronts,
+                                                     const int32_t* __restrict__ imap, int64_t* __restrict__ status) {
+    const int64_t i = find_slot_warp(pre, nfronts, blockIdx.x);
+    const int64_t t = order[i], chunk = blockIdx.x - pre[i];
+    const DFront f = fr[t];
+    const bool kids = f.imap_off >= 0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nt = (fc.u + XT - 1) / XT;
-    const int64_t lt = chunk * 8 + warp;
-    if (lt >= nt * (nt + 1) / 2) return;
+    const int64_t base = kids ? 0 : f.k;  // first row and column of the tile grid
+    const int64_t nt = (f.m - base + XT - 1) / XT, lt = chunk * 8 + warp;
     int64_t ti = (int64_t)((sqrt(8.0 * (double)lt + 1.0) - 1.0) * 0.5);
     while (ti * (ti + 1) / 2 > lt) ti--;
     while ((ti + 1) * (ti + 2) / 2 <= lt) ti++;
     const int64_t tj = lt - ti * (ti + 1) / 2;
-    const int32_t* em = emap + fc.emap_off;
-    const int64_t y = tj * XT + lane;
-    const int64_t py = y < fc.u ? em[y] : -1;
-    const int64_t X0 = ti * XT, X1 = min(fc.u, X0 + XT);
-    // the parent rows of the tile's rows, one per lane, handed out by shuffles: the
-    // parent's loads do not wait for a load of the map
-    const int32_t emx = X0 + lane < X1 ? em[X0 + lane] : 0;
-    // this lane's parent column: in a panel row (column py) or in an update-block row
-    // (column py − k); a parent row px starts at pcol + (px − pshift)·pld
-    const bool in_panel = py < fp.k;
-    T* const pcol = in_panel ? panel + fp.poff + py : upd + fp.uoff + (py - fp.k);
-    const int64_t pld = in_panel ? fp.ldp : fp.ldu, pshift = in_panel ? 0 : fp.k;
-    const T* ucol = upd + fc.uoff + y;
-    constexpr int U = 8;
-    for (int64_t x0 = X0; x0 < X1; x0 += U) {
-        T v[U], old[U];
-        uint32_t okm = 0;  // bit u: row x0 + u is added by this lane
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int64_t x = x0 + u;
-            const bool ok = x < X1 && py >= 0 && y <= x;
-            okm |= (uint32_t)ok << u;
-            v[u] = ok ? ucol[x * fc.ldu] : T(0);
-        }
-        // the parent row offsets are shuffled again for the loads and for the stores
-        // instead of being held in registers across them
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int64_t px = __shfl_sync(0xffffffffu, emx, (int)(x0 + u - X0) & (XT - 1));
-            old[u] = (okm >> u) & 1u ? pcol[(px - pshift) * pld] : T(0);
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int64_t px = __shfl_sync(0xffffffffu, emx, (int)(x0 + u - X0) & (XT - 1));
-            if ((okm >> u) & 1u) pcol[(px - pshift) * pld] = old[u] + v[u];
-        }
+    const int64_t R0 = base + ti * XT, R1 = min(f.m, R0 + XT), c = base + tj * XT + lane;
+    const bool in = lt < nt * (nt + 1) / 2;
+    // the children's rows of this lane's column and of the tile's rows (one per lane, handed
+    // out by shuffles)
+    int32_t c0 = -1, c1 = -1, r0 = -1, r1 = -1;
+    DFront k0{}, k1{};
+    if (kids && f.kid0 >= 0) k0 = fr[f.kid0];
+    if (kids && f.kid1 >= 0) k1 = fr[f.kid1];
+    if (kids && in && c < f.m) {
+        c0 = imap[f.imap_off + c];
+        c1 = imap[f.imap_off + f.m + c];
+    }
+    if (kids && in && R0 + lane < R1) {
+        r0 = imap[f.imap_off + R0 + lane];
+        r1 = imap[f.imap_off + f.m + R0 + lane];
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    if (kids && ((f.kid0 >= 0 && status[f.kid0] != -1) || (f.kid1 >= 0 && status[f.kid1] != -1))) {
+        if (chunk == 0 && threadIdx.x == 0) status[t] = -2;  // an ancestor of a failed front
+        return;
+    }
+    if (!in) return;
+    const int nr = (int)(R1 - R0), cr = (int)min(c - R0, (int64_t)XT);  // this lane's rows start at cr
+    const bool any0 = __any_sync(0xffffffffu, c0 >= 0) && __any_sync(0xffffffffu, r0 >= 0);
+    const bool any1 = __any_sync(0xffffffffu, c1 >= 0) && __any_sync(0xffffffffu, r1 >= 0);
+    if (any0) asm_prefetch(upd + k0.uoff, k0.ldu, r0, c0);
+    if (any1) asm_prefetch(upd + k1.uoff, k1.ldu, r1, c1);
+    const T* const zero = reinterpret_cast<const T*>(&g_zero);
+    const T* const p0 = c0 >= 0 ? upd + k0.uoff + c0 : zero;
+    const T* const p1 = c1 >= 0 ? upd + k1.uoff + c1 : zero;
+    const int s0 = c0 >= 0 ? (int)k0.ldu : 0, s1 = c1 >= 0 ? (int)k1.ldu : 0;
+    // the tile's columns in the panel, then those in the update block (a tile on the border
+    // takes both passes)
+    if (c - lane < f.k && (any0 || any1))
+        asm_rows<T, true, true, true>(panel + f.poff + R0 * f.ldp + c, p0, p1, s0, s1,
+                                      c < f.k && (c0 >= 0 || c1 >= 0), cr, (int)f.ldp, nr, r0, r1);
+    if (c - lane + XT > f.k && R1 > f.k) {
+        T* const col = upd + f.uoff + (R0 - f.k) * f.ldu + (c - f.k);
+        const bool put = c >= f.k;
+        if (any0 && any1)
+            asm_rows<T, false, true, true>(col, p0, p1, s0, s1, put, cr, (int)f.ldu, nr, r0, r1);
+        else if (any0)
+            asm_rows<T, false, true, false>(col, p0, p1, s0, s1, put, cr, (int)f.ldu, nr, r0, r1);
+        else if (any1)
+            asm_rows<T, false, false, true>(col, p0, p1, s0, s1, put, cr, (int)f.ldu, nr, r0, r1);
+        else
+            asm_rows<T, false, false, false>(col, p0, p1, s0, s1, put, cr, (int)f.ldu, nr, r0, r1);
     }
 }
 
@@ -1481,8 +1506,7 @@ void Engine::upload_plan() {
     dp_.pre_scr = up(plan_.pre_scr);
     dp_.panel_mode = up(plan_.panel_mode);
     dp_.outer_mode = up(plan_.outer_mode);
-    dp_.xadd_child = up(plan_.xadd_child);
-    dp_.xadd_fpre = up(plan_.xadd_fpre);
+    dp_.asm_pre = up(plan_.asm_pre);
     dp_.rows = up(plan_.rows);
     dp_.emap = up(plan_.emap);
     dp_.chain_blk = up(plan_.chain_blk);
@@ -1500,11 +1524,6 @@ void Engine::upload_plan() {
         k_imap_fill<<<(unsigned)plan_.nfronts, 128, 0, stream_>>>(dp_.fronts, dp_.emap, dp_.imap);
         RFG_CUDA(cudaGetLastError());
     }
-    level_poff_.assign(plan_.nlevels + 1, plan_.panel_elems);
-    for (int64_t l = 0; l < plan_.nlevels; l++)
-        if (plan_.level_off[l + 1] > plan_.level_off[l]) level_poff_[l] = plan_.fronts[plan_.level_order[plan_.level_off[l]]].poff;
-    for (int64_t l = plan_.nlevels - 1; l >= 0; l--)
-        if (plan_.level_off[l + 1] == plan_.level_off[l]) level_poff_[l] = level_poff_[l + 1];
 }
 
 // The host scatter lists on the device; the host copies of the per-entry lists are
@@ -1632,8 +1651,6 @@ void Engine::build_scatter_device(const CallerPattern& cp) {
     if (!in_arena) dev_free(base, stream_);
     RFG_CUDA(cudaStreamSynchronize(stream_));
     if (flag & 2) throw CudaError("build_scatter_device: an entry's row is not in its front (symbolic mismatch)");
-    scatter_.level_seg.assign(P.nlevels + 1, 0);
-    for (int64_t l = 0; l <= P.nlevels; l++) scatter_.level_seg[l] = scatter_.front_seg[P.level_off[l]];
 }
 
 Engine::Engine(Plan&& plan, Scatter&& scatter, int64_t nsrc, Precision prec, bool use_tc)
@@ -1809,35 +1826,29 @@ void Engine::factor_impl() {
             launches++;
         }
     }
+    if (P.panel_elems > 0) RFG_CUDA(cudaMemsetAsync(panel, 0, P.panel_elems * sizeof(T), stream_));
+    mark(0);
+    if (nseg_ > 0) {
+        const int64_t nb = std::min<int64_t>((nseg_ + 255) / 256, 148 * 16);
+        launch_pdl(true, k_scatter<T>, dim3((unsigned)nb), dim3(256), 0, stream_, panel, (const double*)src_,
+                   (const int64_t*)dp_.seg_dst, (const int64_t*)dp_.seg_ptr, (const int64_t*)dp_.seg_src, (int64_t)0,
+                   nseg_);
+        launches++;
+        mark(0);
+    }
+    if (P.nfronts > 0) {
+        launch_pdl(true, k_capture_diag<T>, dim3((unsigned)P.nfronts), dim3(128), 0, stream_, (const T*)panel, adiag_,
+                   (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, (int64_t)0);
+        launches++;
+        mark(0);
+    }
     for (int64_t l = 0; l < P.nlevels; l++) {
-        int64_t lo = P.level_off[l], nl = P.level_off[l + 1] - lo;
+        const int64_t lo = P.level_off[l], nl = P.level_off[l + 1] - lo;
         if (nl == 0) continue;
-        int64_t pbytes = (level_poff_[l + 1] - level_poff_[l]) * sizeof(T);
-        if (pbytes > 0) RFG_CUDA(cudaMemsetAsync(panel + level_poff_[l], 0, pbytes, stream_));
-        int64_t maxu = 0;
-        for (int64_t i = lo; i < lo + nl; i++) maxu = std::max(maxu, P.fronts[P.level_order[i]].u);
-        const unsigned zy = (unsigned)std::min<int64_t>(256, std::max<int64_t>(1, (maxu + 31) / 32));
-        launch_pdl(true, k_zero_update<T>, dim3((unsigned)nl, zy), dim3(256), 0, stream_, upd,
-                   (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, lo);
-        mark(0);
-        int64_t s0 = scatter_.level_seg[l], s1 = scatter_.level_seg[l + 1];
-        if (s1 > s0) {
-            int64_t nb = std::min<int64_t>((s1 - s0 + 255) / 256, 148 * 16);
-            launch_pdl(true, k_scatter<T>, dim3((unsigned)nb), dim3(256), 0, stream_, panel, (const double*)src_,
-                       (const int64_t*)dp_.seg_dst, (const int64_t*)dp_.seg_ptr, (const int64_t*)dp_.seg_src, s0, s1);
-            launches++;
-            mark(0);
-        }
-        launch_pdl(true, k_capture_diag<T>, dim3((unsigned)nl), dim3(128), 0, stream_, (const T*)panel, adiag_,
-                   (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, lo);
-        launches += 2;
-        mark(0);
-        for (int r = 0; r < 2; r++) {
-            const DXadd& x = P.xadd[2 * l + r];
-            if (x.fnblk == 0) continue;
-            launch_pdl(true, k_extend_add<T>, dim3((unsigned)x.fnblk), dim3(256), 0, stream_, panel, upd,
-                       (const DFront*)dp_.fronts, (const int64_t*)(dp_.xadd_child + x.off),
-                       (const int64_t*)(dp_.xadd_fpre + x.fpre_off), x.nchild, (const int32_t*)dp_.emap, status_);
+        if (P.asm_blocks[l] > 0) {
+            launch_pdl(true, k_assemble<T>, dim3((unsigned)P.asm_blocks[l]), dim3(256), 0, stream_, panel, upd,
+                       (const DFront*)dp_.fronts, (const int64_t*)(dp_.level_order + lo),
+                       (const int64_t*)(dp_.asm_pre + lo + l), nl, (const int32_t*)dp_.imap, status_);
             launches++;
             mark(1);
         }

@@ -473,36 +473,25 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
         }
     }
     timer.lap("steps");
-    // extend-add lists
-    P.xadd.assign(2 * nlev, DXadd{});
-    for (int64_t l = 0; l < nlev; l++)
-        for (int r = 0; r < 2; r++) {
-            DXadd& x = P.xadd[2 * l + r];
-            x.off = (int64_t)P.xadd_child.size();
-            x.fpre_off = (int64_t)P.xadd_fpre.size();
-            P.xadd_fpre.push_back(0);
-            int64_t cnt = 0, fblk = 0;
-            for (int64_t i = P.level_off[l]; i < P.level_off[l + 1]; i++) {
-                const SymFront& f = S.fronts[P.level_order[i]];
-                if (f.nchild <= r) continue;
-                int64_t c = S.children[f.child_off + r];
-                if (S.fronts[c].u == 0) continue;
-                P.xadd_child.push_back(c);
-                const int64_t uc = S.fronts[c].u;
-                const int64_t T = cdiv(uc, XT);
-                fblk += cdiv(T * (T + 1) / 2, 8);
-                P.xadd_fpre.push_back(fblk);
-                cnt++;
-            }
-            x.nchild = cnt;
-            x.fnblk = fblk;
+    // assembly tiles: the front's lower triangle, or the update block's without children
+    P.asm_blocks.assign(nlev, 0);
+    for (int64_t l = 0; l < nlev; l++) {
+        int64_t blk = 0;
+        P.asm_pre.push_back(0);
+        for (int64_t i = P.level_off[l]; i < P.level_off[l + 1]; i++) {
+            const DFront& d = P.fronts[P.level_order[i]];
+            const int64_t T = cdiv(d.imap_off >= 0 ? d.m : d.u, XT);
+            blk += cdiv(T * (T + 1) / 2, 8);
+            P.asm_pre.push_back(blk);
         }
+        P.asm_blocks[l] = blk;
+    }
     if (std::any_of(S.fronts.begin(), S.fronts.end(), [](const SymFront& f) { return f.nchild > 2; }))
         throw std::runtime_error("internal: a front has more than two children");
     P.front_of_dof.assign(S.n, 0);
     for (int64_t t = 0; t < nt; t++)
         for (int64_t q = S.fronts[t].start; q < S.fronts[t].start + S.fronts[t].k; q++) P.front_of_dof[q] = t;
-    timer.lap("extend-add lists");
+    timer.lap("assembly tiles");
     return P;
 }
 
@@ -523,7 +512,6 @@ Scatter scatter_from_lower(const Plan& P, const Symbolic& S, const std::vector<i
                            const std::vector<int64_t>& rowidx) {
     Scatter X;
     LocalRows L(S.n);
-    X.level_seg.assign(P.nlevels + 1, 0);
     X.front_seg.assign(P.nfronts + 1, 0);
     X.seg_ptr.push_back(0);
     for (int64_t l = 0; l < P.nlevels; l++) {
@@ -539,7 +527,6 @@ Scatter scatter_from_lower(const Plan& P, const Symbolic& S, const std::vector<i
                     X.seg_ptr.push_back((int64_t)X.src.size());
                 }
         }
-        X.level_seg[l + 1] = (int64_t)X.dst.size();
     }
     X.front_seg[P.nfronts] = (int64_t)X.dst.size();
     return X;
@@ -552,7 +539,6 @@ Scatter scatter_from_caller_general(const Plan& P, const Symbolic& S, const int6
                                     const std::vector<int64_t>& eq, const std::vector<int64_t>& owner) {
     Scatter X;
     LocalRows L(S.n);
-    X.level_seg.assign(P.nlevels + 1, 0);
     X.front_seg.assign(P.nfronts + 1, 0);
     X.seg_ptr.push_back(0);
     std::vector<std::pair<int64_t, int64_t>> col;  // (dst, p)
@@ -582,7 +568,6 @@ Scatter scatter_from_caller_general(const Plan& P, const Symbolic& S, const int6
                 }
             }
         }
-        X.level_seg[l + 1] = (int64_t)X.dst.size();
     }
     X.front_seg[P.nfronts] = (int64_t)X.dst.size();
     return X;
@@ -625,8 +610,6 @@ Scatter scatter_from_caller(const Plan& P, const Symbolic& S, int64_t ncaller, c
     Scatter X;
     X.front_seg.assign(nt + 1, 0);
     for (int64_t j = 0; j < nt; j++) X.front_seg[j + 1] = X.front_seg[j] + cnt[j + 1];
-    X.level_seg.assign(P.nlevels + 1, 0);
-    for (int64_t l = 0; l <= P.nlevels; l++) X.level_seg[l] = X.front_seg[P.level_off[l]];
     int64_t total = X.front_seg[nt];
     X.dst.resize(total);
     X.src.resize(total);

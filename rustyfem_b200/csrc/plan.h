@@ -41,7 +41,7 @@ constexpr int KO = NBO / NB;
 constexpr int UT = 64;        // Schur-update tile (UT × UT of F)
 constexpr int PR = 128;       // rows of a row chunk of the solve steps
 constexpr int PNR = 64;       // panel rows per CTA
-constexpr int XT = 32;        // factor: tile (XT × XT of a child's update matrix) of one warp of the extend-add
+constexpr int XT = 32;        // tile (XT × XT of a front) of one warp of the assembly
 
 // per-front descriptor used by the kernels (int64 everywhere: offsets exceed 2^31)
 struct DFront {
@@ -94,15 +94,6 @@ struct WStep {
     int64_t n_rows;           // CTAs of the row kernels: max(1, ⌈(m − J1)/PR⌉) per front
     int64_t n_part;           // partial-sum columns of the backward row kernel: Σ CTAs × width
 };
-
-// extend-add work of one level and one child rank
-struct DXadd {
-    int64_t off;              // offset into xadd_child
-    int64_t nchild;
-    int64_t fpre_off;         // offset into xadd_fpre (nchild + 1 entries)
-    int64_t fnblk;            // total CTAs of the factor's extend-add (eight XT × XT tiles each)
-};
-
 
 constexpr uint8_t PANEL_SCR = 1, PANEL_SPLIT = 2;
 constexpr uint8_t OUT_NONE = 0, OUT_FULL = 1, OUT_STRIP = 2, OUT_PAIR = 3;
@@ -165,10 +156,9 @@ struct Plan {
     std::vector<int64_t> chain_colbase;  // per front: its first column piece of its level, or -1
     int64_t chain_colpart = 0;  // partial sums of a level's column pieces (CHAIN_GROUPS row groups), per rhs
     std::vector<uint8_t> front_tc;      // fronts whose large outer updates run on the tensor cores
-    // extend-add lists, per level and rank (2 ranks)
-    std::vector<DXadd> xadd;            // 2·nlevels
-    std::vector<int64_t> xadd_child;    // child ids
-    std::vector<int64_t> xadd_fpre;     // prefix of the children's area-balanced chunks
+    // assembly CTAs (eight tiles each) of each front, as prefix sums per level (the
+    // level's fronts + 1 entries, level l at level_off[l] + l), and each level's total
+    std::vector<int64_t> asm_pre, asm_blocks;
     SegVec rows;                        // global equation of the later rows (Symbolic::rows)
     std::vector<int32_t> emap;          // local index in the parent of each later row
     int64_t panel_elems = 0, upd_elems = 0, vu_rows = 0, imap_elems = 0;
@@ -220,7 +210,6 @@ struct Scatter {
     SegVec dst;                         // panel-arena offset per segment
     std::vector<int64_t> seg_ptr;       // nseg+1
     SegVec src;                         // source index per entry
-    std::vector<int64_t> level_seg;     // nlevels+1: segments of each level are contiguous
     std::vector<int64_t> front_seg;     // nfronts+1: segments of the j-th front in level order
 };
 
