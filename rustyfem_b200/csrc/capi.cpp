@@ -512,18 +512,21 @@ RustyfemHandle* build(size_t n, size_t nn, const int64_t* loc, const double* coo
         // the caller's lower triangle into the internal lower CSC (ffi/src/lib.rs:191-202)
         const Symbolic& S = h->sym;
         std::vector<double> val(h->lrowidx.size(), 0.0);
-        for (int64_t c = 0; c < h->ncaller; c++) {
-            int64_t qc = h->eq[c];
-            if (qc < 0) continue;
-            for (int64_t p = indptr[c]; p < indptr[c + 1]; p++) {
-                int64_t r = indices[p], qr = h->eq[r];
-                if (qr < 0 || r < c) continue;
-                int64_t rr = std::max(qr, qc), cc = std::min(qr, qc);
-                auto b = h->lrowidx.begin() + h->lcolptr[cc], e = h->lrowidx.begin() + h->lcolptr[cc + 1];
-                auto it = std::lower_bound(b, e, rr);
-                val[it - h->lrowidx.begin()] += data[p];
+        // in parallel over the caller's columns: an internal entry receives from one of them only
+        parallel_chunks(h->ncaller, 64, [&](int64_t c0, int64_t c1) {
+            for (int64_t c = c0; c < c1; c++) {
+                int64_t qc = h->eq[c];
+                if (qc < 0) continue;
+                for (int64_t p = indptr[c]; p < indptr[c + 1]; p++) {
+                    int64_t r = indices[p], qr = h->eq[r];
+                    if (qr < 0 || r < c) continue;
+                    int64_t rr = std::max(qr, qc), cc = std::min(qr, qc);
+                    auto b = h->lrowidx.begin() + h->lcolptr[cc], e = h->lrowidx.begin() + h->lcolptr[cc + 1];
+                    auto it = std::lower_bound(b, e, rr);
+                    val[it - h->lrowidx.begin()] += data[p];
+                }
             }
-        }
+        });
         h->ieng.reset(new IndefEngine(S, h->lcolptr, h->lrowidx, 0.01));
         h->t_analyse_ms = ms_since(t0);
         int64_t e = h->ieng->factor(val.data());
@@ -556,19 +559,23 @@ RustyfemHandle* build(size_t n, size_t nn, const int64_t* loc, const double* coo
         // src/sparse/lu.rs:40-47)
         const Symbolic& S = h->sym;
         std::vector<double> lval(h->lrowidx.size(), 0.0), uval(h->lrowidx.size(), 0.0);
-        for (int64_t c = 0; c < h->ncaller; c++) {
-            int64_t qc = h->eq[c];
-            if (qc < 0) continue;
-            for (int64_t p = indptr[c]; p < indptr[c + 1]; p++) {
-                int64_t qr = h->eq[indices[p]];
-                if (qr < 0) continue;
-                // A(qr, qc): lower (qr, qc), or upper_t at row qc of column qr
-                const int64_t rr = qr >= qc ? qr : qc, cc = qr >= qc ? qc : qr;
-                auto b = h->lrowidx.begin() + h->lcolptr[cc], e = h->lrowidx.begin() + h->lcolptr[cc + 1];
-                auto it = std::lower_bound(b, e, rr);
-                (qr >= qc ? lval : uval)[it - h->lrowidx.begin()] += data[p];
+        // in parallel over the caller's columns: an entry of either triangle receives from one of
+        // them only
+        parallel_chunks(h->ncaller, 64, [&](int64_t c0, int64_t c1) {
+            for (int64_t c = c0; c < c1; c++) {
+                int64_t qc = h->eq[c];
+                if (qc < 0) continue;
+                for (int64_t p = indptr[c]; p < indptr[c + 1]; p++) {
+                    int64_t qr = h->eq[indices[p]];
+                    if (qr < 0) continue;
+                    // A(qr, qc): lower (qr, qc), or upper_t at row qc of column qr
+                    const int64_t rr = qr >= qc ? qr : qc, cc = qr >= qc ? qc : qr;
+                    auto b = h->lrowidx.begin() + h->lcolptr[cc], e = h->lrowidx.begin() + h->lcolptr[cc + 1];
+                    auto it = std::lower_bound(b, e, rr);
+                    (qr >= qc ? lval : uval)[it - h->lrowidx.begin()] += data[p];
+                }
             }
-        }
+        });
         h->leng.reset(new LuEngine(S, h->lcolptr, h->lrowidx, 0.01));
         h->t_analyse_ms = ms_since(t0);
         int64_t e = h->leng->factor(lval.data(), uval.data());

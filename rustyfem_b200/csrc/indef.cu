@@ -1135,13 +1135,13 @@ IndefEngine::IndefEngine(const Symbolic& S, const std::vector<int64_t>& colptr, 
     level_order_ = P.level_order;
     nlevels_ = P.nlevels;
     int64_t nt = (int64_t)S.fronts.size();
-    RFG_CUDA(cudaMalloc(&d_desc_, std::max<int64_t>(nt, 1) * sizeof(IFrontDesc)));
-    RFG_CUDA(cudaMalloc(&d_val_, std::max<size_t>(rowidx.size(), 1) * sizeof(double)));
-    RFG_CUDA(cudaMalloc(&d_scale_, std::max<int64_t>(S.n, 1) * sizeof(double)));
+    d_desc_ = (decltype(d_desc_))dev_alloc(std::max<int64_t>(nt, 1) * sizeof(IFrontDesc), stream_);
+    d_val_ = (decltype(d_val_))dev_alloc(std::max<size_t>(rowidx.size(), 1) * sizeof(double), stream_);
+    d_scale_ = (decltype(d_scale_))dev_alloc(std::max<int64_t>(S.n, 1) * sizeof(double), stream_);
     int64_t maxl = 1;
     for (int64_t l = 0; l < nlevels_; l++) maxl = std::max(maxl, level_off_[l + 1] - level_off_[l]);
-    RFG_CUDA(cudaMalloc(&d_tpre_, (maxl + 1) * sizeof(int64_t)));
-    RFG_CUDA(cudaMalloc(&d_active_, sizeof(int64_t)));
+    d_tpre_ = (decltype(d_tpre_))dev_alloc((maxl + 1) * sizeof(int64_t), stream_);
+    d_active_ = (decltype(d_active_))dev_alloc(sizeof(int64_t), stream_);
     int dev = 0;
     RFG_CUDA(cudaGetDevice(&dev));
     RFG_CUDA(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, dev));
@@ -1163,11 +1163,11 @@ void IndefEngine::release_fronts() {
 IndefEngine::~IndefEngine() {
     if (stream_) cudaStreamSynchronize(stream_);
     release_fronts();
-    cudaFree(d_desc_);
-    cudaFree(d_val_);
-    cudaFree(d_scale_);
-    cudaFree(d_tpre_);
-    cudaFree(d_active_);
+    dev_free(d_desc_, stream_);
+    dev_free(d_val_, stream_);
+    dev_free(d_scale_, stream_);
+    dev_free(d_tpre_, stream_);
+    dev_free(d_active_, stream_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -1474,8 +1474,8 @@ void IndefEngine::solve_device(double* X, int64_t nrhs) {
     for (int64_t t = 0; t < nt; t++) xstride = std::max(xstride, npiv_[t]);
     double* xbuf = nullptr;
     int64_t* dids = nullptr;
-    RFG_CUDA(cudaMallocAsync((void**)&xbuf, maxl * xstride * sizeof(double), stream_));
-    RFG_CUDA(cudaMallocAsync((void**)&dids, nt * sizeof(int64_t), stream_));
+    xbuf = (decltype(xbuf))dev_alloc(maxl * xstride * sizeof(double), stream_);
+    dids = (decltype(dids))dev_alloc(nt * sizeof(int64_t), stream_);
     RFG_CUDA(cudaMemcpyAsync(dids, level_order_.data(), nt * sizeof(int64_t), cudaMemcpyHostToDevice, stream_));
     for (int64_t l = 0; l < nlevels_; l++) {
         int64_t lo = level_off_[l], nl = level_off_[l + 1] - lo;
@@ -1487,8 +1487,8 @@ void IndefEngine::solve_device(double* X, int64_t nrhs) {
         k_indef_bwd<<<(unsigned)nl, ET, 0, stream_>>>((IFrontDesc*)d_desc_, dids + lo, X, (int)nrhs, xbuf, xstride);
     }
     RFG_CUDA(cudaGetLastError());
-    RFG_CUDA(cudaFreeAsync(xbuf, stream_));
-    RFG_CUDA(cudaFreeAsync(dids, stream_));
+    dev_free(xbuf, stream_);
+    dev_free(dids, stream_);
 }
 
 }  // namespace rfg

@@ -1517,13 +1517,6 @@ void Engine::upload_plan() {
     dp_.chain_cols = up(plan_.chain_cols);
     dp_.chain_colbase = up(plan_.chain_colbase);
     dp_.blk_width = up(plan_.blk_width);
-    // the child row of each front row, for either child: the inverse of emap, on the device
-    dp_.imap = (int32_t*)dalloc(std::max<int64_t>(plan_.imap_elems, 1) * sizeof(int32_t));
-    RFG_CUDA(cudaMemsetAsync(dp_.imap, 0xff, std::max<int64_t>(plan_.imap_elems, 1) * sizeof(int32_t), stream_));
-    if (plan_.nfronts > 0) {
-        k_imap_fill<<<(unsigned)plan_.nfronts, 128, 0, stream_>>>(dp_.fronts, dp_.emap, dp_.imap);
-        RFG_CUDA(cudaGetLastError());
-    }
 }
 
 // The host scatter lists on the device; the host copies of the per-entry lists are
@@ -1704,8 +1697,10 @@ void Engine::init(bool) {
         // first refined solve), sized for every scattered entry and its mirror
         const int64_t cap = std::max<int64_t>(2 * nseg_, 1);
         a_rowptr_ = (int64_t*)dalloc((plan_.n + 1) * sizeof(int64_t));
-        a_col_ = (int32_t*)dalloc(cap * sizeof(int32_t));
-        a_src_ = (uint32_t*)dalloc(cap * sizeof(uint32_t));
+        // columns and sources in blocks of the values' size: equal blocks find each other's places
+        // when the pool hands a freed handle's memory to the next one
+        a_col_ = (int32_t*)dalloc(cap * sizeof(double));
+        a_src_ = (uint32_t*)dalloc(cap * sizeof(double));
         a_val_ = (double*)dalloc(cap * sizeof(double));
     }
     if (use_tc_) {
@@ -1729,6 +1724,13 @@ void Engine::init(bool) {
         RFG_CUDA(cudaMemsetAsync(scr_uscale_, 0, std::max<int64_t>(plan_.max_scr_rows, 1) * sizeof(float), stream_));
         adiag0_ = (double*)dalloc(std::max<int64_t>(plan_.n, 1) * sizeof(double));
         setup_tc();
+    }
+    // the child row of each front row, for either child: the inverse of emap, on the device
+    dp_.imap = (int32_t*)dalloc(std::max<int64_t>(plan_.imap_elems, 1) * sizeof(int32_t));
+    RFG_CUDA(cudaMemsetAsync(dp_.imap, 0xff, std::max<int64_t>(plan_.imap_elems, 1) * sizeof(int32_t), stream_));
+    if (plan_.nfronts > 0) {
+        k_imap_fill<<<(unsigned)plan_.nfronts, 128, 0, stream_>>>(dp_.fronts, dp_.emap, dp_.imap);
+        RFG_CUDA(cudaGetLastError());
     }
     RFG_CUDA(cudaStreamSynchronize(stream_));
 }
