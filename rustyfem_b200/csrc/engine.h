@@ -43,20 +43,34 @@ inline bool pdl_enabled() {
     }();
     return on;
 }
+// `priority` (0: the stream's) is the launch's priority: its CTAs go before waiting CTAs of lower
+// priority (more negative is higher).
 template <typename... KArgs, typename... Args>
-inline void launch_pdl(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                       Args... args) {
+inline void launch_pdl_prio(int priority, bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                            cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    if (pdl && pdl_enabled()) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (priority != 0) {
+        at[n].id = cudaLaunchAttributePriority;
+        at[n++].val.priority = priority;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = pdl && pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = n;
     RFG_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+template <typename... KArgs, typename... Args>
+inline void launch_pdl(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                       Args... args) {
+    launch_pdl_prio(0, pdl, kern, grid, block, smem, st, args...);
 }
 
 // Device utilities (devutil.cu). exclusive_scan_i64: in-place exclusive prefix sum of
@@ -85,6 +99,8 @@ struct DevPlan {
     int64_t* pre_outer = nullptr;
     int64_t* pre_outer_tc = nullptr;
     int64_t* pre_outer_tc2 = nullptr;
+    int64_t* pre_outer_a = nullptr;     // Plan::pre_outer_a, pre_outer_tc_a
+    int64_t* pre_outer_tc_a = nullptr;
     uint8_t* panel_mode = nullptr;    // Plan::panel_mode
     uint8_t* outer_mode = nullptr;    // Plan::outer_mode
     int64_t* pre_scr = nullptr;
@@ -241,6 +257,10 @@ class Engine {
     int64_t nsrc_;
     Precision prec_;
     cudaStream_t stream_ = nullptr;
+    // the outer updates that run beside the next outer block's steps (FP64)
+    cudaStream_t side_ = nullptr;
+    cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
+    int high_prio_ = 0;
     DevPlan dp_;
     void* panel_ = nullptr;
     void* upd_ = nullptr;

@@ -1092,22 +1092,23 @@ __device__ __forceinline__ double* out_row(double* panel, double* upd, const DFr
 __global__ void __launch_bounds__(DM_THREADS, 2)
     k_schur_dmma(double* __restrict__ panel, double* __restrict__ upd, const DFront* __restrict__ fr,
                  const int64_t* __restrict__ order, int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre_tiles,
-                 const int64_t* __restrict__ pre_scr, int64_t s, const double* __restrict__ scr_w,
-                 const double* __restrict__ scr_l, const int64_t* __restrict__ status) {
+                 const int64_t* __restrict__ pre_a, int part, const int64_t* __restrict__ pre_scr, int64_t s,
+                 const double* __restrict__ scr_w, const double* __restrict__ scr_l,
+                 const int64_t* __restrict__ status) {
     pdl_wait();  // wait first: a dependent launched early may then read our inputs
     pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sbuf = reinterpret_cast<double*>(smem_raw);  // [stage][BT W rows | DM_TN L rows][DM_PITCH]
-    const int64_t b = blockIdx.x >> 1;
     const int half = blockIdx.x & 1;
-    const int64_t i = find_slot_warp(pre_tiles, nact, b);
+    int64_t lt;
+    const int64_t i = find_tile_warp(pre_tiles, pre_a, part, nact, blockIdx.x >> 1, &lt);
     const int64_t t = order[fr_off + i];
     if (status[t] != -1) return;
     const DFront f = fr[t];
     const int64_t J0 = (s / KO) * NBO;
     const int64_t J1e = min(J0 + NBO, f.k);
     const int klen = (int)(J1e - J0);
-    const BigTile bt = big_tile(f, J1e, b - pre_tiles[i]);
+    const BigTile bt = big_tile(f, J1e, lt);
     const int64_t col0 = bt.col0 + half * DM_TN;
     if (col0 >= bt.col_end) return;
     // scratch row of front row r: pre_scr[i] + r − J0
@@ -1237,6 +1238,7 @@ __global__ void __launch_bounds__(128, 2) k_schur_dmma64(double* __restrict__ pa
                                                       const DFront* __restrict__ fr,
                                                       const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
                                                       const int64_t* __restrict__ pre_tiles,
+                                                      const int64_t* __restrict__ pre_a, int part,
                                                       const int64_t* __restrict__ pre_scr, int64_t s,
                                                       const double* __restrict__ scr_w,
                                                       const double* __restrict__ scr_l,
@@ -1245,13 +1247,13 @@ __global__ void __launch_bounds__(128, 2) k_schur_dmma64(double* __restrict__ pa
     pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sbuf = reinterpret_cast<double*>(smem_raw);  // [stage][UT W rows | UT L rows][DM_PITCH]
-    const int64_t b = blockIdx.x;
-    const int64_t i = find_slot_warp(pre_tiles, nact, b);
+    int64_t lt;
+    const int64_t i = find_tile_warp(pre_tiles, pre_a, part, nact, blockIdx.x, &lt);
     const int64_t t = order[fr_off + i];
     if (status[t] != -1) return;
     const DFront f = fr[t];
     const int64_t J0 = (s / KO) * NBO;
-    const SmallTile tl = small_tile<OUTER>(f, s, b - pre_tiles[i]);
+    const SmallTile tl = small_tile<OUTER>(f, s, lt);
     // scratch row of front row r: pre_scr[i] + r − J0; the tile's pivots start at kofs
     const double* wrow = scr_w + (pre_scr[i] - J0 + tl.row0) * NBO + tl.kofs;
     const double* lrow = scr_l + (pre_scr[i] - J0 + tl.col0) * NBO + tl.kofs;
@@ -1503,6 +1505,8 @@ void Engine::upload_plan() {
     dp_.pre_outer = up(plan_.pre_outer);
     dp_.pre_outer_tc = up(plan_.pre_outer_tc);
     dp_.pre_outer_tc2 = up(plan_.pre_outer_tc2);
+    dp_.pre_outer_a = up(plan_.pre_outer_a);
+    dp_.pre_outer_tc_a = up(plan_.pre_outer_tc_a);
     dp_.pre_scr = up(plan_.pre_scr);
     dp_.panel_mode = up(plan_.panel_mode);
     dp_.outer_mode = up(plan_.outer_mode);
@@ -1676,8 +1680,18 @@ void Engine::init(bool) {
     size_t es = prec_ == PREC_FP64 ? sizeof(double) : sizeof(float);
     if (!panel_) panel_ = dalloc(plan_.panel_elems * es);
     if (!upd_) upd_ = dalloc(plan_.upd_elems * es);
-    scr_w_ = dalloc(std::max<int64_t>(plan_.max_scr_rows, 1) * NBO * es);
-    scr_l_ = dalloc(std::max<int64_t>(plan_.max_scr_rows, 1) * NBO * es);
+    // FP64: two buffers, alternating with the parity of the outer block (a block's operands are
+    // still read beside the next block's steps)
+    const int64_t nscr = prec_ == PREC_FP64 ? 2 : 1;
+    scr_w_ = dalloc(nscr * std::max<int64_t>(plan_.max_scr_rows, 1) * NBO * es);
+    scr_l_ = dalloc(nscr * std::max<int64_t>(plan_.max_scr_rows, 1) * NBO * es);
+    if (prec_ == PREC_FP64) {
+        int least = 0;
+        RFG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &high_prio_));
+        RFG_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
+        RFG_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
+        RFG_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
+    }
     d_ = (double*)dalloc(std::max<int64_t>(plan_.n, 1) * sizeof(double));
     linv_ = (double*)dalloc(std::max<int64_t>(plan_.nblocks, 1) * NB * NB * sizeof(double));
     if (plan_.nblocks > 0) {
@@ -1767,7 +1781,9 @@ Engine::~Engine() {
     for (void* p : allocs_) dev_free(p, stream_);
     for (void* p : {(void*)ref_r_, (void*)ref_dx_, (void*)ref_red_}) dev_free(p, stream_);
     if (stream_) cudaStreamSynchronize(stream_);
-    if (ev0_) cudaEventDestroy(ev0_);
+    if (side_) cudaStreamDestroy(side_);
+    for (cudaEvent_t e : {ev_fork_, ev_join_, ev0_})
+        if (e) cudaEventDestroy(e);
     if (ev1_) cudaEventDestroy(ev1_);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -1777,13 +1793,21 @@ void Engine::pivots_to_host(double* out) const {
     RFG_CUDA(cudaStreamSynchronize(stream_));
 }
 
+// CTAs of an outer update's rest from which it runs beside the next block's steps: one per SM
+// (thresholds of 40 and 600 measured the same; below, the rest is shorter than the fork and join).
+// A 64-pivot step is a chain of three launches of a few CTAs, about 33 µs, and four of them wait
+// for each outer update; side by side a factorization of the 33³ cube went from 18.5 to 17.6 ms, of the
+// 22³ from 3.76 to 3.63 ms, of the 45³ from 77.5 to 76.2 ms. (One CTA per SM for the rest, which leaves
+// half of every SM to the steps, was slower: 101 ms at 45³.)
+constexpr int64_t AHEAD_MIN_CTAS = 148;
+
 template <typename T>
 void Engine::factor_impl() {
     using S = typename ScrType<T>::type;
     T* panel = (T*)panel_;
     T* upd = (T*)upd_;
-    S* sw = (S*)scr_w_;
-    S* sl = (S*)scr_l_;
+    S* const sw0 = (S*)scr_w_;
+    S* const sl0 = (S*)scr_l_;
     const Plan& P = plan_;
     int64_t launches = 0;
     size_t schur_smem = 2 * NB * (UT + 1) * sizeof(S);
@@ -1791,7 +1815,7 @@ void Engine::factor_impl() {
     prof_phase_.clear();
     // PROF_SKIP: the interval before a 128-tile outer update at profiling level 2 (not counted)
     constexpr int PROF_SKIP = 7;
-    auto mark = [&](int phase) {
+    auto mark = [&](int phase, cudaStream_t on = nullptr) {
         // an event after each launch; the time since the previous event goes to its phase
         // (level 2: only the events around the 128-tile outer updates)
         if (!profile_) return;
@@ -1803,7 +1827,7 @@ void Engine::factor_impl() {
             prof_ev_.push_back(e);
         }
         // external: under stream capture the record becomes an event-record node of the graph
-        RFG_CUDA(cudaEventRecordWithFlags(prof_ev_[prof_phase_.size() + 1], stream_, cudaEventRecordExternal));
+        RFG_CUDA(cudaEventRecordWithFlags(prof_ev_[prof_phase_.size() + 1], on ? on : stream_, cudaEventRecordExternal));
         prof_phase_.push_back(phase);
     };
     if (profile_) {
@@ -1844,11 +1868,29 @@ void Engine::factor_impl() {
         launches++;
         mark(0);
     }
+    // Look-ahead (FP64): the part of an outer update that the next outer block's steps do not read
+    // runs beside them on the side stream; the steps' launches go first wherever a CTA leaves an SM.
+    // (With profiling on the launches are timed one after another.)
+    const bool use_ahead = side_ != nullptr && profile_ == 0;
+    const int prio = use_ahead ? high_prio_ : 0;
+    int64_t ahead = -1;  // the outer block whose update is on the side stream
+    bool pdl = true;     // false for the launch that follows a wait for the side stream
+    auto join = [&] {
+        if (ahead < 0) return;
+        RFG_CUDA(cudaStreamWaitEvent(stream_, ev_join_, 0));
+        ahead = -1;
+        pdl = false;
+    };
+    auto overlap = [&] {
+        const bool p = pdl;
+        pdl = true;
+        return p;
+    };
     for (int64_t l = 0; l < P.nlevels; l++) {
         const int64_t lo = P.level_off[l], nl = P.level_off[l + 1] - lo;
         if (nl == 0) continue;
         if (P.asm_blocks[l] > 0) {
-            launch_pdl(true, k_assemble<T>, dim3((unsigned)P.asm_blocks[l]), dim3(256), 0, stream_, panel, upd,
+            launch_pdl(overlap(), k_assemble<T>, dim3((unsigned)P.asm_blocks[l]), dim3(256), 0, stream_, panel, upd,
                        (const DFront*)dp_.fronts, (const int64_t*)(dp_.level_order + lo),
                        (const int64_t*)(dp_.asm_pre + lo + l), nl, (const int32_t*)dp_.imap, status_);
             launches++;
@@ -1856,7 +1898,12 @@ void Engine::factor_impl() {
         }
         for (int64_t si = P.step_off[l]; si < P.step_off[l + 1]; si++) {
             const DStep& st = P.steps[si];
-            launch_pdl(true, k_pivot_block<T>, dim3((unsigned)st.nact), dim3(PBT), PB_SMEM, stream_, panel, d_,
+            // this outer block's W and L operands
+            const int64_t sb = sizeof(T) == 8 ? ((st.s / KO) & 1) * std::max<int64_t>(P.max_scr_rows, 1) * NBO : 0;
+            S* const sw = sw0 + sb;
+            S* const sl = sl0 + sb;
+            if (ahead >= 0 && st.s / KO >= ahead + 2) join();  // the buffer is about to be written again
+            launch_pdl_prio(prio, overlap(), k_pivot_block<T>, dim3((unsigned)st.nact), dim3(PBT), PB_SMEM, stream_, panel, d_,
                        (const double*)adiag_, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, st.fr_off,
                        st.s, status_, linv_);
             launches++;
@@ -1864,7 +1911,7 @@ void Engine::factor_impl() {
             if (st.n_panel > 0) {
                 // this outer block's buffer of the split operands
                 const int64_t so = use_tc_ ? ((st.s / KO) & 1) * std::max<int64_t>(plan_.max_scr_rows, 1) * NBO : 0;
-                launch_pdl(true, k_panel<T>, dim3((unsigned)st.n_panel), dim3(PNT),
+                launch_pdl_prio(prio, true, k_panel<T>, dim3((unsigned)st.n_panel), dim3(PNT),
                            PANEL_SMEM, stream_, panel, (const double*)d_,
                            (const double*)linv_, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, st.fr_off,
                            st.nact, (const int64_t*)(dp_.pre_panel + st.pre_off),
@@ -1880,9 +1927,10 @@ void Engine::factor_impl() {
             }
             if (st.n_inner > 0) {
                 if constexpr (sizeof(T) == 8)
-                    launch_pdl(true, k_schur_dmma64<false>, dim3((unsigned)st.n_inner), dim3(128), D64_SMEM, stream_,
+                    launch_pdl_prio(prio, true, k_schur_dmma64<false>, dim3((unsigned)st.n_inner), dim3(128), D64_SMEM,
+                               stream_,
                                panel, upd, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, st.fr_off,
-                               st.nact, (const int64_t*)(dp_.pre_inner + st.pre_off),
+                               st.nact, (const int64_t*)(dp_.pre_inner + st.pre_off), (const int64_t*)nullptr, 0,
                                (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, (const double*)sw, (const double*)sl,
                                (const int64_t*)status_);
                 else
@@ -1900,45 +1948,78 @@ void Engine::factor_impl() {
                 mark(4);
             }
             if (st.n_outer + st.n_outer_tc > 0) {
-                if (st.n_outer > 0) {
-                    if constexpr (sizeof(T) == 8)
-                        launch_pdl(true, k_schur_dmma64<true>, dim3((unsigned)st.n_outer), dim3(128), D64_SMEM,
-                                   stream_, panel, upd, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order,
-                                   st.fr_off, st.nact, (const int64_t*)(dp_.pre_outer + st.pre_off),
-                                   (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, (const double*)sw,
-                                   (const double*)sl, (const int64_t*)status_);
-                    else
+                if constexpr (sizeof(T) == 8) {
+                    // Two outer blocks' updates of one front must follow each other. The tiles of the next
+                    // block's columns (part 1) keep the steps waiting; the rest (part 2), when a launch of it
+                    // fills the GPU and steps follow, runs on the side stream beside them.
+                    const int64_t rest = 2 * (st.n_outer_tc - st.n_outer_tc_a) + (st.n_outer - st.n_outer_a);
+                    const bool split = use_ahead && si + 1 < P.step_off[l + 1] && rest >= AHEAD_MIN_CTAS;
+                    join();
+                    auto outer = [&](int part, cudaStream_t on, int pr, bool chained) {
+                        auto cnt = [&](int64_t all, int64_t a) { return part == 0 ? all : part == 1 ? a : all - a; };
+                        const int64_t n64 = cnt(st.n_outer, st.n_outer_a), n128 = cnt(st.n_outer_tc, st.n_outer_tc_a);
+                        if (n64 > 0) {
+                            launch_pdl_prio(pr, chained, k_schur_dmma64<true>, dim3((unsigned)n64), dim3(128), D64_SMEM, on,
+                                            panel, upd, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order,
+                                            st.fr_off, st.nact, (const int64_t*)(dp_.pre_outer + st.pre_off),
+                                            (const int64_t*)(dp_.pre_outer_a + st.pre_off), part,
+                                            (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, (const double*)sw,
+                                            (const double*)sl, (const int64_t*)status_);
+                            chained = true;
+                            launches++;
+                            mark(5, on);
+                        }
+                        if (n128 > 0) {
+                            mark(PROF_SKIP, on);
+                            launch_pdl_prio(pr, chained, k_schur_dmma, dim3((unsigned)(2 * n128)), dim3(DM_THREADS), DM_SMEM,
+                                            on, panel, upd, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order,
+                                            st.fr_off, st.nact, (const int64_t*)(dp_.pre_outer_tc + st.pre_off),
+                                            (const int64_t*)(dp_.pre_outer_tc_a + st.pre_off), part,
+                                            (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, (const double*)sw,
+                                            (const double*)sl, (const int64_t*)status_);
+                            launches++;
+                            mark(6, on);
+                            nprof += profile_ ? 1 : 0;
+                        }
+                    };
+                    if (split) {
+                        RFG_CUDA(cudaEventRecord(ev_fork_, stream_));
+                        if (st.n_outer_a + st.n_outer_tc_a > 0) outer(1, stream_, prio, overlap());
+                        RFG_CUDA(cudaStreamWaitEvent(side_, ev_fork_, 0));
+                        outer(2, side_, 0, false);
+                        RFG_CUDA(cudaEventRecord(ev_join_, side_));
+                        ahead = st.s / KO;
+                    } else {
+                        outer(0, stream_, prio, overlap());
+                    }
+                } else {
+                    if (st.n_outer > 0) {
                         launch_pdl(true, k_schur<T, S, true>, dim3((unsigned)st.n_outer), dim3(256), schur_smem,
                                    stream_, panel, upd, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order,
                                    st.fr_off, st.nact, (const int64_t*)(dp_.pre_outer + st.pre_off),
                                    (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, (const S*)sw, (const S*)sl,
                                    (const int64_t*)status_);
-                    launches++;
-                    mark(5);
-                }
-                if (st.n_outer_tc > 0) {
-                    mark(PROF_SKIP);
-                    if (use_tc_) {
-                        launch_schur_tc(st);
-                    } else if constexpr (sizeof(T) == 8) {
-                        launch_pdl(true, k_schur_dmma, dim3((unsigned)(2 * st.n_outer_tc)), dim3(DM_THREADS), DM_SMEM, stream_,
-                                   panel, upd, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order, st.fr_off,
-                                   st.nact, (const int64_t*)(dp_.pre_outer_tc + st.pre_off),
-                                   (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, (const double*)sw,
-                                   (const double*)sl, (const int64_t*)status_);
-                    } else {
-                        launch_pdl(true, k_schur_big<T, S>, dim3((unsigned)st.n_outer_tc), dim3(256), big_smem<S>(),
-                                   stream_, panel, upd, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order,
-                                   st.fr_off, st.nact, (const int64_t*)(dp_.pre_outer_tc + st.pre_off),
-                                   (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, (const S*)sw, (const S*)sl,
-                                   (const int64_t*)status_);
+                        launches++;
+                        mark(5);
                     }
-                    launches++;
-                    mark(6);
-                    nprof += profile_ ? 1 : 0;
+                    if (st.n_outer_tc > 0) {
+                        mark(PROF_SKIP);
+                        if (use_tc_)
+                            launch_schur_tc(st);
+                        else
+                            launch_pdl(true, k_schur_big<T, S>, dim3((unsigned)st.n_outer_tc), dim3(256), big_smem<S>(),
+                                       stream_, panel, upd, (const DFront*)dp_.fronts, (const int64_t*)dp_.level_order,
+                                       st.fr_off, st.nact, (const int64_t*)(dp_.pre_outer_tc + st.pre_off),
+                                       (const int64_t*)(dp_.pre_scr + st.scr_off), st.s, (const S*)sw, (const S*)sl,
+                                       (const int64_t*)status_);
+                        launches++;
+                        mark(6);
+                        nprof += profile_ ? 1 : 0;
+                    }
                 }
             }
         }
+        join();
     }
     if (P.nblocks > 0) {
         launch_pdl(true, k_block_inverse, dim3((unsigned)P.nblocks), dim3(128), BI_SMEM, stream_, linv_,

@@ -276,8 +276,10 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
             P.pre_outer.push_back(0);
             P.pre_outer_tc.push_back(0);
             P.pre_outer_tc2.push_back(0);
+            P.pre_outer_a.push_back(0);
+            P.pre_outer_tc_a.push_back(0);
             P.outer_mode.push_back(0);
-            int64_t cot = 0, cot2 = 0, cit = 0;
+            int64_t cot = 0, cot2 = 0, cit = 0, coa = 0, cota = 0;
             for (int64_t i = 0; i < nact; i++) {
                 const DFront& d = P.fronts[P.level_order[lo + i]];
                 int64_t j0 = s * NB;
@@ -333,7 +335,11 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
                         }
                     }
                     P.outer_mode[P.outer_mode.size() - 1] = om;
-                    const int64_t Ws = std::min<int64_t>(NBO, d.k - J1e);  // the strip's columns
+                    const int64_t Ws = std::min<int64_t>(NBO, d.k - J1e);  // the next block's columns
+                    if (big)
+                        cota += tri(cdiv(Ro, TC_TILE), cdiv(Ws, TC_TILE));
+                    else
+                        coa += tri(cdiv(Ro, UT), cdiv(Ws, UT));
                     const int64_t Kp = (J1e - J0) + (om == OUT_PAIR ? NBO : 0);
                     if (big) {
                         P.front_tc[t] = use_tc ? 1 : 0;
@@ -368,6 +374,8 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
                 P.pre_outer.push_back(co);
                 P.pre_outer_tc.push_back(cot);
                 P.pre_outer_tc2.push_back(cot2);
+                P.pre_outer_a.push_back(coa);
+                P.pre_outer_tc_a.push_back(cota);
                 P.outer_mode.push_back(0);
             }
             st.n_panel = cp;
@@ -376,6 +384,8 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
             st.n_outer = co;
             st.n_outer_tc = cot;
             st.n_outer_tc2 = cot2;
+            st.n_outer_a = coa;
+            st.n_outer_tc_a = cota;
             P.big_tiles += cot;
             P.small_tiles += co;
             st.inner_flops = fi;

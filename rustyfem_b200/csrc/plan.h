@@ -76,6 +76,8 @@ struct DStep {
                               // cores in the mixed path, CUDA cores in the FP64 path)
     int64_t n_outer_tc2;      // the same trailing matrices in 128×256 tiles (persistent
                               // tensor-core kernel)
+    int64_t n_outer_a;        // of n_outer and n_outer_tc, the tiles of the next outer block's columns
+    int64_t n_outer_tc_a;
     int64_t scr_rows;         // scratch rows of the outer block
     int64_t scr_off_prev;     // the previous outer block's scratch prefix (two-block passes)
     double inner_flops;       // algorithmic flops of the inner updates
@@ -114,6 +116,9 @@ struct Plan {
     // prefix arrays (per step, nact+1 entries each, concatenated): panel CTAs,
     // inner tiles, outer tiles (0 for fronts before out_lo); pre_scr per outer block
     std::vector<int64_t> pre_panel, pre_inner, pre_inner_tc, pre_outer, pre_outer_tc, pre_outer_tc2, pre_scr;
+    // of pre_outer and pre_outer_tc, the tiles of the next outer block's columns (the first ones of a
+    // front's list): what its panels wait for
+    std::vector<int64_t> pre_outer_a, pre_outer_tc_a;
     std::vector<uint8_t> front_tc_inner;  // fronts whose inner updates may run on the tensor cores
     // per step and active front (the layout of pre_panel): what the panel kernel writes
     // besides L — PANEL_SCR: the W and L rows in the storage precision (read by the

@@ -186,4 +186,35 @@ __device__ __forceinline__ int64_t find_slot_warp(const int64_t* __restrict__ pr
     return lo;
 }
 
+// The tile of CTA b in a part of a step's outer update: pre (and pre_a of it, the tiles of the next
+// outer block's columns, first in each front's list) are the prefix sums over the fronts. Part 0:
+// all tiles, 1: those of pre_a, 2: the others. Returns the front's slot and its tile index in
+// *tile. All 32 lanes of a warp with the same b.
+__device__ __forceinline__ int64_t find_tile_warp(const int64_t* __restrict__ pre, const int64_t* __restrict__ pre_a,
+                                                  int part, int64_t n, int64_t b, int64_t* tile) {
+    if (part == 0) {
+        const int64_t i = find_slot_warp(pre, n, b);
+        *tile = b - pre[i];
+        return i;
+    }
+    if (part == 1) {
+        const int64_t i = find_slot_warp(pre_a, n, b);
+        *tile = b - pre_a[i];
+        return i;
+    }
+    const int lane = threadIdx.x & 31;
+    int64_t lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int64_t step = (hi - lo + 31) / 32;
+        const int64_t idx = lo + lane * step;
+        const bool ok = idx < hi && pre[idx] - pre_a[idx] <= b;
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        const int k = 31 - __clz(m);
+        lo += k * step;
+        hi = min(hi, lo + step);
+    }
+    *tile = b - (pre[lo] - pre_a[lo]) + (pre_a[lo + 1] - pre_a[lo]);
+    return lo;
+}
+
 }  // namespace rfg
