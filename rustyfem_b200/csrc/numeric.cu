@@ -1083,6 +1083,40 @@ constexpr int DM_BK = 16, DM_PITCH = 20, DM_STAGES = 3, DM_TN = 64, DM_THREADS =
 constexpr int DM_STAGE = (BT + DM_TN) * DM_PITCH;  // doubles per stage: W rows, then L rows
 constexpr size_t DM_SMEM = (size_t)DM_STAGES * DM_STAGE * sizeof(double);
 
+// Operand loads of the FP64 updates: ROWS scratch rows of W and then of L, DM_BK pivots each, 128
+// threads. Thread (tid / 8, tid % 8) copies the 16 bytes of pivots 2·(tid % 8) of every 16th row, all
+// from one pointer at constant offsets: with two warps per scheduler the instructions around the
+// products are what keeps the tensor pipe waiting, so there are no bounds. Rows past the front's
+// are another front's or the scratch's spare rows (DM_SPARE): they meet outputs that are not
+// stored. Pivots past the block's are zeros that the panel stored. (With bounds and zero fill per
+// copy there were 4.8 other instructions per product and the tensor pipe was 75 % active in a
+// large launch of the 33³ cube; a factorization went from 76.2 to 71.1 ms at 45³, 17.6 to 16.9 ms at
+// 33³, 3.63 to 3.49 ms at 22³.)
+constexpr int DM_SPARE = 128;
+__device__ __forceinline__ void cp_async16_full(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+struct DmLoader {
+    const double *w, *l;
+    uint32_t s;
+    __device__ __forceinline__ DmLoader(const double* wrow, const double* lrow, double* sbuf) {
+        const int r = threadIdx.x >> 3, c = (threadIdx.x & 7) * 2;
+        w = wrow + r * NBO + c;
+        l = lrow + r * NBO + c;
+        s = (uint32_t)__cvta_generic_to_shared(sbuf + r * DM_PITCH + c);
+    }
+    // the next chunk of pivots into the stage at byte offset off
+    template <int WR, int LR>
+    __device__ __forceinline__ void next(uint32_t off) {
+#pragma unroll
+        for (int i = 0; i < WR / 16; i++) cp_async16_full(s + off + i * 16 * DM_PITCH * 8, w + i * 16 * NBO);
+#pragma unroll
+        for (int i = 0; i < LR / 16; i++) cp_async16_full(s + off + (WR + i * 16) * DM_PITCH * 8, l + i * 16 * NBO);
+        w += DM_BK;
+        l += DM_BK;
+    }
+};
+
 // Start of front row r in the output of an outer-update tile, indexed by front column:
 // the panel row (columns < k) or the update-block row (columns >= k).
 __device__ __forceinline__ double* out_row(double* panel, double* upd, const DFront& f, bool in_panel, int64_t r) {
@@ -1114,8 +1148,6 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
     // scratch row of front row r: pre_scr[i] + r − J0
     const double* wrow = scr_w + (pre_scr[i] - J0 + bt.row0) * NBO;
     const double* lrow = scr_l + (pre_scr[i] - J0 + col0) * NBO;
-    const int nra = (int)min((int64_t)BT, f.m - bt.row0);
-    const int nrb = (int)min((int64_t)DM_TN, bt.col_end - col0);
     const int nk = (klen + DM_BK - 1) / DM_BK;
     {
         // L2 prefetch of this CTA's output rows (in range only), read back at the end
@@ -1127,18 +1159,13 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
             asm volatile("prefetch.global.L2 [%0];" ::"l"(rowp + cend - 1));
         }
     }
-    auto load = [&](int kc) {
-        double* st = sbuf + (kc % DM_STAGES) * DM_STAGE;
-        const int k0 = kc * DM_BK;
-        cp_async_tile(st, DM_PITCH, wrow + k0, NBO, nra, klen - k0, BT, DM_BK, DM_THREADS);
-        cp_async_tile(st + BT * DM_PITCH, DM_PITCH, lrow + k0, NBO, nrb, klen - k0, DM_TN, DM_BK, DM_THREADS);
-    };
+    DmLoader ld(wrow, lrow, sbuf);
+    constexpr uint32_t STB = DM_STAGE * sizeof(double);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
     const int wm = warp & 1, wn = warp >> 1;  // warp tile rows [64·wm, +64), columns [32·wn, +32)
     const int aoff = (wm * 64 + g) * DM_PITCH + q, boff = (BT + wn * 32 + g) * DM_PITCH + q;
-    auto frag = [&](double* fa, double* fb, int kc, int kk) {
-        const double* st = sbuf + (kc % DM_STAGES) * DM_STAGE + kk;
+    auto frag = [&](double* fa, double* fb, const double* st) {
 #pragma unroll
         for (int a = 0; a < 8; a++) fa[a] = st[aoff + a * 8 * DM_PITCH];
 #pragma unroll
@@ -1150,29 +1177,33 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
 #pragma unroll
         for (int c = 0; c < 4; c++) acc[a][c][0] = acc[a][c][1] = 0.0;
     double fa[2][8], fb[2][4];
-    load(0);
+    ld.next<BT, DM_TN>(0);
     cp_async_commit();
-    if (nk > 1) load(1);
+    if (nk > 1) ld.next<BT, DM_TN>(STB);
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
-    if (nk > 2) load(2);
+    if (nk > 2) ld.next<BT, DM_TN>(2 * STB);
     cp_async_commit();
-    frag(fa[0], fb[0], 0, 0);
+    const double* st = sbuf;  // chunk kc's stage
+    uint32_t soff = 0;        // its byte offset
+    frag(fa[0], fb[0], st);
     for (int kc = 0; kc < nk; kc++) {
 #pragma unroll
         for (int j = 0; j < DM_BK / 4; j++) {
             const int cur = j & 1, nxt = cur ^ 1;
             if (j + 1 < DM_BK / 4) {
-                frag(fa[nxt], fb[nxt], kc, (j + 1) * 4);
+                frag(fa[nxt], fb[nxt], st + (j + 1) * 4);
             } else if (kc + 1 < nk) {
                 // chunk kc + 1 is in once at most one group is pending; after the barrier no
                 // warp reads chunk kc's stage any more, so chunk kc + 3 may replace it
                 cp_async_wait<1>();
                 __syncthreads();
-                if (kc + 3 < nk) load(kc + 3);
+                if (kc + 3 < nk) ld.next<BT, DM_TN>(soff);
                 cp_async_commit();
-                frag(fa[nxt], fb[nxt], kc + 1, 0);
+                soff = soff == 2 * STB ? 0 : soff + STB;
+                st = sbuf + soff / sizeof(double);
+                frag(fa[nxt], fb[nxt], st);
             }
 #pragma unroll
             for (int a = 0; a < 8; a++)
@@ -1258,21 +1289,14 @@ __global__ void __launch_bounds__(128, 2) k_schur_dmma64(double* __restrict__ pa
     const double* wrow = scr_w + (pre_scr[i] - J0 + tl.row0) * NBO + tl.kofs;
     const double* lrow = scr_l + (pre_scr[i] - J0 + tl.col0) * NBO + tl.kofs;
     const int klen = (int)tl.klen;
-    const int nra = (int)min((int64_t)UT, f.m - tl.row0);
-    const int nrb = (int)min((int64_t)UT, tl.col_end - tl.col0);
     const int nk = (klen + DM_BK - 1) / DM_BK;
-    auto load = [&](int kc) {
-        double* st = sbuf + (kc % DM_STAGES) * D64_STAGE;
-        const int k0 = kc * DM_BK;
-        cp_async_tile(st, DM_PITCH, wrow + k0, NBO, nra, klen - k0, UT, DM_BK, 128);
-        cp_async_tile(st + UT * DM_PITCH, DM_PITCH, lrow + k0, NBO, nrb, klen - k0, UT, DM_BK, 128);
-    };
+    DmLoader ld(wrow, lrow, sbuf);
+    constexpr uint32_t STB = D64_STAGE * sizeof(double);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
     const int wm = warp & 1, wn = warp >> 1;  // warp tile rows [32·wm, +32), columns [32·wn, +32)
     const int aoff = (wm * 32 + g) * DM_PITCH + q, boff = (UT + wn * 32 + g) * DM_PITCH + q;
-    auto frag = [&](double* fa, double* fb, int kc, int kk) {
-        const double* st = sbuf + (kc % DM_STAGES) * D64_STAGE + kk;
+    auto frag = [&](double* fa, double* fb, const double* st) {
 #pragma unroll
         for (int a = 0; a < 4; a++) fa[a] = st[aoff + a * 8 * DM_PITCH];
 #pragma unroll
@@ -1284,27 +1308,31 @@ __global__ void __launch_bounds__(128, 2) k_schur_dmma64(double* __restrict__ pa
 #pragma unroll
         for (int c = 0; c < 4; c++) acc[a][c][0] = acc[a][c][1] = 0.0;
     double fa[2][4], fb[2][4];
-    load(0);
+    ld.next<UT, UT>(0);
     cp_async_commit();
-    if (nk > 1) load(1);
+    if (nk > 1) ld.next<UT, UT>(STB);
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
-    if (nk > 2) load(2);
+    if (nk > 2) ld.next<UT, UT>(2 * STB);
     cp_async_commit();
-    frag(fa[0], fb[0], 0, 0);
+    const double* st = sbuf;
+    uint32_t soff = 0;
+    frag(fa[0], fb[0], st);
     for (int kc = 0; kc < nk; kc++) {
 #pragma unroll
         for (int j = 0; j < DM_BK / 4; j++) {
             const int cur = j & 1, nxt = cur ^ 1;
             if (j + 1 < DM_BK / 4) {
-                frag(fa[nxt], fb[nxt], kc, (j + 1) * 4);
+                frag(fa[nxt], fb[nxt], st + (j + 1) * 4);
             } else if (kc + 1 < nk) {
                 cp_async_wait<1>();
                 __syncthreads();
-                if (kc + 3 < nk) load(kc + 3);
+                if (kc + 3 < nk) ld.next<UT, UT>(soff);
                 cp_async_commit();
-                frag(fa[nxt], fb[nxt], kc + 1, 0);
+                soff = soff == 2 * STB ? 0 : soff + STB;
+                st = sbuf + soff / sizeof(double);
+                frag(fa[nxt], fb[nxt], st);
             }
 #pragma unroll
             for (int a = 0; a < 4; a++)
@@ -1683,8 +1711,9 @@ void Engine::init(bool) {
     // FP64: two buffers, alternating with the parity of the outer block (a block's operands are
     // still read beside the next block's steps)
     const int64_t nscr = prec_ == PREC_FP64 ? 2 : 1;
-    scr_w_ = dalloc(nscr * std::max<int64_t>(plan_.max_scr_rows, 1) * NBO * es);
-    scr_l_ = dalloc(nscr * std::max<int64_t>(plan_.max_scr_rows, 1) * NBO * es);
+    const int64_t scr_elems = (nscr * std::max<int64_t>(plan_.max_scr_rows, 1) + DM_SPARE) * NBO;
+    scr_w_ = dalloc(scr_elems * es);
+    scr_l_ = dalloc(scr_elems * es);
     if (prec_ == PREC_FP64) {
         int least = 0;
         RFG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &high_prio_));
