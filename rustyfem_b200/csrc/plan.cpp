@@ -280,6 +280,19 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
             P.pre_outer_tc_a.push_back(0);
             P.outer_mode.push_back(0);
             int64_t cot = 0, cot2 = 0, cit = 0, coa = 0, cota = 0;
+            // FP64: outer updates with few 128-tiles in all run on 64-tiles
+            bool small_outer = false;
+            if (!use_tc) {
+                int64_t n128 = 0;
+                for (int64_t i = st.out_lo; i < nact; i++) {
+                    const DFront& d = P.fronts[P.level_order[lo + i]];
+                    const int64_t J1e = std::min<int64_t>(J1, d.k), Ro = d.m - J1e;
+                    if (Ro >= tun.big_min_rows && (d.u == 0 || d.u >= TC_TILE))
+                        n128 += tri(cdiv(Ro, TC_TILE), cdiv(d.k - J1e, TC_TILE)) +
+                                cdiv(d.u, TC_TILE) * (cdiv(d.u, TC_TILE) + 1) / 2;
+                }
+                small_outer = n128 < FP64_MIN_TILES;
+            }
             for (int64_t i = 0; i < nact; i++) {
                 const DFront& d = P.fronts[P.level_order[lo + i]];
                 int64_t j0 = s * NB;
@@ -316,7 +329,7 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
                     // 128-tiles for large trailing matrices whose update block is empty (a root) or
                     // fills whole tiles; the panel part is then either empty (k <= NBO) or at least
                     // NBO wide
-                    const bool big = Ro >= tun.big_min_rows && (d.u == 0 || d.u >= TC_TILE);
+                    const bool big = !small_outer && Ro >= tun.big_min_rows && (d.u == 0 || d.u >= TC_TILE);
                     // the kind of a tensor-core update: a block whose front has a next block that
                     // also ends with a tensor-core update passes only over the next block's columns
                     // (strip), and the next block passes over the rest with both blocks' pivots
