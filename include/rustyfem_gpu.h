@@ -200,13 +200,16 @@ int32_t rfg_solve_device(const RustyfemHandle* h, size_t nrhs, double* b_device,
  *  - Same input and result as rfg_solve_device on a positive definite handle (b_device:
  *    caller numbering, column-major n × nrhs, solved in place), but with no iterative
  *    refinement and no statistics: the result is the handle's factor applied once, the
- *    same values rfg_solve_device gives with refine_max_iter = 0 and stats = NULL.
+ *    same values rfg_solve_device gives with refine_max_iter = 0 and stats = NULL (to
+ *    rounding when the chains of the top levels do not fit in the scratch, below).
  *  - Returns 0, or -1 with rfg_last_error() set: an indefinite handle, or a handle whose
  *    scratch need (n × min(nrhs, 32) values twice, the per-front update vectors and
- *    per-CTA partial sums of one 32-column sweep) exceeds 16 MiB; then nothing was
- *    launched.
- *  - Nothing in the scratch need be zero beforehand: every call zeroes the update
- *    vectors and the ticket counters itself.
+ *    per-CTA partial sums of one sweep of min(nrhs, 32) columns) exceeds 16 MiB; then
+ *    nothing was launched. The flags of the top levels' chains and, for an FP64 factor,
+ *    their partial sums are not part of the need: they are taken when they fit beside
+ *    it, otherwise those levels run step by step.
+ *  - Nothing in the scratch need be zero beforehand: every call writes what it reads, and
+ *    clears the chains' flags and counters itself.
  *  - Stream order as for rfg_solve_device (above); the call returns when its result is
  *    in b_device: it synchronizes the handle's stream.
  *  - The scratch is one per device and shared by every handle: two calls that overlap

@@ -977,10 +977,14 @@ int32_t rfg_solve_device_noalloc(const RustyfemHandle* h, size_t nrhs_, double* 
         if (h->eng) {
             const int64_t xb = r256(h->n_sym * nr_max * 8);
             need = xb + h->eng->sweep_workspace_bytes(nr_max, chain);
-            if (need > NOALLOC_SCRATCH_BYTES && chain && h->eng->precision() == PREC_FP64) {
-                // an FP64 sweep whose solve chains do not fit runs every level stepped
+            if (need > NOALLOC_SCRATCH_BYTES && chain) {
+                // a sweep whose solve chains do not fit runs every level stepped; in the mixed path
+                // only the chains' flags may be what does not fit (its column pieces' partial sums
+                // are part of the need)
                 chain = false;
-                need = xb + h->eng->sweep_workspace_bytes(nr_max, chain);
+                need = h->eng->precision() == PREC_FP64
+                           ? xb + h->eng->sweep_workspace_bytes(nr_max, chain)
+                           : need - h->eng->sweep_flag_bytes(true) + h->eng->sweep_flag_bytes(false);
             }
         }
         if (need > NOALLOC_SCRATCH_BYTES) {

@@ -183,6 +183,7 @@ class Engine {
     };
     bool has_chain() const { return chain_inv_ != nullptr; }
     int64_t sweep_workspace_bytes(int64_t nrhs, bool chain) const;
+    int64_t sweep_flag_bytes(bool chain) const;  // of it, the chains' flags
     SweepWorkspace carve_sweep_workspace(void* base, int64_t nrhs, bool chain) const;
     void solve_sweep_on(double* X, int64_t nrhs, const SweepWorkspace& ws);
 

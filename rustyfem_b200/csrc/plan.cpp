@@ -405,7 +405,6 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
             st.outer_flops = fo;
             P.inner_flops += fi;
             P.outer_flops += fo;
-            P.max_nact = std::max(P.max_nact, nact);
             P.steps.push_back(st);
         }
         P.step_off[l + 1] = (int64_t)P.steps.size();
@@ -435,7 +434,6 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
                 P.pre_wrows.push_back(w.n_rows);
                 P.pre_wpart.push_back(w.n_part);
             }
-            P.max_wrows = std::max(P.max_wrows, w.n_rows);
             P.max_wpart = std::max(P.max_wpart, w.n_part);
             P.wsteps.push_back(w);
         }

@@ -144,7 +144,7 @@ struct Plan {
     std::vector<WStep> wsteps;
     std::vector<int64_t> wstep_off;     // nlevels + 1
     std::vector<int64_t> pre_wrows, pre_wpart;
-    int64_t max_wrows = 0, max_wpart = 0;
+    int64_t max_wpart = 0;
     // Solve chains. On the levels with at most chain_fronts fronts (the top of the tree,
     // where a step's launches have a few CTAs of work) a sweep
     // runs as one launch per level and direction instead of
@@ -174,7 +174,6 @@ struct Plan {
     std::vector<int32_t> emap;          // local index in the parent of each later row
     int64_t panel_elems = 0, upd_elems = 0, vu_rows = 0, imap_elems = 0;
     int64_t max_scr_rows = 0;           // largest scratch over all steps
-    int64_t max_nact = 0;               // largest number of active fronts of a step
     int64_t nblocks = 0;                // NB×NB diagonal blocks of all fronts
     std::vector<uint8_t> blk_width;     // their pivots (NB but for a front's last block)
     std::vector<int64_t> front_of_dof;  // front owning each equation

@@ -1722,8 +1722,10 @@ void Engine::chain_check() {
 int64_t Engine::sweep_workspace_bytes(int64_t nrhs, bool chain) const {
     const Plan& P = plan_;
     return round256(std::max<int64_t>(P.n * nrhs, 1) * 8) + round256(std::max<int64_t>(P.vu_rows * nrhs, 1) * 8) +
-           round256(std::max<int64_t>(partial_rows(chain) * nrhs, 1) * 8) + round256(flag_words(chain) * 4);
+           round256(std::max<int64_t>(partial_rows(chain) * nrhs, 1) * 8) + sweep_flag_bytes(chain);
 }
+
+int64_t Engine::sweep_flag_bytes(bool chain) const { return round256(flag_words(chain) * 4); }
 
 Engine::SweepWorkspace Engine::carve_sweep_workspace(void* base, int64_t nrhs, bool chain) const {
     const Plan& P = plan_;
