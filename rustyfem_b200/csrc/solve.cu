@@ -75,16 +75,18 @@ __device__ __forceinline__ int64_t find_slot2(const int64_t* pre, int64_t n, int
 constexpr int PF_MAXR = 4;
 
 // row tile of the rows / partial kernels: PF_RPC rows (half of a PR-row chunk of the plan)
-// × cols floats (cols = the step's widest block rounded up to 32), row pitch cols + 4
+// × cols floats (cols = the step's widest block rounded up to 32), row pitch cols + 8
 // (16-byte rows, conflict-free row reads); three such CTAs fit on an SM
 constexpr int PF_RPC = PR / 2;
 // The rows kernel takes 64 rows of an FP32 factor per CTA and 32 of an FP64 one (the same bytes);
 // the partial sums take 64 in both, so that the partial blocks of a chunk stay two.
 template <typename T>
 constexpr int PF_ROWS = PF_RPC * 4 / (int)sizeof(T);
-// row pitches: FP32 rows are read in two halves, FP64 rows by four lanes in 64-byte groups
+// row pitch: the lanes of a row (two for FP32, four for FP64) read its 16-byte groups in turn, and the
+// pitch keeps eight lanes' reads in different banks. (FP32 rows read in two halves at a pitch of
+// cols + 4 met every bank twice: the refined solve of the 60³ cube 17.93 ms, now 17.56.)
 template <typename T>
-__host__ __device__ inline int pf_pitch(int cols) { return cols + (sizeof(T) == 4 ? 4 : 8); }
+__host__ __device__ inline int pf_pitch(int cols) { return cols + 8; }
 inline int pf_cols(int64_t wb_max) { return (int)((wb_max + 31) / 32 * 32); }
 template <typename T>
 size_t pf_rows_smem(int cols, int nrhs) {
@@ -282,13 +284,11 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
     double acc[R][2];
 #pragma unroll
     for (int j = 0; j < R; j++) acc[j][0] = acc[j][1] = 0.0;
-    // FP32: each thread a half of the row; FP64: every fourth 16-byte group
     const int nq = cols / (VEC * TPR);
-    const int q0 = sizeof(T) == 4 ? h * nq : h, dq = sizeof(T) == 4 ? 1 : TPR;
     const VT* row = reinterpret_cast<const VT*>(Lt + rr * pitch);
 #pragma unroll 4
     for (int u = 0; u < nq; u++) {
-        const int q = q0 + u * dq;
+        const int q = h + u * TPR;
         const VT lv = row[q];
         const T* l = reinterpret_cast<const T*>(&lv);
 #pragma unroll
