@@ -107,6 +107,7 @@ struct DevPlan {
     int64_t* asm_pre = nullptr;       // Plan::asm_pre
     int64_t* pre_wrows = nullptr;
     int64_t* pre_wpart = nullptr;
+    int2* wrow_slot = nullptr;   // Plan::wrow_slot
     int64_t* rows = nullptr;
     int32_t* emap = nullptr;
     int64_t* seg_dst = nullptr;

@@ -1530,6 +1530,7 @@ void Engine::upload_plan() {
     dp_.pre_inner_tc = up(plan_.pre_inner_tc);
     dp_.pre_wrows = up(plan_.pre_wrows);
     dp_.pre_wpart = up(plan_.pre_wpart);
+    dp_.wrow_slot = (int2*)up(plan_.wrow_slot);
     dp_.pre_outer = up(plan_.pre_outer);
     dp_.pre_outer_tc = up(plan_.pre_outer_tc);
     dp_.pre_outer_tc2 = up(plan_.pre_outer_tc2);

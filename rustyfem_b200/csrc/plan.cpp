@@ -423,6 +423,7 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
             w.fr_off = lo;
             while (lo + w.nact < hi && (S2 == 0 || S.fronts[P.level_order[lo + w.nact]].k > S2 * WS)) w.nact++;
             w.pre_off = (int64_t)P.pre_wrows.size();
+            w.row_off = (int64_t)P.wrow_slot.size();
             P.pre_wrows.push_back(0);
             P.pre_wpart.push_back(0);
             for (int64_t i = 0; i < w.nact; i++) {
@@ -431,6 +432,7 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
                 const int64_t c = std::max<int64_t>(1, cdiv(d.m - J1, PR));
                 w.n_rows += c;
                 w.n_part += c * wb;
+                P.wrow_slot.insert(P.wrow_slot.end(), c, {(int32_t)i, (int32_t)P.level_order[lo + i]});
                 P.pre_wrows.push_back(w.n_rows);
                 P.pre_wpart.push_back(w.n_part);
             }

@@ -254,8 +254,8 @@ __global__ void __launch_bounds__(256) k_wfwd_diag_pf(const double* __restrict__
 template <typename T, int R>
 __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, double* __restrict__ V,
                                                      const double* __restrict__ Y, const T* __restrict__ panel,
-                                                     const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                     int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
+                                                     const DFront* __restrict__ fr, const int2* __restrict__ slots,
+                                                     const int64_t* __restrict__ pre,
                                                      int64_t S, int cols, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
@@ -265,9 +265,9 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
     T* Lt = reinterpret_cast<T*>(sm);                              // [RPC][pitch]
     double* yB = sm + RPC * pitch * sizeof(T) / sizeof(double);    // [WS][R]
     const int64_t b = blockIdx.x / SUB;
-    const int64_t i = find_slot_warp(pre, nact, b);
-    const int64_t chunk = b - pre[i];
-    const DFront f = fr[order[fr_off + i]];
+    const int2 sf = __ldg(slots + b);
+    const int64_t i = sf.x, chunk = b - pre[i];
+    const DFront f = fr[sf.y];
     const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
     const int wb = (int)(J1 - J0);
     const int64_t r0 = J1 + chunk * PR + (blockIdx.x % SUB) * RPC;
@@ -323,8 +323,8 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
 // thread groups take every G-th row, their sums added in group order.
 template <typename T, int R>
 __global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__ Y, const T* __restrict__ panel,
-                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                      int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
+                                                      const DFront* __restrict__ fr, const int2* __restrict__ slots,
+                                                      const int64_t* __restrict__ pre,
                                                       const int64_t* __restrict__ pre_part,
                                                       const int64_t* __restrict__ rows, int64_t S,
                                                       double* __restrict__ partial, int cols) {
@@ -335,9 +335,9 @@ __global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__
     double* yr = sm + PF_RPC * pitch * sizeof(T) / sizeof(double);  // [PF_RPC][R]
     double* red = yr + PF_RPC * R;                                  // [256][R]
     const int64_t b = blockIdx.x >> 1;
-    const int64_t i = find_slot_warp(pre, nact, b);
-    const int64_t chunk = b - pre[i];
-    const DFront f = fr[order[fr_off + i]];
+    const int2 sf = __ldg(slots + b);
+    const int64_t i = sf.x, chunk = b - pre[i];
+    const DFront f = fr[sf.y];
     const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
     const int wb = (int)(J1 - J0);
     const int64_t r0 = J1 + chunk * PR + (blockIdx.x & 1) * PF_RPC;
@@ -875,8 +875,8 @@ __global__ void __launch_bounds__(256) k_mm_fwd_diag(const double* __restrict__ 
 template <typename T, int NT>
 __global__ void __launch_bounds__(256) k_mm_fwd_rows(double* __restrict__ X, double* __restrict__ V,
                                                      const double* __restrict__ Y, const T* __restrict__ panel,
-                                                     const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                     int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
+                                                     const DFront* __restrict__ fr, const int2* __restrict__ slots,
+                                                     const int64_t* __restrict__ pre,
                                                      int64_t S, int nrhs, int cols, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
@@ -885,9 +885,9 @@ __global__ void __launch_bounds__(256) k_mm_fwd_rows(double* __restrict__ X, dou
     double* yB = sm;                                 // [cols][VP]
     T* Lt = reinterpret_cast<T*>(sm + cols * VP);    // [MM_ROWS][pitch]
     const int64_t b = blockIdx.x >> 1;
-    const int64_t i = find_slot_warp(pre, nact, b);
-    const int64_t chunk = b - pre[i];
-    const DFront f = fr[order[fr_off + i]];
+    const int2 sf = __ldg(slots + b);
+    const int64_t i = sf.x, chunk = b - pre[i];
+    const DFront f = fr[sf.y];
     const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
     const int wb = (int)(J1 - J0);
     const int64_t r0 = J1 + chunk * PR + (blockIdx.x & 1) * MM_ROWS;
@@ -938,8 +938,8 @@ __global__ void __launch_bounds__(256) k_mm_fwd_rows(double* __restrict__ X, dou
 // block of partials per chunk; warp w takes the columns 8w + 64i ....
 template <typename T, int NT>
 __global__ void __launch_bounds__(256) k_mm_bwd_part(const double* __restrict__ Y, const T* __restrict__ panel,
-                                                     const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                     int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre,
+                                                     const DFront* __restrict__ fr, const int2* __restrict__ slots,
+                                                     const int64_t* __restrict__ pre,
                                                      const int64_t* __restrict__ pre_part,
                                                      const int64_t* __restrict__ rows, int64_t S, int nrhs,
                                                      double* __restrict__ partial, int cols) {
@@ -949,9 +949,9 @@ __global__ void __launch_bounds__(256) k_mm_bwd_part(const double* __restrict__ 
     const int pitch = mm_part_pitch<T>(cols);
     double* yr = sm;                            // [PR][VP]
     T* ring = reinterpret_cast<T*>(sm + PR * VP);  // [2][ST][pitch]
-    const int64_t i = find_slot_warp(pre, nact, blockIdx.x);
-    const int64_t chunk = blockIdx.x - pre[i];
-    const DFront f = fr[order[fr_off + i]];
+    const int2 sf = __ldg(slots + blockIdx.x);
+    const int64_t i = sf.x, chunk = blockIdx.x - pre[i];
+    const DFront f = fr[sf.y];
     const int64_t J0 = S * WS, J1 = min(J0 + WS, f.k);
     const int wb = (int)(J1 - J0);
     const int64_t r0 = J1 + chunk * PR;
@@ -1393,14 +1393,14 @@ void wfwd_pf(const WStep& w, int nbw_max, int cols, double* X, double* Y, double
         launch_chained(true, k_wfwd_diag_pd<R>, (unsigned)w.nact, 256, pd_diag_smem(nbw_max, R), st, X, Y, panel, linv,
                        dp.fronts, dp.level_order, w.fr_off, w.S, nbw_max, V, imap);
     launch_chained(true, k_wfwd_rows_pf<T, R>, (unsigned)(PR / PF_ROWS<T> * w.n_rows), PR, pf_rows_smem<T>(cols, R), st,
-                   X, V, Y, panel, dp.fronts, dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, w.S, cols, imap);
+                   X, V, Y, panel, dp.fronts, dp.wrow_slot + w.row_off, dp.pre_wrows + w.pre_off, w.S, cols, imap);
 }
 template <typename T, int R>
 void wbwd_pf(const WStep& w, int nbw_max, int cols, double* Y, const T* panel, const double* linv,
              const double* d, const DevPlan& dp, double* partial, cudaStream_t st) {
     launch_chained(true, k_wbwd_part_pf<T, R>, (unsigned)(2 * w.n_rows), 256, pf_part_smem<T>(cols, R), st, Y, panel,
-                   dp.fronts, dp.level_order, w.fr_off, w.nact, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off,
-                   dp.rows, w.S, partial, cols);
+                   dp.fronts, dp.wrow_slot + w.row_off, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off, dp.rows, w.S,
+                   partial, cols);
     if constexpr (sizeof(T) == 4)
         launch_chained(true, k_wbwd_diag_pf<R>, (unsigned)w.nact, 256, pf_diag_smem(nbw_max, R), st, Y, panel, linv,
                        dp.fronts, dp.level_order, w.fr_off, dp.pre_wrows + w.pre_off, dp.pre_wpart + w.pre_off, w.S,
@@ -1420,14 +1420,14 @@ void wfwd_mm(const WStep& w, int nbw_max, int cols, double* X, double* Y, double
                (const double*)X, Y, (const double*)V, panel, linv, (const DFront*)dp.fronts,
                (const int64_t*)dp.level_order, w.fr_off, w.S, nrhs, nbw_max, (const int32_t*)dp.imap);
     launch_pdl(true, k_mm_fwd_rows<T, NT>, dim3((unsigned)(2 * w.n_rows)), dim3(256), mm_rows_smem<T>(cols, NT), st, X,
-               V, (const double*)Y, panel, (const DFront*)dp.fronts, (const int64_t*)dp.level_order, w.fr_off, w.nact,
+               V, (const double*)Y, panel, (const DFront*)dp.fronts, (const int2*)(dp.wrow_slot + w.row_off),
                (const int64_t*)(dp.pre_wrows + w.pre_off), w.S, nrhs, cols, (const int32_t*)dp.imap);
 }
 template <typename T, int NT>
 void wbwd_mm(const WStep& w, int nbw_max, int cols, double* Y, const T* panel, const double* linv, const double* d,
              const DevPlan& dp, double* partial, int nrhs, cudaStream_t st) {
     launch_pdl(true, k_mm_bwd_part<T, NT>, dim3((unsigned)w.n_rows), dim3(256), mm_part_smem<T>(cols, NT), st,
-               (const double*)Y, panel, (const DFront*)dp.fronts, (const int64_t*)dp.level_order, w.fr_off, w.nact,
+               (const double*)Y, panel, (const DFront*)dp.fronts, (const int2*)(dp.wrow_slot + w.row_off),
                (const int64_t*)(dp.pre_wrows + w.pre_off), (const int64_t*)(dp.pre_wpart + w.pre_off),
                (const int64_t*)dp.rows, w.S, nrhs, partial, cols);
     launch_pdl(true, k_mm_bwd_diag<T>, dim3((unsigned)w.nact, NT), dim3(256), mm_diag_smem(nbw_max), st, Y, panel, linv,
