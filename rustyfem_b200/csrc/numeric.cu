@@ -865,8 +865,6 @@ __global__ void __launch_bounds__(256) k_schur(T* __restrict__ panel, T* __restr
                                                const int64_t* __restrict__ pre_tiles, const int64_t* __restrict__ pre_scr,
                                                int64_t s, const S* __restrict__ scr_w, const S* __restrict__ scr_l,
                                                const int64_t* __restrict__ status) {
-    pdl_wait();  // wait first: a dependent launched early may then read our inputs
-    pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     S* As = reinterpret_cast<S*>(smem_raw);  // [NB][UT + 1]
     S* Bs = As + NB * (UT + 1);
@@ -874,8 +872,10 @@ __global__ void __launch_bounds__(256) k_schur(T* __restrict__ panel, T* __restr
     int64_t i = find_slot_warp(pre_tiles, nact, b);
     int64_t lt = b - pre_tiles[i];
     int64_t t = order[fr_off + i];
-    if (status[t] != -1) return;
     const DFront f = fr[t];
+    pdl_wait();  // before this only plan data is read, which no kernel writes
+    pdl_launch_dependents();
+    if (status[t] != -1) return;
     const int64_t J0 = (s / KO) * NBO;
     const SmallTile st = small_tile<OUTER>(f, s, lt);
     const int64_t row0 = st.row0, col0 = st.col0, col_end = st.col_end, kofs = st.kofs, klen = st.klen;
@@ -982,16 +982,16 @@ __global__ void __launch_bounds__(256) k_schur_big(T* __restrict__ panel, T* __r
                                                    const int64_t* __restrict__ pre_scr, int64_t s,
                                                    const S* __restrict__ scr_w, const S* __restrict__ scr_l,
                                                    const int64_t* __restrict__ status) {
-    pdl_wait();  // wait first: a dependent launched early may then read our inputs
-    pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     S* sbuf = reinterpret_cast<S*>(smem_raw);  // [2 stages][A|B][BK][BT + 1]
     int64_t b = blockIdx.x;
     int64_t i = find_slot_warp(pre_tiles, nact, b);
     int64_t lt = b - pre_tiles[i];
     int64_t t = order[fr_off + i];
-    if (status[t] != -1) return;
     const DFront f = fr[t];
+    pdl_wait();  // before this only plan data is read, which no kernel writes
+    pdl_launch_dependents();
+    if (status[t] != -1) return;
     int64_t J0 = (s / KO) * NBO;
     int64_t J1e = min(J0 + NBO, f.k);
     int64_t klen = J1e - J0;
@@ -1129,16 +1129,16 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
                  const int64_t* __restrict__ pre_a, int part, const int64_t* __restrict__ pre_scr, int64_t s,
                  const double* __restrict__ scr_w, const double* __restrict__ scr_l,
                  const int64_t* __restrict__ status) {
-    pdl_wait();  // wait first: a dependent launched early may then read our inputs
-    pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sbuf = reinterpret_cast<double*>(smem_raw);  // [stage][BT W rows | DM_TN L rows][DM_PITCH]
     const int half = blockIdx.x & 1;
     int64_t lt;
     const int64_t i = find_tile_warp(pre_tiles, pre_a, part, nact, blockIdx.x >> 1, &lt);
     const int64_t t = order[fr_off + i];
-    if (status[t] != -1) return;
     const DFront f = fr[t];
+    pdl_wait();  // before this only plan data is read, which no kernel writes
+    pdl_launch_dependents();
+    if (status[t] != -1) return;
     const int64_t J0 = (s / KO) * NBO;
     const int64_t J1e = min(J0 + NBO, f.k);
     const int klen = (int)(J1e - J0);
@@ -1274,15 +1274,15 @@ __global__ void __launch_bounds__(128, 2) k_schur_dmma64(double* __restrict__ pa
                                                       const double* __restrict__ scr_w,
                                                       const double* __restrict__ scr_l,
                                                       const int64_t* __restrict__ status) {
-    pdl_wait();  // wait first: a dependent launched early may then read our inputs
-    pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sbuf = reinterpret_cast<double*>(smem_raw);  // [stage][UT W rows | UT L rows][DM_PITCH]
     int64_t lt;
     const int64_t i = find_tile_warp(pre_tiles, pre_a, part, nact, blockIdx.x, &lt);
     const int64_t t = order[fr_off + i];
-    if (status[t] != -1) return;
     const DFront f = fr[t];
+    pdl_wait();  // before this only plan data is read, which no kernel writes
+    pdl_launch_dependents();
+    if (status[t] != -1) return;
     const int64_t J0 = (s / KO) * NBO;
     const SmallTile tl = small_tile<OUTER>(f, s, lt);
     // scratch row of front row r: pre_scr[i] + r − J0; the tile's pivots start at kofs
