@@ -238,10 +238,9 @@ struct TileInfo {
 };
 
 __device__ __forceinline__ TileInfo decode_tile(const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre_tiles,
-                                                int64_t s, int64_t b, DFront* fout, uint8_t mode) {
+                                                int64_t fr_off, const int64_t* __restrict__ pre_tiles,
+                                                int64_t s, int64_t b, int64_t i, DFront* fout, uint8_t mode) {
     TileInfo ti;
-    int64_t i = find_slot_tc(pre_tiles, nact, b);
     int64_t lt = b - pre_tiles[i];
     ti.i = i;
     ti.t = order[fr_off + i];
@@ -288,10 +287,9 @@ __device__ __forceinline__ TileInfo decode_tile(const DFront* __restrict__ fr, c
 // column tile by column tile; columns at or beyond J1e are not written.
 __device__ __forceinline__ TileInfo decode_tile_inner(const DFront* __restrict__ fr,
                                                       const int64_t* __restrict__ order, int64_t fr_off,
-                                                      int64_t nact, const int64_t* __restrict__ pre_tiles,
-                                                      int64_t s, int64_t b, DFront* fout) {
+                                                      const int64_t* __restrict__ pre_tiles, int64_t s,
+                                                      int64_t b, int64_t i, DFront* fout) {
     TileInfo ti;
-    int64_t i = find_slot_tc(pre_tiles, nact, b);
     int64_t lt = b - pre_tiles[i];
     ti.i = i;
     ti.t = order[fr_off + i];
@@ -323,10 +321,9 @@ __device__ __forceinline__ TileInfo decode_tile_inner(const DFront* __restrict__
 // strict upper part of the tiles on the diagonal are computed and not written (beyond the
 // map) or written into entries that nothing reads.
 __device__ __forceinline__ TileInfo decode_tile_wide(const DFront* __restrict__ fr, const int64_t* __restrict__ order,
-                                                     int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre_tiles,
-                                                     int64_t s, int64_t b, DFront* fout, uint8_t mode) {
+                                                     int64_t fr_off, const int64_t* __restrict__ pre_tiles,
+                                                     int64_t s, int64_t b, int64_t i, DFront* fout, uint8_t mode) {
     TileInfo ti;
-    int64_t i = find_slot_tc(pre_tiles, nact, b);
     int64_t lt = b - pre_tiles[i];
     ti.i = i;
     ti.t = order[fr_off + i];
@@ -365,17 +362,70 @@ __device__ __forceinline__ TileInfo decode_tile_wide(const DFront* __restrict__ 
     return ti;
 }
 
+// What the three roles of the persistent kernel need of a tile.
+struct PsTile {
+    int live;              // its front is not stopped
+    int t, row0, col0;
+    int klen, klen0, k0;
+    int xmax, cbase;       // bound and origin of the map's columns (and rows, of the update block)
+    int ya, yb, ya0, yb0;  // scratch rows of A and B in this block's buffer and in the previous one's
+    int in_panel;
+};
+
+// A warp decodes 32 of its CTA's tiles at a time, one per lane, and hands them out by shuffles: a
+// tile's description is a chain of dependent loads (slot, order, front, scratch rows), which one
+// thread at a time would go through between two tiles. The first 32 are decoded before the wait for
+// the previous kernel (plan data only). A mixed factorization of the 60³ cube takes 64.4 ms so and
+// 65.5 with a decode per tile and role, one of the hex20 20³ cube 7.65 and 7.88.
+// Lane's tile b; live = 0 past the last one.
 template <int TN>
-__device__ __forceinline__ TileInfo decode_any(bool inner, const DFront* __restrict__ fr,
-                                               const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
-                                               const int64_t* __restrict__ pre_tiles, int64_t s, int64_t b,
-                                               DFront* fout, const uint8_t* __restrict__ omode) {
-    if (inner) return decode_tile_inner(fr, order, fr_off, nact, pre_tiles, s, b, fout);
-    // the front's kind of outer update at this step (full, strip or the pair's second pass)
+__device__ __forceinline__ PsTile ps_decode(bool inner, const DFront* __restrict__ fr,
+                                            const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
+                                            const int64_t* __restrict__ pre_tiles, int64_t ntiles, int64_t s, int64_t b,
+                                            const uint8_t* __restrict__ omode, const int64_t* __restrict__ pre_scr,
+                                            const int64_t* __restrict__ pre_scr_prev) {
+    PsTile p{};
+    if (b >= ntiles) return p;
     const int64_t i = find_slot_tc(pre_tiles, nact, b);
-    const uint8_t mode = omode ? omode[i] : OUT_FULL;
-    return TN == 256 ? decode_tile_wide(fr, order, fr_off, nact, pre_tiles, s, b, fout, mode)
-                     : decode_tile(fr, order, fr_off, nact, pre_tiles, s, b, fout, mode);
+    DFront f;
+    TileInfo ti;
+    if (inner) {
+        ti = decode_tile_inner(fr, order, fr_off, pre_tiles, s, b, i, &f);
+    } else {
+        // the front's kind of outer update at this step (full, strip or the pair's second pass)
+        const uint8_t mode = omode ? omode[i] : OUT_FULL;
+        ti = TN == 256 ? decode_tile_wide(fr, order, fr_off, pre_tiles, s, b, i, &f, mode)
+                       : decode_tile(fr, order, fr_off, pre_tiles, s, b, i, &f, mode);
+    }
+    p.live = 1;
+    p.t = (int)ti.t;
+    p.row0 = (int)ti.row0;
+    p.col0 = (int)ti.col0;
+    p.klen = (int)ti.klen;
+    p.klen0 = (int)ti.klen0;
+    p.k0 = (int)ti.k0;
+    p.xmax = (int)ti.xmax;
+    p.cbase = ti.in_panel ? 0 : (int)f.k;
+    p.in_panel = ti.in_panel;
+    // this block's rows in its scratch layout, and for the second pass of a pair the previous
+    // block's (the other buffer)
+    p.ya = (int)(pre_scr[i] + (ti.row0 - ti.J0));
+    p.yb = (int)(pre_scr[i] + (ti.col0 - ti.J0));
+    if (ti.klen0) {
+        p.ya0 = (int)(pre_scr_prev[i] + (ti.row0 - (ti.J0 - NBO)));
+        p.yb0 = (int)(pre_scr_prev[i] + (ti.col0 - (ti.J0 - NBO)));
+    }
+    return p;
+}
+
+__device__ __forceinline__ PsTile ps_shfl(const PsTile& p, int src) {
+    constexpr int N = sizeof(PsTile) / sizeof(int);
+    PsTile r;
+    const int* a = reinterpret_cast<const int*>(&p);
+    int* o = reinterpret_cast<int*>(&r);
+#pragma unroll
+    for (int k = 0; k < N; k++) o[k] = __shfl_sync(0xffffffffu, a[k], src);
+    return r;
 }
 
 template <int TN, bool H16>
@@ -417,26 +467,34 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
+    auto decode = [&](int64_t n) {
+        return ps_decode<TN>(inner != 0, fr, order, fr_off, nact, pre_tiles, ntiles, s, blockIdx.x + n * gridDim.x, omode,
+                             pre_scr, pre_scr_prev);
+    };
+    PsTile mine = decode(lane);
     // the set-up above overlaps the previous kernel (programmatic launch); the operands and
     // the front are touched only after it has completed
     pdl_wait();
     pdl_launch_dependents();
+    if (mine.live) mine.live = status[mine.t] == -1;
+    // the CTA's n-th tile, on all lanes of the warp (n goes up by one from call to call)
+    auto tile = [&](int64_t n) {
+        if (n > 0 && (n & 31) == 0) {
+            mine = decode(n + lane);
+            if (mine.live) mine.live = status[mine.t] == -1;
+        }
+        return ps_shfl(mine, (int)(n & 31));
+    };
+    const int64_t my_tiles = ntiles > blockIdx.x ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
     if (warp == 0) {
-        if (lane == 0) {
-            int64_t g = 0;  // chunk counter over all tiles of this CTA
-            for (int64_t b = blockIdx.x; b < ntiles && ok; b += gridDim.x) {
-                DFront f;
-                TileInfo ti = decode_any<TN>(inner != 0, fr, order, fr_off, nact, pre_tiles, s, b, &f, omode);
-                if (status[ti.t] != -1) continue;
+        int64_t g = 0;  // chunk counter over all tiles of this CTA
+        for (int64_t n = 0; n < my_tiles; n++) {
+            const PsTile ti = tile(n);
+            if (!ti.live) continue;
+            if (lane == 0) {
                 const int par = (int)((s / KO) & 1);
-                // this block's rows in its scratch layout, and for the second pass of a pair the
-                // previous block's (the other buffer)
-                const int srowA = (int)(pre_scr[ti.i] + (ti.row0 - ti.J0));
-                const int srowB = (int)(pre_scr[ti.i] + (ti.col0 - ti.J0));
-                const int srowA0 = ti.klen0 ? (int)(pre_scr_prev[ti.i] + (ti.row0 - (ti.J0 - NBO))) : 0;
-                const int srowB0 = ti.klen0 ? (int)(pre_scr_prev[ti.i] + (ti.col0 - (ti.J0 - NBO))) : 0;
                 const int nk = (int)((ti.klen + KC - 1) / KC);
                 for (int kc = 0; kc < nk; kc++, g++) {
                     int st = (int)(g % L::STAGES);
@@ -448,8 +506,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
                     tc::mbar_expect_tx(&full[st], L::STAGE);
                     const bool prev = kc * KC < ti.klen0;
                     const int p = prev ? par ^ 1 : par;
-                    const int x = prev ? kc * KC : (int)ti.k0 + (kc * KC - (int)ti.klen0);
-                    const int ya = prev ? srowA0 : srowA, yb = prev ? srowB0 : srowB;
+                    const int x = prev ? kc * KC : ti.k0 + (kc * KC - ti.klen0);
+                    const int ya = prev ? ti.ya0 : ti.ya, yb = prev ? ti.yb0 : ti.yb;
                     if constexpr (H16) {
                         tc::tma_load_2d(sb, &maps.uhi[p], x, ya, &full[st]);
                         tc::tma_load_2d(sb + L::OPA, &maps.ulo[p], x, ya, &full[st]);
@@ -465,20 +523,17 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
                     }
                 }
             }
+            if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = H16 ? tc::idesc_f16(TCM, TN, true) : tc::idesc_tf32(TCM, TN, true);
-            int64_t g = 0, tl = 0;
-            for (int64_t b = blockIdx.x; b < ntiles && ok; b += gridDim.x) {
-                DFront f;
-                TileInfo ti = decode_any<TN>(inner != 0, fr, order, fr_off, nact, pre_tiles, s, b, &f, omode);
-                if (status[ti.t] != -1) continue;
-                const int a = (int)(tl & 1);
-                if (tl >= 2 && !tc::mbar_wait(&tempty[a], (uint32_t)(((tl >> 1) - 1) & 1), err, 12)) {
-                    ok = false;
-                    break;
-                }
+        constexpr uint32_t idesc = H16 ? tc::idesc_f16(TCM, TN, true) : tc::idesc_tf32(TCM, TN, true);
+        int64_t g = 0, tl = 0;
+        for (int64_t n = 0; n < my_tiles; n++) {
+            const PsTile ti = tile(n);
+            if (!ti.live) continue;
+            const int a = (int)(tl & 1);
+            if (lane == 0 && tl >= 2 && !tc::mbar_wait(&tempty[a], (uint32_t)(((tl >> 1) - 1) & 1), err, 12)) ok = false;
+            if (lane == 0 && ok) {
                 tc::tc_fence_after();
                 const uint32_t acc = tmem + a * TN;
                 const int nk = (int)((ti.klen + KC - 1) / KC);
@@ -510,8 +565,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
                     tc::mma_commit(&empty[st]);
                 }
                 tc::mma_commit(&tfull[a]);
-                tl++;
             }
+            tl++;
+            if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
         }
     } else {
         // epilogue warps 2..5: TMEM lane quarter (warp % 4)
@@ -519,32 +575,30 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         const int et = threadIdx.x - 64;  // 0..127
         const int rl = q * 32 + lane;     // tile row of this thread
         int64_t tl = 0, nbox = 0;
-        for (int64_t b = blockIdx.x; b < ntiles; b += gridDim.x) {
-            DFront f;
-            TileInfo ti = decode_any<TN>(inner != 0, fr, order, fr_off, nact, pre_tiles, s, b, &f, omode);
-            if (status[ti.t] != -1) continue;
+        for (int64_t n = 0; n < my_tiles; n++) {
+            const PsTile ti = tile(n);
+            if (!ti.live) continue;
             const int a = (int)(tl & 1);
+            float rinv = 1.f;
+            if constexpr (H16) {
+                // the scales of the tile's rows and columns (rows past the scratch belong to
+                // tiles' padding, whose results are not written), while the tile is multiplied: cinv
+                // was last read before the previous tile's last barrier. A row's scale depends on
+                // the row alone (its original diagonal), so the two blocks of a pair share it: this
+                // block's scratch layout gives it
+                const int64_t ra = (int64_t)ti.ya + rl;
+                rinv = ra < scale_rows ? 1.f / uscale[ra] : 0.f;
+                for (int c = et; c < TN; c += 128)
+                    cinv[c] = (int64_t)ti.yb + c < scale_rows ? 1.f / uscale[ti.yb + c] : 0.f;
+            }
             // one thread waits (bounded) and tells the other 127 through shared memory, so
             // that all epilogue threads take the same branch at every named barrier
             if (et == 0) *eflag = tc::mbar_wait(&tfull[a], (uint32_t)((tl >> 1) & 1), err, 14) ? 1u : 0u;
             tc::named_barrier(1, 128);
             if (*eflag == 0) break;
             tc::tc_fence_after();
-            float rinv = 1.f;
-            if constexpr (H16) {
-                // the scales of the tile's rows and columns (rows past the scratch belong to
-                // tiles' padding, whose results are not written)
-                const int64_t srA = pre_scr[ti.i] + (ti.row0 - ti.J0), srB = pre_scr[ti.i] + (ti.col0 - ti.J0);
-                // a row's scale depends on the row alone (its original diagonal), so the two
-                // blocks of a pair share it: this block's scratch layout gives it
-                const int64_t ra = srA + rl;
-                rinv = ra < scale_rows ? 1.f / uscale[ra] : 0.f;
-                for (int c = et; c < TN; c += 128) cinv[c] = srB + c < scale_rows ? 1.f / uscale[srB + c] : 0.f;
-                tc::named_barrier(1, 128);
-            }
             const CUtensorMap* cm = &cmaps[2 * ti.t + (ti.in_panel ? 0 : 1)];
-            const int64_t cbase = ti.in_panel ? 0 : f.k;
-            const int64_t width = ti.xmax;
+            const int cbase = ti.cbase, width = ti.xmax;
             for (int cb = 0; cb < TN / 32; cb++, nbox++) {
                 uint32_t v[32];
                 tc::tmem_ld32(tmem + a * TN + ((uint32_t)(q * 32) << 16) + cb * 32, v);
@@ -572,8 +626,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
                 tc::fence_proxy_async_smem();
                 tc::named_barrier(1, 128);
                 if (et == 0) {
-                    int64_t x = (ti.col0 - cbase) + cb * 32;
-                    if (x < width) tc::tma_reduce_add_2d(cm, (int)x, (int)(ti.row0 - cbase), box);
+                    const int x = (ti.col0 - cbase) + cb * 32;
+                    if (x < width) tc::tma_reduce_add_2d(cm, x, ti.row0 - cbase, box);
                     tc::bulk_commit();
                 }
             }
