@@ -193,7 +193,8 @@ __global__ void __launch_bounds__(256, 6) k_assemble(T* __restrict__ panel, T* _
 // the length of that chain. The block is factored in sub-panels of PB = 8 pivots. Warps 0 and 1
 // hold one row below the sub-panel's diagonal 8×8 block per lane, and every lane also holds the
 // whole diagonal block and eliminates it for itself: from pivot to pivot there is no exchange,
-// only the reciprocal and one multiply-add on registers. The sub-panel's rank-8 update of the
+// only the reciprocal and one multiply-add on registers. (One barrier of the two warps stands
+// between their loads of the block and the store of its factor in its place.) The sub-panel's rank-8 update of the
 // trailing block runs on the FP64 tensor-core path (two m8n8k4 products per 8×8 tile), first for
 // the next sub-panel's columns, then, while the next sub-panel is eliminated, for the rest
 // (warps 2 to 6); warp 7 tests the pivots and inverts the finished 16×16 diagonal blocks. The block's slot of `linv`
@@ -377,6 +378,10 @@ __global__ void __launch_bounds__(PBT, 2) k_pivot_block(T* __restrict__ panel, d
                 a[k] = v.x;
                 a[k + 1] = v.y;
             }
+            // Both warps hold the diagonal block before thread 32 stores its factor over it. (A
+            // named barrier of the 64 threads: the six other warps are in the previous
+            // sub-panel's update.)
+            asm volatile("bar.sync 1, 64;" ::: "memory");
             // the eight pivots without a branch: the rule is checked on all of them afterwards (a
             // bad pivot spoils only values that nobody reads, the front stops here)
 #pragma unroll
