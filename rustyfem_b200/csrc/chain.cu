@@ -189,8 +189,8 @@ __device__ __forceinline__ void fwd_tiles(double (&acc)[R], T* ring, double* yb,
 
 template <typename T, int R>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
-    k_chain_fwd(const double* __restrict__ X, double* __restrict__ Y, const T* __restrict__ panel,
-                const double* __restrict__ V, const int32_t* __restrict__ imap,
+    k_chain_fwd(const double* X, double* __restrict__ Y, const T* __restrict__ panel,
+                const double* V, const int32_t* __restrict__ imap,
                 const double* __restrict__ cinv, const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
                 const int64_t* __restrict__ items, int64_t nitems, int* __restrict__ flags, int* __restrict__ counter,
                 int* __restrict__ err) {
@@ -231,7 +231,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
 #pragma unroll
             for (int r = 0; r < R; r++)
                 xo[i * R + r] =
-                    i < nr ? kids_add(X[(f.start + r0 + i) * R + r], V, imap, f, r0 + i, R, r) - acc[r] : 0.0;
+                    i < nr ? kids_add(__ldcg(X + (f.start + r0 + i) * R + r), V, imap, f, r0 + i, R, r) - acc[r] : 0.0;
         }
         cluster.sync();
         for (int e = tid; e < WS * R; e += CT) {
@@ -261,7 +261,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
 // The later rows of a chain level's fronts after the level's chain: V[rows] = (children's V) −
 // L21·y over all the front's pivots, one CTA per CHAIN_PIECE rows.
 template <typename T, int R>
-__global__ void __launch_bounds__(CT) k_chain_rows(const double* __restrict__ Y, double* __restrict__ V,
+__global__ void __launch_bounds__(CT) k_chain_rows(const double* Y, double* __restrict__ V,
                                                    const int32_t* __restrict__ imap, const T* __restrict__ panel,
                                                    const DFront* __restrict__ fr, const int64_t* __restrict__ items) {
     pdl_launch_dependents();
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(CT) k_chain_rows(const double* __restrict__ Y,
                         __syncthreads();
                         const int wbj = (int)min((int64_t)WS, f.k - j * WS);
                         const double* ys = Y + (f.start + j * WS) * R;
-                        for (int e = tid; e < WS * R; e += CT) yb[e] = e < wbj * R ? ys[e] : 0.0;
+                        for (int e = tid; e < WS * R; e += CT) yb[e] = e < wbj * R ? __ldcg(ys + e) : 0.0;
                     });
     quad_sum<R>(acc);
     if (q == 0 && i < nr) {
@@ -349,12 +349,12 @@ __device__ __forceinline__ void col_sum(double (&acc)[R], double* red) {
 // minus the later rows' part (the row groups of k_chain_cols in order; cb < 0: no later rows).
 __device__ __forceinline__ double chain_z(const double* Y, const double* d, const double* part, int64_t cb,
                                           const DFront& f, int64_t col, int nrhs, int r) {
-    double z = Y[(f.start + col) * nrhs + r] / d[f.start + col];
+    double z = __ldcg(Y + (f.start + col) * nrhs + r) / d[f.start + col];
     if (cb >= 0) {
         const double* p = part + ((cb + col / CQ) * CHAIN_GROUPS * CQ + col % CQ) * (int64_t)nrhs + r;
         double sum = 0.0;
 #pragma unroll
-        for (int g = 0; g < CHAIN_GROUPS; g++) sum += p[(int64_t)g * CQ * nrhs];
+        for (int g = 0; g < CHAIN_GROUPS; g++) sum += __ldcg(p + (int64_t)g * CQ * nrhs);
         z -= sum;
     }
     return z;
@@ -363,7 +363,7 @@ __device__ __forceinline__ double chain_z(const double* Y, const double* d, cons
 template <typename T, int R>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     k_chain_bwd(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ cinv,
-                const double* __restrict__ d, const double* __restrict__ part, const int64_t* __restrict__ colbase,
+                const double* __restrict__ d, const double* part, const int64_t* __restrict__ colbase,
                 const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk, const int64_t* __restrict__ items,
                 int64_t nitems, int* __restrict__ flags, int* __restrict__ counter, int* __restrict__ err) {
     pdl_launch_dependents();
@@ -447,7 +447,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
 
 // y of the later rows of a chain level's fronts into V (contiguous per front), before the
 // level's backward: V[vuoff + i] = Y[rows[rows_off + i]], one CTA per CHAIN_PIECE rows.
-__global__ void __launch_bounds__(CT) k_chain_gather(const double* __restrict__ Y, double* __restrict__ V,
+__global__ void __launch_bounds__(CT) k_chain_gather(const double* Y, double* __restrict__ V,
                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ rows,
                                                      const int64_t* __restrict__ items, int nrhs) {
     pdl_launch_dependents();
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(CT) k_chain_gather(const double* __restrict__ 
     const int nr = (int)min((int64_t)CQ, f.u - i0);
     for (int e = threadIdx.x; e < nr * nrhs; e += CT) {
         const int ii = e / nrhs, r = e - ii * nrhs;
-        V[(f.vuoff + i0 + ii) * nrhs + r] = Y[rows[f.rows_off + i0 + ii] * nrhs + r];
+        V[(f.vuoff + i0 + ii) * nrhs + r] = __ldcg(Y + rows[f.rows_off + i0 + ii] * nrhs + r);
     }
 }
 
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(CT) k_chain_gather(const double* __restrict__ 
 // part[(item · CHAIN_GROUPS + group) · CHAIN_PIECE + column]; the chain subtracts them in
 // group order (chain_z).
 template <typename T, int R>
-__global__ void __launch_bounds__(CT) k_chain_cols(double* __restrict__ part, const double* __restrict__ V,
+__global__ void __launch_bounds__(CT) k_chain_cols(double* __restrict__ part, const double* V,
                                                    const T* __restrict__ panel, const DFront* __restrict__ fr,
                                                    const int64_t* __restrict__ items) {
     pdl_launch_dependents();
@@ -540,8 +540,8 @@ __device__ __forceinline__ int vsw(int k, int n) { return k * MG + (n ^ ((k & 2)
 
 template <typename T>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
-    k_chain_fwd_mm(const double* __restrict__ X, double* __restrict__ Y, const T* __restrict__ panel,
-                   const double* __restrict__ V, const int32_t* __restrict__ imap, const double* __restrict__ cinv,
+    k_chain_fwd_mm(const double* X, double* __restrict__ Y, const T* __restrict__ panel,
+                   const double* V, const int32_t* __restrict__ imap, const double* __restrict__ cinv,
                    const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
                    const int64_t* __restrict__ items, int64_t nitems, int nrhs, int64_t nblocks,
                    int* __restrict__ flags0, int* __restrict__ counter, int* __restrict__ err) {
@@ -609,7 +609,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
             const int i = 8 * w + g, n = 2 * q + e;
             double x = 0.0;
             if (i < nr && n < rc)
-                x = kids_add(X[(f.start + r0 + i) * nrhs + j0 + n], V, imap, f, r0 + i, nrhs, j0 + n) - (a0[e] + a1[e]);
+                x = kids_add(__ldcg(X + (f.start + r0 + i) * nrhs + j0 + n), V, imap, f, r0 + i, nrhs, j0 + n) - (a0[e] + a1[e]);
             xo[i * MG + n] = x;
         }
         cluster.sync();
@@ -641,7 +641,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
 template <typename T>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     k_chain_bwd_mm(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ cinv,
-                   const double* __restrict__ d, const double* __restrict__ part, const int64_t* __restrict__ colbase,
+                   const double* __restrict__ d, const double* part, const int64_t* __restrict__ colbase,
                    const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
                    const int64_t* __restrict__ items, int64_t nitems, int nrhs, int64_t nblocks,
                    int* __restrict__ flags0, int* __restrict__ counter, int* __restrict__ err) {
@@ -767,7 +767,7 @@ __device__ __forceinline__ void vec_piece(double* dst, const double* src, int n,
 }
 
 template <typename T, int NT>
-__global__ void __launch_bounds__(CT) k_chain_rows_mm(const double* __restrict__ Y, double* __restrict__ V,
+__global__ void __launch_bounds__(CT) k_chain_rows_mm(const double* Y, double* __restrict__ V,
                                                       const int32_t* __restrict__ imap, const T* __restrict__ panel,
                                                       const DFront* __restrict__ fr, const int64_t* __restrict__ items,
                                                       int nrhs) {
@@ -820,7 +820,7 @@ __global__ void __launch_bounds__(CT) k_chain_rows_mm(const double* __restrict__
 }
 
 template <typename T, int NT>
-__global__ void __launch_bounds__(CT) k_chain_cols_mm(double* __restrict__ part, const double* __restrict__ V,
+__global__ void __launch_bounds__(CT) k_chain_cols_mm(double* __restrict__ part, const double* V,
                                                       const T* __restrict__ panel, const DFront* __restrict__ fr,
                                                       const int64_t* __restrict__ items, int nrhs) {
     pdl_launch_dependents();

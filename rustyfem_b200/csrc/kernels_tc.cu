@@ -433,8 +433,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     k_schur_tc_persistent(const __grid_constant__ TcMaps maps, const CUtensorMap* __restrict__ cmaps,
                           const DFront* __restrict__ fr, const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
                           const int64_t* __restrict__ pre_tiles, int64_t ntiles, const int64_t* __restrict__ pre_scr,
-                          int64_t s, const int64_t* __restrict__ status, int* __restrict__ err, int inner,
-                          const float* __restrict__ uscale, int64_t scale_rows, const uint8_t* __restrict__ omode,
+                          int64_t s, const int64_t* status, int* __restrict__ err, int inner,
+                          const float* uscale, int64_t scale_rows, const uint8_t* __restrict__ omode,
                           const int64_t* __restrict__ pre_scr_prev) {
     using L = PsLayout<TN>;
     constexpr int KC = H16 ? 64 : TCK;  // K per stage
@@ -587,9 +587,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
                 // the row alone (its original diagonal), so the two blocks of a pair share it: this
                 // block's scratch layout gives it
                 const int64_t ra = (int64_t)ti.ya + rl;
-                rinv = ra < scale_rows ? 1.f / uscale[ra] : 0.f;
+                rinv = ra < scale_rows ? 1.f / __ldcg(uscale + ra) : 0.f;
                 for (int c = et; c < TN; c += 128)
-                    cinv[c] = (int64_t)ti.yb + c < scale_rows ? 1.f / uscale[ti.yb + c] : 0.f;
+                    cinv[c] = (int64_t)ti.yb + c < scale_rows ? 1.f / __ldcg(uscale + ti.yb + c) : 0.f;
             }
             // one thread waits (bounded) and tells the other 127 through shared memory, so
             // that all epilogue threads take the same branch at every named barrier

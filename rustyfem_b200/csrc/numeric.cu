@@ -62,12 +62,12 @@ __global__ void k_scatter(T* __restrict__ panel, const double* __restrict__ src,
 }
 
 template <typename T>
-__global__ void k_capture_diag(const T* __restrict__ panel, double* __restrict__ adiag, const DFront* __restrict__ fr,
+__global__ void k_capture_diag(const T* panel, double* __restrict__ adiag, const DFront* __restrict__ fr,
                                const int64_t* __restrict__ order, int64_t lo) {
     pdl_wait();  // wait first: a dependent launched early may then read our inputs
     pdl_launch_dependents();
     const DFront f = fr[order[lo + blockIdx.x]];
-    for (int64_t i = threadIdx.x; i < f.k; i += blockDim.x) adiag[f.start + i] = (double)panel[f.poff + i * f.ldp + i];
+    for (int64_t i = threadIdx.x; i < f.k; i += blockDim.x) adiag[f.start + i] = (double)__ldcg(panel + f.poff + i * f.ldp + i);
 }
 
 // Children's update matrices into the fronts of a level, by gathering: the lower triangle of a
@@ -309,7 +309,7 @@ __device__ __noinline__ void pb_diag_inverse(const double* A, double* S, double*
 
 template <typename T>
 __global__ void __launch_bounds__(PBT, 2) k_pivot_block(T* __restrict__ panel, double* __restrict__ d,
-                                                        const double* __restrict__ adiag,
+                                                        const double* adiag,
                                                         const DFront* __restrict__ fr, const int64_t* __restrict__ order,
                                                         int64_t fr_off, int64_t s, int64_t* __restrict__ status,
                                                         double* __restrict__ linv) {
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(PBT, 2) k_pivot_block(T* __restrict__ panel, d
             v[i] = VT{};
             if (r < jb && 2 * lane <= r) v[i] = *reinterpret_cast<const VT*>(blk + (int64_t)r * f.ldp + 2 * lane);
         }
-        for (int p = tid; p < NB; p += PBT) orig[p] = p < jb ? adiag[f.start + j0 + p] : 1.0;
+        for (int p = tid; p < NB; p += PBT) orig[p] = p < jb ? __ldcg(adiag + f.start + j0 + p) : 1.0;
         if (tid == 0) bad = NB;
 #pragma unroll
         for (int i = 0; i < NB / 8; i++) {
@@ -622,15 +622,15 @@ __device__ __forceinline__ void panel_group(double (&acc)[2][4], const double (&
 }
 
 template <typename T>
-__global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const double* __restrict__ d,
-                                               const double* __restrict__ linv, const DFront* __restrict__ fr,
+__global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const double* d,
+                                               const double* linv, const DFront* __restrict__ fr,
                                                const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
                                                const int64_t* __restrict__ pre_panel, const int64_t* __restrict__ pre_scr,
                                                int64_t s, T* __restrict__ scr_w, T* __restrict__ scr_l,
-                                               const int64_t* __restrict__ status, float* __restrict__ whi,
+                                               const int64_t* status, float* __restrict__ whi,
                                                float* __restrict__ wlo, float* __restrict__ lhi, float* __restrict__ llo,
                                                const uint8_t* __restrict__ mode, const int64_t* __restrict__ rows,
-                                               const double* __restrict__ adiag0, __half* __restrict__ uhi,
+                                               const double* adiag0, __half* __restrict__ uhi,
                                                __half* __restrict__ ulo, float* __restrict__ uscale,
                                                int* __restrict__ err) {
     extern __shared__ __align__(16) double pnl_smem[];
@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const doub
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
     // the chunk's rows of the step's columns are final once the update kernel before the
     // pivot kernel has completed, which the pivot kernel waited for before it let this
-    // kernel start (programmatic launch): they are loaded while the pivot block is factored.
+    // kernel start (programmatic launch): they are loaded, from L2, while the pivot block is factored.
     // A group of four columns that starts below jb ends inside the row's padding (zeros).
     double F[4][2][4];
 #pragma unroll
@@ -662,15 +662,15 @@ __global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const doub
             const bool ok = rr < nr && c < jb;
             const T* p = panel + f.poff + (r0 + rr) * f.ldp + j0 + c;
             if constexpr (sizeof(T) == 4) {
-                const float4 v = ok ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 v = ok ? __ldcg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 F[G][m][0] = v.x;
                 F[G][m][1] = v.y;
                 F[G][m][2] = v.z;
                 F[G][m][3] = v.w;
             } else {
                 const double2 z = make_double2(0.0, 0.0);
-                const double2 u = ok ? *reinterpret_cast<const double2*>(p) : z;
-                const double2 v = ok ? *reinterpret_cast<const double2*>(p + 2) : z;
+                const double2 u = ok ? __ldcg(reinterpret_cast<const double2*>(p)) : z;
+                const double2 v = ok ? __ldcg(reinterpret_cast<const double2*>(p + 2)) : z;
                 F[G][m][0] = u.x;
                 F[G][m][1] = u.y;
                 F[G][m][2] = v.x;
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const doub
         // the rows' scales from their original diagonal (known since the assembly), also
         // kept per scratch row for the tensor-core epilogue: while the pivot block runs
         const int64_t r = r0 + 16 * w + lane;
-        rsc = u16_row_scale(adiag0[r < f.k ? f.start + r : rows[f.rows_off + r - f.k]]);
+        rsc = u16_row_scale(__ldcg(adiag0 + (r < f.k ? f.start + r : rows[f.rows_off + r - f.k])));
         if (rsc == 0.f) atomicExch(err, 21);
         uscale[sr0 + 16 * w + lane] = rsc;
     }
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const doub
         constexpr int PER = NB * NB / 2 / PNT;  // 16-byte loads per thread, all issued before any store
         double2 v[PER];
 #pragma unroll
-        for (int u = 0; u < PER; u++) v[u] = __ldg(reinterpret_cast<const double2*>(li) + u * PNT + tid);
+        for (int u = 0; u < PER; u++) v[u] = __ldcg(reinterpret_cast<const double2*>(li) + u * PNT + tid);
 #pragma unroll
         for (int u = 0; u < PER; u++) {
             const int e = 2 * (u * PNT + tid), r = e / NB, c = e % NB;
@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(PNT) k_panel(T* __restrict__ panel, const doub
         }
     }
     if (tid < NB) {
-        const double dv = tid < jb ? d[f.start + j0 + tid] : 0.0;
+        const double dv = tid < jb ? __ldcg(d + f.start + j0 + tid) : 0.0;
         dinv[tid] = tid < jb ? 1.0 / dv : 0.0;
         if (sizeof(T) == sizeof(float)) usq[tid] = tid < jb ? (float)sqrt(dv) : 0.f;
     }
@@ -868,8 +868,8 @@ template <typename T, typename S, bool OUTER>
 __global__ void __launch_bounds__(256) k_schur(T* __restrict__ panel, T* __restrict__ upd, const DFront* __restrict__ fr,
                                                const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
                                                const int64_t* __restrict__ pre_tiles, const int64_t* __restrict__ pre_scr,
-                                               int64_t s, const S* __restrict__ scr_w, const S* __restrict__ scr_l,
-                                               const int64_t* __restrict__ status) {
+                                               int64_t s, const S* scr_w, const S* scr_l,
+                                               const int64_t* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     S* As = reinterpret_cast<S*>(smem_raw);  // [NB][UT + 1]
     S* Bs = As + NB * (UT + 1);
@@ -901,8 +901,8 @@ __global__ void __launch_bounds__(256) k_schur(T* __restrict__ panel, T* __restr
             int rr = idx / NB, kk = idx - rr * NB;
             int64_t r = row0 + rr, c = col0 + rr;
             bool kin = kk < kc;
-            As[kk * (UT + 1) + rr] = (kin && r < f.m) ? wbase[r * NBO + k0 + kk] : (S)0;
-            Bs[kk * (UT + 1) + rr] = (kin && c < col_end) ? lbase[c * NBO + k0 + kk] : (S)0;
+            As[kk * (UT + 1) + rr] = (kin && r < f.m) ? __ldcg(wbase + r * NBO + k0 + kk) : (S)0;
+            Bs[kk * (UT + 1) + rr] = (kin && c < col_end) ? __ldcg(lbase + c * NBO + k0 + kk) : (S)0;
         }
         __syncthreads();
 #pragma unroll 8
@@ -985,8 +985,8 @@ __global__ void __launch_bounds__(256) k_schur_big(T* __restrict__ panel, T* __r
                                                    const int64_t* __restrict__ order, int64_t fr_off, int64_t nact,
                                                    const int64_t* __restrict__ pre_tiles,
                                                    const int64_t* __restrict__ pre_scr, int64_t s,
-                                                   const S* __restrict__ scr_w, const S* __restrict__ scr_l,
-                                                   const int64_t* __restrict__ status) {
+                                                   const S* scr_w, const S* scr_l,
+                                                   const int64_t* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     S* sbuf = reinterpret_cast<S*>(smem_raw);  // [2 stages][A|B][BK][BT + 1]
     int64_t b = blockIdx.x;
@@ -1132,8 +1132,8 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
     k_schur_dmma(double* __restrict__ panel, double* __restrict__ upd, const DFront* __restrict__ fr,
                  const int64_t* __restrict__ order, int64_t fr_off, int64_t nact, const int64_t* __restrict__ pre_tiles,
                  const int64_t* __restrict__ pre_a, int part, const int64_t* __restrict__ pre_scr, int64_t s,
-                 const double* __restrict__ scr_w, const double* __restrict__ scr_l,
-                 const int64_t* __restrict__ status) {
+                 const double* scr_w, const double* scr_l,
+                 const int64_t* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sbuf = reinterpret_cast<double*>(smem_raw);  // [stage][BT W rows | DM_TN L rows][DM_PITCH]
     const int half = blockIdx.x & 1;
@@ -1276,9 +1276,9 @@ __global__ void __launch_bounds__(128, 2) k_schur_dmma64(double* __restrict__ pa
                                                       const int64_t* __restrict__ pre_tiles,
                                                       const int64_t* __restrict__ pre_a, int part,
                                                       const int64_t* __restrict__ pre_scr, int64_t s,
-                                                      const double* __restrict__ scr_w,
-                                                      const double* __restrict__ scr_l,
-                                                      const int64_t* __restrict__ status) {
+                                                      const double* scr_w,
+                                                      const double* scr_l,
+                                                      const int64_t* status) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sbuf = reinterpret_cast<double*>(smem_raw);  // [stage][UT W rows | UT L rows][DM_PITCH]
     int64_t lt;

@@ -149,11 +149,11 @@ __device__ __forceinline__ void warp_sum8(const double (&v)[8][R], double (&out)
 // four sub-blocks the inverse block of sub-block 3 is copied into the space of column
 // block 0 once stage 0 is done.
 template <int R>
-__global__ void __launch_bounds__(256) k_wfwd_diag_pf(const double* __restrict__ X, double* __restrict__ Y,
+__global__ void __launch_bounds__(256) k_wfwd_diag_pf(const double* X, double* __restrict__ Y,
                                                       const float* __restrict__ panel, const double* __restrict__ linv,
                                                       const DFront* __restrict__ fr, const int64_t* __restrict__ order,
                                                       int64_t fr_off, int64_t S, int nbw_max,
-                                                      const double* __restrict__ V, const int32_t* __restrict__ imap) {
+                                                      const double* V, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
     double* Li = sm;                                                     // [nli][NB][NB]
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256) k_wfwd_diag_pf(const double* __restrict__
         const int p = threadIdx.x;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            double x = p < wb ? xs[p * R + r] : 0.0;
+            double x = p < wb ? __ldcg(xs + p * R + r) : 0.0;
             if (S == 0 && p < wb) x = kids_add(x, V, imap, f, p, R, r);
             xB[p * R + r] = x;
         }
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(256) k_wfwd_diag_pf(const double* __restrict__
 // row tile prefetched before the wait for y_B.
 template <typename T, int R>
 __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, double* __restrict__ V,
-                                                     const double* __restrict__ Y, const T* __restrict__ panel,
+                                                     const double* Y, const T* __restrict__ panel,
                                                      const DFront* __restrict__ fr, const int2* __restrict__ slots,
                                                      const int64_t* __restrict__ pre,
                                                      int64_t S, int cols, const int32_t* __restrict__ imap) {
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
     pdl_wait();
     if (nr == 0) return;
     const double* ys = Y + (f.start + J0) * R;
-    for (int idx = threadIdx.x; idx < cols * R; idx += PR) yB[idx] = idx < wb * R ? ys[idx] : 0.0;
+    for (int idx = threadIdx.x; idx < cols * R; idx += PR) yB[idx] = idx < wb * R ? __ldcg(ys + idx) : 0.0;
     cp_async_wait<0>();
     __syncthreads();
     const int rr = threadIdx.x / TPR, h = threadIdx.x % TPR;
@@ -310,10 +310,10 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
         if (S == 0) {
             // the first step of the front: the children's part on the way (V starts from it)
 #pragma unroll
-            for (int j = 0; j < R; j++) tgt[j] = kids_add(r < f.k ? tgt[j] : 0.0, V, imap, f, r, R, j) - v[j];
+            for (int j = 0; j < R; j++) tgt[j] = kids_add(r < f.k ? __ldcg(tgt + j) : 0.0, V, imap, f, r, R, j) - v[j];
         } else {
 #pragma unroll
-            for (int j = 0; j < R; j++) tgt[j] -= v[j];
+            for (int j = 0; j < R; j++) tgt[j] = __ldcg(tgt + j) - v[j];
         }
     }
 }
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(PR) k_wfwd_rows_pf(double* __restrict__ X, dou
 // rows (two CTAs per PR-row chunk, each with its own block of partials); G = 256/cols
 // thread groups take every G-th row, their sums added in group order.
 template <typename T, int R>
-__global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__ Y, const T* __restrict__ panel,
+__global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* Y, const T* __restrict__ panel,
                                                       const DFront* __restrict__ fr, const int2* __restrict__ slots,
                                                       const int64_t* __restrict__ pre,
                                                       const int64_t* __restrict__ pre_part,
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(256) k_wbwd_part_pf(const double* __restrict__
         if (rr < nr) {
             const int64_t r = r0 + rr;
             const int64_t q = r < f.k ? f.start + r : rows[f.rows_off + r - f.k];
-            v = Y[q * R + j];
+            v = __ldcg(Y + q * R + j);
         }
         yr[idx] = v;
     }
@@ -425,7 +425,7 @@ __device__ __forceinline__ void wbwd_sum_partials(double* z, const double* Y, co
                 for (int u = 0; u < 8; u++) v += t[u];
             }
             for (; c < nc; c++) v += __ldcg(&pbase[c * nout + o]);
-            v = Y[(f.start + J0) * R + o] / d[f.start + J0 + o / R] - v;
+            v = __ldcg(Y + (f.start + J0) * R + o) / d[f.start + J0 + o / R] - v;
         }
         z[o] = v;
     }
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pf(double* __restrict__ Y, co
                                                       const int64_t* __restrict__ order, int64_t fr_off,
                                                       const int64_t* __restrict__ pre,
                                                       const int64_t* __restrict__ pre_part, int64_t S,
-                                                      const double* __restrict__ partial, int nbw_max,
+                                                      const double* partial, int nbw_max,
                                                       const double* __restrict__ d) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
@@ -559,11 +559,11 @@ __device__ __forceinline__ void pd_issue(double* sm, int tile, const double* pan
 }
 
 template <int R>
-__global__ void __launch_bounds__(256) k_wfwd_diag_pd(const double* __restrict__ X, double* __restrict__ Y,
+__global__ void __launch_bounds__(256) k_wfwd_diag_pd(const double* X, double* __restrict__ Y,
                                                       const double* __restrict__ panel, const double* __restrict__ linv,
                                                       const DFront* __restrict__ fr, const int64_t* __restrict__ order,
                                                       int64_t fr_off, int64_t S, int nbw_max,
-                                                      const double* __restrict__ V, const int32_t* __restrict__ imap) {
+                                                      const double* V, const int32_t* __restrict__ imap) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
     double* xB = sm + pd_slots(nbw_max) * NB * NB;  // [WS][R]
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(256) k_wfwd_diag_pd(const double* __restrict__
         const int p = threadIdx.x;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            double x = p < wb ? xs[p * R + r] : 0.0;
+            double x = p < wb ? __ldcg(xs + p * R + r) : 0.0;
             if (S == 0 && p < wb) x = kids_add(x, V, imap, f, p, R, r);
             xB[p * R + r] = x;
         }
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pd(double* __restrict__ Y, co
                                                       const int64_t* __restrict__ order, int64_t fr_off,
                                                       const int64_t* __restrict__ pre,
                                                       const int64_t* __restrict__ pre_part, int64_t S,
-                                                      const double* __restrict__ partial, int nbw_max,
+                                                      const double* partial, int nbw_max,
                                                       const double* __restrict__ d) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
@@ -800,8 +800,8 @@ __device__ __forceinline__ void mm_issue(double* sm, int tile, int ntile, const 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_mm_fwd_diag(const double* __restrict__ X, double* __restrict__ Y,
-                                                     const double* __restrict__ V, const T* __restrict__ panel,
+__global__ void __launch_bounds__(256) k_mm_fwd_diag(const double* X, double* __restrict__ Y,
+                                                     const double* V, const T* __restrict__ panel,
                                                      const double* __restrict__ linv, const DFront* __restrict__ fr,
                                                      const int64_t* __restrict__ order, int64_t fr_off, int64_t S,
                                                      int nrhs, int nbw_max, const int32_t* __restrict__ imap) {
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(256) k_mm_fwd_diag(const double* __restrict__ 
         const int p = e >> 3, n = e & 7;
         double x = 0.0;
         if (p < wb && n < rc) {
-            x = X[(f.start + J0 + p) * nrhs + j0 + n];
+            x = __ldcg(X + (f.start + J0 + p) * nrhs + j0 + n);
             if (S == 0) x = kids_add(x, V, imap, f, p, nrhs, j0 + n);
         }
         xB[p * MM_V + n] = x;
@@ -874,7 +874,7 @@ __global__ void __launch_bounds__(256) k_mm_fwd_diag(const double* __restrict__ 
 // CTA (two CTAs per PR-row chunk), warp w rows 8w ....
 template <typename T, int NT>
 __global__ void __launch_bounds__(256) k_mm_fwd_rows(double* __restrict__ X, double* __restrict__ V,
-                                                     const double* __restrict__ Y, const T* __restrict__ panel,
+                                                     const double* Y, const T* __restrict__ panel,
                                                      const DFront* __restrict__ fr, const int2* __restrict__ slots,
                                                      const int64_t* __restrict__ pre,
                                                      int64_t S, int nrhs, int cols, const int32_t* __restrict__ imap) {
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(256) k_mm_fwd_rows(double* __restrict__ X, dou
     const double* ys = Y + (f.start + J0) * nrhs;
     for (int e = threadIdx.x; e < cols * 8 * NT; e += 256) {
         const int p = e / (8 * NT), n = e % (8 * NT);
-        yB[p * VP + n] = (p < wb && n < nrhs) ? ys[p * nrhs + n] : 0.0;
+        yB[p * VP + n] = (p < wb && n < nrhs) ? __ldcg(ys + p * nrhs + n) : 0.0;
     }
     cp_async_wait<0>();
     __syncthreads();
@@ -928,7 +928,7 @@ __global__ void __launch_bounds__(256) k_mm_fwd_rows(double* __restrict__ X, dou
         for (int e = 0; e < 2; e++) {
             const int j = 8 * n + 2 * q + e;
             if (j >= nrhs) continue;
-            double x = (S > 0 || r < f.k) ? tgt[j] : 0.0;
+            double x = (S > 0 || r < f.k) ? __ldcg(tgt + j) : 0.0;
             if (S == 0) x = kids_add(x, V, imap, f, r, nrhs, j);
             tgt[j] = x - (acc[0][n][e] + acc[1][n][e]);
         }
@@ -937,7 +937,7 @@ __global__ void __launch_bounds__(256) k_mm_fwd_rows(double* __restrict__ X, dou
 // Backward partial sums: out[p][j] = Σ_rr L[r0+rr][J0+p]·y(r0+rr)[j] over a chunk's PR rows, one
 // block of partials per chunk; warp w takes the columns 8w + 64i ....
 template <typename T, int NT>
-__global__ void __launch_bounds__(256) k_mm_bwd_part(const double* __restrict__ Y, const T* __restrict__ panel,
+__global__ void __launch_bounds__(256) k_mm_bwd_part(const double* Y, const T* __restrict__ panel,
                                                      const DFront* __restrict__ fr, const int2* __restrict__ slots,
                                                      const int64_t* __restrict__ pre,
                                                      const int64_t* __restrict__ pre_part,
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(256) k_mm_bwd_part(const double* __restrict__ 
         double v = 0.0;
         if (rr < nr && n < nrhs) {
             const int64_t r = r0 + rr;
-            v = Y[(r < f.k ? f.start + r : rows[f.rows_off + r - f.k]) * nrhs + n];
+            v = __ldcg(Y + (r < f.k ? f.start + r : rows[f.rows_off + r - f.k]) * nrhs + n);
         }
         yr[rr * VP + n] = v;
     }
@@ -1021,7 +1021,7 @@ __global__ void __launch_bounds__(256) k_mm_bwd_diag(double* __restrict__ Y, con
                                                      const DFront* __restrict__ fr, const int64_t* __restrict__ order,
                                                      int64_t fr_off, const int64_t* __restrict__ pre,
                                                      const int64_t* __restrict__ pre_part, int64_t S, int nrhs,
-                                                     int nbw_max, const double* __restrict__ partial) {
+                                                     int nbw_max, const double* partial) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) double sm[];
     double* z = sm + mm_slots(nbw_max) * MM_TILE;  // [nbw·NB][MM_V]
@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(256) k_mm_bwd_diag(double* __restrict__ Y, con
                     for (int u = 0; u < 8; u++) v += t[u];
                 }
                 for (; c < nc; c++) v += __ldcg(pe + c * bs);
-                v = Y[(f.start + J0 + p) * nrhs + j0 + n] / d[f.start + J0 + p] - v;
+                v = __ldcg(Y + (f.start + J0 + p) * nrhs + j0 + n) / d[f.start + J0 + p] - v;
             }
             z[p * MM_V + n] = v;
         }

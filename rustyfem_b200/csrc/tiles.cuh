@@ -38,8 +38,8 @@ __device__ __forceinline__ double kids_add(double x, const double* V, const int3
                                            const DFront& f, int64_t p, int nrhs, int j) {
     if (f.imap_off < 0) return x;
     const int32_t i0 = imap[f.imap_off + p], i1 = imap[f.imap_off + f.m + p];
-    if (i0 >= 0) x += V[(f.kv0 + i0) * nrhs + j];
-    if (i1 >= 0) x += V[(f.kv1 + i1) * nrhs + j];
+    if (i0 >= 0) x += __ldcg(V + (f.kv0 + i0) * nrhs + j);
+    if (i1 >= 0) x += __ldcg(V + (f.kv1 + i1) * nrhs + j);
     return x;
 }
 
@@ -50,6 +50,13 @@ __device__ __forceinline__ double kids_add(double x, const double* V, const int3
 // reads or writes nothing that its predecessors produce or consume before it;
 // pdl_launch_dependents() lets the next kernel start once every CTA of this grid has
 // issued it.
+// A kernel that starts early shares its lifetime with the kernels that write its inputs. What an
+// earlier kernel of the chain wrote therefore never comes in as `const T* __restrict__` and is never
+// read by __ldg (either lets the compiler take the non-coherent path, which holds only for data that
+// nobody writes while the kernel lives): such parameters carry no __restrict__, and values that are
+// read once or staged in shared memory are read from L2 (__ldcg, cp.async.cg), whatever an SM's L1
+// kept from a kernel before. const __restrict__ stays on what is constant for the whole chain: the
+// plan's arrays and, in the sweeps, the factor.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
