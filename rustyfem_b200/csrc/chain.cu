@@ -9,15 +9,24 @@
 //   forward, block B of a front, CTA s owning the rows B·WS + 64s ... + 63:
 //       x_s = X[rows] + (children's V) − Σ_{J < B} L[rows, J]·y_J   (tile J as soon as block
 //             J's flag is up)
-//       x_B gathered from the cluster's CTAs (distributed shared memory),
-//       y[rows] = inv(L_BB)[rows, :]·x_B, then the block's flag is raised;
+//       y of the block (below), then the block's flag is raised;
 //   forward, later rows: V[rows] = (children's V) − Σ_J L[rows, J]·y_J over all blocks J;
 //   backward, block B, CTA s owning the columns B·WS + 64s ... + 63:
 //       z_s = Y[cols]/D − Σ_{r later} L[r, cols]·y_r − Σ_{J > B} L[J, cols]ᵀ·y_J,
-//       y[cols] = inv(L_BB)[:, cols]ᵀ·z_B.
+//       y of the block.
 // The tiles of a block stream through a ring of four cp.async stages while the CTA waits
 // for the flags; the dependency chain from block to block is one flag wait, the last
-// tile, a cluster barrier and one product with the WS × WS inverse.
+// tile and the solve with the block's diagonal block, for which two ways stand:
+//   FP32 factor: x_B (z_B) gathered from the cluster's CTAs (distributed shared memory) and one
+//       product with the explicit WS × WS inverse of L_BB (k_chain_inverse);
+//   FP64 factor: substitution over the CTAs in turn, forward y_s = inv(L_ss)·x_s with the
+//       factorization's 64 × 64 inverse, y_s to the CTAs after s, x_t −= L_ts·y_s there (backward
+//       the same from the last one, transposed). Three cluster barriers more in the chain from block to
+//       block (a solve call of the 33³ cube 1.57 ms, 1.42 with the inverse), for the rounding of the
+//       stepped sweeps: an FP64 solve is not refined unless the caller asks, and with the WS × WS
+//       inverse its residuals were 1.02 to 1.10 times as large in the 2-norm and up to 1.5 times in the
+//       maximum norm (means over right-hand sides; hex8 17³ to 45³, hex20 20³, one and six of them). Now
+//       0.98 to 1.003 and 0.95 to 1.06 times.
 //
 // Items are taken in the plan's order from a counter, by the first CTA of a cluster when
 // its previous item is done. Every item depends only on items before it in that order and
@@ -68,11 +77,10 @@ static_assert(CL == 4 && CT == 4 * CQ, "four CTAs of 256 threads per block");
 static_assert(CQ == CHAIN_PIECE, "the later-row pieces of the plan are one CTA's rows or columns");
 
 constexpr size_t fwd_smem(int R) {
-    return (size_t)CQ * FLP * 8 + (size_t)4 * CQ * FQP<float> * sizeof(float) + (size_t)WS * R * 8 + (size_t)CQ * R * 8;
+    return (size_t)CQ * FLP * 8 + (size_t)4 * CQ * FQP<float> * sizeof(float) + (size_t)2 * WS * R * 8;
 }
 constexpr size_t bwd_smem(int R) {
-    return (size_t)WS * CQ * 8 + (size_t)4 * BRC<float> * BTP * sizeof(float) + (size_t)4 * CQ * R * 8 + (size_t)WS * R * 8 +
-           (size_t)CQ * R * 8;
+    return (size_t)WS * CQ * 8 + (size_t)4 * BRC<float> * BTP * sizeof(float) + (size_t)4 * CQ * R * 8 + (size_t)2 * WS * R * 8;
 }
 static_assert(FQP<float> * sizeof(float) == FQP<double> * sizeof(double) && BRC<float> * sizeof(float) == BRC<double> * sizeof(double),
               "the rings of both precisions have one size");
@@ -146,6 +154,24 @@ __device__ __forceinline__ void quad_sum(double (&a)[R]) {
     }
 }
 
+// a += b, b = 0. The products of each block of WS rows or columns are summed by themselves before they
+// join the others: one running sum over thousands of terms rounds at the size of the whole sum each time
+// (hex20 20³, six right-hand sides, FP64: residual 2-norms 1.04 times those of the stepped sweeps so,
+// 1.00 now).
+template <int R>
+__device__ __forceinline__ void fold(double (&a)[R], double (&b)[R]) {
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        a[r] += b[r];
+        b[r] = 0.0;
+    }
+}
+template <int N>
+__device__ __forceinline__ void fold(double (&a)[N][2], double (&b)[N][2]) {
+#pragma unroll
+    for (int n = 0; n < N; n++) fold(a[n], b[n]);
+}
+
 // Forward tiles: acc (thread (i, q): row i, 16-byte groups q, q + 4, ... of each piece's row)
 // += Σ_{Q < nq} L[r0 + i, piece Q]·y over the pieces of the blocks 0, 1, ...; piece Q in
 // ring slot Q & 3, three pieces in flight. yload(j) fills yb with y_j (all threads,
@@ -163,10 +189,14 @@ __device__ __forceinline__ void fwd_tiles(double (&acc)[R], T* ring, double* yb,
         cp_async_commit();
     };
     for (int Q = 0; Q < min(3, nq); Q++) issue(Q);
+    double tot[R] = {};
     for (int Q = 0; Q < nq; Q++) {
         const int64_t j = Q / PB;
         const int qq = Q % PB;
-        if (qq == 0) yload(j);
+        if (qq == 0) {
+            fold(tot, acc);
+            yload(j);
+        }
         cp_wait_upto(min(2, nq - 1 - Q));
         __syncthreads();  // piece Q and y_j visible; every thread is done with piece Q − 1
         if (Q + 3 < nq) issue(Q + 3);
@@ -185,13 +215,44 @@ __device__ __forceinline__ void fwd_tiles(double (&acc)[R], T* ring, double* yb,
             }
         }
     }
+    fold(acc, tot);
+}
+
+// What CTA s of a forward block needs of the diagonal block, into Lv. FP32 factor: its rows of the
+// WS × WS inverse. FP64: its rows of L left of the diagonal (from prow) and inv(L_ss) after them.
+template <typename T>
+__device__ __forceinline__ void load_fwd_block(double* Lv, const double* inv, const T* prow, const DFront& f, int64_t cb,
+                                               int64_t b, int s, int nr) {
+    if constexpr (sizeof(T) == 4) {
+        const int cmax = CQ * (s + 1);  // inverse row 64s + i ends at the diagonal
+        cp_async_tile<double>(Lv, FLP, inv + (cb * WS + s * CQ) * (int64_t)WS, WS, CQ, cmax, CQ, cmax, CT);
+    } else {
+        if (nr <= 0) return;
+        if (s > 0) cp_async_tile<double>(Lv, FLP, prow, f.ldp, nr, CQ * s, CQ, CQ * s, CT);
+        cp_async_tile<double>(Lv + CQ * s, FLP, inv + (f.blk_off + CL * b + s) * (int64_t)(NB * NB), NB, NB, NB, NB, NB, CT);
+    }
+}
+
+// The same for the columns of a backward block, into Lc (rows of pitch P): FP32 its columns of the
+// inverse from the diagonal on; FP64 inv(L_ss), then its columns of L below (from pcol, nrr rows).
+template <typename T, int P>
+__device__ __forceinline__ void load_bwd_block(double* Lc, const double* inv, const T* pcol, const DFront& f, int64_t cb,
+                                               int64_t b, int s, int nc, int nrr) {
+    if constexpr (sizeof(T) == 4) {
+        const int ninv = WS - s * CQ;  // inverse column 64s + c starts at its diagonal row
+        cp_async_tile<double>(Lc, P, inv + (cb * WS + s * CQ) * (int64_t)WS + s * CQ, WS, ninv, CQ, ninv, CQ, CT);
+    } else {
+        if (nc <= 0) return;
+        cp_async_tile<double>(Lc, P, inv + (f.blk_off + CL * b + s) * (int64_t)(NB * NB), NB, NB, NB, NB, NB, CT);
+        if (nrr > 0) cp_async_tile<double>(Lc + CQ * P, P, pcol, f.ldp, nrr, nc, WS - CQ * (s + 1), CQ, CT);
+    }
 }
 
 template <typename T, int R>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     k_chain_fwd(const double* X, double* __restrict__ Y, const T* __restrict__ panel,
                 const double* V, const int32_t* __restrict__ imap,
-                const double* __restrict__ cinv, const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
+                const double* __restrict__ inv, const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
                 const int64_t* __restrict__ items, int64_t nitems, int* __restrict__ flags, int* __restrict__ counter,
                 int* __restrict__ err) {
     pdl_launch_dependents();
@@ -199,10 +260,11 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     cg::cluster_group cluster = cg::this_cluster();
     const int s = (int)cluster.block_rank();
     extern __shared__ __align__(16) double sm[];
-    double* Lv = sm;                                                   // [CQ][FLP]: inverse rows 64s ..
+    double* Lv = sm;                                                   // [CQ][FLP]: inverse rows 64s .., or L_st and inv(L_ss)
     T* ring = reinterpret_cast<T*>(sm + CQ * FLP);                     // [4][CQ][FQP]: tile pieces
     double* yb = reinterpret_cast<double*>(ring + 4 * CQ * FQP<T>);    // [WS][R]: y_J, then x_B
     double* xo = yb + WS * R;                                          // [CQ][R]: this CTA's rows of x_B
+    double* yr = xo + CQ * R;                                          // [WS - CQ][R]: y_t of the cluster's other CTAs
     __shared__ int64_t s_item;
     const int tid = threadIdx.x, i = tid >> 2, q = tid & 3;
     for (;;) {
@@ -213,8 +275,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
         const int64_t cb0 = chain_blk[t];
         const int64_t r0 = b * WS + s * CQ;
         const int nr = (int)max((int64_t)0, min((int64_t)CQ, f.k - r0));
-        const int cmax = CQ * (s + 1);  // inverse row 64s + i ends at the diagonal
-        cp_async_tile<double>(Lv, FLP, cinv + ((cb0 + b) * WS + s * CQ) * (int64_t)WS, WS, CQ, cmax, CQ, cmax, CT);
+        load_fwd_block<T>(Lv, inv, panel + f.poff + r0 * f.ldp + b * WS, f, cb0 + b, b, s, nr);
         cp_async_commit();
         double acc[R];
 #pragma unroll
@@ -233,25 +294,68 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
                 xo[i * R + r] =
                     i < nr ? kids_add(__ldcg(X + (f.start + r0 + i) * R + r), V, imap, f, r0 + i, R, r) - acc[r] : 0.0;
         }
-        cluster.sync();
-        for (int e = tid; e < WS * R; e += CT) {
-            const int rk = e / (CQ * R);
-            yb[e] = cluster.map_shared_rank(xo, rk)[e - rk * CQ * R];
-        }
-        cp_async_wait<0>();
-        __syncthreads();
+        // a = Σ_c Lv[i, c0 + c]·v[c] over n columns, a multiple of CQ
+        auto row_product = [&](double (&a)[R], int c0, int n, const double* v) {
+            double a2[R] = {};
+#pragma unroll
+            for (int r = 0; r < R; r++) a[r] = 0.0;
+            for (int cb = 0; cb < n; cb += CQ) {
+#pragma unroll
+                for (int u = 0; u < CQ / 4; u += 2) {
+                    const int c = cb + q + 4 * u;
+                    const double l0 = Lv[i * FLP + c0 + c], l1 = Lv[i * FLP + c0 + c + 4];
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        a[r] = fma(l0, v[c * R + r], a[r]);
+                        a2[r] = fma(l1, v[(c + 4) * R + r], a2[r]);
+                    }
+                }
+            }
+            fold(a, a2);
+            quad_sum<R>(a);
+        };
+        auto put_y = [&](const double (&a)[R]) {
+            if (q == 0 && i < nr) {
+#pragma unroll
+                for (int r = 0; r < R; r++) Y[(f.start + r0 + i) * R + r] = a[r];
+            }
+        };
         double a[R];
+        if constexpr (sizeof(T) == 4) {
+            cluster.sync();
+            for (int e = tid; e < WS * R; e += CT) {
+                const int rk = e / (CQ * R);
+                yb[e] = cluster.map_shared_rank(xo, rk)[e - rk * CQ * R];
+            }
+            cp_async_wait<0>();
+            __syncthreads();
+            row_product(a, 0, CQ * (s + 1), yb);  // inverse row 64s + i ends at the diagonal
+            put_y(a);
+        } else {
+            cp_async_wait<0>();
+            __syncthreads();
+            const int nsub = (int)min((int64_t)CL, (f.k - b * WS + CQ - 1) / CQ);
+            for (int t = 0; t < nsub; t++) {
+                if (s == t) {
+                    row_product(a, CQ * t, CQ, xo);
+                    put_y(a);
+                    if (q > t) {  // the lanes of a row take a rank each
+                        double* o = cluster.map_shared_rank(yr, q) + (CQ * t + i) * R;
 #pragma unroll
-        for (int r = 0; r < R; r++) a[r] = 0.0;
-        for (int c = q; c < cmax; c += 4) {
-            const double l = Lv[i * FLP + c];
+                        for (int r = 0; r < R; r++) o[r] = a[r];
+                    }
+                }
+                if (t + 1 == nsub) break;
+                cluster.sync();
+                if (s > t && s < nsub) {
+                    row_product(a, CQ * t, CQ, yr + CQ * t * R);
+                    if (q == 0) {
 #pragma unroll
-            for (int r = 0; r < R; r++) a[r] = fma(l, yb[c * R + r], a[r]);
-        }
-        quad_sum<R>(a);
-        if (q == 0 && i < nr) {
-#pragma unroll
-            for (int r = 0; r < R; r++) Y[(f.start + r0 + i) * R + r] = a[r];
+                        for (int r = 0; r < R; r++) xo[i * R + r] -= a[r];
+                    }
+                    __syncthreads();
+                }
+            }
         }
         chain_signal(&flags[cb0 + b]);
         cluster.sync();  // the cluster's x_B pieces may be overwritten after this
@@ -310,9 +414,11 @@ __device__ __forceinline__ void bwd_tiles(double (&acc)[R], T* ring, const T* pc
         cp_async_commit();
     };
     for (int h = 0; h < min(3, nh); h++) issue(h);
+    double tot[R] = {};
     for (int h = 0; h < nh; h++) {
         int64_t ra;
         const int nrr = rows_of(h, ra);
+        if (h % BPB<T> == 0) fold(tot, acc);
         const double* yv = yload(h);
         cp_wait_upto(min(2, nh - 1 - h));
         __syncthreads();  // chunk h visible; every thread is done with chunk h − 1
@@ -328,6 +434,7 @@ __device__ __forceinline__ void bwd_tiles(double (&acc)[R], T* ring, const T* pc
             }
         }
     }
+    fold(acc, tot);
 }
 
 // Σ over the four row groups of a column, in group order (threads tid < CQ get the total
@@ -362,7 +469,7 @@ __device__ __forceinline__ double chain_z(const double* Y, const double* d, cons
 
 template <typename T, int R>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
-    k_chain_bwd(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ cinv,
+    k_chain_bwd(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ inv,
                 const double* __restrict__ d, const double* part, const int64_t* __restrict__ colbase,
                 const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk, const int64_t* __restrict__ items,
                 int64_t nitems, int* __restrict__ flags, int* __restrict__ counter, int* __restrict__ err) {
@@ -371,11 +478,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     cg::cluster_group cluster = cg::this_cluster();
     const int s = (int)cluster.block_rank();
     extern __shared__ __align__(16) double sm[];
-    double* Lc = sm;                                               // [WS][CQ]: rows 64s .. of inverse columns 64s ..
+    double* Lc = sm;                                               // [WS][CQ]: rows 64s .. of inverse columns 64s .., or inv(L_ss) and L_ts
     T* ring = reinterpret_cast<T*>(sm + WS * CQ);                  // [4][BRC][BTP]: tile chunks
     double* yp = reinterpret_cast<double*>(ring + 4 * BRC<T> * BTP);  // [WS][R]: y of a later block; then z_B
     double* red = yp + WS * R;                                     // [4][CQ][R]
     double* zo = red + 4 * CQ * R;                                 // [CQ][R]: this CTA's columns of z_B
+    double* yr = zo + CQ * R;                                      // [WS - CQ][R]: y_t of the cluster's other CTAs
     __shared__ int64_t s_item;
     const int tid = threadIdx.x, c = tid & (CQ - 1), g = tid >> 6;
     for (;;) {
@@ -387,9 +495,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
         const int64_t col0 = b * WS + s * CQ;
         const int nc = (int)max((int64_t)0, min((int64_t)CQ, f.k - col0));
         const int64_t nb = (f.k + WS - 1) / WS;
-        const int ninv = WS - s * CQ;  // inverse column 64s + c starts at its diagonal row
-        cp_async_tile<double>(Lc, CQ, cinv + ((cb0 + b) * WS + s * CQ) * (int64_t)WS + s * CQ, WS, ninv, CQ, ninv, CQ,
-                              CT);
+        const int wb = (int)min((int64_t)WS, f.k - b * WS);
+        load_bwd_block<T, CQ>(Lc, inv, panel + f.poff + (b * WS + CQ * (s + 1)) * f.ldp + col0, f, cb0 + b, b, s, nc,
+                              wb - CQ * (s + 1));
         cp_async_commit();
         double acc[R];
 #pragma unroll
@@ -419,26 +527,70 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
             for (int r = 0; r < R; r++)
                 zo[c * R + r] = c < nc ? chain_z(Y, d, part, colbase[t], f, col0 + c, R, r) - acc[r] : 0.0;
         }
-        cluster.sync();
-        double* zf = yp;
-        for (int e = tid; e < WS * R; e += CT) {
-            const int rk = e / (CQ * R);
-            zf[e] = cluster.map_shared_rank(zo, rk)[e - rk * CQ * R];
-        }
-        cp_async_wait<0>();
-        __syncthreads();
+        // threads tid < CQ: a = Σ_rr Lc[r0 + rr, c]·v[rr] over n rows, a multiple of CQ
+        auto col_product = [&](double (&a)[R], int r0, int n, const double* v) {
+            double a2[R] = {};
+#pragma unroll
+            for (int r = 0; r < R; r++) a[r] = 0.0;
+            for (int rb = 0; rb < n; rb += CQ) {
+#pragma unroll
+                for (int u = 0; u < CQ / 4; u += 2) {
+                    const int rr = rb + g + 4 * u;
+                    const double l0 = Lc[(r0 + rr) * CQ + c], l1 = Lc[(r0 + rr + 4) * CQ + c];
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        a[r] = fma(l0, v[rr * R + r], a[r]);
+                        a2[r] = fma(l1, v[(rr + 4) * R + r], a2[r]);
+                    }
+                }
+            }
+            fold(a, a2);
+            col_sum<R>(a, red);
+        };
+        auto put_y = [&](const double (&a)[R]) {
+            if (tid < nc) {
+#pragma unroll
+                for (int r = 0; r < R; r++) Y[(f.start + col0 + c) * R + r] = a[r];
+            }
+        };
         double a[R];
+        if constexpr (sizeof(T) == 4) {
+            cluster.sync();
+            double* zf = yp;
+            for (int e = tid; e < WS * R; e += CT) {
+                const int rk = e / (CQ * R);
+                zf[e] = cluster.map_shared_rank(zo, rk)[e - rk * CQ * R];
+            }
+            cp_async_wait<0>();
+            __syncthreads();
+            col_product(a, 0, WS - s * CQ, zf + s * CQ * R);
+            put_y(a);
+        } else {
+            cp_async_wait<0>();
+            __syncthreads();
+            for (int t = (wb + CQ - 1) / CQ - 1; t >= 0; t--) {
+                if (s == t) {
+                    col_product(a, 0, CQ, zo);
+                    put_y(a);
+                    if (tid < CQ) {
+                        for (int rk = 0; rk < t; rk++) {
+                            double* o = cluster.map_shared_rank(yr, rk) + (CQ * (t - 1) + c) * R;
 #pragma unroll
-        for (int r = 0; r < R; r++) a[r] = 0.0;
-        for (int rr = g; rr < ninv; rr += 4) {
-            const double l = Lc[rr * CQ + c];
+                            for (int r = 0; r < R; r++) o[r] = a[r];
+                        }
+                    }
+                }
+                if (t == 0) break;
+                cluster.sync();
+                if (s < t) {
+                    col_product(a, CQ * (t - s), CQ, yr + CQ * (t - 1) * R);
+                    if (tid < CQ) {
 #pragma unroll
-            for (int r = 0; r < R; r++) a[r] = fma(l, zf[(s * CQ + rr) * R + r], a[r]);
-        }
-        col_sum<R>(a, red);
-        if (tid < nc) {
-#pragma unroll
-            for (int r = 0; r < R; r++) Y[(f.start + col0 + c) * R + r] = a[r];
+                        for (int r = 0; r < R; r++) zo[c * R + r] -= a[r];
+                    }
+                    __syncthreads();
+                }
+            }
         }
         chain_signal(&flags[cb0 + b]);
         cluster.sync();  // the cluster's z_B pieces may be overwritten after this
@@ -541,7 +693,7 @@ __device__ __forceinline__ int vsw(int k, int n) { return k * MG + (n ^ ((k & 2)
 template <typename T>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
     k_chain_fwd_mm(const double* X, double* __restrict__ Y, const T* __restrict__ panel,
-                   const double* V, const int32_t* __restrict__ imap, const double* __restrict__ cinv,
+                   const double* V, const int32_t* __restrict__ imap, const double* __restrict__ inv,
                    const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
                    const int64_t* __restrict__ items, int64_t nitems, int nrhs, int64_t nblocks,
                    int* __restrict__ flags0, int* __restrict__ counter, int* __restrict__ err) {
@@ -567,9 +719,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
         int* flags = flags0 + jg * nblocks + chain_blk[t];
         const int64_t r0 = b * WS + s * CQ;
         const int nr = (int)max((int64_t)0, min((int64_t)CQ, f.k - r0));
-        const int cmax = CQ * (s + 1);  // inverse row 64s + i ends at the diagonal
-        cp_async_tile<double>(Lv, FLP, cinv + ((chain_blk[t] + b) * WS + s * CQ) * (int64_t)WS, WS, CQ, cmax, CQ, cmax,
-                              CT);
+        load_fwd_block<T>(Lv, inv, panel + f.poff + r0 * f.ldp + b * WS, f, chain_blk[t] + b, b, s, nr);
         cp_async_commit();
         const T* prow = panel + f.poff + r0 * f.ldp;
         const int nq = PB * (int)b;
@@ -577,10 +727,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
             if (nr > 0) cp_async_tile<T>(ring + (Q & 3) * CQ * QP, QP, prow + (int64_t)Q * QC, f.ldp, nr, QC, CQ, QC, CT);
             cp_async_commit();
         };
-        double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+        double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0}, tot[2] = {0.0, 0.0};
         for (int Q = 0; Q < min(3, nq); Q++) issue(Q);
         for (int Q = 0; Q < nq; Q++) {
             if (Q % PB == 0) {
+                fold(a0, a1);
+                fold(tot, a0);
                 const int64_t j = Q / PB;
                 if (tid == 0) chain_wait(&flags[j], CL, err);
                 __syncthreads();
@@ -603,34 +755,69 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
                 }
             }
         }
-        __syncthreads();  // the ring is idle: it takes x_s
+        double x[2];  // row 8w + g of x_s, right-hand sides 2q, 2q + 1
+        const int i = 8 * w + g;
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-            const int i = 8 * w + g, n = 2 * q + e;
-            double x = 0.0;
+            const int n = 2 * q + e;
+            x[e] = 0.0;
             if (i < nr && n < rc)
-                x = kids_add(__ldcg(X + (f.start + r0 + i) * nrhs + j0 + n), V, imap, f, r0 + i, nrhs, j0 + n) - (a0[e] + a1[e]);
-            xo[i * MG + n] = x;
+                x[e] = kids_add(__ldcg(X + (f.start + r0 + i) * nrhs + j0 + n), V, imap, f, r0 + i, nrhs, j0 + n) - (tot[e] + (a0[e] + a1[e]));
         }
-        cluster.sync();
-        for (int e = tid; e < WS * MG; e += CT) {
-            const int k = e / MG;
-            yb[vsw(k, e % MG)] = cluster.map_shared_rank(xo, k / CQ)[e - (k / CQ) * CQ * MG];
-        }
-        cp_async_wait<0>();
-        __syncthreads();
-        {
+        // y = Σ_k Lv[i, k0 + k]·yb[k0 + k] over n columns
+        double y[2];
+        auto row_product = [&](int k0, int n) {
             double acc[2][2] = {};
-            const double* Lr = Lv + (8 * w + g) * FLP + q;
-            const int kmax = s * CQ + 8 * w + 8;  // the inverse rows 8w .. 8w+7 end at their diagonal
-            for (int k = 0; k < kmax; k += 8) {
-                dmma_884(acc[0][0], acc[0][1], Lr[k], yb[vsw(k + q, g)]);
-                dmma_884(acc[1][0], acc[1][1], Lr[k + 4], yb[vsw(k + 4 + q, g)]);
+            const double* Lr = Lv + (8 * w + g) * FLP + q + k0;
+            for (int k = 0; k < n; k += 8) {
+                dmma_884(acc[0][0], acc[0][1], Lr[k], yb[vsw(k0 + k + q, g)]);
+                dmma_884(acc[1][0], acc[1][1], Lr[k + 4], yb[vsw(k0 + k + 4 + q, g)]);
             }
+            y[0] = acc[0][0] + acc[1][0];
+            y[1] = acc[0][1] + acc[1][1];
+        };
+        auto put_y = [&] {
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int i = 8 * w + g, n = 2 * q + e;
-                if (i < nr && n < rc) Y[(f.start + r0 + i) * nrhs + j0 + n] = acc[0][e] + acc[1][e];
+            for (int e = 0; e < 2; e++)
+                if (i < nr && 2 * q + e < rc) Y[(f.start + r0 + i) * nrhs + j0 + 2 * q + e] = y[e];
+        };
+        __syncthreads();  // the ring is idle: it takes x_s
+        if constexpr (sizeof(T) == 4) {
+            xo[i * MG + 2 * q] = x[0];
+            xo[i * MG + 2 * q + 1] = x[1];
+            cluster.sync();
+            for (int e = tid; e < WS * MG; e += CT) {
+                const int k = e / MG;
+                yb[vsw(k, e % MG)] = cluster.map_shared_rank(xo, k / CQ)[e - (k / CQ) * CQ * MG];
+            }
+            cp_async_wait<0>();
+            __syncthreads();
+            row_product(0, s * CQ + 8 * w + 8);  // the inverse rows 8w .. 8w+7 end at their diagonal
+            put_y();
+        } else {
+            cp_async_wait<0>();
+            cluster.sync();  // every CTA is past its tiles: y_t comes into the rows 64t of yb, x_s stands in its own
+            const int nsub = (int)min((int64_t)CL, (f.k - b * WS + CQ - 1) / CQ);
+            for (int t = 0; t < nsub; t++) {
+                if (s == t) {
+                    yb[vsw(CQ * t + i, 2 * q)] = x[0];
+                    yb[vsw(CQ * t + i, 2 * q + 1)] = x[1];
+                    __syncthreads();
+                    row_product(CQ * t, 8 * w + 8);
+                    put_y();
+                    for (int rk = t + 1; rk < nsub; rk++) {
+                        double* o = cluster.map_shared_rank(yb, rk);
+                        o[vsw(CQ * t + i, 2 * q)] = y[0];
+                        o[vsw(CQ * t + i, 2 * q + 1)] = y[1];
+                    }
+                }
+                if (t + 1 == nsub) break;
+                cluster.sync();
+                if (s > t && s < nsub) {
+                    row_product(CQ * t, CQ);
+                    x[0] -= y[0];
+                    x[1] -= y[1];
+                }
             }
         }
         chain_signal(&flags[b]);
@@ -640,7 +827,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
 
 template <typename T>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
-    k_chain_bwd_mm(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ cinv,
+    k_chain_bwd_mm(double* __restrict__ Y, const T* __restrict__ panel, const double* __restrict__ inv,
                    const double* __restrict__ d, const double* part, const int64_t* __restrict__ colbase,
                    const DFront* __restrict__ fr, const int64_t* __restrict__ chain_blk,
                    const int64_t* __restrict__ items, int64_t nitems, int nrhs, int64_t nblocks,
@@ -668,9 +855,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
         const int64_t col0 = b * WS + s * CQ;
         const int nc = (int)max((int64_t)0, min((int64_t)CQ, f.k - col0));
         const int64_t nb = (f.k + WS - 1) / WS;
-        const int ninv = WS - s * CQ;  // inverse column 64s + c starts at its diagonal row
-        cp_async_tile<double>(Lc, MLP, cinv + ((chain_blk[t] + b) * WS + s * CQ) * (int64_t)WS + s * CQ, WS, ninv, CQ,
-                              ninv, CQ, CT);
+        const int wb = (int)min((int64_t)WS, f.k - b * WS);
+        load_bwd_block<T, MLP>(Lc, inv, panel + f.poff + (b * WS + CQ * (s + 1)) * f.ldp + col0, f, chain_blk[t] + b, b, s,
+                               nc, wb - CQ * (s + 1));
         cp_async_commit();
         // the chunks of blocks nb − 1, ..., b + 1, PB per block
         const T* pcol = panel + f.poff + col0;
@@ -683,10 +870,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
                                  CT);
             cp_async_commit();
         };
-        double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0};
+        double a0[2] = {0.0, 0.0}, a1[2] = {0.0, 0.0}, tot[2] = {0.0, 0.0};
         for (int h = 0; h < min(3, nh); h++) issue(h);
         for (int h = 0; h < nh; h++) {
             if (h % PB == 0) {
+                fold(a0, a1);
+                fold(tot, a0);
                 const int64_t bb = nb - 1 - h / PB;
                 if (tid == 0) chain_wait(&flags[bb], CL, err);
                 __syncthreads();
@@ -710,32 +899,66 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
                 }
             }
         }
-        __syncthreads();  // the ring is idle: it takes z_s
+        double z[2];  // column 8w + g of z_s, right-hand sides 2q, 2q + 1
+        const int c = 8 * w + g;
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-            const int c = 8 * w + g, n = 2 * q + e;
-            zo[c * MG + n] =
-                c < nc && n < rc ? chain_z(Y, d, part, colbase[t], f, col0 + c, nrhs, j0 + n) - (a0[e] + a1[e]) : 0.0;
+            const int n = 2 * q + e;
+            z[e] = c < nc && n < rc ? chain_z(Y, d, part, colbase[t], f, col0 + c, nrhs, j0 + n) - (tot[e] + (a0[e] + a1[e])) : 0.0;
         }
-        cluster.sync();
-        for (int e = tid; e < WS * MG; e += CT) {
-            const int k = e / MG;
-            yp[vsw(k, e % MG)] = cluster.map_shared_rank(zo, k / CQ)[e - (k / CQ) * CQ * MG];
-        }
-        cp_async_wait<0>();
-        __syncthreads();
-        {
+        // y = Σ_k Lc[k, c]·yp[64s + k] over the rows [k0, k1) (relative to 64s)
+        double y[2];
+        auto col_product = [&](int k0, int k1) {
             double acc[2][2] = {};
             const double* Lq = Lc + q * MLP + 8 * w + g;
-            // inverse columns 64s + 8w ...: rows from 8w (relative to 64s) to the block's end
-            for (int k = 8 * w; k < ninv; k += 8) {
+            for (int k = k0; k < k1; k += 8) {
                 dmma_884(acc[0][0], acc[0][1], Lq[k * MLP], yp[vsw(s * CQ + k + q, g)]);
                 dmma_884(acc[1][0], acc[1][1], Lq[(k + 4) * MLP], yp[vsw(s * CQ + k + 4 + q, g)]);
             }
+            y[0] = acc[0][0] + acc[1][0];
+            y[1] = acc[0][1] + acc[1][1];
+        };
+        auto put_y = [&] {
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int c = 8 * w + g, n = 2 * q + e;
-                if (c < nc && n < rc) Y[(f.start + col0 + c) * nrhs + j0 + n] = acc[0][e] + acc[1][e];
+            for (int e = 0; e < 2; e++)
+                if (c < nc && 2 * q + e < rc) Y[(f.start + col0 + c) * nrhs + j0 + 2 * q + e] = y[e];
+        };
+        __syncthreads();  // the ring is idle: it takes z_s
+        if constexpr (sizeof(T) == 4) {
+            zo[c * MG + 2 * q] = z[0];
+            zo[c * MG + 2 * q + 1] = z[1];
+            cluster.sync();
+            for (int e = tid; e < WS * MG; e += CT) {
+                const int k = e / MG;
+                yp[vsw(k, e % MG)] = cluster.map_shared_rank(zo, k / CQ)[e - (k / CQ) * CQ * MG];
+            }
+            cp_async_wait<0>();
+            __syncthreads();
+            col_product(8 * w, WS - s * CQ);  // the inverse's columns start at their diagonal
+            put_y();
+        } else {
+            cp_async_wait<0>();
+            cluster.sync();  // every CTA is past its tiles: y_t comes into the rows 64t of yp, z_s stands in its own
+            for (int t = (wb + CQ - 1) / CQ - 1; t >= 0; t--) {
+                if (s == t) {
+                    yp[vsw(CQ * t + c, 2 * q)] = z[0];
+                    yp[vsw(CQ * t + c, 2 * q + 1)] = z[1];
+                    __syncthreads();
+                    col_product(8 * w, CQ);
+                    put_y();
+                    for (int rk = 0; rk < t; rk++) {
+                        double* o = cluster.map_shared_rank(yp, rk);
+                        o[vsw(CQ * t + c, 2 * q)] = y[0];
+                        o[vsw(CQ * t + c, 2 * q + 1)] = y[1];
+                    }
+                }
+                if (t == 0) break;
+                cluster.sync();
+                if (s < t) {
+                    col_product(CQ * (t - s), CQ * (t - s) + CQ);
+                    z[0] -= y[0];
+                    z[1] -= y[1];
+                }
             }
         }
         chain_signal(&flags[b]);
@@ -791,9 +1014,10 @@ __global__ void __launch_bounds__(CT) k_chain_rows_mm(const double* Y, double* _
         vec_piece<NT>(yr + (Q & 3) * QC * VP, Y + (f.start + c0) * nrhs, ncol, nrhs, QC);
         cp_async_commit();
     };
-    double acc[NT][2] = {};
+    double acc[NT][2] = {}, tot[NT][2] = {};
     for (int Q = 0; Q < min(3, nq); Q++) issue(Q);
     for (int Q = 0; Q < nq; Q++) {
+        if (Q % FPB<T> == 0) fold(tot, acc);
         cp_wait_upto(min(2, nq - 1 - Q));
         __syncthreads();
         if (Q + 3 < nq) issue(Q + 3);
@@ -814,7 +1038,7 @@ __global__ void __launch_bounds__(CT) k_chain_rows_mm(const double* Y, double* _
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 const int j = n * MG + 2 * q + e;
-                if (j < nrhs) vt[j] = kids_add(0.0, V, imap, f, r0 + i, nrhs, j) - acc[n][e];
+                if (j < nrhs) vt[j] = kids_add(0.0, V, imap, f, r0 + i, nrhs, j) - (tot[n][e] + acc[n][e]);
             }
     }
 }
@@ -844,9 +1068,10 @@ __global__ void __launch_bounds__(CT) k_chain_cols_mm(double* __restrict__ part,
         vec_piece<NT>(yr + (h & 3) * RC * VP, V + (f.vuoff + ra) * nrhs, nrr, nrhs, RC);
         cp_async_commit();
     };
-    double acc[NT][2] = {};
+    double acc[NT][2] = {}, tot[NT][2] = {};
     for (int h = 0; h < min(3, nh); h++) issue(h);
     for (int h = 0; h < nh; h++) {
+        if (h % BPB<T> == 0) fold(tot, acc);
         cp_wait_upto(min(2, nh - 1 - h));
         __syncthreads();
         if (h + 3 < nh) issue(h + 3);
@@ -865,7 +1090,7 @@ __global__ void __launch_bounds__(CT) k_chain_cols_mm(double* __restrict__ part,
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int j = n * MG + 2 * q + e;
-            if (j < nrhs) out[j] = acc[n][e];
+            if (j < nrhs) out[j] = tot[n][e] + acc[n][e];
         }
 }
 
@@ -874,11 +1099,11 @@ __global__ void __launch_bounds__(CT) k_chain_cols_mm(double* __restrict__ part,
 // The block columns are independent: one CTA (8 warps of 32×16 outputs) each, its M_tj kept
 // in shared memory, the products on the FP64 tensor-core path. It is bound by the chain of
 // 64³ products of block column 0 (nine for a full block) and by the loads of L between them.
+// For an FP32 factor; an FP64 one is solved by substitution (the head of this file).
 constexpr int IVP = NB + 4;  // pitch (doubles): fragment loads of both operands without conflicts
 constexpr size_t INV_SMEM = (size_t)5 * NB * IVP * sizeof(double);
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_chain_inverse(double* __restrict__ cinv, const T* __restrict__ panel,
+__global__ void __launch_bounds__(256) k_chain_inverse(double* __restrict__ cinv, const float* __restrict__ panel,
                                                        const double* __restrict__ linv, const DFront* __restrict__ fr,
                                                        const int64_t* __restrict__ chain_blk,
                                                        const int64_t* __restrict__ chain_bfront) {
@@ -1007,7 +1232,6 @@ void set_chain_attrs(ChainDev& d) {
 }
 template <typename T>
 void set_chain_attrs_all(ChainDev& d) {
-    set_smem(k_chain_inverse<T>, INV_SMEM);
     set_chain_attrs<T, 1>(d);
     set_chain_attrs<T, 2>(d);
     set_chain_attrs<T, 3>(d);
@@ -1025,6 +1249,7 @@ const ChainDev& chain_dev() {
     std::lock_guard<std::mutex> lock(mu);
     ChainDev& d = devs[dev];
     if (!d.done) {
+        set_smem(k_chain_inverse, INV_SMEM);
         set_chain_attrs_all<float>(d);
         set_chain_attrs_all<double>(d);
         d.done = true;
@@ -1037,19 +1262,24 @@ unsigned grid_for_items(int fit, int64_t nitems) {
     return (unsigned)(std::min<int64_t>(fit, nitems) * CL);
 }
 
+// what the chains multiply by in a block's solve
+template <typename T>
+const double* block_inverses(const ChainArgs& c) {
+    return sizeof(T) == 8 ? c.linv : c.cinv;
+}
+
 void check_nrhs(int nrhs) {
     if (nrhs < 1 || nrhs > 4 * MG) throw CudaError("solve chain: 1 to 32 right-hand sides");
 }
 
 }  // namespace
 
-template <typename T>
-void launch_chain_inverse(double* cinv, const T* panel, const double* linv, const DFront* fronts,
+void launch_chain_inverse(double* cinv, const float* panel, const double* linv, const DFront* fronts,
                           const int64_t* chain_blk, const int64_t* chain_bfront, int64_t nblocks, cudaStream_t st) {
     if (nblocks <= 0) return;
     chain_dev();
-    k_chain_inverse<T><<<dim3((unsigned)nblocks, CL), 256, INV_SMEM, st>>>(cinv, panel, linv, fronts, chain_blk,
-                                                                          chain_bfront);
+    k_chain_inverse<<<dim3((unsigned)nblocks, CL), 256, INV_SMEM, st>>>(cinv, panel, linv, fronts, chain_blk,
+                                                                       chain_bfront);
     RFG_CUDA(cudaGetLastError());
 }
 
@@ -1080,12 +1310,12 @@ void launch_chain_fwd(int nrhs, int64_t nitems, const double* X, double* Y, cons
     if (nrhs > 4) {
         const int64_t n = nitems * ((nrhs + MG - 1) / MG);
         launch_pdl(true, k_chain_fwd_mm<T>, dim3(grid_for_items(d.fwd[chain_kind<T>][0], n)), dim3(CT), mm_fwd_smem<T>,
-                   st, X, Y, panel, V, c.imap, c.cinv, c.fronts, c.blk, items, nitems, nrhs, c.nblocks, flags, counter,
+                   st, X, Y, panel, V, c.imap, block_inverses<T>(c), c.fronts, c.blk, items, nitems, nrhs, c.nblocks, flags, counter,
                    c.err);
         return;
     }
     RFG_CHAIN_BY_R(nrhs, launch_pdl(true, k_chain_fwd<T, R>, dim3(grid_for_items(d.fwd[chain_kind<T>][R], nitems)),
-                                    dim3(CT), fwd_smem(R), st, X, Y, panel, V, c.imap, c.cinv, c.fronts, c.blk, items,
+                                    dim3(CT), fwd_smem(R), st, X, Y, panel, V, c.imap, block_inverses<T>(c), c.fronts, c.blk, items,
                                     nitems, flags, counter, c.err));
 }
 
@@ -1134,20 +1364,18 @@ void launch_chain_bwd(int nrhs, int64_t nitems, double* Y, const double* part, c
     if (nrhs > 4) {
         const int64_t n = nitems * ((nrhs + MG - 1) / MG);
         launch_pdl(true, k_chain_bwd_mm<T>, dim3(grid_for_items(d.bwd[chain_kind<T>][0], n)), dim3(CT), mm_bwd_smem<T>,
-                   st, Y, panel, c.cinv, c.d, part, c.colbase, c.fronts, c.blk, items, nitems, nrhs, c.nblocks, flags,
+                   st, Y, panel, block_inverses<T>(c), c.d, part, c.colbase, c.fronts, c.blk, items, nitems, nrhs, c.nblocks, flags,
                    counter, c.err);
         return;
     }
     RFG_CHAIN_BY_R(nrhs, launch_pdl(true, k_chain_bwd<T, R>, dim3(grid_for_items(d.bwd[chain_kind<T>][R], nitems)),
-                                    dim3(CT), bwd_smem(R), st, Y, panel, c.cinv, c.d, part, c.colbase, c.fronts, c.blk,
+                                    dim3(CT), bwd_smem(R), st, Y, panel, block_inverses<T>(c), c.d, part, c.colbase, c.fronts, c.blk,
                                     items, nitems, flags, counter, c.err));
 }
 
 #undef RFG_CHAIN_BY_R
 
 #define RFG_CHAIN_INSTANCE(T)                                                                                        \
-    template void launch_chain_inverse<T>(double*, const T*, const double*, const DFront*, const int64_t*,           \
-                                          const int64_t*, int64_t, cudaStream_t);                                    \
     template void launch_chain_fwd<T>(int, int64_t, const double*, double*, const double*, const T*,                 \
                                       const ChainArgs&, const int64_t*, int*, int*, cudaStream_t);                   \
     template void launch_chain_rows<T>(int, int64_t, const double*, double*, const T*, const ChainArgs&,             \

@@ -29,7 +29,8 @@ struct ChainArgs {
     const int32_t* imap;     // DevPlan::imap
     const int64_t* blk;      // Plan::chain_blk
     const int64_t* colbase;  // Plan::chain_colbase
-    const double* cinv;      // the blocks' inverses
+    const double* linv;      // inverses of the NB × NB diagonal blocks (FP64 factor)
+    const double* cinv;      // inverses of the chain blocks (FP32 factor)
     const double* d;         // pivots
     int64_t nblocks;         // Plan::chain_blocks
     int* err;                // set to 1 when a wait gave up (sticky)
@@ -37,9 +38,8 @@ struct ChainArgs {
 
 // The inverse of every chain block's unit-lower diagonal block, WS × WS in FP64 (row-major,
 // zero above the diagonal and beyond the block's width), from the NB × NB inverses of the
-// factorization and the factor: cinv[(cb·WS + r)·WS + c].
-template <typename T>
-void launch_chain_inverse(double* cinv, const T* panel, const double* linv, const DFront* fronts,
+// factorization and the FP32 factor: cinv[(cb·WS + r)·WS + c].
+void launch_chain_inverse(double* cinv, const float* panel, const double* linv, const DFront* fronts,
                           const int64_t* chain_blk, const int64_t* chain_bfront, int64_t nblocks, cudaStream_t st);
 
 // Forward chain of one level: Y[pivot rows] = L⁻¹ x for the level's fronts, x = X plus the

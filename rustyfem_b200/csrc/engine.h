@@ -182,7 +182,7 @@ class Engine {
         int* flags;       // the flag words of the solve chains
         bool chain;       // room for the solve chains; without it every level is stepped
     };
-    bool has_chain() const { return chain_inv_ != nullptr; }
+    bool has_chain() const { return chain_err_ != nullptr; }
     int64_t sweep_workspace_bytes(int64_t nrhs, bool chain) const;
     int64_t sweep_flag_bytes(bool chain) const;  // of it, the chains' flags
     SweepWorkspace carve_sweep_workspace(void* base, int64_t nrhs, bool chain) const;
@@ -286,7 +286,7 @@ class Engine {
     bool tc_persistent_ = true;
     double* d_ = nullptr;
     double* linv_ = nullptr;      // inverse of each unit-lower NB×NB diagonal block (solves)
-    double* chain_inv_ = nullptr; // inverse of each solve-chain block (WS × WS)
+    double* chain_inv_ = nullptr; // inverse of each solve-chain block (WS × WS), mixed precision
     int* chain_err_ = nullptr;    // set by a solve-chain wait that gave up
     int64_t chain_inv_at_ = -1;   // the numeric phase (factor_calls_) chain_inv_ was formed for
     double* adiag_ = nullptr;

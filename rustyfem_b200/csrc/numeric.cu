@@ -1734,7 +1734,8 @@ void Engine::init(bool) {
         RFG_CUDA(cudaGetLastError());
     }
     if (plan_.chain_blocks > 0) {
-        chain_inv_ = (double*)dalloc(plan_.chain_blocks * (int64_t)WS * WS * sizeof(double));
+        if (prec_ == PREC_MIXED)
+            chain_inv_ = (double*)dalloc(plan_.chain_blocks * (int64_t)WS * WS * sizeof(double));
         chain_err_ = (int*)dalloc(sizeof(int));
         RFG_CUDA(cudaMemsetAsync(chain_err_, 0, sizeof(int), stream_));
     }

@@ -156,8 +156,9 @@ struct Plan {
     // runs as one launch per level and direction instead of
     // two per WS-wide step: each WS-wide diagonal block of a front is one work item, done
     // by a cluster of four CTAs that waits for the blocks it depends on (chain.cu). The
-    // block's solve multiplies by the inverse of its unit-lower diagonal block (WS × WS,
-    // FP64), formed from the factor before the first sweep.
+    // block's solve multiplies an FP32 factor's vectors by the inverse of its unit-lower diagonal
+    // block (WS × WS, FP64), formed from the factor before the first sweep; an FP64 factor's are
+    // solved by substitution over the cluster's CTAs.
     std::vector<uint8_t> level_chain;    // per level: 1 when its sweeps run as chains
     std::vector<int64_t> chain_blk;      // per front: its first chain block, or -1
     std::vector<int64_t> chain_bfront;   // per chain block: its front

@@ -1465,7 +1465,7 @@ void launch_scatter_rhs(double* b, const double* X, const int64_t* eq, const int
 }
 
 ChainArgs Engine::chain_args() const {
-    return ChainArgs{dp_.fronts, dp_.rows, dp_.imap, dp_.chain_blk, dp_.chain_colbase, chain_inv_, d_,
+    return ChainArgs{dp_.fronts, dp_.rows, dp_.imap, dp_.chain_blk, dp_.chain_colbase, linv_, chain_inv_, d_,
                      plan_.chain_blocks, chain_err_};
 }
 
@@ -1683,7 +1683,7 @@ int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }
 }  // namespace
 
 bool Engine::chain_on(int64_t nrhs) const {
-    return chain_inv_ != nullptr && nrhs >= 1 && nrhs <= MAXR;
+    return has_chain() && nrhs >= 1 && nrhs <= MAXR;
 }
 
 int64_t Engine::partial_rows(bool chain) const {
@@ -1694,16 +1694,12 @@ int64_t Engine::flag_words(bool chain) const {
     return std::max<int64_t>(1, chain ? chain_flag_words(plan_) : 0);
 }
 
-// The chain blocks' inverses for the current factor: formed by the first sweep after each
+// The chain blocks' inverses for the current FP32 factor: formed by the first sweep after each
 // numeric phase (on the engine's stream, before that sweep's launches or graph).
 void Engine::ensure_chain_inverse() {
-    if (chain_inv_at_ == factor_calls_) return;
-    if (prec_ == PREC_FP64)
-        launch_chain_inverse(chain_inv_, (const double*)panel_, linv_, dp_.fronts, dp_.chain_blk, dp_.chain_bfront,
-                             plan_.chain_blocks, stream_);
-    else
-        launch_chain_inverse(chain_inv_, (const float*)panel_, linv_, dp_.fronts, dp_.chain_blk, dp_.chain_bfront,
-                             plan_.chain_blocks, stream_);
+    if (!chain_inv_ || chain_inv_at_ == factor_calls_) return;
+    launch_chain_inverse(chain_inv_, (const float*)panel_, linv_, dp_.fronts, dp_.chain_blk, dp_.chain_bfront,
+                         plan_.chain_blocks, stream_);
     solve_launches++;
     chain_inv_at_ = factor_calls_;
 }
