@@ -41,7 +41,7 @@ PLAN = {"fr", "order", "pre", "pre_tiles", "pre_a", "pre_scr", "pre_scr_prev", "
         "imap", "mode", "omode", "slots", "items", "colbase", "chain_blk", "dst", "seg_ptr", "seg_src", "src",
         "width", "cmaps"}
 # and during the sweeps the factor
-FACTOR = {"panel", "linv", "cinv", "d"}
+FACTOR = {"panel", "linv", "inv", "d"}
 
 
 def chained_kernels(name):
