@@ -30,6 +30,10 @@ Newton loop that refactors the same pattern.
            oracle's element loop, and the skewed 24³ cube through rustyfem_factor_unsym
            (skipped with --no-extras)
 
+The line is printed in any case; a record that misses its bar (backward error 1e-12, relative error
+against the oracle 1e-10 for FP64, equal inertia, delayed pivots and assembled bits) is listed under
+missed_bars and ends the run with an error.
+
 ``--impl reference`` times the reference's CPU algorithm (the oracle port: the
 reference is Rust and cannot be built here) on the same workload: its K timed
 steps together run one whole factor + solve of the cube (analysis, the
@@ -370,11 +374,11 @@ def measure_unsym(n: int, oracle: bool) -> dict:
 
 def run_hex20(args):
     n = 40 if args.n == WORKLOAD_N else args.n
-    print(json.dumps(measure_hex20(n, args.steps, args.warmup)), flush=True)
+    finish(measure_hex20(n, args.steps, args.warmup))
 
 
 def run_plates(args):
-    print(json.dumps(measure_plates(args.steps, args.warmup)), flush=True)
+    finish(measure_plates(args.steps, args.warmup))
 
 
 def run_profile_case(args):
@@ -535,6 +539,47 @@ def rel_err(x, xo) -> float:
     import numpy as np
 
     return float(np.linalg.norm(x - xo) / np.linalg.norm(xo))
+
+
+# ---------------------------------------------------------------------------
+# the bars a printed record has to meet
+# ---------------------------------------------------------------------------
+BACKWARD_ERROR_BAR = 1e-12
+# relative error against the oracle's solution; the mixed path is held to its backward error (on the
+# graded cube the matrix's condition alone leaves 1e-7 of it)
+ORACLE_BARS = {"fp64": 1e-10, "indefinite": 1e-9, "unsymmetric": 1e-10}
+
+
+def missed_bars(record, kind=None, path="") -> list[str]:
+    """What in a record (and the records in it) misses its bar: backward errors, relative errors
+    against the oracle (by the path's kind), equalities with the oracle. A NaN misses."""
+    missed = []
+    for key, v in record.items():
+        at = path + key
+        if isinstance(v, dict):
+            # "fp64_last_step_parts" is a record of the FP64 path too
+            k = next((n for n in ORACLE_BARS if key.startswith(n)), "mixed" if key.startswith("mixed") else kind)
+            missed += missed_bars(v, k, at + ".")
+        elif key == "backward_error":
+            if v is not None and not v <= BACKWARD_ERROR_BAR:
+                missed.append(f"{at} = {v:.3e} (bar {BACKWARD_ERROR_BAR:g})")
+        elif key == "rel_err_vs_oracle":
+            bar = ORACLE_BARS.get(kind)
+            if v is not None and bar is not None and not v <= bar:
+                missed.append(f"{at} = {v:.3e} (bar {bar:g})")
+        elif key in ("inertia_equal", "delayed_equal", "bit_identical_to_oracle") and v is not True:
+            missed.append(f"{at} = {v}")
+    return missed
+
+
+def finish(out, kind=None) -> None:
+    """Prints the line; ends with an error when a record in it misses its bar."""
+    missed = missed_bars(out, kind)
+    if missed:
+        out["missed_bars"] = missed
+    print(json.dumps(out), flush=True)
+    if missed:
+        sys.exit("bench: wrong result: " + "; ".join(missed))
 
 
 # ---------------------------------------------------------------------------
@@ -886,7 +931,7 @@ def run_b200(args, rank, world, local_rank):
         dist.barrier()
         dist.destroy_process_group()
     if out is not None:
-        print(json.dumps(out), flush=True)
+        finish(out)
 
 
 # ---------------------------------------------------------------------------
@@ -1001,16 +1046,16 @@ def main():
         run_hex20(args)
         return
     if args.workload == "assembly":
-        print(json.dumps(measure_assembly(args.n, not args.no_oracle)), flush=True)
+        finish(measure_assembly(args.n, not args.no_oracle))
         return
     if args.workload == "unsym":
-        print(json.dumps(measure_unsym(args.n, not args.no_oracle)), flush=True)
+        finish(measure_unsym(args.n, not args.no_oracle), "unsymmetric")
         return
     if args.workload == "plates":
         run_plates(args)
         return
     if args.workload == "indef":
-        print(json.dumps(measure_indef(30 if args.n == WORKLOAD_N else args.n, not args.no_oracle)), flush=True)
+        finish(measure_indef(30 if args.n == WORKLOAD_N else args.n, not args.no_oracle), "indefinite")
         return
     run_b200(args, rank, world, local_rank)
 
