@@ -438,6 +438,7 @@ bool finish_model(RustyfemHandle* h, const int64_t* indptr, const int64_t* indic
     bool use_tc = h->opt.precision == RFG_MIXED && !(h->opt.flags & RFG_FLAG_NO_TENSOR_CORES);
     Precision prec = h->opt.precision == RFG_MIXED ? PREC_MIXED : PREC_FP64;
     Tuning tun;
+    tun.fp64 = prec == PREC_FP64;
     if (const char* e = getenv("RFG_TC_OUTER_TN")) tun.outer_tn = atoi(e) == 128 ? 128 : TC_WIDE;
     // two-block passes of the tensor-core outer update (the persistent kernel only)
     if (const char* e = getenv("RFG_TC_PAIR")) tun.pair_blocks = e[0] != '0';

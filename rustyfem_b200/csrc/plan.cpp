@@ -282,7 +282,7 @@ Plan build_plan(const Symbolic& S, bool use_tc, const Tuning& tun) {
             int64_t cot = 0, cot2 = 0, cit = 0, coa = 0, cota = 0;
             // FP64: outer updates with few 128-tiles in all run on 64-tiles
             bool small_outer = false;
-            if (!use_tc) {
+            if (!use_tc && tun.fp64) {
                 int64_t n128 = 0;
                 for (int64_t i = st.out_lo; i < nact; i++) {
                     const DFront& d = P.fronts[P.level_order[lo + i]];

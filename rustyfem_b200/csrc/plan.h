@@ -202,6 +202,7 @@ struct Tuning {
     bool pair_blocks = true;             // tensor-core outer updates in two-block passes
     int64_t chain_fronts = -1;           // solve chains on levels of at most this many fronts
                                          // (-1: RFG_SOLVE_CHAIN, else CHAIN_FRONTS; 0: none)
+    bool fp64 = true;                    // without tensor cores: an FP64 factor (FP64_MIN_TILES), else FP32
 };
 constexpr int64_t CHAIN_FRONTS = 16;
 // Levels whose fronts are all one block wide have no chain to shorten: their two step launches
