@@ -210,7 +210,8 @@ class Engine {
     // Splits the internal rows into independent systems (offsets off[0] = 0 < ... <=
     // off[g] ... = n, one per model of a batched factorization): the refined solve
     // then measures the backward error of every system on its own and iterates until
-    // the worst one meets the tolerance. Without it the rows form one system.
+    // the worst one meets the tolerance. Without it the rows form one system. Once per
+    // engine, before its first refined solve.
     void set_segments(const std::vector<int64_t>& off);
 
     const Plan& plan() const { return plan_; }

@@ -1782,20 +1782,13 @@ void* noalloc_scratch() {
 
 void Engine::set_segments(const std::vector<int64_t>& off) {
     if (off.size() < 2 || off.front() != 0 || off.back() != plan_.n) throw CudaError("set_segments: bad offsets");
+    // the norms kept from solve to solve, and the buffers, belong to the systems
+    if (!seg_off_.empty()) throw CudaError("set_segments: the systems of a handle are set once, before its first refined solve");
     int64_t nseg = (int64_t)off.size() - 1;
     std::vector<int64_t> pre(nseg + 1, 0);
     for (int64_t g = 0; g < nseg; g++) {
         if (off[g + 1] < off[g]) throw CudaError("set_segments: offsets must not decrease");
         pre[g + 1] = pre[g] + (off[g + 1] - off[g] + SEG_ROWS - 1) / SEG_ROWS;
-    }
-    if (ref_red_ && (int64_t)seg_off_.size() != nseg + 1) {
-        dev_free(ref_red_, stream_);
-        ref_red_ = nullptr;
-        ref_nrhs_ = 0;
-        if (ref_r_) dev_free(ref_r_, stream_);
-        if (ref_dx_) dev_free(ref_dx_, stream_);
-        ref_r_ = ref_dx_ = nullptr;
-        a_val_at_ = -1;
     }
     seg_off_ = off;
     seg_blocks_ = pre[nseg];
