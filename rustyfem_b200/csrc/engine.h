@@ -182,6 +182,7 @@ class Engine {
         int* flags;       // the flag words of the solve chains
         bool chain;       // room for the solve chains; without it every level is stepped
     };
+    // the sweeps run the solve chains of the plan's chain levels
     bool has_chain() const { return chain_err_ != nullptr; }
     int64_t sweep_workspace_bytes(int64_t nrhs, bool chain) const;
     int64_t sweep_flag_bytes(bool chain) const;  // of it, the chains' flags
@@ -240,8 +241,6 @@ class Engine {
     template <typename T>
     int64_t backward_steps(int64_t level, double* Y, double* V, int nrhs, double* partial, int* chain);
     ChainArgs chain_args() const;
-    // the sweeps of nrhs right-hand sides run the solve chains of the plan's chain levels
-    bool chain_on(int64_t nrhs) const;
     void ensure_chain_inverse();
     int64_t flag_words(bool chain) const;
     int64_t partial_rows(bool chain) const;  // partial-sum values per right-hand side of a sweep

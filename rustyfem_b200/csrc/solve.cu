@@ -1551,7 +1551,7 @@ void Engine::solve_impl(double* X, int64_t nrhs_total) {
         return;
     }
     int nrhs = (int)nrhs_total;
-    int* chain = chain_on(nrhs) ? counters_ : nullptr;
+    int* chain = has_chain() ? counters_ : nullptr;
     if (chain) RFG_CUDA(cudaMemsetAsync(chain, 0, chain_flag_words(P) * sizeof(int), stream_));
     for (int64_t l = 0; l < P.nlevels; l++) launches += forward_steps<T>(l, X, ybuf_, vupd_, nrhs, chain);
     for (int64_t l = P.nlevels - 1; l >= 0; l--)
@@ -1630,7 +1630,7 @@ void Engine::solve_device(double* X, int64_t nrhs, bool allow_graph) {
         counters_ = (int*)dalloc(flag_words(has_chain()) * sizeof(int));
         ws_nrhs_ = w;
     }
-    if (chain_on(nrhs)) ensure_chain_inverse();
+    ensure_chain_inverse();
     if (use_graphs_ && nrhs <= MAXR) {
         cudaGraphExec_t ex = nullptr;
         for (auto& g : solve_graphs_)
@@ -1681,10 +1681,6 @@ void Engine::solve_device(double* X, int64_t nrhs, bool allow_graph) {
 namespace {
 int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }
 }  // namespace
-
-bool Engine::chain_on(int64_t nrhs) const {
-    return has_chain() && nrhs >= 1 && nrhs <= MAXR;
-}
 
 int64_t Engine::partial_rows(bool chain) const {
     return std::max<int64_t>(2 * plan_.max_wpart, chain ? plan_.chain_colpart : 0);
@@ -1743,7 +1739,7 @@ template <typename T>
 void Engine::solve_sweep_impl(double* X, int64_t nrhs_total, const SweepWorkspace& ws) {
     const Plan& P = plan_;
     int nrhs = (int)nrhs_total;
-    int* chain = ws.chain && chain_on(nrhs) ? ws.flags : nullptr;
+    int* chain = ws.chain ? ws.flags : nullptr;
     if (chain) RFG_CUDA(cudaMemsetAsync(chain, 0, chain_flag_words(P) * sizeof(int), stream_));
     for (int64_t l = 0; l < P.nlevels; l++) forward_steps<T>(l, X, ws.y, ws.v, nrhs, chain);
     for (int64_t l = P.nlevels - 1; l >= 0; l--) backward_steps<T>(l, ws.y, ws.v, nrhs, ws.partial, chain);
@@ -1755,7 +1751,7 @@ void Engine::solve_sweep_on(double* X, int64_t nrhs, const SweepWorkspace& ws) {
     if (nrhs <= 0 || plan_.n == 0) return;
     if (nrhs > MAXR) throw CudaError("solve_sweep_on: at most 32 right-hand sides per sweep");
     solve_set_attributes();
-    if (ws.chain && chain_on(nrhs)) ensure_chain_inverse();
+    if (ws.chain) ensure_chain_inverse();
     if (prec_ == PREC_FP64)
         solve_sweep_impl<double>(X, nrhs, ws);
     else
