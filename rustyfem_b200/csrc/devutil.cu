@@ -153,13 +153,13 @@ void sort_rows_u64(uint64_t* key, const int64_t* rp, int64_t nrows, cudaStream_t
 namespace {
 __global__ void k_selftest_reciprocal(const double* __restrict__ x, double* __restrict__ r, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        r[i] = recip_newton(x[i]);
+        r[i] = recip_chebyshev(x[i]);
 }
 }  // namespace
 
 }  // namespace rfg
 
-// The pivot blocks' reciprocal (recip_newton) on the current device for n host values
+// The pivot blocks' reciprocal (recip_chebyshev) on the current device for n host values
 // x > 0, into r: lets a test compare it with the correctly rounded 1/x.
 extern "C" int32_t rfg_selftest_reciprocal(const double* x, double* r, size_t n) {
     using namespace rfg;

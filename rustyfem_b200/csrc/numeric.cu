@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(PBT, 2) k_pivot_block(T* __restrict__ panel, d
             // bad pivot spoils only values that nobody reads, the front stops here)
 #pragma unroll
             for (int j = 0; j < PB; j++) {
-                const double rinv = recip_newton(D[j][j]);
+                const double rinv = recip_chebyshev(D[j][j]);
                 double l[PB];
 #pragma unroll
                 for (int i = j + 1; i < PB; i++) {

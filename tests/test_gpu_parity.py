@@ -255,7 +255,7 @@ def test_device_entry_points_wait_for_the_callers_stream(gpu):
 
 
 def test_pivot_reciprocal_within_one_ulp(gpu):
-    """The pivot blocks divide by each pivot through a Newton–Raphson reciprocal instead of
+    """The pivot blocks divide by each pivot through one Chebyshev step of the approximate reciprocal instead of
     the IEEE division: within one unit in the last place of the correctly rounded 1/x over
     twenty decades and at the ends of the mantissa."""
     import ctypes
