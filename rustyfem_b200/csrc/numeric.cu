@@ -1747,10 +1747,8 @@ void Engine::init(bool) {
         // first refined solve), sized for every scattered entry and its mirror
         const int64_t cap = std::max<int64_t>(2 * nseg_, 1);
         a_rowptr_ = (int64_t*)dalloc((plan_.n + 1) * sizeof(int64_t));
-        // columns and sources in blocks of the values' size: equal blocks find each other's places
-        // when the pool hands a freed handle's memory to the next one
-        a_col_ = (int32_t*)dalloc(cap * sizeof(double));
-        a_src_ = (uint32_t*)dalloc(cap * sizeof(double));
+        a_col_ = (int32_t*)dalloc(cap * sizeof(int32_t));
+        a_src_ = (uint32_t*)dalloc(cap * sizeof(uint32_t));
         a_val_ = (double*)dalloc(cap * sizeof(double));
     }
     if (use_tc_) {
