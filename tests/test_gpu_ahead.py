@@ -26,3 +26,30 @@ def test_side_stream(gpu, n):
             assert np.array_equal(h.solve(m.rhs), x), level
     finally:
         h.free()
+
+
+@pytest.mark.parametrize("n", [17, 27])
+def test_forks_and_other_values(gpu, n):
+    """The look-ahead runs (a step that forks with a next block's columns launches its outer update in two
+    parts): four of the five forked steps of the 17³ cube have their rest on 64-tiles alone, fourteen of the
+    27³ cube's eighteen on 128-tiles alone. With other values in between every factorization gives the bits of a fresh
+    handle's."""
+    ms = [W.hex8_cube(n, emod=W.log_uniform_moduli(n, 1e9, 1e11, seed=s)).full() for s in range(3)]
+    want = []
+    for m in ms:
+        h, _, _ = ffi.factor(m)
+        assert h is not None, ffi.last_error()
+        want.append(h.solve(m.rhs))
+        h.free()
+    h, _, _ = ffi.factor(ms[0])
+    try:
+        launches = h.stats()["launches"]
+        h.set_profiling(1)
+        assert h.refactor(ms[1].data) == -1
+        assert launches > h.stats()["launches"]
+        h.set_profiling(0)
+        for i in (1, 2, 0, 2, 1, 0):
+            assert h.refactor(ms[i].data) == -1
+            assert np.array_equal(h.solve(ms[i].rhs), want[i]), i
+    finally:
+        h.free()
