@@ -42,6 +42,32 @@ def test_same_bits(gpu, n, times, nrhs):
         h.free()
 
 
+def test_same_bits_beside_other_handles(gpu):
+    # three threads with a handle each, so that launches, CTAs and warps meet in other orders
+    import threading
+
+    jobs = [(graded(25), ffi.FP64, 1), (graded(21), ffi.FP64, 6), (graded(21), ffi.MIXED, 1)]
+    failed = []
+
+    def run(m, precision, nrhs):
+        rhs = np.random.default_rng(nrhs).standard_normal((nrhs, m.n))
+        h, _, _ = ffi.factor(m, precision=precision)
+        try:
+            first = h.solve(rhs)
+            for i in range(100):
+                if h.refactor(m.data) != -1 or not np.array_equal(h.solve(rhs), first):
+                    failed.append((m.name, precision, i, ffi.last_error()))
+        finally:
+            h.free()
+
+    threads = [threading.Thread(target=run, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+
+
 @pytest.mark.parametrize("front", ["root", "largest below the root"])
 def test_refused_beside_an_update(gpu, front):
     m = W.hex8_cube(27).full()
