@@ -67,7 +67,10 @@ class IndefEngine {
     int64_t* d_tpre_ = nullptr;    // prefix of trailing-update tiles over a level's fronts
     int64_t* d_active_ = nullptr;  // fronts of the level not yet done
     int num_sms_ = 148;
-    // fronts from this size run their block rounds on a cluster of CTAs (shifted 24³ Laplacian: 24.7 ms a call at 768, 22.6 at 384, 22.7 at 128)
+    // fronts from this size run their block rounds on a cluster of CTAs. A call at 128 / 256 / 384 / 768 / 1536,
+    // ms: shifted Laplacian 12³ 5.5 / 4.9 / 4.8 / 4.8 / 4.8, 18³ 14.1 / 14.5 / 13.7 / 14.4 / 14.5, 24³ 22.4 / 21.8 /
+    // 22.1 / 24.4 / 26.9, 30³ 39.9 / 38.6 / 37.9 / 37.8 / 57; shifted hex8 20³ 80.6 / 76.9 / 76.6 / 79.9 / 103, 30³
+    // 305 / 294 / 291 / 288 / 295
     int64_t cluster_rows_ = 384;
     void* d_desc_ = nullptr;     // IFrontDesc[nfronts]
     std::vector<void*> front_bufs_;

@@ -70,7 +70,9 @@ class LuEngine {
     int64_t* d_rpre_ = nullptr;   // prefix of the row-block-update tiles
     int64_t* d_active_ = nullptr;
     int num_sms_ = 148;
-    // fronts from this size run their block rounds on a cluster of CTAs (unsymmetric 13³: 29.5 ms a call at 768, 26.6 at 384, 27.2 at 128)
+    // fronts from this size run their block rounds on a cluster of CTAs. A call at 128 / 256 / 384 / 768 / 1536,
+    // ms, skewed hex8: 7³ 5.4 / 5.1 / 5.1 / 5.1 / 5.1, 10³ 13.1 / 13.1 / 13.0 / 14.5 / 14.5, 13³ 23.9 / 23.4 / 24.0 /
+    // 26.4 / 28.8, 18³ 67.2 / 65.7 / 65.9 / 71.5 / 90, 24³ 144 / 140 / 138 / 141 / 146
     int64_t cluster_rows_ = 384;
     void* d_desc_ = nullptr;  // LFrontDesc[nfronts]
     std::vector<void*> front_bufs_, level_bufs_;

@@ -1830,9 +1830,10 @@ void Engine::pivots_to_host(double* out) const {
 // CTAs of an outer update's rest from which it runs beside the next block's steps: one per SM
 // (thresholds of 40 and 600 measured the same; below, the rest is shorter than the fork and join).
 // A 64-pivot step is a chain of three launches of a few CTAs, about 33 µs, and four of them wait
-// for each outer update; side by side a factorization of the 33³ cube went from 18.5 to 17.6 ms, of the
-// 22³ from 3.76 to 3.63 ms, of the 45³ from 77.5 to 76.2 ms. (One CTA per SM for the rest, which leaves
-// half of every SM to the steps, was slower: 101 ms at 45³.)
+// for each outer update; a factorization takes, with the rest on the one stream and beside the steps,
+// 3.42 and 3.33 ms at 22³, 17.22 and 16.47 at 33³, 71.6 and 70.6 at 45³, 336.3 and 334.7 at 60³. (One
+// CTA per SM for the rest, which leaves half of every SM to the steps, was slower: 88 against 71 ms at
+// 45³.)
 constexpr int64_t AHEAD_MIN_CTAS = 148;
 
 template <typename T>

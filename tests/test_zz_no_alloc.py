@@ -3,8 +3,8 @@
 The no-allocation entry point runs the same sweep kernels on a fixed device scratch
 array instead of the handle's own buffers. With refinement off (refine_max_iter = 0,
 no statistics) rfg_solve_device applies the factor once, so both must give the same
-values bit for bit, on every call (the backward sweep's ticket counters live in the
-shared scratch and must be back at zero for the next call). The call must take no
+values bit for bit, on every call (the flags and counters of the solve chains live in
+the shared scratch and every call clears them). The call must take no
 device memory, and a handle whose scratch need is above the fixed size is refused
 before anything runs. This file is named to be collected last, so that it also runs
 after every other GPU test has loaded and used the library.
