@@ -22,7 +22,7 @@
 //   FP64 factor: substitution over the CTAs in turn, forward y_s = inv(L_ss)·x_s with the
 //       factorization's 64 × 64 inverse, y_s to the CTAs after s, x_t −= L_ts·y_s there (backward
 //       the same from the last one, transposed). Three cluster barriers more in the chain from block to
-//       block (a solve call of the 33³ cube 1.57 ms, 1.42 with the inverse), for the rounding of the
+//       block (a solve call of the 33³ cube 1.55 ms, 1.42 with the inverse), for the rounding of the
 //       stepped sweeps: an FP64 solve is not refined unless the caller asks, and with the WS × WS
 //       inverse its residuals were 1.02 to 1.10 times as large in the 2-norm and up to 1.5 times in the
 //       maximum norm (means over right-hand sides; hex8 17³ to 45³, hex20 20³, one and six of them). Now
@@ -338,15 +338,16 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
             for (int t = 0; t < nsub; t++) {
                 if (s == t) {
                     row_product(a, CQ * t, CQ, xo);
-                    put_y(a);
                     if (q > t) {  // the lanes of a row take a rank each
                         double* o = cluster.map_shared_rank(yr, q) + (CQ * t + i) * R;
 #pragma unroll
                         for (int r = 0; r < R; r++) o[r] = a[r];
                     }
                 }
+                // Y after the barrier: its release would wait for stores to global memory too
+                if (t + 1 < nsub) cluster.sync();
+                if (s == t) put_y(a);
                 if (t + 1 == nsub) break;
-                cluster.sync();
                 if (s > t && s < nsub) {
                     row_product(a, CQ * t, CQ, yr + CQ * t * R);
                     if (q == 0) {
@@ -571,7 +572,6 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
             for (int t = (wb + CQ - 1) / CQ - 1; t >= 0; t--) {
                 if (s == t) {
                     col_product(a, 0, CQ, zo);
-                    put_y(a);
                     if (tid < CQ) {
                         for (int rk = 0; rk < t; rk++) {
                             double* o = cluster.map_shared_rank(yr, rk) + (CQ * (t - 1) + c) * R;
@@ -580,8 +580,9 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
                         }
                     }
                 }
+                if (t > 0) cluster.sync();
+                if (s == t) put_y(a);
                 if (t == 0) break;
-                cluster.sync();
                 if (s < t) {
                     col_product(a, CQ * (t - s), CQ, yr + CQ * (t - 1) * R);
                     if (tid < CQ) {
@@ -804,15 +805,15 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
                     yb[vsw(CQ * t + i, 2 * q + 1)] = x[1];
                     __syncthreads();
                     row_product(CQ * t, 8 * w + 8);
-                    put_y();
                     for (int rk = t + 1; rk < nsub; rk++) {
                         double* o = cluster.map_shared_rank(yb, rk);
                         o[vsw(CQ * t + i, 2 * q)] = y[0];
                         o[vsw(CQ * t + i, 2 * q + 1)] = y[1];
                     }
                 }
+                if (t + 1 < nsub) cluster.sync();
+                if (s == t) put_y();
                 if (t + 1 == nsub) break;
-                cluster.sync();
                 if (s > t && s < nsub) {
                     row_product(CQ * t, CQ);
                     x[0] -= y[0];
@@ -945,15 +946,15 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(CT, 1)
                     yp[vsw(CQ * t + c, 2 * q + 1)] = z[1];
                     __syncthreads();
                     col_product(8 * w, CQ);
-                    put_y();
                     for (int rk = 0; rk < t; rk++) {
                         double* o = cluster.map_shared_rank(yp, rk);
                         o[vsw(CQ * t + c, 2 * q)] = y[0];
                         o[vsw(CQ * t + c, 2 * q + 1)] = y[1];
                     }
                 }
+                if (t > 0) cluster.sync();
+                if (s == t) put_y();
                 if (t == 0) break;
-                cluster.sync();
                 if (s < t) {
                     col_product(CQ * (t - s), CQ * (t - s) + CQ);
                     z[0] -= y[0];

@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(256) k_wbwd_diag_pf(double* __restrict__ Y, co
 // A step is bound by the latency of its chain of launches and barriers, not by the factor's
 // bytes: with these kernels (launched as programmatic dependents) and the solve chains instead
 // of the plain step kernels, a refined-solve call with the FP64 factor of the 33³ cube went
-// from 3.72 to 1.79 ms (now 1.57), of the 45³ cube from 6.25 to 3.26 ms, of a 410-equation plate
+// from 3.72 to 1.79 ms (now 1.55), of the 45³ cube from 6.25 to 3.26 ms, of a 410-equation plate
 // from 0.224 to 0.181 ms (now 0.10).
 template <bool FWD>
 __device__ __forceinline__ void pd_issue(double* sm, int tile, const double* panel, const DFront& f,
